@@ -1,0 +1,594 @@
+// Training kernels that WALK a layer's connection graph: forward, and backward_w + backward_x in one pass.
+//
+// Take the layer's inputs as nodes and its neurons as edges (a neuron joins its two input rows).  A walk along edges
+// meets the neurons in an order in which each neuron shares an input row with the one before it, so a row that was
+// loaded for one neuron is still in registers for the next: one row load per neuron instead of two.  The order in which
+// neurons are processed is free -- every neuron writes its own output row -- so the walk is computed once per layer
+// (dl_build_walk, on the host) and the kernels follow it.
+//
+// In a square layer with random connections every input feeds exactly two neurons: the graph is a set of closed
+// walks, every node lies on one of them once, and both terms of its input gradient come from two neighbouring steps.
+// The backward kernel then carries the first term in a register to the next step and stores the finished row: per neuron
+// it reads one row of x and one of grad_y and writes one of grad_x, and the four batch sums of the weight gradient come
+// from the same registers.  The two gather kernels of train.cu (backward_w: three rows read; backward_x: four read, one
+// written) move eight rows for the same result.
+//
+// Bound by memory: measured per launch in a captured chain, 64000 x 64000 at batch 1024: forward 118 -> 89 us (81 us for its
+// bytes at the measured copy bandwidth), both gradients with Adam 316 (199 + 116 one after the other) -> 149 us (127);
+// 128000 x 128000 at batch 256: 66 -> 45 us and 168 -> 95 us.
+//
+// A walk is cut into chunks; a chunk's warps handle up to 128 batch columns each.  What a chunk needs from the step
+// before it (the carried gradient term) it recomputes from that step's operands: two extra row loads per chunk.
+#include <stdlib.h>
+
+#include <vector>
+
+#include "adam_math.cuh"
+#include "common.cuh"
+#include "gates.cuh"
+
+namespace dl {
+
+constexpr int kWalkSteps = 8;          // steps that a lane group takes between two reductions, all their loads in flight
+constexpr int kWalkWarps = kThreads / 32;
+
+// Entry of a walk, two int32:
+//   x = node << 1 | store     the input row this step stands on; store: its gradient is complete here and is stored
+//   y = neuron << 2 | flip << 1 | emit, or -1 when no neuron leads on (the end of an open walk, a node nobody reads)
+//                             flip: the row stood on is the neuron's SECOND input; emit: the neuron's outputs belong to
+//                             this entry (an entry in front of a closed walk repeats its last one without store and emit)
+// The neuron leads to the node of the next entry.
+
+// Four values of a row per lane.  VEC: four adjacent ones (16-byte loads); else four that lie G lanes apart, so that
+// rows of any length and alignment are read in whole sectors.
+template <int G, bool VEC>
+struct RowIo {
+    int64_t col;    // first column of this lane
+    int live;       // bit i: component i lies inside the row
+    __device__ __forceinline__ RowIo(int64_t col0, int lane, int64_t batch) {
+        if (VEC) {
+            col = col0 + lane * 4;
+            live = col < batch ? 15 : 0;
+        } else {
+            col = col0 + lane;
+            live = 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) live |= (col + i * G < batch ? 1 : 0) << i;
+        }
+    }
+    __device__ __forceinline__ float4 load(const float *__restrict__ m, int64_t row, int64_t batch) const {
+        const float *p = m + row * batch + col;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (VEC) {
+            if (live) v = __ldg(reinterpret_cast<const float4 *>(p));
+        } else {
+            if (live & 1) v.x = __ldg(p);
+            if (live & 2) v.y = __ldg(p + G);
+            if (live & 4) v.z = __ldg(p + 2 * G);
+            if (live & 8) v.w = __ldg(p + 3 * G);
+        }
+        return v;
+    }
+    __device__ __forceinline__ void store(float *__restrict__ m, int64_t row, int64_t batch, const float4 &v) const {
+        float *p = m + row * batch + col;
+        if (VEC) {
+            if (live) *reinterpret_cast<float4 *>(p) = v;
+        } else {
+            if (live & 1) p[0] = v.x;
+            if (live & 2) p[G] = v.y;
+            if (live & 4) p[2 * G] = v.z;
+            if (live & 8) p[3 * G] = v.w;
+        }
+    }
+};
+
+// ---------------------------------------------------------------------------------------------
+// forward along the walk: y[j] = mix(x[a_j], x[b_j]), the coefficients of the CTA's neurons computed by four lanes each
+// while the first rows are in flight
+// ---------------------------------------------------------------------------------------------
+template <int G, bool VEC>
+__global__ void __launch_bounds__(kThreads, 4)
+walk_forward_kernel(const float *__restrict__ x, const float *__restrict__ w, int w_mode, float *__restrict__ y,
+                    float4 *__restrict__ coef_out, const int2 *__restrict__ walk, int entries, int64_t batch, int wc, int ncb) {
+    constexpr int N = kWalkWarps * (32 / G) * kWalkSteps;  // entries per CTA
+    __shared__ int s_node[N + 1], s_edge[N + 1];
+    __shared__ float4 s_coef[N];  // {c0, c of the row stood on, c of the row led to, cab}
+
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % G;
+    const int first = blockIdx.x * N;
+    for (int t = tid; t <= N; t += kThreads) {
+        const int2 e = first + t < entries ? __ldg(walk + first + t) : make_int2(-1, -1);
+        s_node[t] = e.x >> 1;
+        s_edge[t] = e.y;
+        if (t < N && e.y >= 0) prefetch_l2(w + (int64_t)(e.y >> 2) * 16);
+    }
+    __syncthreads();
+    grid_dependency_wait();
+    grid_dependents_launch();
+
+    const int wcol = warp % wc;
+    const int p = ((warp / wc) * (32 / G) + (tid % 32) / G) * (kWalkSteps * wc);  // this chunk's first entry
+    float4 xin = make_float4(0.f, 0.f, 0.f, 0.f), xn[kWalkSteps];
+    auto fetch = [&](const RowIo<G, VEC> &io, int q) {
+#pragma unroll
+        for (int i = 0; i < kWalkSteps; ++i) {
+            xn[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            const int node = s_node[q + i + 1];
+            if (node >= 0) xn[i] = io.load(x, node, batch);
+        }
+    };
+    auto begin = [&](const RowIo<G, VEC> &io) {
+        const int node = s_node[p];
+        xin = node >= 0 ? io.load(x, node, batch) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    int cb = wcol;
+    if (cb < ncb) {
+        const RowIo<G, VEC> io((int64_t)cb * (4 * G), lane, batch);
+        begin(io);
+        fetch(io, p);
+    }
+    for (int t = tid; t < N * 4; t += kThreads) {
+        const int nl = t >> 2, q = t & 3, e = s_edge[nl];
+        const bool live = e >= 0 && (e & 1);
+        const int64_t j = live ? e >> 2 : 0;
+        const float4 c = quad_coef(w + j * 16 + q * 4, live, q, w_mode);
+        if (q == 0 && live) {
+            s_coef[nl] = (e & 2) ? make_float4(c.x, c.z, c.y, c.w) : c;
+            if (coef_out != nullptr) coef_out[j] = c;
+        }
+    }
+    __syncthreads();
+    bool fetched = true;
+    for (; cb < ncb; cb += wc) {
+        const RowIo<G, VEC> io((int64_t)cb * (4 * G), lane, batch);
+        if (!fetched) begin(io);
+        for (int sb = 0; sb < wc; ++sb) {
+            const int q = p + sb * kWalkSteps;
+            if (!fetched) fetch(io, q);
+            fetched = false;
+#pragma unroll
+            for (int i = 0; i < kWalkSteps; ++i) {
+                const int e = s_edge[q + i];
+                if (e >= 0 && (e & 1)) io.store(y, e >> 2, batch, mixv(s_coef[q + i], xin, xn[i]));
+                xin = xn[i];
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// backward along the walk
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ float sum4(const float4 &v) { return (v.x + v.y) + (v.z + v.w); }
+__device__ __forceinline__ float4 mul4(const float4 &a, const float4 &b) {
+    return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w);
+}
+__device__ __forceinline__ float4 scale4(const float4 &a, float s) { return make_float4(a.x * s, a.y * s, a.z * s, a.w * s); }
+// (c + cab * p) * g, and the same added to acc
+__device__ __forceinline__ float4 term4(float c, float cab, const float4 &p, const float4 &g) {
+    return make_float4(fmaf(cab, p.x, c) * g.x, fmaf(cab, p.y, c) * g.y, fmaf(cab, p.z, c) * g.z, fmaf(cab, p.w, c) * g.w);
+}
+__device__ __forceinline__ float4 term4_add(float c, float cab, const float4 &p, const float4 &g, const float4 &acc) {
+    return make_float4(fmaf(fmaf(cab, p.x, c), g.x, acc.x), fmaf(fmaf(cab, p.y, c), g.y, acc.y),
+                       fmaf(fmaf(cab, p.z, c), g.z, acc.z), fmaf(fmaf(cab, p.w, c), g.w, acc.w));
+}
+
+// Sums over the G lanes of a group for 32 values per lane at once: at every step a lane hands half of its values to its
+// partner and keeps the other half, so 32 sums cost 31 (G = 32) shuffles instead of 160.  Afterwards v[0 .. 32/G) of lane l
+// hold the sums of values l * 32/G ...
+template <int G>
+__device__ __forceinline__ void transpose_sum(float (&v)[4 * kWalkSteps], int lane) {
+    int n = 4 * kWalkSteps;
+#pragma unroll
+    for (int h = G / 2; h >= 1; h >>= 1) {
+        n >>= 1;
+        const bool up = (lane & h) != 0;
+#pragma unroll
+        for (int i = 0; i < 2 * kWalkSteps; ++i) {
+            if (i < n) {
+                const float give = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ void async_copy16(void *dst_smem, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void async_copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Optional Adam step in the epilogue, as in train.cu's backward_w: moments of this layer, state = {steps done, ticket}.
+struct WalkAdam {
+    float *m, *v;
+    int *state;
+    float lr, beta1, beta2, eps, grad_scale;
+};
+
+// GX: grad_x is wanted and the walk passes every input row once (WalkPlan complete); else only the weight gradients.
+template <int G, bool VEC, bool GX>
+__global__ void __launch_bounds__(kThreads, 2)
+walk_backward_kernel(const float *__restrict__ x, const float *__restrict__ gy, const float4 *__restrict__ coef, const float *w,
+                     float *__restrict__ grad_w, float *__restrict__ gx, float scale, const int2 *__restrict__ walk, int entries,
+                     int64_t batch, int wc, int ncb, int gy_group, WalkAdam adam) {
+    constexpr int N = kWalkWarps * (32 / G) * kWalkSteps;
+    constexpr bool kStaged = N * 4 == kThreads;  // one quarter neuron per thread: weights and moments are fetched ahead
+    __shared__ int s_node[N + 2], s_edge[N + 2], s_gy[N + 2];  // index t: entry first - 1 + t
+    __shared__ float4 s_coef[N + 1];                           // {c of the row stood on, c of the row led to, cab, -}
+    __shared__ float s_sum[G == 32 ? kWalkWarps * N * 4 : N * 4];
+    __shared__ float4 s_ahead[kStaged ? 3 * kThreads : 1];
+    __shared__ float s_step_size, s_bc2_sqrt;
+
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % G;
+    const int first = blockIdx.x * N;
+    for (int t = tid; t < N + 2; t += kThreads) {
+        const int at = first - 1 + t;
+        const int2 e = at >= 0 && at < entries ? __ldg(walk + at) : make_int2(-1, -1);
+        s_node[t] = e.x;
+        s_edge[t] = e.y;
+        s_gy[t] = e.y < 0 ? 0 : gy_group == 1 ? e.y >> 2 : (e.y >> 2) / gy_group;
+    }
+    if (adam.m != nullptr && tid == 0) {
+        const float t = (float)(adam.state[0] + 1);
+        s_step_size = adam.lr / (1.f - powf(adam.beta1, t));
+        s_bc2_sqrt = sqrtf(1.f - powf(adam.beta2, t));
+    }
+    __syncthreads();
+    // the quarter neuron of this thread in the epilogue (kStaged); its moments are touched by this kernel only, one step
+    // apart, so they may be fetched before the kernel in front is through
+    const int my_edge = kStaged ? s_edge[(tid >> 2) + 1] : -1;
+    const bool my_emit = kStaged && my_edge >= 0 && (my_edge & 1);
+    const int64_t my_at = (int64_t)(my_edge >> 2) * 16 + (tid & 3) * 4;
+    if (my_emit && adam.m != nullptr) {
+        async_copy16(s_ahead + kThreads + tid, adam.m + my_at);
+        async_copy16(s_ahead + 2 * kThreads + tid, adam.v + my_at);
+    }
+    grid_dependency_wait();
+    grid_dependents_launch();
+    if (my_emit) async_copy16(s_ahead + tid, w + my_at);
+
+    const int wcol = warp % wc;
+    const int p = ((warp / wc) * (32 / G) + (tid % 32) / G) * (kWalkSteps * wc) + 1;  // this chunk's first entry, as an index t
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 xin = zero4, xh = zero4, gh = zero4, dprev = zero4, xn[kWalkSteps], g[kWalkSteps];
+    auto begin = [&](const RowIo<G, VEC> &io) {
+        xin = s_node[p] >= 0 ? io.load(x, s_node[p] >> 1, batch) : zero4;
+        if (GX) {
+            xh = gh = zero4;
+            if (s_edge[p - 1] >= 0) {
+                xh = io.load(x, s_node[p - 1] >> 1, batch);
+                gh = io.load(gy, s_gy[p - 1], batch);
+            }
+        }
+    };
+    auto fetch = [&](const RowIo<G, VEC> &io, int q) {
+#pragma unroll
+        for (int i = 0; i < kWalkSteps; ++i) {
+            xn[i] = g[i] = zero4;
+            if (s_node[q + i + 1] >= 0) xn[i] = io.load(x, s_node[q + i + 1] >> 1, batch);
+            if (s_edge[q + i] >= 0) g[i] = io.load(gy, s_gy[q + i], batch);
+        }
+    };
+    float4 my_coef[(N + kThreads) / kThreads];
+#pragma unroll
+    for (int r = 0; r < (N + kThreads) / kThreads; ++r) {
+        const int t = tid + r * kThreads;
+        my_coef[r] = zero4;
+        if (t <= N && s_edge[t] >= 0) my_coef[r] = __ldg(coef + (s_edge[t] >> 2));
+    }
+    int cb = wcol;
+    if (cb < ncb) {
+        const RowIo<G, VEC> io((int64_t)cb * (4 * G), lane, batch);
+        begin(io);
+        fetch(io, p);
+    }
+#pragma unroll
+    for (int r = 0; r < (N + kThreads) / kThreads; ++r) {
+        const int t = tid + r * kThreads;
+        if (t <= N) {
+            const float4 c = my_coef[r];
+            s_coef[t] = (s_edge[t] & 2) ? make_float4(c.z, c.y, c.w, 0.f) : make_float4(c.y, c.z, c.w, 0.f);
+        }
+    }
+    __syncthreads();
+    bool fetched = true;
+    for (; cb < ncb; cb += wc) {
+        const RowIo<G, VEC> io((int64_t)cb * (4 * G), lane, batch);
+        if (!fetched) begin(io);
+        if (GX) {
+            const float4 c = s_coef[p - 1];
+            dprev = s_edge[p - 1] >= 0 ? term4(c.y, c.z, xh, gh) : zero4;
+        }
+        for (int sb = 0; sb < wc; ++sb) {
+            const int q = p + sb * kWalkSteps;
+            if (!fetched) fetch(io, q);
+            fetched = false;
+            float v[4 * kWalkSteps];
+#pragma unroll
+            for (int i = 0; i < kWalkSteps; ++i) {
+                const int e = s_edge[q + i];
+                if (GX) {
+                    const int node = s_node[q + i];
+                    float4 acc = dprev;
+                    dprev = zero4;
+                    if (e >= 0) {
+                        const float4 c = s_coef[q + i];
+                        acc = term4_add(c.x, c.z, xn[i], g[i], acc);
+                        dprev = term4(c.y, c.z, xin, g[i]);
+                    }
+                    if (node >= 0 && (node & 1)) io.store(gx, node >> 1, batch, scale4(acc, scale));
+                }
+                const float4 ag = mul4(xin, g[i]);
+                v[4 * i] = sum4(g[i]);
+                v[4 * i + 1] = sum4(ag);
+                v[4 * i + 2] = sum4(mul4(xn[i], g[i]));
+                v[4 * i + 3] = sum4(mul4(ag, xn[i]));
+                xin = xn[i];
+            }
+            transpose_sum<G>(v, lane);
+            float *dst = s_sum + (G == 32 ? wcol * N * 4 : 0) + (q - 1) * 4 + lane * (32 / G);
+#pragma unroll
+            for (int i = 0; i < 32 / G; ++i) dst[i] = cb == wcol ? v[i] : dst[i] + v[i];
+        }
+    }
+    async_copies_wait();
+    __syncthreads();
+
+    // ---- epilogue: four lanes per neuron, four gates each: 16 gradients, softmax backward, Adam
+    const int parts = wc < ncb ? wc : ncb;
+    for (int t = tid; t < N * 4; t += kThreads) {
+        const int e = s_edge[(t >> 2) + 1], q = t & 3;
+        const bool emit = e >= 0 && (e & 1);
+        const int64_t at = (int64_t)(e >> 2) * 16 + q * 4;
+        float mine = 0.f;
+        for (int r = 0; r < parts; ++r) mine += s_sum[r * N * 4 + t];
+        const int base = tid & 28;
+        const float s0 = __shfl_sync(0xffffffffu, mine, base), s1 = __shfl_sync(0xffffffffu, mine, base + 1),
+                    s2 = __shfl_sync(0xffffffffu, mine, base + 2), sab = __shfl_sync(0xffffffffu, mine, base + 3);
+        const float sa = (e & 2) ? s2 : s1, sb = (e & 2) ? s1 : s2;
+        float4 w4 = make_float4(0.f, 0.f, 0.f, 0.f), m4 = w4, v4 = w4;
+        if (emit) {
+            if (kStaged) {
+                w4 = s_ahead[tid];
+            } else {
+                w4 = *reinterpret_cast<const float4 *>(w + at);
+            }
+            if (adam.m != nullptr) {
+                m4 = kStaged ? s_ahead[kThreads + tid] : *reinterpret_cast<const float4 *>(adam.m + at);
+                v4 = kStaged ? s_ahead[2 * kThreads + tid] : *reinterpret_cast<const float4 *>(adam.v + at);
+            }
+        }
+        float pr[4] = {w4.x, w4.y, w4.z, w4.w}, out[4];
+        float mx = fmaxf(fmaxf(pr[0], pr[1]), fmaxf(pr[2], pr[3]));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { pr[i] = expf(pr[i] - mx); s += pr[i]; }
+        s = quad_sum(s);
+        float dot = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            pr[i] = pr[i] / s;
+            out[i] = gate_grad_from_sums(4 * q + i, s0, sa, sb, sab);
+            dot += pr[i] * out[i];
+        }
+        dot = quad_sum(dot);
+        float4 o = make_float4(pr[0] * (out[0] - dot), pr[1] * (out[1] - dot), pr[2] * (out[2] - dot), pr[3] * (out[3] - dot));
+        if (emit) {
+            if (grad_w != nullptr) *reinterpret_cast<float4 *>(grad_w + at) = o;
+            if (adam.m != nullptr) {
+                const AdamConsts consts = {1.f - adam.beta1, adam.beta2, 1.f - adam.beta2, s_step_size, s_bc2_sqrt, adam.eps};
+                o = make_float4(__fmul_rn(o.x, adam.grad_scale), __fmul_rn(o.y, adam.grad_scale), __fmul_rn(o.z, adam.grad_scale),
+                                __fmul_rn(o.w, adam.grad_scale));
+                adam_update4(w4, o, m4, v4, consts);
+                *reinterpret_cast<float4 *>(const_cast<float *>(w) + at) = w4;
+                *reinterpret_cast<float4 *>(adam.m + at) = m4;
+                *reinterpret_cast<float4 *>(adam.v + at) = v4;
+            }
+        }
+    }
+    if (adam.m != nullptr && tid == 0) {
+        // thread 0 of every CTA has read the step count at its start; the last one to get here advances it
+        if (atomicAdd(adam.state + 1, 1) == (int)gridDim.x - 1) {
+            adam.state[1] = 0;
+            adam.state[0] = adam.state[0] + 1;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------------
+// Lanes per row, warps side by side over the columns, column blocks of 4 * G.  As many warps as there are column blocks
+// (a power of two, at most 8) share a chunk unless that leaves more than a quarter of them idle.
+struct WalkShape {
+    int G, wc, ncb;
+};
+static WalkShape walk_shape(int64_t batch) {
+    const int64_t lanes = ceil_div(batch, 4);
+    WalkShape s;
+    s.G = lanes <= 8 ? 8 : lanes <= 16 ? 16 : 32;
+    s.ncb = (int)ceil_div(batch, 4 * s.G);
+    s.wc = kWalkWarps;
+    while (s.wc > 1 && ceil_div(s.ncb, s.wc) * s.wc * 4 > (int64_t)s.ncb * 5) s.wc /= 2;
+    return s;
+}
+static int64_t walk_ctas(int G, int64_t entries) { return ceil_div(entries, (int64_t)kWalkWarps * (32 / G) * kWalkSteps); }
+
+}  // namespace dl
+
+using namespace dl;
+
+// Walk of a layer's connection graph, built on the host from HOST copies of a and b.  out: int32 pairs (format above), room
+// for dl_walk_capacity(n_in, n_out) of them.  *entries: how many were written; *complete: 1 when no input feeds more than two
+// neurons, so that the walk passes every input row exactly once (grad_x can be formed along it).
+extern "C" DL_API int64_t dl_walk_capacity(int64_t n_in, int64_t n_out) { return n_in + 3 * n_out + 1; }
+
+extern "C" DL_API int dl_build_walk(const int64_t *a, const int64_t *b, int64_t n_in, int64_t n_out, int32_t *out, int64_t *entries,
+                                    int *complete) {
+    DL_REQUIRE(n_in > 0 && n_out > 0 && a && b && out && entries && complete, DL_ERR_INVALID_ARG, "dl_build_walk: null pointer or size");
+    DL_REQUIRE(n_in < ((int64_t)1 << 30) && n_out < ((int64_t)1 << 28), DL_ERR_TOO_LARGE, "dl_build_walk: too many rows");
+    struct Ends {
+        int32_t a, b;
+    };
+    struct Reach {
+        int32_t next, end;
+    };
+    std::vector<Ends> ends(n_out);
+    std::vector<int32_t> degree(n_in, 0);
+    int32_t most = 0;
+    for (int64_t j = 0; j < n_out; ++j) {
+        DL_REQUIRE(a[j] >= 0 && a[j] < n_in && b[j] >= 0 && b[j] < n_in, DL_ERR_INVALID_ARG,
+                   "dl_build_walk: connection of neuron %lld outside [0, %lld)", (long long)j, (long long)n_in);
+        ends[j] = {(int32_t)a[j], (int32_t)b[j]};
+        const int32_t da = ++degree[a[j]], db = ++degree[b[j]];
+        most = da > most ? da : most;
+        most = db > most ? db : most;
+    }
+    int64_t n = 0;
+    auto put = [&](int32_t node, int store, int32_t edge) {
+        out[2 * n] = node << 1 | store;
+        out[2 * n + 1] = edge;
+        ++n;
+    };
+    if (most <= 2) {
+        // every input lies on one walk, once: from an input the walk goes on by the neuron that it did not come by
+        std::vector<Ends> readers(n_in, {-1, -1});
+        for (int32_t j = 0; j < (int32_t)n_out; ++j)
+            for (const int32_t v : {ends[j].a, ends[j].b}) (readers[v].a < 0 ? readers[v].a : readers[v].b) = j;
+        std::vector<uint8_t> seen(n_in, 0);
+        auto follow = [&](int32_t v, bool closed) {
+            const int32_t home = v;
+            const int64_t head = n;
+            if (closed) put(v, 0, -1);  // becomes the repetition of the walk's last step
+            int32_t came = -1;          // neuron the walk came by (its first neuron at home)
+            do {
+                seen[v] = 1;
+                const int32_t j = readers[v].a != came ? readers[v].a : readers[v].b;
+                const bool loop = j >= 0 && ends[j].a == ends[j].b;
+                if (j < 0) break;
+                const int flip = ends[j].a != v ? 2 : 0;
+                put(v, 1, j << 2 | flip | 1);
+                v = flip ? ends[j].a : ends[j].b;
+                came = j;
+                if (loop) break;
+            } while (v != home);
+            if (closed) {
+                out[2 * head] = out[2 * (n - 1)] & ~1;
+                out[2 * head + 1] = out[2 * (n - 1) + 1] & ~1;
+                put(v, 0, -1);
+            } else {
+                put(v, 1, -1);
+            }
+        };
+        for (int32_t i = 0; i < (int32_t)n_in; ++i)  // open walks begin and end at inputs that feed one neuron (or none)
+            if (degree[i] < 2 && !seen[i]) follow(i, false);
+        for (int32_t i = 0; i < (int32_t)n_in; ++i)
+            if (!seen[i]) follow(i, true);
+        *entries = n;
+        *complete = 1;
+        return DL_OK;
+    }
+    std::vector<Reach> reach(n_in);
+    std::vector<int32_t> list(2 * n_out);
+    int32_t at = 0;
+    for (int64_t i = 0; i < n_in; ++i) {
+        reach[i] = {at, at};
+        at += degree[i];
+    }
+    for (int32_t j = 0; j < (int32_t)n_out; ++j) {
+        list[reach[ends[j].a].end++] = j;
+        list[reach[ends[j].b].end++] = j;
+    }
+    std::vector<uint8_t> used(n_out, 0);
+    auto follow = [&](int32_t v) {  // by unused neurons until there are none
+        bool any = false;
+        for (;;) {
+            Reach &r = reach[v];
+            while (r.next < r.end && used[list[r.next]]) ++r.next;
+            if (r.next == r.end) break;
+            const int32_t j = list[r.next++];
+            used[j] = 1;
+            const int flip = ends[j].a != v ? 2 : 0;
+            put(v, 0, j << 2 | flip | 1);
+            v = flip ? ends[j].a : ends[j].b;
+            any = true;
+        }
+        if (any) put(v, 0, -1);
+        return any;
+    };
+    for (int32_t i = 0; i < (int32_t)n_in; ++i)  // open walks begin and end at inputs that feed an odd number of neurons
+        if (degree[i] % 2 == 1) follow(i);
+    for (int32_t i = 0; i < (int32_t)n_in; ++i)
+        while (follow(i)) {
+        }
+    *entries = n;
+    *complete = 0;
+    return DL_OK;
+}
+
+static int walk_checks(const char *who, const int32_t *walk, int64_t entries, int64_t n_in, int64_t n_out, int64_t batch) {
+    DL_REQUIRE(walk != nullptr && aligned_to(walk, 8) && entries > 0 && entries <= INT32_MAX, DL_ERR_INVALID_ARG, "%s: bad walk", who);
+    DL_REQUIRE(n_in > 0 && n_out > 0 && batch > 0, DL_ERR_INVALID_ARG, "%s: sizes must be positive", who);
+    DL_REQUIRE(n_in < ((int64_t)1 << 30) && n_out < ((int64_t)1 << 28) && batch < ((int64_t)1 << 31), DL_ERR_TOO_LARGE, "%s: too large", who);
+    return DL_OK;
+}
+
+extern "C" DL_API int dl_forward_walk_f32(const float *x, const float *w, int w_mode, float *y, float *coef, const int32_t *walk,
+                                          int64_t entries, int64_t n_in, int64_t n_out, int64_t batch, int flags, void *stream) {
+    if (int s = walk_checks("dl_forward_walk_f32", walk, entries, n_in, n_out, batch)) return s;
+    DL_REQUIRE(w_mode >= DL_W_LOGITS && w_mode <= DL_W_ARGMAX, DL_ERR_INVALID_ARG, "dl_forward_walk_f32: unknown w_mode %d", w_mode);
+    DL_REQUIRE(x && w && y, DL_ERR_INVALID_ARG, "dl_forward_walk_f32: null pointer");
+    DL_REQUIRE(coef == nullptr || aligned_to(coef, 16), DL_ERR_INVALID_ARG, "dl_forward_walk_f32: coef must be 16-byte aligned");
+    const WalkShape s = walk_shape(batch);
+    const bool vec = batch % 4 == 0 && aligned_to(x, 16) && aligned_to(y, 16);
+    const bool overlap = (flags & DL_LAUNCH_OVERLAP_SETUP) != 0;
+    const dim3 grid((unsigned)walk_ctas(s.G, entries));
+    const int2 *wk = reinterpret_cast<const int2 *>(walk);
+    float4 *c4 = reinterpret_cast<float4 *>(coef);
+#define DL_WF(GG)                                                                                                                     \
+    case GG:                                                                                                                          \
+        if (vec) launch_dependent(overlap, walk_forward_kernel<GG, true>, grid, dim3(kThreads), 0, as_stream(stream), x, w, w_mode, y, c4, \
+                                  wk, (int)entries, batch, s.wc, s.ncb);                                                              \
+        else launch_dependent(overlap, walk_forward_kernel<GG, false>, grid, dim3(kThreads), 0, as_stream(stream), x, w, w_mode, y, c4,    \
+                              wk, (int)entries, batch, s.wc, s.ncb);                                                                  \
+        break;
+    switch (s.G) { DL_WF(8) DL_WF(16) DL_WF(32) }
+#undef DL_WF
+    return launch_status("dl_forward_walk_f32");
+}
+
+extern "C" DL_API int dl_backward_walk_f32(const float *x, const float *grad_y, const float *coef, float *w, float *grad_w, float *grad_x,
+                                           float grad_scale, const int32_t *walk, int64_t entries, int complete, int64_t n_in,
+                                           int64_t n_out, int64_t batch, int64_t rows_per_class, float *exp_avg, float *exp_avg_sq,
+                                           float lr, float beta1, float beta2, float eps, float adam_grad_scale, int32_t *state, int flags,
+                                           void *stream) {
+    const char *who = "dl_backward_walk_f32";
+    if (int s = walk_checks(who, walk, entries, n_in, n_out, batch)) return s;
+    DL_REQUIRE(rows_per_class >= 1 && rows_per_class <= INT32_MAX && n_out % rows_per_class == 0, DL_ERR_INVALID_ARG,
+               "%s: n_out (%lld) is not a multiple of the rows per class (%lld)", who, (long long)n_out, (long long)rows_per_class);
+    DL_REQUIRE(x && grad_y && coef && w && (grad_w || exp_avg), DL_ERR_INVALID_ARG, "%s: null pointer", who);
+    DL_REQUIRE(grad_x == nullptr || complete, DL_ERR_INVALID_ARG, "%s: grad_x needs a walk that passes every input once", who);
+    DL_REQUIRE((exp_avg == nullptr) == (exp_avg_sq == nullptr) && (exp_avg == nullptr || state), DL_ERR_INVALID_ARG, "%s: null pointer", who);
+    DL_REQUIRE(aligned_to(coef, 16) && aligned_to(w, 16) && aligned_to(grad_w, 16) && aligned_to(exp_avg, 16) && aligned_to(exp_avg_sq, 16),
+               DL_ERR_INVALID_ARG, "%s: coef, w, grad_w and the moments must be 16-byte aligned", who);
+    const WalkShape s = walk_shape(batch);
+    const bool vec = batch % 4 == 0 && aligned_to(x, 16) && aligned_to(grad_y, 16) && aligned_to(grad_x, 16);
+    const bool overlap = (flags & DL_LAUNCH_OVERLAP_SETUP) != 0;
+    const dim3 grid((unsigned)walk_ctas(s.G, entries));
+    const WalkAdam adam = {exp_avg, exp_avg_sq, reinterpret_cast<int *>(state), lr, beta1, beta2, eps, adam_grad_scale};
+    auto launch = [&](auto kernel) {
+        launch_dependent(overlap, kernel, grid, dim3(kThreads), 0, as_stream(stream), x, grad_y, reinterpret_cast<const float4 *>(coef), w,
+                         grad_w, grad_x, grad_scale, reinterpret_cast<const int2 *>(walk), (int)entries, batch, s.wc, s.ncb,
+                         (int)rows_per_class, adam);
+    };
+#define DL_WB(GG)                                                                                                        \
+    case GG:                                                                                                             \
+        if (grad_x != nullptr) vec ? launch(walk_backward_kernel<GG, true, true>) : launch(walk_backward_kernel<GG, false, true>); \
+        else vec ? launch(walk_backward_kernel<GG, true, false>) : launch(walk_backward_kernel<GG, false, false>);       \
+        break;
+    switch (s.G) { DL_WB(8) DL_WB(16) DL_WB(32) }
+#undef DL_WB
+    return launch_status(who);
+}

@@ -109,7 +109,8 @@ class LogicLayer(torch.nn.Module):
 
         `given_x_indices_of_y_start` / `given_x_indices_of_y` have the reference's meaning
         (difflogic.py:56-69); `_plan` is the same index with the partner row and the input slot
-        resolved, which is what the kernel walks."""
+        resolved, which is what the gather kernel follows; `_walk` is the order in which the walk kernels
+        take the neurons (ops.build_walk)."""
         a, b = self.indices
         self.indices = (a.contiguous(), b.contiguous())
         a, b = self.indices
@@ -120,11 +121,12 @@ class LogicLayer(torch.nn.Module):
             self._plan = ops.build_backward_plan(a, b, self.given_x_indices_of_y_start, self.given_x_indices_of_y)
             if _DEBUG_CHECKS:
                 ops.check_connections(a, b, self.in_dim, self.given_x_indices_of_y_start, self.given_x_indices_of_y, self._plan)
+            self._walk = ops.build_walk(a, b, self.in_dim)
             # the layer's kernels may read these index tensors ahead of the kernel that precedes them in the
             # stream (DL_LAUNCH_OVERLAP_SETUP), so they must be final before any such launch is queued
             torch.cuda.current_stream(a.device).synchronize()
         else:
-            self._plan = None
+            self._plan = self._walk = None
 
     def set_connections(self, a, b):
         """Replaces the connection indices (e.g. to copy them from another model) and rebuilds the inverse index."""
@@ -193,10 +195,10 @@ class LogicLayer(torch.nn.Module):
         a, b = self.indices
         if self.training:
             y = LogicLayerFunction.apply(x, self.weights, a, b, self.given_x_indices_of_y_start, self._plan,
-                                         float(self.grad_factor), getattr(self.weights, '_dl_grad_out', None))
+                                         float(self.grad_factor), getattr(self.weights, '_dl_grad_out', None), self._walk)
         else:
             with torch.no_grad():
-                y, _ = ops.logic_forward(x, a, b, self.weights, ops.W_ARGMAX, overlap=True)
+                y, _ = _forward(x, a, b, self.weights, self._walk, ops.W_ARGMAX)
         return y.transpose(0, 1)
 
     def forward_cuda_eval(self, x: PackBitsTensor):
@@ -256,6 +258,12 @@ class GroupSum(torch.nn.Module):
 ########################################################################################################################
 
 
+def _forward(x, a, b, weights, walk, w_mode, want_coef=False):
+    if walk is not None and x.shape[1] > 0:
+        return ops.logic_forward_walk(x, weights, walk, w_mode, want_coef=want_coef, overlap=True)
+    return ops.logic_forward(x, a, b, weights, w_mode, want_coef=want_coef, overlap=True)
+
+
 def _run_backward_w(x, a, b, grad, weights, grad_out, rows_per_class=1):
     """backward_w of a layer; with an optimizer that steps inside backward (FlatAdam.enable_step_in_backward) the
     weights are updated by the same kernel and there is no gradient to return."""
@@ -271,6 +279,44 @@ def _run_backward_w(x, a, b, grad, weights, grad_out, rows_per_class=1):
     return ops.logic_backward_w(x, a, b, grad, weights, ops.W_LOGITS, out=grad_out, overlap=True, rows_per_class=rows_per_class)
 
 
+def _run_backward(ctx, x, weights, a, b, start, plan, coef, grad_y, rows_per_class=1):
+    """(grad_x, grad_w) of a layer, None for what is not wanted.  One kernel along the layer's walk gives both (or the
+    weight gradient alone); layers whose walk cannot give grad_x, and those whose gradients are sent to other GPUs by
+    backward_w itself, run the two gather kernels."""
+    want_x, want_w = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
+    walk = ctx.walk
+    grad_x = grad_w = None
+    exchange = getattr(weights, '_dl_exchange', None)
+    if (walk is not None and want_w and (walk[1] or not want_x) and x.shape[1] > 0
+            and (exchange is None or exchange.gradient_by_plain_kernel(weights))
+            and weights.data_ptr() % 16 == 0 and (ctx.grad_out is None or ctx.grad_out.data_ptr() % 16 == 0)):
+        opt = getattr(weights, '_dl_adam', None)
+        grad_x, grad_w = ops.logic_backward_walk(
+            x, grad_y, coef, weights.data, walk, ctx.grad_factor, want_grad_x=want_x, grad_out=None if opt is not None else ctx.grad_out,
+            adam=opt.backward_args(weights) if opt is not None else None, overlap=True, rows_per_class=rows_per_class)
+        if exchange is not None:
+            exchange.gradient_queued(weights)
+    else:
+        side = _backward_w_stream if (want_x and want_w) else None
+        if side is not None:
+            # fork: backward_w on the side stream, backward_x stays on the stream the next layer is waiting on
+            main = torch.cuda.current_stream(x.device)
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                grad_w = _run_backward_w(x, a, b, grad_y, weights, ctx.grad_out, rows_per_class)
+            for t in (x, grad_y, weights):
+                t.record_stream(side)
+        if want_x:
+            grad_x = ops.logic_backward_x(x, coef, grad_y, start, plan, ctx.grad_factor, overlap=True, rows_per_class=rows_per_class)
+        if want_w and side is None:
+            grad_w = _run_backward_w(x, a, b, grad_y, weights, ctx.grad_out, rows_per_class)
+    if grad_w is not None and ctx.grad_out is not None:
+        # a fresh alias that nothing else references: autograd then adopts it as `weights.grad` instead of copying it, so
+        # the gradient stays inside the flat bucket
+        grad_w = grad_w.view(grad_w.shape)
+    return grad_x, grad_w
+
+
 class LogicLayerFunction(torch.autograd.Function):
     """Autograd node of one logic layer on feature-major tensors, from the raw weights.
 
@@ -278,38 +324,17 @@ class LogicLayerFunction(torch.autograd.Function):
     in front of it and the GradFactor node before the layer."""
 
     @staticmethod
-    def forward(ctx, x, weights, a, b, start, plan, grad_factor, grad_out=None):
-        y, coef = ops.logic_forward(x, a, b, weights, ops.W_LOGITS, want_coef=True, overlap=True)
+    def forward(ctx, x, weights, a, b, start, plan, grad_factor, grad_out=None, walk=None):
+        y, coef = _forward(x, a, b, weights, walk, ops.W_LOGITS, want_coef=True)
         ctx.save_for_backward(x, weights, a, b, start, plan, coef)
-        ctx.grad_factor = grad_factor
+        ctx.grad_factor, ctx.walk = grad_factor, walk
         ctx.grad_out = grad_out  # optional [out_dim, 16] buffer (a slice of a flat gradient bucket) for backward_w
         return y
 
     @staticmethod
     def backward(ctx, grad_y):
         x, weights, a, b, start, plan, coef = ctx.saved_tensors
-        grad_y = grad_y.contiguous()
-        grad_x = grad_w = None
-        side = _backward_w_stream if (ctx.needs_input_grad[0] and ctx.needs_input_grad[1]) else None
-        if side is not None:
-            # fork: backward_w on the side stream, backward_x stays on the stream the next layer is waiting on
-            main = torch.cuda.current_stream(x.device)
-            side.wait_stream(main)
-            with torch.cuda.stream(side):
-                grad_w = _run_backward_w(x, a, b, grad_y, weights, ctx.grad_out)
-            for t in (x, grad_y, weights):
-                t.record_stream(side)
-            grad_x = ops.logic_backward_x(x, coef, grad_y, start, plan, ctx.grad_factor, overlap=True)
-        else:
-            if ctx.needs_input_grad[0]:
-                grad_x = ops.logic_backward_x(x, coef, grad_y, start, plan, ctx.grad_factor, overlap=True)
-            if ctx.needs_input_grad[1]:
-                grad_w = _run_backward_w(x, a, b, grad_y, weights, ctx.grad_out)
-        if grad_w is not None and ctx.grad_out is not None:
-            # a fresh alias that nothing else references: autograd then adopts it as `weights.grad`
-            # instead of copying it, so the gradient stays inside the flat bucket
-            grad_w = grad_w.view(grad_w.shape)
-        return grad_x, grad_w, None, None, None, None, None, None
+        return _run_backward(ctx, x, weights, a, b, start, plan, coef, grad_y.contiguous()) + (None,) * 7
 
 
 class LogicLayerHeadFunction(torch.autograd.Function):
@@ -324,16 +349,16 @@ class LogicLayerHeadFunction(torch.autograd.Function):
     `loss_fn(model(x), y)` (experiments/main.py:175) with the same numbers."""
 
     @staticmethod
-    def forward(ctx, x, weights, a, b, start, plan, grad_factor, grad_out, target, k, tau):
+    def forward(ctx, x, weights, a, b, start, plan, grad_factor, grad_out, target, k, tau, walk=None):
         n_out = weights.shape[0]
         if ops.forward_head_applicable(n_out, x.shape[1], k):
             # the layer's rows are added up per class inside the forward kernel; its output is never stored
             loss, scores, grad_classes, coef = ops.logic_forward_head(x, a, b, weights, target, k, tau)
         else:
-            y, coef = ops.logic_forward(x, a, b, weights, ops.W_LOGITS, want_coef=True, overlap=True)
+            y, coef = _forward(x, a, b, weights, walk, ops.W_LOGITS, want_coef=True)
             loss, scores, grad_classes = ops.groupsum_cross_entropy(y, target, k, tau)
         ctx.save_for_backward(x, weights, a, b, start, plan, coef, grad_classes)
-        ctx.grad_factor, ctx.grad_out, ctx.rows_per_class = grad_factor, grad_out, n_out // k
+        ctx.grad_factor, ctx.grad_out, ctx.rows_per_class, ctx.walk = grad_factor, grad_out, n_out // k, walk
         ctx.mark_non_differentiable(scores)
         ctx.set_materialize_grads(False)
         return loss, scores
@@ -341,29 +366,11 @@ class LogicLayerHeadFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_loss, _grad_scores):
         if grad_loss is None:
-            return (None,) * 11
+            return (None,) * 12
         x, weights, a, b, start, plan, coef, grad_classes = ctx.saved_tensors
         if not getattr(grad_loss, '_dl_is_one', False):
             grad_classes = grad_classes * grad_loss     # a gradient other than the marked unit tensor: scale (one more kernel)
-        m = ctx.rows_per_class
-        grad_x = grad_w = None
-        side = _backward_w_stream if (ctx.needs_input_grad[0] and ctx.needs_input_grad[1]) else None
-        if side is not None:
-            main = torch.cuda.current_stream(x.device)
-            side.wait_stream(main)
-            with torch.cuda.stream(side):
-                grad_w = _run_backward_w(x, a, b, grad_classes, weights, ctx.grad_out, rows_per_class=m)
-            for t in (x, grad_classes, weights):
-                t.record_stream(side)
-            grad_x = ops.logic_backward_x(x, coef, grad_classes, start, plan, ctx.grad_factor, overlap=True, rows_per_class=m)
-        else:
-            if ctx.needs_input_grad[0]:
-                grad_x = ops.logic_backward_x(x, coef, grad_classes, start, plan, ctx.grad_factor, overlap=True, rows_per_class=m)
-            if ctx.needs_input_grad[1]:
-                grad_w = _run_backward_w(x, a, b, grad_classes, weights, ctx.grad_out, rows_per_class=m)
-        if grad_w is not None and ctx.grad_out is not None:
-            grad_w = grad_w.view(grad_w.shape)  # a fresh alias: autograd adopts it as `weights.grad` without copying
-        return (grad_x, grad_w) + (None,) * 9
+        return _run_backward(ctx, x, weights, a, b, start, plan, coef, grad_classes, ctx.rows_per_class) + (None,) * 10
 
 
 def logic_layer_head(layer, x, target, k, tau):
@@ -379,7 +386,7 @@ def logic_layer_head(layer, x, target, k, tau):
     a, b = layer.indices
     return LogicLayerHeadFunction.apply(xt, layer.weights, a, b, layer.given_x_indices_of_y_start, layer._plan,
                                         float(layer.grad_factor), getattr(layer.weights, '_dl_grad_out', None),
-                                        target.contiguous(), int(k), float(tau))
+                                        target.contiguous(), int(k), float(tau), layer._walk)
 
 
 class LogicLayerCudaFunction(torch.autograd.Function):

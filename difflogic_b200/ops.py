@@ -193,6 +193,66 @@ def build_backward_plan(a, b, start, lst):
     return plan
 
 
+def build_walk(a, b, n_in):
+    """Walk of a layer's connection graph for logic_forward_walk / logic_backward_walk: (entries int32 [n, 2] on a's device,
+    complete), or None for sizes or indices it does not take.  Built on the host (dl_build_walk)."""
+    import ctypes
+    n_out = a.numel()
+    if n_out == 0 or n_in == 0:
+        return None
+    ah, bh = a.cpu().contiguous(), b.cpu().contiguous()
+    out = torch.empty((N.lib().dl_walk_capacity(int(n_in), n_out), 2), dtype=torch.int32)
+    entries, complete = ctypes.c_int64(), ctypes.c_int()
+    if N.lib().dl_build_walk(ah.data_ptr(), bh.data_ptr(), int(n_in), n_out, out.data_ptr(), ctypes.addressof(entries),
+                             ctypes.addressof(complete)) != N.DL_OK:
+        return None
+    return out[:entries.value].to(a.device), bool(complete.value)
+
+
+def logic_forward_walk(x, w, walk, w_mode=W_LOGITS, want_coef=False, overlap=False):
+    """logic_forward along the layer's walk (build_walk): same result, one row load per neuron."""
+    _f32_matrix(x, "x")
+    _f32_matrix(w, "w")
+    n_in, batch = x.shape
+    n_out = w.shape[0]
+    _need(w.shape[1] == 16, "w must be [n_out, 16]")
+    y = torch.empty((n_out, batch), dtype=torch.float32, device=x.device)
+    coef = torch.empty((n_out, 4), dtype=torch.float32, device=x.device) if want_coef else None
+    with torch.cuda.device(x.device):
+        N.check(N.lib().dl_forward_walk_f32(x.data_ptr(), w.data_ptr(), w_mode, y.data_ptr(), N.ptr(coef), walk[0].data_ptr(),
+                                            walk[0].shape[0], n_in, n_out, batch, int(overlap), N.stream_of(x)))
+    return y, coef
+
+
+def logic_backward_walk(x, grad_y, coef, w, walk, grad_scale=1.0, want_grad_x=True, grad_out=None, adam=None, overlap=False,
+                        rows_per_class=1):
+    """backward_w and backward_x of a layer in one pass along its walk: (grad_x or None, grad_w or None).  adam: what
+    FlatAdam.backward_args gives; the weights are then updated in place and grad_w is stored only into grad_out."""
+    _f32_matrix(x, "x")
+    _f32_matrix(grad_y, "grad_y")
+    _f32_matrix(coef, "coef")
+    _f32_matrix(w, "w")
+    n_in, batch = x.shape
+    n_out = w.shape[0]
+    rows_per_class = int(rows_per_class)
+    _need(tuple(grad_y.shape) == (n_out // max(rows_per_class, 1), batch), "grad_y does not fit x and w")
+    _need(tuple(w.shape) == (n_out, 16) and tuple(coef.shape) == (n_out, 4), "w must be [n_out, 16] and coef [n_out, 4]")
+    gx = torch.empty_like(x) if want_grad_x else None
+    if adam is None and grad_out is None:
+        grad_out = torch.empty((n_out, 16), dtype=torch.float32, device=x.device)
+    if grad_out is not None:
+        _f32_matrix(grad_out, "grad_out")
+        _need(tuple(grad_out.shape) == (n_out, 16), "grad_out must be [n_out, 16]")
+    a = adam or {}
+    with torch.cuda.device(x.device):
+        N.check(N.lib().dl_backward_walk_f32(x.data_ptr(), grad_y.data_ptr(), coef.data_ptr(), w.data_ptr(), N.ptr(grad_out), N.ptr(gx),
+                                             float(grad_scale), walk[0].data_ptr(), walk[0].shape[0], int(walk[1]), n_in, n_out, batch,
+                                             rows_per_class, N.ptr(a.get("exp_avg")), N.ptr(a.get("exp_avg_sq")), float(a.get("lr", 0.0)),
+                                             float(a.get("beta1", 0.0)), float(a.get("beta2", 0.0)), float(a.get("eps", 0.0)),
+                                             float(a.get("grad_scale", 1.0)), N.ptr(a.get("state")), int(overlap), N.stream_of(x)))
+    return gx, grad_out
+
+
 _VIOLATIONS = {1: "connection index outside [0, in_dim)", 2: "inverse-index offsets are not 0 = start[0] <= ... <= start[in_dim] = 2 * out_dim",
                3: "inverse-index entry outside [0, out_dim)", 4: "gather-plan entry out of range",
                5: "gather-plan entry does not match the connections"}

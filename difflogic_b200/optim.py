@@ -237,6 +237,19 @@ class FlatAdam(torch.optim.Optimizer):
                                                 self._bucket_kernels[bi:], len(self._buckets[bi][2]))
         else:
             out = ops.logic_backward_w(x, a, b, grad_y, p, ops.W_LOGITS, out=grad_out, overlap=True, rows_per_class=rows_per_class)
+        self.gradient_queued(p)
+        return out
+
+    def gradient_by_plain_kernel(self, p):
+        """True when nothing but the gradient itself is asked of the kernel that computes p's: any kernel that writes it may
+        then be launched in backward_w's place, followed by gradient_queued(p)."""
+        return not (self._push_in_backward if self._bucket_of[p] in self._packet_form else self._announce_in_backward)
+
+    def gradient_queued(self, p):
+        """The kernel that writes p's gradient is in the current stream's queue: launches the exchange of p's bucket once that
+        holds for all of the bucket's parameters."""
+        rank, world = self._exchange
+        bi = self._bucket_of[p]
         if not self._bucket_launched[bi]:
             self._bucket_pending[bi] -= 1
             if self._bucket_pending[bi] <= 0:
@@ -250,7 +263,6 @@ class FlatAdam(torch.optim.Optimizer):
                         self._one_pass.add(bi)
                     self._forms_fixed = last
                 self._launch_bucket(bi, behind_backward_w=last, announce_here=not self._announce_in_backward)
-        return out
 
     def _launch_bucket(self, bi, behind_backward_w, announce_here):
         rank, world = self._exchange

@@ -191,14 +191,14 @@ class TrainStep:
         if self._on_gpu and (self._unit_grad is None or self._unit_grad.device != loss.device):
             self._unit_grad = torch.ones((), dtype=loss.dtype, device=loss.device)
             self._unit_grad._dl_is_one = True   # lets the fused head skip the multiplication by the incoming gradient
-        # backward_w of every layer runs on a side stream, off the chain of backward_x kernels -- unless gradient
-        # hooks (the NCCL path) need the gradients in stream order
+        # backward_w of the layers that do not run both gradients in one kernel goes to a side stream, off the chain of
+        # backward_x kernels -- unless gradient hooks (the NCCL path) need the gradients in stream order
         side = self._bw_stream if (self._on_gpu and not self._hooks) else None
         if side is not None:
+            side.wait_stream(torch.cuda.current_stream())   # joined below whether or not a layer makes use of it
             _dl.set_backward_w_stream(side)
             if hasattr(self.optimizer, "prefetch_state") and not self._in_backward:
                 # warm the optimizer's moments in L2 beside the backward pass
-                side.wait_stream(torch.cuda.current_stream())
                 with torch.cuda.stream(side):
                     self.optimizer.prefetch_state()
         if self._in_backward:

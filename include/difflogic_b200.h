@@ -154,6 +154,31 @@ DL_API int dl_backward_x_f32(const float *x, const float *coef, const float *gra
 DL_API int dl_build_backward_plan(const int64_t *a, const int64_t *b, const int64_t *start, const int64_t *list,
                            int32_t *plan, int64_t n_in, int64_t n_out, void *stream);
 
+/* ------------------------------------------------------------------------------------------
+ * Training kernels along a walk of the connection graph (inputs are nodes, a neuron joins its two input rows): every
+ * neuron shares an input row with the one before it, so a row is loaded once for both.  Same results as dl_forward_f32,
+ * dl_backward_w_f32 (DL_W_LOGITS) / dl_backward_w_adam_f32 and dl_backward_x_f32; no counterpart in the reference, whose
+ * kernels gather both rows of every neuron.
+ *
+ * dl_build_walk runs on the HOST, on host copies of a and b, once per layer.  out has room for dl_walk_capacity() pairs of
+ * int32; *entries of them are written: {node << 1 | store, neuron << 2 | flip << 1 | emit} or {node << 1 | store, -1}.
+ * *complete = 1 when no input feeds more than two neurons (square layers with random connections): the walk then passes
+ * every input row once and grad_x can be formed along it.
+ * An index outside its range is refused (DL_ERR_INVALID_ARG).
+ * ---------------------------------------------------------------------------------------- */
+DL_API int64_t dl_walk_capacity(int64_t n_in, int64_t n_out);
+DL_API int dl_build_walk(const int64_t *a, const int64_t *b, int64_t n_in, int64_t n_out, int32_t *out, int64_t *entries, int *complete);
+/* dl_forward_f32 along the walk (device copy of out). */
+DL_API int dl_forward_walk_f32(const float *x, const float *w, int w_mode, float *y, float *coef, const int32_t *walk, int64_t entries,
+                               int64_t n_in, int64_t n_out, int64_t batch, int flags, void *stream);
+/* backward_w and, when grad_x is not NULL (complete walks only), backward_x in one pass.  coef: as dl_forward_f32 wrote it from w.
+ * grad_y: one row per neuron, or one per class of rows_per_class neurons.  grad_w may be NULL when exp_avg / exp_avg_sq are given:
+ * Adam then updates w, as dl_backward_w_adam_f32 does (state: this layer's {steps done, 0}). */
+DL_API int dl_backward_walk_f32(const float *x, const float *grad_y, const float *coef, float *w, float *grad_w, float *grad_x,
+                                float grad_scale, const int32_t *walk, int64_t entries, int complete, int64_t n_in, int64_t n_out,
+                                int64_t batch, int64_t rows_per_class, float *exp_avg, float *exp_avg_sq, float lr, float beta1,
+                                float beta2, float eps, float adam_grad_scale, int32_t *state, int flags, void *stream);
+
 /* Debug aid: checks a layer's index arrays on the device, once, instead of bounds checks on every access (the arrays
  * are fixed when a layer is built, and every kernel here trusts them).  Checked: a[j], b[j] in [0, n_in);
  * 0 = start[0] <= ... <= start[n_in] = 2 n_out; list entries in [0, n_out); plan entries in range and consistent with
