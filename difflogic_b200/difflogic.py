@@ -210,8 +210,15 @@ class LogicLayer(torch.nn.Module):
         x._push_layer(self)  # evaluated when x.t is read, or fused with the other layers by GroupSum
         return x
 
+    def train(self, mode=True):
+        # Kernels (an optimizer's, a replayed graph's) write the weights without autograd's version counter noticing; what was
+        # derived from the weights in eval mode does not outlive a change of mode.
+        self._gate_cache = None
+        return super().train(mode)
+
     def _gate_ids(self):
-        """uint8 arg-max gate per neuron, cached until the weights change."""
+        """uint8 arg-max gate per neuron, cached until the weights change (their version counter moves, which FlatAdam and
+        TrainStep see to for the updates that their kernels make) or the mode is set."""
         w = self.weights
         key = (w.data_ptr(), w._version)
         cached = getattr(self, '_gate_cache', None)

@@ -433,6 +433,11 @@ class FlatAdam(torch.optim.Optimizer):
             for t in (self.exp_avg, self.exp_avg_sq):
                 N.check(N.lib().dl_prefetch_l2(t.data_ptr(), t.numel() * 4, st))
 
+    def mark_updated(self):
+        """Moves the version counters of the parameters: the kernels that update them go past autograd's bookkeeping, and
+        what others have derived from the weights (arg-max gates for packed inference) is kept by version."""
+        torch.autograd.graph.increment_version(self._params)
+
     def grad_view(self, p):
         off, n = self._slices[p]
         return self.flat_grad[off:off + n].view_as(p)
@@ -466,10 +471,12 @@ class FlatAdam(torch.optim.Optimizer):
             for done in self._bucket_done:
                 current.wait_event(done)
             self._begin_exchange_step()
+            self.mark_updated()
             return loss
         with torch.cuda.device(self.flat_param.device):
             N.check(N.lib().dl_adam_step_f32(self.flat_param.data_ptr(), self.flat_grad.data_ptr(), self.exp_avg.data_ptr(),
                                              self.exp_avg_sq.data_ptr(), self.flat_param.numel(), float(g['lr']), float(beta1),
                                              float(beta2), float(g['eps']), float(self.grad_scale), self.state_t.data_ptr(),
                                              N.stream_of(self.flat_param)))
+        self.mark_updated()
         return loss

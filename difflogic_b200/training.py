@@ -212,8 +212,10 @@ class TrainStep:
                 _dl.set_backward_w_stream(None)
                 torch.cuda.current_stream().wait_stream(side)
         self._join_comm()
-        if not self._in_backward:    # else the backward_w kernels have applied the update
+        if not self._in_backward:    # else the backward kernels have applied the update
             self.optimizer.step()
+        else:
+            self.optimizer.mark_updated()
         return loss.detach()
 
     def __call__(self, x, y):
@@ -223,7 +225,12 @@ class TrainStep:
         self._static_x.copy_(x, non_blocking=True)
         self._static_y.copy_(y, non_blocking=True)
         self._graph.replay()
+        self._mark_updated()
         return self._static_loss
+
+    def _mark_updated(self):
+        """A replayed graph has updated the parameters: their version counters move as they would in an eager step."""
+        torch.autograd.graph.increment_version(self.params)
 
     def capture(self, x, y, warmup=3):
         """Captures the step in a CUDA graph.  `x`, `y` give the shapes; their contents are used for
@@ -262,6 +269,7 @@ class TrainStep:
         """Replays the step captured on resident batch i (whatever that batch's tensors hold now)."""
         graph, loss = self._resident[i][0], self._resident[i][1]
         graph.replay()
+        self._mark_updated()
         return loss
 
     @property
@@ -271,6 +279,7 @@ class TrainStep:
     def replay(self):
         """Replays the captured step on whatever the static input buffers hold."""
         self._graph.replay()
+        self._mark_updated()
         return self._static_loss
 
     def close(self):
