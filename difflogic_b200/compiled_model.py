@@ -303,7 +303,8 @@ void apply_logic_gate_net(bool const *inp, int *out, size_t len) {
         if x.dtype != torch.bool:
             x = x.ne(0)
         assert x.shape[1] == self.num_inputs, (x.shape, self.num_inputs)
-        words, pad_len = ops.packbits_batch_major(x.contiguous(), self.num_bits)
+        words, _ = ops.packbits_batch_major(x.contiguous(), self.num_bits, padded=True)
+        pad_len = words.shape[1] * self.num_bits - x.shape[0]
         for a, b, gate in self._cuda_plan[:-1]:
             words = ops.eval_packed(words, a, b, gate)
         a, b, gate = self._cuda_plan[-1]

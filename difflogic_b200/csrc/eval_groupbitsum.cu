@@ -502,7 +502,7 @@ using namespace dl;
 // dl_groupbitsum one after the other).
 extern "C" DL_API int dl_eval_groupbitsum_applicable(const void *x, int64_t n_in, int64_t n_out, int64_t words, int bit_count,
                                                      int64_t k) {
-    if (!(bit_count == 8 || bit_count == 16 || bit_count == 32 || bit_count == 64)) return 0;
+    if (!(bit_count == 8 || bit_count == 16 || bit_count == 32 || bit_count == 64 || bit_count == 128)) return 0;
     if (n_in <= 0 || n_out <= 0 || k <= 0 || words <= 0 || n_out % k != 0) return 0;
     const int64_t row_bytes = words * (bit_count / 8), m = n_out / k;
     if (row_bytes % 16 != 0 || row_bytes < 512 || !aligned_to(x, 16)) return 0;

@@ -340,8 +340,9 @@ static int launch_groupbitsum(const void *x, int32_t *out, int64_t n, int64_t ro
 
 using namespace dl;
 
+// 128: rows counted in units of 16 bytes, whatever the width of the caller's words (rows padded to whole units)
 static int check_bits(const char *who, int bit_count) {
-    if (bit_count == 8 || bit_count == 16 || bit_count == 32 || bit_count == 64) return DL_OK;
+    if (bit_count == 8 || bit_count == 16 || bit_count == 32 || bit_count == 64 || bit_count == 128) return DL_OK;
     return fail(DL_ERR_BAD_BIT_COUNT, "%s: `bit_count` has to be in { 8, 16, 32, 64 }, got %d", who, bit_count);
 }
 

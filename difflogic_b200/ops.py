@@ -396,21 +396,25 @@ def packbits(t, bit_count):
     return out, (bit_count - batch % bit_count) % bit_count
 
 
-def packbits_batch_major(t, bit_count):
-    """bool [batch, n] (as the user holds it) -> (words [n, ceil(batch/bit_count)], pad_len)."""
+ROW_UNIT_BITS = 128   # rows padded to units of 16 bytes: what the packed kernels move at a time
+
+
+def packbits_batch_major(t, bit_count, padded=False):
+    """bool [batch, n] (as the user holds it) -> (words [n, ceil(batch/bit_count)], pad_len).  padded: the rows are filled
+    up with zero words to whole units of 16 bytes."""
     _check_bit_count(bit_count)
     t = _as_bool_bytes(t)
     batch, n = t.shape
-    words = -(-batch // bit_count)
-    out = torch.empty((n, words), dtype=_BITS_TO_DTYPE[bit_count], device=t.device)
+    unit = ROW_UNIT_BITS if padded else bit_count
+    out = torch.empty((n, -(-batch // unit) * (unit // bit_count)), dtype=_BITS_TO_DTYPE[bit_count], device=t.device)
     with torch.cuda.device(t.device):
-        N.check(N.lib().dl_packbits_batch_major(t.data_ptr(), out.data_ptr(), n, batch, bit_count, N.stream_of(t)))
+        N.check(N.lib().dl_packbits_batch_major(t.data_ptr(), out.data_ptr(), n, batch, unit, N.stream_of(t)))
     return out, (bit_count - batch % bit_count) % bit_count
 
 
-def threshold_packbits_batch_major(t, thresholds, bit_count):
+def threshold_packbits_batch_major(t, thresholds, bit_count, padded=False):
     """uint8 [batch, n] -> (words [len(thresholds)*n, ceil(batch/bit_count)], pad_len); bit s of row i*n+f is
-    t[s, f] > thresholds[i] (thermometer encoding and packing in one kernel)."""
+    t[s, f] > thresholds[i] (thermometer encoding and packing in one kernel).  padded: as in packbits_batch_major."""
     import ctypes
     _check_bit_count(bit_count)
     N.require_cuda(t)
@@ -418,21 +422,31 @@ def threshold_packbits_batch_major(t, thresholds, bit_count):
     thresholds = [int(v) for v in thresholds]
     _need(1 <= len(thresholds) <= 16 and all(0 <= v <= 255 for v in thresholds), "1..16 thresholds in 0..255")
     batch, n = t.shape
-    words = -(-batch // bit_count)
-    out = torch.empty((len(thresholds) * n, words), dtype=_BITS_TO_DTYPE[bit_count], device=t.device)
+    unit = ROW_UNIT_BITS if padded else bit_count
+    out = torch.empty((len(thresholds) * n, -(-batch // unit) * (unit // bit_count)), dtype=_BITS_TO_DTYPE[bit_count], device=t.device)
     arr = (ctypes.c_ubyte * len(thresholds))(*thresholds)
     with torch.cuda.device(t.device):
         N.check(N.lib().dl_threshold_packbits_batch_major(t.data_ptr(), ctypes.addressof(arr), len(thresholds), out.data_ptr(),
-                                                          n, batch, bit_count, N.stream_of(t)))
+                                                          n, batch, unit, N.stream_of(t)))
     return out, (bit_count - batch % bit_count) % bit_count
+
+
+def _row_units(x, pad_len):
+    """(units, bits per unit) of the rows of x for a count that leaves out their last pad_len samples: its words, or, when
+    whole words are left out (rows padded to 16 bytes), units of 16 bytes."""
+    bits = bits_of(x)
+    words = x.shape[1]
+    if pad_len >= bits and words * bits % ROW_UNIT_BITS == 0:
+        return words * bits // ROW_UNIT_BITS, ROW_UNIT_BITS
+    return words, bits
 
 
 def groupbitsum(x, pad_len, k):
     """words [n, W] -> int32 [W*bits - pad_len, k] class counts."""
     N.require_cuda(x)
     _need(x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D tensor")
-    bits = bits_of(x)
-    n, words = x.shape
+    words, bits = _row_units(x, int(pad_len))
+    n = x.shape[0]
     k = int(k)
     if k <= 0 or n % k != 0:
         raise ValueError("in_dim (%d) has to be divisible by k (%d) but it is not" % (n, k))
@@ -458,8 +472,8 @@ def eval_groupbitsum(x, a, b, gate, pad_len, k):
     _need(x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D tensor")
     _need(a.dtype == torch.int64 and b.dtype == torch.int64 and gate.dtype == torch.uint8, "a, b int64 and gate uint8")
     _need(a.numel() == b.numel() == gate.numel(), "a, b and gate must have one entry per gate")
-    bits = bits_of(x)
-    n_in, words = x.shape
+    words, bits = _row_units(x, int(pad_len))
+    n_in = x.shape[0]
     n_out, k = a.numel(), int(k)
     if k <= 0 or n_out % k != 0:
         raise ValueError("in_dim (%d) has to be divisible by k (%d) but it is not" % (n_out, k))

@@ -4,6 +4,9 @@ Drop-in for the reference class (difflogic/packbitstensor.py:6-41): `.t` is the 
 `[features, ceil(batch / bit_count)]` of dtype int{bit_count}, `.pad_len` the number of unused
 high bits in the last word, sample s being bit s % bit_count (LSB first) of word s // bit_count.
 
+Rows are kept padded to whole units of 16 bytes while layers are applied, so that a batch of any size is moved 16 bytes
+at a time by the kernels for long rows; `.t` shows the words of the batch only.
+
 Evaluation is lazy.  A LogicLayer in eval mode does not compute at once; it appends itself to the
 tensor's list of pending layers.  Reading `.t` runs the pending layers one kernel per layer, exactly
 as the reference does.  `group_sum(k)` -- what GroupSum calls -- runs all pending layers but the last
@@ -37,7 +40,8 @@ class PackBitsTensor:
             if t.dtype != torch.bool:
                 t = t != 0
             # transpose and pack in one kernel, straight from the batch-major matrix
-            self._t, self.pad_len = ops.packbits_batch_major(t.contiguous(), self.bit_count)
+            self._t, self.pad_len = ops.packbits_batch_major(t.contiguous(), self.bit_count, padded=True)
+            self._words = -(-t.shape[0] // self.bit_count)
         else:
             raise NotImplementedError(device)
 
@@ -48,6 +52,7 @@ class PackBitsTensor:
         self.bit_count = ops.bits_of(words)
         self.device = device
         self._t = words
+        self._words = words.shape[1]
         self._pending = []
         self.pad_len = int(pad_len)
         return self
@@ -58,8 +63,10 @@ class PackBitsTensor:
         Feature `i * n + f` of the result is `t[:, f] > thresholds[i]` with f running over the flattened trailing
         dimensions -- the layout of `torch.cat([x > (i+1)/4 ...], dim=1)` followed by Flatten on `x = t / 255`."""
         t = t.to(device).reshape(t.shape[0], -1).contiguous()
-        words, pad_len = ops.threshold_packbits_batch_major(t, thresholds, bit_count)
-        return cls.from_packed(words, pad_len, device=device)
+        words, pad_len = ops.threshold_packbits_batch_major(t, thresholds, bit_count, padded=True)
+        self = cls.from_packed(words, pad_len, device=device)
+        self._words = -(-t.shape[0] // bit_count)
+        return self
 
     # -- lazy layer application ------------------------------------------------------------------
 
@@ -67,12 +74,15 @@ class PackBitsTensor:
     def t(self):
         """The packed tensor after every layer applied so far (pending layers run now, one kernel each)."""
         self._materialize()
+        if self._t.shape[1] != self._words:
+            self._t = self._t[:, :self._words].contiguous()
         return self._t
 
     @t.setter
     def t(self, value):
         self._pending = []
         self._t = value
+        self._words = value.shape[1]
 
     def _push_layer(self, layer):
         """Called by LogicLayer.forward_cuda_eval: remember the layer (its connections and current arg-max gates)."""
@@ -88,6 +98,7 @@ class PackBitsTensor:
 
     def group_sum(self, k):
         assert torch.device(self.device).type == 'cuda', self.device
+        pad_len = self.pad_len + (self._t.shape[1] - self._words) * self.bit_count
         if self._pending and FUSED_LAST_LAYER:
             # all layers but the last run now; the last one is counted as it is computed, its output never stored
             (layer, gate) = self._pending.pop()
@@ -95,8 +106,9 @@ class PackBitsTensor:
             self._pending.append((layer, gate))  # still pending: `.t` would run it as a kernel of its own
             if ops.eval_groupbitsum_applicable(self._t, layer.out_dim, k):
                 a, b = layer.indices
-                return ops.eval_groupbitsum(self._t, a, b, gate, self.pad_len, k)
-        return ops.groupbitsum(self.t, self.pad_len, k)
+                return ops.eval_groupbitsum(self._t, a, b, gate, pad_len, k)
+        self._materialize()
+        return ops.groupbitsum(self._t, pad_len, k)
 
     def flatten(self, start_dim=0, end_dim=-1, **kwargs):
         """Returns the object itself so that torch.nn.Flatten passes it through; arguments are ignored."""

@@ -10,7 +10,9 @@
  * Layouts.  Float activations are feature-major: x[n_in][batch], y[n_out][batch], batch is
  * the fastest dimension.  Packed activations are feature-major rows of words along the batch:
  * t[n][words], word = bit_count bits (8, 16, 32 or 64), sample s is bit (s % bit_count) of
- * word (s / bit_count), least-significant bit first.  Connection indices a[], b[] are int64,
+ * word (s / bit_count), least-significant bit first.  The packers, dl_eval_packed, dl_groupbitsum and
+ * dl_eval_groupbitsum also take bit_count = 128: rows counted in units of 16 bytes, for callers that pad
+ * their rows to whole units (the bit order is the same for every word width).  Connection indices a[], b[] are int64,
  * as the Python API stores them.
  *
  * Each declaration names the interface of the reference implementation
