@@ -43,6 +43,10 @@ SIGNATURES = {
                                     _f32, _f32, _f32, _f32, _f32, _ptr, _int, _ptr]),
     "dl_eval_packed": (_int, [_ptr, _ptr, _ptr, _ptr, _ptr, _i64, _i64, _i64, _int, _ptr]),
     "dl_eval_packed_pitched": (_int, [_ptr, _i64, _ptr, _ptr, _ptr, _ptr, _i64, _i64, _i64, _i64, _ptr]),
+    "dl_eval_network_applicable": (_int, [_ptr, _ptr, _int, _i64, _i64, _i64]),
+    "dl_network_program_words": (_i64, [_ptr, _int]),
+    "dl_network_program": (_int, [_ptr, _ptr, _ptr, _ptr, _int, _ptr, _ptr]),
+    "dl_eval_network": (_int, [_ptr, _ptr, _ptr, _int, _ptr, _ptr, _i64, _i64, _i64, _ptr]),
     "dl_argmax_gate_u8": (_int, [_ptr, _ptr, _i64, _ptr]),
     "dl_packbits": (_int, [_ptr, _ptr, _i64, _i64, _int, _ptr]),
     "dl_packbits_batch_major": (_int, [_ptr, _ptr, _i64, _i64, _int, _ptr]),

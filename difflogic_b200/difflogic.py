@@ -210,10 +210,19 @@ class LogicLayer(torch.nn.Module):
         x._push_layer(self)  # evaluated when x.t is read, or fused with the other layers by GroupSum
         return x
 
+    # Program of the packed network that ends with this layer (PackBitsTensor._network).  It follows from the layers' tensors,
+    # so it is left out of copies and files.
+    _network = None
+
+    def __getstate__(self):
+        state = self.__dict__.copy()
+        state.pop('_network', None)
+        return state
+
     def train(self, mode=True):
         # Kernels (an optimizer's, a replayed graph's) write the weights without autograd's version counter noticing; what was
         # derived from the weights in eval mode does not outlive a change of mode.
-        self._gate_cache = None
+        self._gate_cache = self._network = None
         return super().train(mode)
 
     def _gate_ids(self):

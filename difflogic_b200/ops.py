@@ -486,6 +486,69 @@ def eval_groupbitsum(x, a, b, gate, pad_len, k):
     return out
 
 
+class NetworkProgram:
+    """What dl_eval_network needs of a network: its row counts and its program (dl_network_program), built from the layers'
+    connections and arg-max gates.  `layers`: (a, b, gate) of every layer, in order; they are kept, so that `matches` can
+    tell a network by its tensors."""
+
+    def __init__(self, n_in, layers):
+        import ctypes
+        self.layers = [(a, b, gate, a._version, b._version) for a, b, gate in layers]
+        count = len(layers)
+        self.sizes = network_sizes(n_in, layers)
+        device = layers[0][2].device
+        for a, b, gate in layers:
+            _index(a, "a", gate.numel())
+            _index(b, "b", gate.numel())
+        self.program = torch.empty(N.lib().dl_network_program_words(self.sizes, count), dtype=torch.int32, device=device)
+        pointers = [(ctypes.c_void_p * count)(*[t.data_ptr() for t in column]) for column in zip(*layers)]
+        with torch.cuda.device(device):
+            stream = torch.cuda.current_stream(device)
+            N.check(N.lib().dl_network_program(pointers[0], pointers[1], pointers[2], self.sizes, count, self.program.data_ptr(),
+                                               stream.cuda_stream))
+            # other threads and streams may take it from here on
+            stream.synchronize()
+        self.stream = stream.cuda_stream
+
+    def matches(self, layers):
+        return len(layers) == len(self.layers) and all(
+            a is p[0] and b is p[1] and gate is p[2] and a._version == p[3] and b._version == p[4]
+            for (a, b, gate), p in zip(layers, self.layers))
+
+
+def network_sizes(n_in, layers):
+    import ctypes
+    return (ctypes.c_int64 * (len(layers) + 1))(n_in, *[gate.numel() for _, _, gate in layers])
+
+
+def eval_network_applicable(x, sizes, batch, k):
+    """True when the one-kernel network evaluation takes layers of these sizes on packed words x."""
+    if not (x.is_cuda and x.dim() == 2 and x.is_contiguous() and x.dtype in _DTYPE_TO_BITS and x.shape[0] == sizes[0]):
+        return False
+    return N.lib().dl_eval_network_applicable(x.data_ptr(), sizes, len(sizes) - 1, x.shape[1] * (bits_of(x) // 8), int(batch), int(k)) != 0
+
+
+def eval_network(x, network, batch, k=None):
+    """All layers of a NetworkProgram on packed words x in one kernel: int32 [batch, k] class counts, or without k the last
+    layer's rows as packed words."""
+    _need(x.is_cuda and x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D CUDA tensor")
+    sizes, words = network.sizes, x.shape[1]
+    _need(x.shape[0] == sizes[0] and x.device == network.program.device, "x does not fit the network")
+    row_bytes = words * (bits_of(x) // 8)
+    if k is None:
+        out = torch.empty((sizes[len(sizes) - 1], words), dtype=x.dtype, device=x.device)
+    else:
+        out = torch.empty((int(batch), int(k)), dtype=torch.int32, device=x.device)
+    with torch.cuda.device(x.device):
+        stream = torch.cuda.current_stream(x.device)
+        if stream.cuda_stream != network.stream:
+            network.program.record_stream(stream)
+        N.check(N.lib().dl_eval_network(x.data_ptr(), network.program.data_ptr(), sizes, len(sizes) - 1,
+                                        0 if k is None else out.data_ptr(), out.data_ptr() if k is None else 0, row_bytes, int(batch),
+                                        1 if k is None else int(k), stream.cuda_stream))
+    return out
+
+
 # ------------------------------------------------------------------------------------------------
 # float GroupSum
 # ------------------------------------------------------------------------------------------------

@@ -8,9 +8,10 @@ Rows are kept padded to whole units of 16 bytes while layers are applied, so tha
 at a time by the kernels for long rows; `.t` shows the words of the batch only.
 
 Evaluation is lazy.  A LogicLayer in eval mode does not compute at once; it appends itself to the
-tensor's list of pending layers.  Reading `.t` runs the pending layers one kernel per layer, exactly
-as the reference does.  `group_sum(k)` -- what GroupSum calls -- runs all pending layers but the last
-one kernel each and hands the last layer together with the bit-sum to ONE kernel that never stores the
+tensor's list of pending layers.  Layers of up to 16384 rows run in ONE kernel that keeps the activations
+in shared memory (ops.eval_network): `group_sum(k)` -- what GroupSum calls -- gets the class counts from it,
+reading `.t` the last layer's rows.  Wider ones run one kernel per layer, exactly as the reference does, and
+`group_sum(k)` hands the last layer together with the bit-sum to one kernel that never stores the
 layer's output (ops.eval_groupbitsum) when the sizes are in that kernel's range.  The counts are
 identical either way; the in-place semantics of the reference (the layer returns the same object, `.t`
 then holds the layer's output) are kept.
@@ -90,7 +91,30 @@ class PackBitsTensor:
         assert rows == layer.in_dim, ((rows,), layer.in_dim)
         self._pending.append((layer, layer._gate_ids()))
 
+    def _network(self, batch, k):
+        """The pending layers as a program for the one-kernel evaluation, or None when that kernel does not take them.  The
+        program stays with the last layer until a layer's gates or connections are others.  Not while a CUDA graph is being
+        captured: the graph would outlive a program that a change of the weights replaces."""
+        layers = [layer.indices + (gate,) for layer, gate in self._pending]
+        sizes = ops.network_sizes(self._t.shape[0], layers)
+        if not ops.eval_network_applicable(self._t, sizes, batch, k) or torch.cuda.is_current_stream_capturing():
+            return None
+        last = self._pending[-1][0]
+        network = last._network
+        if network is None or not network.matches(layers):
+            if any(t.device != self._t.device for layer in layers for t in layer):
+                return None
+            last._network = None      # given back before the next one is made
+            network = last._network = ops.NetworkProgram(self._t.shape[0], layers)
+        return network
+
     def _materialize(self):
+        if len(self._pending) > 1:
+            batch = self._t.shape[1] * self.bit_count
+            network = self._network(batch, 1)
+            if network is not None:
+                self._t, self._pending = ops.eval_network(self._t, network, batch), []
+                return
         pending, self._pending = self._pending, []
         for layer, gate in pending:
             a, b = layer.indices
@@ -100,6 +124,10 @@ class PackBitsTensor:
         assert torch.device(self.device).type == 'cuda', self.device
         pad_len = self.pad_len + (self._t.shape[1] - self._words) * self.bit_count
         if self._pending and FUSED_LAST_LAYER:
+            batch = self._t.shape[1] * self.bit_count - pad_len
+            network = self._network(batch, k)
+            if network is not None:
+                return ops.eval_network(self._t, network, batch, k)   # all layers are still pending
             # all layers but the last run now; the last one is counted as it is computed, its output never stored
             (layer, gate) = self._pending.pop()
             self._materialize()

@@ -208,6 +208,24 @@ DL_API int dl_eval_packed(const void *x, const int64_t *a, const int64_t *b, con
 DL_API int dl_eval_packed_pitched(const void *x, int64_t x_pitch, const int64_t *a, const int64_t *b, const uint8_t *gate,
                                   void *y, int64_t y_pitch, int64_t n_in, int64_t n_out, int64_t row_bytes, void *stream);
 
+/* A whole packed network in one kernel: activations stay in shared memory (resident.cu).  n: HOST array of layers + 1 row
+ * counts (input, then every layer); 1 .. 32 layers of 1 .. 16384 rows.
+ *   dl_eval_network_applicable  bytes of a row that a block takes (16, 8 or 4), or 0 when the kernel does not take the sizes:
+ *                               rows of whole 16 bytes, 16-byte aligned, n[layers] divisible by k, and the widest layer plus
+ *                               the counts of a block within shared memory.
+ *   dl_network_program          order of evaluation and gate masks from every layer's connections and gate ids (HOST arrays of
+ *                               device pointers) into dl_network_program_words() 32-bit words.  Connections outside the
+ *                               layer's input read row 0.
+ *   dl_eval_network             x [n[0]][row_bytes] -> out [batch][k] class counts, or the last layer's rows
+ *                               rows_out [n[layers]][row_bytes]; one of the two is null.
+ * The counts and rows are those of dl_eval_packed per layer followed by dl_groupbitsum. */
+DL_API int dl_eval_network_applicable(const void *x, const int64_t *n, int layers, int64_t row_bytes, int64_t batch, int64_t k);
+DL_API int64_t dl_network_program_words(const int64_t *n, int layers);
+DL_API int dl_network_program(const int64_t *const *a, const int64_t *const *b, const uint8_t *const *gate, const int64_t *n,
+                              int layers, uint32_t *program, void *stream);
+DL_API int dl_eval_network(const void *x, const uint32_t *program, const int64_t *n, int layers, int32_t *out, void *rows_out,
+                           int64_t row_bytes, int64_t batch, int64_t k, void *stream);
+
 /* argmax over the 16 gate weights -> uint8 gate id, first maximum on ties
  * (weights.argmax(-1).to(uint8), difflogic/difflogic.py:146). */
 DL_API int dl_argmax_gate_u8(const float *w, uint8_t *gate, int64_t n_out, void *stream);

@@ -1,0 +1,117 @@
+"""The one-kernel evaluation of a packed network against the oracle and the layer-by-layer kernels: counts and rows."""
+import copy
+
+import numpy as np
+import pytest
+import torch
+
+import difflogic_b200 as D
+from difflogic_b200 import _native as N
+from difflogic_b200 import ops
+from oracle import logic_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+# (rows of the input and of every layer, k, batch, bytes of a row per block): every block width, one and several CTAs per SM,
+# one layer and the most there may be, layers of different widths, an odd number of rows, rows at the limit of a block width,
+# classes shorter and longer than a warp's run of rows, the last block full, almost full and almost empty
+CASES = [([5, 3], 1, 1, 4), ([40, 60, 60], 2, 100, 4), ([784] + 4 * [8000], 10, 100, 4), ([300, 1001, 1001], 7, 128, 4),
+         ([64, 16384, 16384], 2, 33, 4), ([50, 640, 320, 640], 64, 7000, 8), ([100, 10241, 10241], 11, 8 * 64 * 148, 8),
+         ([16384, 16384], 1, 40000, 8), ([30, 10240, 10240], 10, 128 * 148 - 127, 16), ([33, 2000, 2000, 999], 999, 20, 4),
+         ([70] + 32 * [100], 100, 30001, 16), ([117, 5000, 5120], 16, 50000, 16), ([400, 2560, 2561], 13, 40001, 16),
+         ([20, 12, 300], 300, 25000, 8)]
+
+
+def _network(dims, seed):
+    g = torch.Generator().manual_seed(seed)
+    layers = []
+    for n_in, n_out in zip(dims[:-1], dims[1:]):
+        a, b = torch.randint(0, n_in, (2, n_out), generator=g)
+        b[:: 17] = a[:: 17]                                     # neurons that read one row twice
+        layers.append((a, b, (torch.arange(n_out) % 16)[torch.randperm(n_out, generator=g)].to(torch.uint8)))
+    return layers
+
+
+@pytest.mark.parametrize("dims,k,batch,width", CASES)
+def test_counts_and_rows(dims, k, batch, width):
+    layers = _network(dims, batch)
+    words = -(-batch // 128) * 2
+    g = torch.Generator().manual_seed(1)
+    x = torch.randint(-2 ** 63, 2 ** 63 - 1, (dims[0], words), generator=g)
+    device_layers = [tuple(t.cuda() for t in layer) for layer in layers]
+    xd, sizes = x.cuda(), ops.network_sizes(dims[0], layers)
+    assert N.lib().dl_eval_network_applicable(xd.data_ptr(), sizes, len(layers), words * 8, batch, k) == width
+    network = ops.NetworkProgram(dims[0], device_layers)
+    rows, hidden = xd, x.numpy()
+    for (a, b, gate), (ha, hb, hg) in zip(device_layers, layers):
+        rows = ops.eval_packed(rows, a, b, gate)
+        hidden = O.eval_packed(hidden, ha.numpy(), hb.numpy(), hg.numpy())
+    assert torch.equal(ops.eval_network(xd, network, words * 64), rows) and np.array_equal(rows.cpu().numpy(), hidden)
+    counts = ops.eval_network(xd, network, batch, k)
+    assert counts.shape == (batch, k) and counts.dtype == torch.int32
+    want = ((hidden.view(np.uint64)[:, None, :] >> np.arange(64, dtype=np.uint64)[None, :, None]) & 1) if dims[-1] * words < 60000 else None
+    if want is not None:
+        want = want.transpose(0, 2, 1).reshape(k, dims[-1] // k, -1).sum(1).T[:batch]
+        assert np.array_equal(counts.cpu().numpy(), want)
+    assert torch.equal(counts, ops.groupbitsum(rows, words * 64 - batch, k) if words * 64 - batch < 64 else
+                       ops.groupbitsum(rows, 0, k)[:batch])
+
+
+def test_sizes_outside_the_range():
+    x = torch.zeros(64, 4, dtype=torch.int64, device="cuda")
+
+    def takes(dims, batch=256, k=1, x=x, row_bytes=32):
+        return N.lib().dl_eval_network_applicable(x.data_ptr(), ops.network_sizes(dims[0], [(0, 0, torch.empty(n)) for n in dims[1:]]),
+                                                  len(dims) - 1, row_bytes, batch, k)
+    assert takes([64, 100])
+    assert not takes([64, 16385]) and not takes([16385, 100]) and not takes([64] + 33 * [100]) and not takes([64])
+    assert not takes([64, 100], k=3) and not takes([64, 100], k=0) and not takes([64, 100], batch=0) and not takes([64, 100], batch=257)
+    assert not takes([64, 100], row_bytes=24) and not takes([64, 16384], k=16384)
+
+
+def test_programs_follow_the_network():
+    """A remembered program is not used for other gates, connections or layers, nor copied along with a layer."""
+    torch.manual_seed(3)
+    first, other, last = D.LogicLayer(50, 300), D.LogicLayer(50, 300), D.LogicLayer(300, 200)
+    x = torch.rand(1000, 50, device="cuda") < 0.5
+
+    def check(*layers):
+        model = torch.nn.Sequential(*layers, D.GroupSum(10)).eval()
+        h = x.cpu().numpy()
+        with torch.no_grad():
+            counts = model(D.PackBitsTensor(x))
+            packed = D.PackBitsTensor(x)
+            for layer in layers:
+                packed = layer(packed)
+            assert torch.equal(ops.groupbitsum(packed.t, packed.pad_len, 10), counts)
+        want = O.packed_net_counts(h, [l.indices[0].cpu() for l in layers], [l.indices[1].cpu() for l in layers],
+                                   [l.weights.detach().argmax(1).cpu().numpy().astype(np.uint8) for l in layers], 10, 32)
+        assert np.array_equal(counts.cpu().numpy(), want)
+
+    check(first, last)
+    check(other, last)
+    check(first, last)
+    with torch.no_grad():
+        first.weights.copy_(first.weights[torch.randperm(300, device="cuda")])
+    check(first, last)
+    first.set_connections(*[i[torch.randperm(300, device="cuda")] for i in first.indices])
+    check(first, last)
+    last.indices[0].copy_(last.indices[0].flip(0))
+    check(first, last)
+    twin = copy.deepcopy(last)
+    assert twin._network is None and last._network is not None
+    check(first, twin)
+    check(first)
+
+
+def test_a_graph_keeps_its_own_gates():
+    torch.manual_seed(4)
+    model = torch.nn.Sequential(D.LogicLayer(64, 320), D.LogicLayer(320, 320), D.GroupSum(10)).eval()
+    x = torch.rand(640, 64, device="cuda") < 0.5
+    with torch.no_grad():
+        want = model(D.PackBitsTensor(x))
+        graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=stream):
+            counts = model(D.PackBitsTensor(x))
+        graph.replay()
+    assert torch.equal(counts, want)
