@@ -109,8 +109,7 @@ class LogicLayer(torch.nn.Module):
 
         `given_x_indices_of_y_start` / `given_x_indices_of_y` have the reference's meaning
         (difflogic.py:56-69); `_plan` is the same index with the partner row and the input slot
-        resolved, which is what the gather kernel follows; `_walk` is the order in which the walk kernels
-        take the neurons (ops.build_walk)."""
+        resolved, which is what the gather kernel follows."""
         a, b = self.indices
         self.indices = (a.contiguous(), b.contiguous())
         a, b = self.indices
@@ -121,12 +120,29 @@ class LogicLayer(torch.nn.Module):
             self._plan = ops.build_backward_plan(a, b, self.given_x_indices_of_y_start, self.given_x_indices_of_y)
             if _DEBUG_CHECKS:
                 ops.check_connections(a, b, self.in_dim, self.given_x_indices_of_y_start, self.given_x_indices_of_y, self._plan)
-            self._walk = ops.build_walk(a, b, self.in_dim)
             # the layer's kernels may read these index tensors ahead of the kernel that precedes them in the
             # stream (DL_LAUNCH_OVERLAP_SETUP), so they must be final before any such launch is queued
             torch.cuda.current_stream(a.device).synchronize()
         else:
-            self._plan = self._walk = None
+            self._plan = None
+        self._walk = None
+
+    def _walk_for(self, batch):
+        """The order in which the walk kernels take the neurons (ops.build_walk), or None where the gather kernels are to be
+        used.  Built on the host by the first call that wants it (not while a graph is being captured: it synchronises).
+
+        A CTA of the walk kernels takes 64 neurons through the whole batch: narrow layers leave SMs idle, and with few columns
+        the walk's longer chain from load to store shows.  Captured step, four layers, walk against gather kernels: 8000 wide,
+        batch 256: 68 / 64 us, 2048: 338 / 340; 4000 wide, batch 2048: 279 / 175; 16000 wide, batch 64: 67 / 56, 128: 65 / 67, 512:
+        133 / 192; 64000 wide, batch 32: 108 / 128, 64 (two columns of 16 lanes): 133 / 130, 512: 491 / 781."""
+        if self.out_dim < 12000 or self.out_dim * batch < 2000000 or 32 < batch <= 64:
+            return None
+        walk = getattr(self, '_walk', None)
+        if walk is None and not torch.cuda.is_current_stream_capturing():
+            walk = ops.build_walk(self.indices[0], self.indices[1], self.in_dim) or (None, False)
+            torch.cuda.current_stream(self.indices[0].device).synchronize()    # read ahead of the preceding kernel, as the indices
+            self._walk = walk
+        return walk if walk is not None and walk[0] is not None else None
 
     def set_connections(self, a, b):
         """Replaces the connection indices (e.g. to copy them from another model) and rebuilds the inverse index."""
@@ -195,10 +211,10 @@ class LogicLayer(torch.nn.Module):
         a, b = self.indices
         if self.training:
             y = LogicLayerFunction.apply(x, self.weights, a, b, self.given_x_indices_of_y_start, self._plan,
-                                         float(self.grad_factor), getattr(self.weights, '_dl_grad_out', None), self._walk)
+                                         float(self.grad_factor), getattr(self.weights, '_dl_grad_out', None), self._walk_for(x.shape[1]))
         else:
             with torch.no_grad():
-                y, _ = _forward(x, a, b, self.weights, self._walk, ops.W_ARGMAX)
+                y, _ = _forward(x, a, b, self.weights, self._walk_for(x.shape[1]), ops.W_ARGMAX)
         return y.transpose(0, 1)
 
     def forward_cuda_eval(self, x: PackBitsTensor):
@@ -211,12 +227,13 @@ class LogicLayer(torch.nn.Module):
         return x
 
     # Program of the packed network that ends with this layer (PackBitsTensor._network).  It follows from the layers' tensors,
-    # so it is left out of copies and files.
+    # as the walk follows from the connections; both are left out of copies and files.
     _network = None
 
     def __getstate__(self):
         state = self.__dict__.copy()
         state.pop('_network', None)
+        state['_walk'] = None
         return state
 
     def train(self, mode=True):
@@ -402,7 +419,7 @@ def logic_layer_head(layer, x, target, k, tau):
     a, b = layer.indices
     return LogicLayerHeadFunction.apply(xt, layer.weights, a, b, layer.given_x_indices_of_y_start, layer._plan,
                                         float(layer.grad_factor), getattr(layer.weights, '_dl_grad_out', None),
-                                        target.contiguous(), int(k), float(tau), layer._walk)
+                                        target.contiguous(), int(k), float(tau), layer._walk_for(x.shape[0]))
 
 
 class LogicLayerCudaFunction(torch.autograd.Function):
