@@ -543,16 +543,15 @@ check_connections_kernel(const int64_t *__restrict__ a, const int64_t *__restric
 // ---------------------------------------------------------------------------------------------
 static inline unsigned slab_grid(int64_t nslabs) { return (unsigned)(nslabs < 65535 ? nslabs : 65535); }
 
+constexpr int kFillCtas = 148;  // one CTA per SM
 constexpr int kForwardU = 4;  // passes of a CTA of the forward kernel over its row groups
 static inline int64_t forward_rows_per_cta(int G) { return (kThreads / G) * kForwardU; }
 
-template <bool VEC4, bool CLASSSUM = false>
-static int launch_forward(bool overlap, int G, const float *x, const int64_t *a, const int64_t *b, const float *w, int w_mode, float *y,
-                          float *coef, int64_t n_out, int64_t batch, int64_t ncols, cudaStream_t st, int64_t class_rows = 0) {
-    constexpr int U = kForwardU;
+template <int U, bool VEC4, bool CLASSSUM>
+static int launch_forward_passes(bool overlap, int G, const float *x, const int64_t *a, const int64_t *b, const float *w, int w_mode, float *y,
+                          float *coef, int64_t n_out, int64_t batch, int64_t ncols, cudaStream_t st, int64_t class_rows) {
     const int64_t nslabs = ceil_div(ncols, G);
-    const int64_t nb = forward_rows_per_cta(G);
-    const dim3 grid((unsigned)ceil_div(n_out, nb), slab_grid(nslabs));
+    const dim3 grid((unsigned)ceil_div(n_out, (kThreads / G) * U), slab_grid(nslabs));
     float4 *c4 = reinterpret_cast<float4 *>(coef);
 #define DL_FWD(GG)                                                                                              \
     case GG:                                                                                                    \
@@ -563,6 +562,26 @@ static int launch_forward(bool overlap, int G, const float *x, const int64_t *a,
     }
 #undef DL_FWD
     return launch_status("dl_forward_f32");
+}
+
+// A CTA takes kForwardU passes over its row groups, or one where that leaves SMs without a CTA.
+template <bool VEC4, bool CLASSSUM = false>
+static int launch_forward(bool overlap, int G, const float *x, const int64_t *a, const int64_t *b, const float *w, int w_mode, float *y,
+                          float *coef, int64_t n_out, int64_t batch, int64_t ncols, cudaStream_t st, int64_t class_rows = 0) {
+    if constexpr (!CLASSSUM) {
+        if (ceil_div(n_out, forward_rows_per_cta(G)) * ceil_div(ncols, G) < kFillCtas)
+            return launch_forward_passes<1, VEC4, false>(overlap, G, x, a, b, w, w_mode, y, coef, n_out, batch, ncols, st, class_rows);
+    }
+    return launch_forward_passes<kForwardU, VEC4, CLASSSUM>(overlap, G, x, a, b, w, w_mode, y, coef, n_out, batch, ncols, st, class_rows);
+}
+
+// Lanes per neuron in backward_w: a quarter of the row's vectors, so that a lane has four loads per row in flight; but four at
+// least, because the lanes also share the neuron's 16 weights (one lane alone touches 64 bytes of its own: 15 us for 1000 neurons
+// at batch 16), and up to 16 while the grid leaves SMs without a CTA.
+static int backward_w_lanes(int64_t ncols, int64_t n_out) {
+    int G = pow2_at_least(ceil_div(ncols, 4), 32);
+    while (G < 4 || (G < 16 && ceil_div(n_out * G, kThreads) < kFillCtas)) G *= 2;
+    return G;
 }
 
 template <bool VEC4>
@@ -699,7 +718,7 @@ static int backward_w_entry(const float *x, const int64_t *a, const int64_t *b, 
     DL_REQUIRE(w_mode != DL_W_LOGITS || w, DL_ERR_INVALID_ARG, "dl_backward_w_f32: DL_W_LOGITS needs the raw weights");
     const bool vec = batch % 4 == 0 && aligned_to(x, 16) && aligned_to(grad_y, 16);
     const int64_t ncols = vec ? batch / 4 : batch;
-    const int G = pow2_at_least(ceil_div(ncols, 4), 32);
+    const int G = backward_w_lanes(ncols, n_out);
     const bool overlap = (flags & DL_LAUNCH_OVERLAP_SETUP) != 0;
     return vec ? launch_backward_w<true>(overlap, G, x, a, b, grad_y, w, w_mode, grad_w, n_out, batch, ncols, (int)gy_group, adam, ann, push, as_stream(stream))
                : launch_backward_w<false>(overlap, G, x, a, b, grad_y, w, w_mode, grad_w, n_out, batch, ncols, (int)gy_group, adam, ann, push, as_stream(stream));
