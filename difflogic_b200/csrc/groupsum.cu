@@ -305,38 +305,56 @@ groupsum_ce_kernel(const float *__restrict__ x, const int64_t *__restrict__ targ
 // groups of 128 threads add the class's pieces in a fixed order (piece p goes to group p % 8, the groups are added in
 // order) and write the scores; the CTA that holds the ticket computes the loss and the class-row gradients as in
 // groupsum_ce_kernel.  Reads pieces * batch floats per class that the forward kernel has just written (L2).
+// S: CTAs (a cluster) per (columns, class), each adding every S-th round of pieces; their sums meet in the first one's shared
+// memory.  Eight of them where the classes are long and (columns, class) pairs too few to fill the GPU: for 4000 runs, 10 classes
+// and 256 columns one CTA per pair, 20 in all, waited for one load after the other: 31 us.
 constexpr int kCsThreads = 1024;
 constexpr int kCsGroups = kCsThreads / kGsCols;  // 8
 
+template <int S>
 __global__ void __launch_bounds__(kCsThreads)
 class_sums_ce_kernel(const float *__restrict__ sums, const int64_t *__restrict__ target, float *__restrict__ scores,
                      float *__restrict__ loss, float *__restrict__ grad_classes, unsigned int *__restrict__ counter, int64_t batch, int k,
                      int m, int nb, float tau) {
     __shared__ float s_part[kCsGroups][kGsCols];
+    __shared__ float s_all[S][kGsCols];
     __shared__ float s_red[kCsThreads / 32];
     __shared__ bool s_last;
+    const unsigned q = S > 1 ? cooperative_groups::this_cluster().block_rank() : 0u;
     const int tid = threadIdx.x, g = tid / kGsCols, col = tid % kGsCols;
     const int c = blockIdx.y;
     const int64_t gcol = (int64_t)blockIdx.x * kGsCols + col;
     const unsigned row0 = (unsigned)c * (unsigned)m;  // n < 2^31
     const unsigned first = row0 / (unsigned)nb, last = (row0 + (unsigned)m - 1u) / (unsigned)nb;  // runs that hold rows of class c
+    if (S > 1) cooperative_groups::this_cluster().sync();  // the first CTA runs before the others write to it
     grid_dependency_wait();  // sums is the output of the kernel just before
     float acc = 0.f;
     if (gcol < batch) {
 #pragma unroll 8
-        for (unsigned i = first + (unsigned)g; i <= last; i += kCsGroups) {
+        for (unsigned i = first + q * kCsGroups + (unsigned)g; i <= last; i += S * kCsGroups) {
             const unsigned e = i * (unsigned)nb >= row0 ? 0u : 1u;  // the run's first row is of class c, or of the class before it
             acc += __ldcg(sums + (int64_t)(2u * i + e) * batch + gcol);
         }
     }
     s_part[g][col] = acc;
     __syncthreads();
-    if (g == 0 && gcol < batch) {
-        float total = 0.f;
+    float total = 0.f;
+    if (g == 0) {
 #pragma unroll
         for (int gg = 0; gg < kCsGroups; ++gg) total += s_part[gg][col];
-        scores[gcol * k + c] = total / tau;
     }
+    if (S > 1) {
+        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+        if (g == 0) *cluster.map_shared_rank(&s_all[q][col], 0) = total;
+        cluster.sync();
+        if (q != 0) return;
+        if (g == 0) {
+            total = 0.f;
+#pragma unroll
+            for (int r = 0; r < S; ++r) total += s_all[r][col];
+        }
+    }
+    if (g == 0 && gcol < batch) scores[gcol * k + c] = total / tau;
     // ---- ticket: the CTA that gets here last computes the loss over all samples
     __threadfence();
     __syncthreads();
@@ -638,9 +656,23 @@ extern "C" DL_API int dl_class_sums_cross_entropy_f32(const float *class_sums, c
         cudaLaunchKernelEx(&cfg, kernel, class_sums, target, scores, loss, grad_classes, batch, (int)k, (int)(n / k), (int)rows_per_run, tau);
         return launch_status("dl_class_sums_cross_entropy_f32");
     }
-    launch_dependent(true, class_sums_ce_kernel, dim3((unsigned)colblocks, (unsigned)k), dim3(kCsThreads), 0, as_stream(stream), class_sums, target,
-                     scores, loss, grad_classes, reinterpret_cast<unsigned int *>(counter), batch, (int)k, (int)(n / k), (int)rows_per_run,
-                     tau);
+    constexpr int kSplit = 8;
+    const bool split = pieces >= 8 * kCsGroups && colblocks * k < 148;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)colblocks, (unsigned)k, split ? kSplit : 1);
+    cfg.blockDim = dim3(kCsThreads);
+    cfg.stream = as_stream(stream);
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = kSplit;
+    cfg.attrs = attr;
+    cfg.numAttrs = split ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, split ? class_sums_ce_kernel<kSplit> : class_sums_ce_kernel<1>, class_sums, target, scores, loss, grad_classes,
+                       reinterpret_cast<unsigned int *>(counter), batch, (int)k, (int)(n / k), (int)rows_per_run, tau);
     return launch_status("dl_class_sums_cross_entropy_f32");
 }
 
