@@ -1,27 +1,24 @@
 // Transpose-and-pack of a batch-major byte matrix t[batch][n] into feature-major bit rows, shared by the bool packer
 // (packed.cu) and the thermometer packer (threshold_pack.cu).
 //
-// A CTA of 256 threads takes 256 features x 512 samples.  Warp w owns the 64 samples of one output word, lane l eight
-// adjacent features: one 8-byte load per sample, so a warp reads 256 contiguous bytes of a sample's row.  No bit is
-// moved on its own:
-//   * a predicate turns the 8 bytes of a load into 8 bits (bit f = feature f selected): two multiplies and a shift;
-//   * 8 samples give an 8 x 8 bit matrix (byte = sample, bit = feature) that is transposed in registers by three delta
-//     swaps: byte f then holds the 8 samples' bits of feature f;
-//   * after 8 such groups an 8 x 8 BYTE transpose across the 8 registers (byte permutes) gives the 8 output words, one
-//     per feature.
-// The words of the 8 warps meet in shared memory so that a feature's 64 bytes (512 samples) leave as 16-byte stores
-// (words stored straight from the registers, 8 bytes at a time to 8 different rows per thread, measured slower: 382
-// against 337 us for 2^20 x 784 bools, and twice as slow with three outputs).
-// Needs n % 8 == 0 and an 8-byte aligned source; rows of the output need no alignment (ragged ends go byte by byte).
+// A thread owns eight adjacent features and reads eight samples of them at a time, eight bytes each.  No bit is moved on its
+// own: a predicate turns the 8 bytes of a load into 8 bits (two multiplies and a shift), and the 8 x 8 bit matrix of eight
+// samples is transposed in registers by three delta swaps: byte f then holds the 8 samples' bits of feature f.
+//
+// A CTA of 256 threads takes 8 * WF features x 8 * K * (256 / WF) samples: WF threads side by side over the features, each going
+// through 8 * K samples.  The bytes meet in shared memory, so that a feature's samples leave as one run of K * 256 / WF bytes.
+//   WF = 32, K = 1   256 features, 64 samples, one round of loads per thread: thousands of short CTAs
+//   WF =  8, K = 4   64 features, 1024 samples, runs of 128 bytes: for matrices too narrow for 256 features, whose lanes would
+//                    be idle, and for very long rows
+//
+// Rows of the source that do not start at 8-byte boundaries (n % 8 != 0) are read as three aligned 4-byte words and shifted
+// into place; the words that hold the matrix's first and last byte are the only ones that reach beyond it, by less than 4 bytes.
+// Rows of the output need no alignment (ragged ends go byte by byte).
 #pragma once
 
 #include "common.cuh"
 
 namespace dl {
-
-constexpr int kPackFeatures = 256;  // per CTA
-constexpr int kPackSamples = 512;   // per CTA and pass
-constexpr int kPackRow = 8 * 33 + 1;  // shared-memory row (one per warp): 8 blocks of 32 lanes, padded
 
 // 0x01 in every selected byte of lo / hi -> 8 bits (byte 0 of lo to bit 0): the two products put the bytes' low bits
 // next to each other in bits 24..31 and overlap nowhere, so the sum cannot carry
@@ -53,74 +50,122 @@ __device__ __forceinline__ void transpose_bytes_4x4(uint32_t a, uint32_t b, uint
     r[3] = __byte_perm(t2, t3, 0x7632);
 }
 
-// MASK: functor (lo, hi: the 8 bytes of one load; i: which of the NT outputs) -> 8 bits, bit f set when feature f is selected
-// for output i.  The source is read ONCE for all NT outputs (e.g. NT thermometer thresholds).  Output i goes to the rows
-// starting at dst + i * out_stride (row_bytes bytes per feature row); s_words: kPackRow * 8 words.  Samples beyond the
-// batch give zero bits.
-template <int NT, typename MASK>
-__device__ __forceinline__ void pack_tile(const uint8_t *__restrict__ t, uint8_t *__restrict__ dst, int64_t out_stride, int64_t n,
-                                          int64_t batch, int64_t row_bytes, int64_t f0, int64_t sblk, unsigned long long *s_words,
-                                          MASK mask) {
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int64_t f = f0 + lane * 8;
-    const int64_t s0 = sblk * kPackSamples + warp * 64;
-    const int live = f < n ? (int)max((int64_t)0, min((int64_t)64, batch - s0)) : 0;  // samples of this thread's item that exist
-    const uint8_t *src = t + s0 * n + f;
-    unsigned long long grp[NT][8];  // per output and group of 8 samples: byte f = the 8 samples' bits of feature f
+struct PackShape {
+    int64_t n, batch, row_bytes;
+};
+
+// The eight bytes of features f .. f + 7 of one sample; features beyond n give any value.
+template <bool ALIGNED>
+__device__ __forceinline__ uint2 load_features(const uint8_t *__restrict__ p, int features) {
+    if (ALIGNED) return __ldg(reinterpret_cast<const uint2 *>(p));
+    const uint32_t off = (uint32_t)reinterpret_cast<uintptr_t>(p) & 3u;
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(p - off);
+    const uint32_t need = off + (uint32_t)features;  // a word is read only when it holds a byte that is wanted
+    const uint32_t w0 = __ldg(w), w1 = need > 4 ? __ldg(w + 1) : 0u, w2 = need > 8 ? __ldg(w + 2) : 0u;
+    return make_uint2(__funnelshift_r(w0, w1, 8 * off), __funnelshift_r(w1, w2, 8 * off));
+}
+
+// Eight samples from src on, `live` of which exist: out[i] byte f = their bits of feature f for output i.  MASK: functor (lo, hi:
+// the 8 bytes of one load; i: which of the NT outputs) -> 8 bits, bit f set when feature f is selected for output i.
+template <int NT, bool ALIGNED, typename MASK>
+__device__ __forceinline__ void pack_eight(const uint8_t *__restrict__ src, int64_t n, int features, int live, MASK mask,
+                                           unsigned long long (&out)[NT]) {
+    uint2 v[8];
 #pragma unroll
-    for (int g = 0; g < 8; ++g) {
-        uint2 v[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            v[r] = make_uint2(0u, 0u);
-            if (g * 8 + r < live) v[r] = __ldg(reinterpret_cast<const uint2 *>(src + (int64_t)(g * 8 + r) * n));
-        }
-#pragma unroll
-        for (int i = 0; i < NT; ++i) {
-            uint32_t xlo = 0u, xhi = 0u;  // byte r = the mask of sample r
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                xlo |= (g * 8 + r < live ? mask(v[r].x, v[r].y, i) : 0u) << (8 * r);
-                xhi |= (g * 8 + 4 + r < live ? mask(v[4 + r].x, v[4 + r].y, i) : 0u) << (8 * r);
-            }
-            grp[i][g] = transpose_bits_8x8((unsigned long long)xlo | ((unsigned long long)xhi << 32));
-        }
+    for (int r = 0; r < 8; ++r) {
+        v[r] = make_uint2(0u, 0u);
+        if (r < live) v[r] = load_features<ALIGNED>(src + (int64_t)r * n, features);
     }
-    const int64_t byte0 = sblk * (kPackSamples / 8);
-    const bool wide = row_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(dst) % 16) == 0 && out_stride % 16 == 0;
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
-        // word of feature q: byte g = grp[g] byte q
-        uint32_t lo_a[4], lo_b[4], hi_a[4], hi_b[4];
-        transpose_bytes_4x4((uint32_t)grp[i][0], (uint32_t)grp[i][1], (uint32_t)grp[i][2], (uint32_t)grp[i][3], lo_a);  // features 0..3, groups 0..3
-        transpose_bytes_4x4((uint32_t)grp[i][4], (uint32_t)grp[i][5], (uint32_t)grp[i][6], (uint32_t)grp[i][7], lo_b);  // features 0..3, groups 4..7
-        transpose_bytes_4x4((uint32_t)(grp[i][0] >> 32), (uint32_t)(grp[i][1] >> 32), (uint32_t)(grp[i][2] >> 32),
-                            (uint32_t)(grp[i][3] >> 32), hi_a);                                                       // features 4..7
-        transpose_bytes_4x4((uint32_t)(grp[i][4] >> 32), (uint32_t)(grp[i][5] >> 32), (uint32_t)(grp[i][6] >> 32),
-                            (uint32_t)(grp[i][7] >> 32), hi_b);
+        uint32_t lo = 0u, hi = 0u;  // byte r = the mask of sample r
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            s_words[warp * kPackRow + q * 33 + lane] = (unsigned long long)lo_a[q] | ((unsigned long long)lo_b[q] << 32);
-            s_words[warp * kPackRow + (q + 4) * 33 + lane] = (unsigned long long)hi_a[q] | ((unsigned long long)hi_b[q] << 32);
+        for (int r = 0; r < 4; ++r) {
+            lo |= (r < live ? mask(v[r].x, v[r].y, i) : 0u) << (8 * r);
+            hi |= (4 + r < live ? mask(v[4 + r].x, v[4 + r].y, i) : 0u) << (8 * r);
+        }
+        out[i] = transpose_bits_8x8((unsigned long long)lo | ((unsigned long long)hi << 32));
+    }
+}
+
+// Shared memory of a tile: [feature % 8][feature / 8, one more than WF][bytes of the run + 16], so that neither the writes, eight
+// features apart, nor the 16-byte reads pile up on banks.
+template <int WF, int K>
+struct PackTile {
+    static constexpr int kFeatures = 8 * WF, kRun = K * (kThreads / WF), kPitch = kRun + (kRun > 8 ? 16 : 0);
+    static constexpr int kShared = 8 * (WF + 1) * kPitch;  // bytes
+};
+
+// Output i goes to the rows starting at dst + i * out_stride (row_bytes bytes per feature row).  Samples beyond the batch give
+// zero bits.  fblk, sblk: which tile.
+template <int NT, int WF, int K, bool ALIGNED, typename MASK>
+__device__ __forceinline__ void pack_tile(const uint8_t *__restrict__ t, uint8_t *__restrict__ dst, int64_t out_stride, const PackShape &sh,
+                                          int64_t fblk, int64_t sblk, uint8_t *s_bytes, MASK mask) {
+    using Tile = PackTile<WF, K>;
+    static_assert(K == 1 || K == 4, "a thread's bytes are written one or four at a time");
+    const int group = threadIdx.x / WF, octet = threadIdx.x % WF;
+    const int64_t f0 = fblk * Tile::kFeatures, f = f0 + octet * 8, byte0 = sblk * Tile::kRun, s0 = (byte0 + group * K) * 8;
+    const int live = f < sh.n ? (int)max((int64_t)0, min((int64_t)(8 * K), sh.batch - s0)) : 0;
+    const int features = (int)min((int64_t)8, sh.n - f);
+    unsigned long long bits[K][NT];  // per round of 8 samples and output: byte f = the samples' bits of feature f
+#pragma unroll
+    for (int g = 0; g < K; ++g) pack_eight<NT, ALIGNED>(t + (s0 + g * 8) * sh.n + f, sh.n, features, live - g * 8, mask, bits[g]);
+    constexpr int kPiece = Tile::kRun >= 16 ? 16 : 8, kPieces = Tile::kRun / kPiece;
+    const bool wide = sh.row_bytes % kPiece == 0 && (reinterpret_cast<uintptr_t>(dst) % kPiece) == 0 && out_stride % kPiece == 0;
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+        uint8_t *mine = s_bytes + octet * Tile::kPitch + group * K;
+        if constexpr (K == 1) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) mine[q * (WF + 1) * Tile::kPitch] = (uint8_t)(bits[0][i] >> (8 * q));
+        } else {
+            uint32_t lo[4], hi[4];  // a feature's four bytes
+            transpose_bytes_4x4((uint32_t)bits[0][i], (uint32_t)bits[1][i], (uint32_t)bits[2][i], (uint32_t)bits[3][i], lo);
+            transpose_bytes_4x4((uint32_t)(bits[0][i] >> 32), (uint32_t)(bits[1][i] >> 32), (uint32_t)(bits[2][i] >> 32),
+                                (uint32_t)(bits[3][i] >> 32), hi);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                *reinterpret_cast<uint32_t *>(mine + q * (WF + 1) * Tile::kPitch) = lo[q];
+                *reinterpret_cast<uint32_t *>(mine + (q + 4) * (WF + 1) * Tile::kPitch) = hi[q];
+            }
         }
         __syncthreads();
-        // a feature's eight words (64 bytes) leave as four 16-byte stores; ragged ends and unaligned rows byte by byte
         uint8_t *rows = dst + (int64_t)i * out_stride;
-        for (int idx = threadIdx.x; idx < kPackFeatures * 4; idx += kThreads) {
-            const int fl = idx / 4, piece = idx % 4;
-            if (f0 + fl >= n) continue;
-            const int at = (fl % 8) * 33 + fl / 8;
-            const unsigned long long w0 = s_words[(2 * piece) * kPackRow + at], w1 = s_words[(2 * piece + 1) * kPackRow + at];
-            uint8_t *o = rows + (f0 + fl) * row_bytes + byte0 + 16 * piece;
-            const int64_t left = row_bytes - (byte0 + 16 * piece);
-            if (left >= 16 && wide) {
-                *reinterpret_cast<uint4 *>(o) = make_uint4((uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1, (uint32_t)(w1 >> 32));
+        for (int idx = threadIdx.x; idx < Tile::kFeatures * kPieces; idx += kThreads) {
+            const int fl = idx / kPieces, piece = idx % kPieces;
+            if (f0 + fl >= sh.n) continue;
+            const uint8_t *from = s_bytes + ((fl % 8) * (WF + 1) + fl / 8) * Tile::kPitch + piece * kPiece;
+            uint8_t *to = rows + (f0 + fl) * sh.row_bytes + byte0 + piece * kPiece;
+            const int64_t left = sh.row_bytes - (byte0 + piece * kPiece);
+            if (left >= kPiece && wide) {
+                if constexpr (kPiece == 16) *reinterpret_cast<uint4 *>(to) = *reinterpret_cast<const uint4 *>(from);
+                else *reinterpret_cast<uint2 *>(to) = *reinterpret_cast<const uint2 *>(from);
             } else {
-                for (int by = 0; by < 16 && by < left; ++by) o[by] = (uint8_t)((by < 8 ? w0 : w1) >> (8 * (by % 8)));
+                for (int by = 0; by < kPiece && by < left; ++by) to[by] = from[by];
             }
         }
         __syncthreads();
     }
+}
+
+// Tile of a packer launch: kind 0 or 1 in the order of the list above.
+template <int KIND>
+using PackTileOf = PackTile<(KIND == 0 ? 32 : 8), (KIND == 0 ? 1 : 4)>;
+
+struct PackGrid {
+    int kind;
+    dim3 grid;
+};
+// Measured (us, 64 x 1024 tile / 256 x 64 tile; n x batch): 784 x 10000: 6.4 / 4.1; 784 x 100000: 23.9 / 22.9; 784 x 2^20: 227 / 232;
+// 783 x 2^20: 344 / 464; 30 x 2^20: 24 / 73; 117 x 10000: 10.8 / 4.0; 9216 x 10000: 29 / 22.
+static inline PackGrid pack_grid(const PackShape &sh) {
+    auto grid = [&](int64_t features, int64_t bytes) {
+        const int64_t sb = ceil_div(sh.row_bytes, bytes);
+        return dim3((unsigned)ceil_div(sh.n, features), (unsigned)(sb < 65535 ? sb : 65535));
+    };
+    const PackGrid small = {0, grid(256, 8)}, large = {1, grid(64, 128)};
+    const int64_t tiles = (int64_t)large.grid.x * large.grid.y;
+    return tiles >= 16 * 148 || (sh.n <= 128 && tiles >= 4 * 148) ? large : small;
 }
 
 }  // namespace dl

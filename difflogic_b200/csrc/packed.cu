@@ -132,70 +132,27 @@ packbits_kernel(const uint8_t *__restrict__ t, uint8_t *__restrict__ out, int64_
     }
 }
 
-// packbits from the batch-major matrix t[batch][n], n % 8 == 0: transpose and pack in one pass, 8-byte loads, bits moved
-// eight by eight (pack_tile.cuh).
+// packbits from the batch-major matrix t[batch][n]: transpose and pack in one pass, bits moved eight by eight (pack_tile.cuh).
 struct MaskNonZero {
     __device__ __forceinline__ uint32_t operator()(uint32_t lo, uint32_t hi, int) const {
         return squeeze8_ones(nonzero_bytes(lo), nonzero_bytes(hi));
     }
 };
 
+template <int KIND, bool ALIGNED>
 __global__ void __launch_bounds__(kThreads)
-packbits_bm8_kernel(const uint8_t *__restrict__ t, uint8_t *__restrict__ out, int64_t n, int64_t batch, int64_t row_bytes) {
-    __shared__ unsigned long long s_words[8 * kPackRow];
-    const int64_t f0 = (int64_t)blockIdx.x * kPackFeatures;
-    for (int64_t sblk = blockIdx.y; sblk * kPackSamples < row_bytes * 8; sblk += gridDim.y)
-        pack_tile<1>(t, out, 0, n, batch, row_bytes, f0, sblk, s_words, MaskNonZero());
+packbits_bm_kernel(const uint8_t *__restrict__ t, uint8_t *__restrict__ out, PackShape sh) {
+    using Tile = PackTileOf<KIND>;
+    __shared__ __align__(16) uint8_t s_bytes[Tile::kShared];
+    for (int64_t sblk = blockIdx.y; sblk * Tile::kRun < sh.row_bytes; sblk += gridDim.y)
+        pack_tile<1, Tile::kFeatures / 8, KIND == 0 ? 1 : 4, ALIGNED>(t, out, 0, sh, blockIdx.x, sblk, s_bytes, MaskNonZero());
 }
 
-// The same for any n (and any alignment): 4-byte or single-byte loads, one bit at a time.
-// A CTA takes 128 features x 512 samples.  Warp w owns 64 samples (one 64-bit word); its lanes
-// each own four adjacent features, read as one 32-bit load per sample (coalesced along the
-// features) and shifted into four words.  The 8 warps' words go through shared memory so that
-// a feature's eight words leave as one 64-byte run.
-template <bool VEC4>
-__global__ void __launch_bounds__(kThreads)
-packbits_bm_kernel(const uint8_t *__restrict__ t, uint8_t *__restrict__ out, int64_t n, int64_t batch, int64_t row_bytes) {
-    __shared__ unsigned long long s_words[128][9];  // [feature][word], padded
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int64_t f0 = (int64_t)blockIdx.x * 128;
-    for (int64_t sblk = blockIdx.y; sblk * 512 < batch; sblk += gridDim.y) {
-        const int64_t s0 = sblk * 512 + warp * 64;
-        unsigned long long wd[4] = {0ull, 0ull, 0ull, 0ull};
-        const int64_t f = f0 + lane * 4;
-        if (VEC4) {
-            if (f < n) {  // n % 4 == 0, so all four features exist
-#pragma unroll 16
-                for (int s = 0; s < 64; ++s) {
-                    if (s0 + s < batch) {
-                        const uint32_t v = __vsetne4(__ldg(reinterpret_cast<const uint32_t *>(t + (s0 + s) * n + f)), 0u);
-                        wd[0] |= (unsigned long long)(v & 1u) << s;
-                        wd[1] |= (unsigned long long)((v >> 8) & 1u) << s;
-                        wd[2] |= (unsigned long long)((v >> 16) & 1u) << s;
-                        wd[3] |= (unsigned long long)((v >> 24) & 1u) << s;
-                    }
-                }
-            }
-        } else {
-            for (int s = 0; s < 64; ++s) {
-                if (s0 + s < batch) {
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (f + q < n) wd[q] |= (unsigned long long)(__ldg(t + (s0 + s) * n + f + q) != 0) << s;
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) s_words[lane * 4 + q][warp] = wd[q];
-        __syncthreads();
-        // write: byte granularity so that any bit_count / ragged row length works
-        const int64_t byte0 = sblk * 64;  // first output byte of this sample block
-        for (int idx = threadIdx.x; idx < 128 * 64; idx += kThreads) {
-            const int fl = idx / 64, by = idx % 64;
-            if (f0 + fl < n && byte0 + by < row_bytes)
-                out[(f0 + fl) * row_bytes + byte0 + by] = (uint8_t)(s_words[fl][by / 8] >> (8 * (by % 8)));
-        }
-        __syncthreads();
+template <bool ALIGNED>
+static void launch_packbits_bm(const PackGrid &g, const uint8_t *t, uint8_t *out, const PackShape &sh, cudaStream_t st) {
+    switch (g.kind) {
+        case 0: packbits_bm_kernel<0, ALIGNED><<<g.grid, kThreads, 0, st>>>(t, out, sh); break;
+        default: packbits_bm_kernel<1, ALIGNED><<<g.grid, kThreads, 0, st>>>(t, out, sh); break;
     }
 }
 
@@ -401,17 +358,10 @@ extern "C" DL_API int dl_packbits_batch_major(const uint8_t *t, void *out, int64
     if (n == 0 || batch == 0) return DL_OK;
     DL_REQUIRE(t && out, DL_ERR_INVALID_ARG, "dl_packbits_batch_major: null pointer");
     const int64_t row_bytes = ceil_div(batch, bit_count) * (bit_count / 8);
-    const int64_t sblocks = ceil_div(row_bytes, 64);  // 512 samples each; covers the pad bytes too
-    const dim3 grid((unsigned)ceil_div(n, 128), (unsigned)(sblocks < 65535 ? sblocks : 65535));
     uint8_t *o = reinterpret_cast<uint8_t *>(out);
-    if (n % 8 == 0 && aligned_to(t, 8)) {
-        const int64_t sb = ceil_div(row_bytes, kPackSamples / 8);
-        const dim3 grid8((unsigned)ceil_div(n, kPackFeatures), (unsigned)(sb < 65535 ? sb : 65535));
-        packbits_bm8_kernel<<<grid8, kThreads, 0, as_stream(stream)>>>(t, o, n, batch, row_bytes);
-    } else if (n % 4 == 0 && aligned_to(t, 4))
-        packbits_bm_kernel<true><<<grid, kThreads, 0, as_stream(stream)>>>(t, o, n, batch, row_bytes);
-    else
-        packbits_bm_kernel<false><<<grid, kThreads, 0, as_stream(stream)>>>(t, o, n, batch, row_bytes);
+    const PackShape sh = {n, batch, row_bytes};
+    if (n % 8 == 0 && aligned_to(t, 8)) launch_packbits_bm<true>(pack_grid(sh), t, o, sh, as_stream(stream));
+    else launch_packbits_bm<false>(pack_grid(sh), t, o, sh, as_stream(stream));
     return launch_status("dl_packbits_batch_major");
 }
 
