@@ -305,9 +305,10 @@ groupsum_ce_kernel(const float *__restrict__ x, const int64_t *__restrict__ targ
 // groups of 128 threads add the class's pieces in a fixed order (piece p goes to group p % 8, the groups are added in
 // order) and write the scores; the CTA that holds the ticket computes the loss and the class-row gradients as in
 // groupsum_ce_kernel.  Reads pieces * batch floats per class that the forward kernel has just written (L2).
-// S: CTAs (a cluster) per (columns, class), each adding every S-th round of pieces; their sums meet in the first one's shared
-// memory.  Eight of them where the classes are long and (columns, class) pairs too few to fill the GPU: for 4000 runs, 10 classes
-// and 256 columns one CTA per pair, 20 in all, waited for one load after the other: 31 us.
+// S = 8: eight CTAs (a cluster) per (columns, class), one for each of the groups, whose 1024 threads fetch 64 of the group's pieces
+// at a time into shared memory for 128 of them to add.  For long classes and too few (columns, class) pairs to fill the GPU: with
+// 4000 runs, 10 classes and 256 columns one CTA per pair, 20 in all, waited for one load after the other (31 us).  The order of
+// the additions is that of S = 1: the scores, which the softmax magnifies every rounding of, are the same to the bit.
 constexpr int kCsThreads = 1024;
 constexpr int kCsGroups = kCsThreads / kGsCols;  // 8
 
@@ -317,9 +318,12 @@ class_sums_ce_kernel(const float *__restrict__ sums, const int64_t *__restrict__
                      float *__restrict__ loss, float *__restrict__ grad_classes, unsigned int *__restrict__ counter, int64_t batch, int k,
                      int m, int nb, float tau) {
     __shared__ float s_part[kCsGroups][kGsCols];
+    constexpr int kChunk = 64;
+    __shared__ float s_chunk[S > 1 ? kChunk : 1][kGsCols];
     __shared__ float s_all[S][kGsCols];
     __shared__ float s_red[kCsThreads / 32];
     __shared__ bool s_last;
+    static_assert(S == 1 || S == kCsGroups, "a CTA per group");
     const unsigned q = S > 1 ? cooperative_groups::this_cluster().block_rank() : 0u;
     const int tid = threadIdx.x, g = tid / kGsCols, col = tid % kGsCols;
     const int c = blockIdx.y;
@@ -328,28 +332,45 @@ class_sums_ce_kernel(const float *__restrict__ sums, const int64_t *__restrict__
     const unsigned first = row0 / (unsigned)nb, last = (row0 + (unsigned)m - 1u) / (unsigned)nb;  // runs that hold rows of class c
     if (S > 1) cooperative_groups::this_cluster().sync();  // the first CTA runs before the others write to it
     grid_dependency_wait();  // sums is the output of the kernel just before
-    float acc = 0.f;
-    if (gcol < batch) {
+    auto piece = [&](unsigned i) {
+        const unsigned e = i * (unsigned)nb >= row0 ? 0u : 1u;  // the run's first row is of class c, or of the class before it
+        return __ldcg(sums + (int64_t)(2u * i + e) * batch + gcol);
+    };
+    float acc = 0.f, total = 0.f;
+    if (S == 1) {
+        if (gcol < batch) {
 #pragma unroll 8
-        for (unsigned i = first + q * kCsGroups + (unsigned)g; i <= last; i += S * kCsGroups) {
-            const unsigned e = i * (unsigned)nb >= row0 ? 0u : 1u;  // the run's first row is of class c, or of the class before it
-            acc += __ldcg(sums + (int64_t)(2u * i + e) * batch + gcol);
+            for (unsigned i = first + (unsigned)g; i <= last; i += kCsGroups) acc += piece(i);
         }
-    }
-    s_part[g][col] = acc;
-    __syncthreads();
-    float total = 0.f;
-    if (g == 0) {
+        s_part[g][col] = acc;
+        __syncthreads();
+        if (g == 0) {
 #pragma unroll
-        for (int gg = 0; gg < kCsGroups; ++gg) total += s_part[gg][col];
-    }
-    if (S > 1) {
+            for (int gg = 0; gg < kCsGroups; ++gg) total += s_part[gg][col];
+        }
+    } else {
+        for (unsigned from = first + q; from <= last; from += kChunk * kCsGroups) {
+            const unsigned have = min((unsigned)kChunk, (last - from) / kCsGroups + 1u);
+            float v[kChunk / kCsGroups];
+#pragma unroll
+            for (int u = 0; u < kChunk / kCsGroups; ++u) {
+                const unsigned t = (unsigned)(g + u * kCsGroups);
+                v[u] = t < have && gcol < batch ? piece(from + t * kCsGroups) : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < kChunk / kCsGroups; ++u) s_chunk[g + u * kCsGroups][col] = v[u];
+            __syncthreads();
+            if (g == 0) {
+#pragma unroll 8
+                for (unsigned t = 0; t < have; ++t) acc += s_chunk[t][col];
+            }
+            __syncthreads();
+        }
         cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-        if (g == 0) *cluster.map_shared_rank(&s_all[q][col], 0) = total;
+        if (g == 0) *cluster.map_shared_rank(&s_all[q][col], 0) = acc;
         cluster.sync();
         if (q != 0) return;
         if (g == 0) {
-            total = 0.f;
 #pragma unroll
             for (int r = 0; r < S; ++r) total += s_all[r][col];
         }

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 # (n_out, k, batch): 64 and 63 runs of 32 rows per class, classes that end inside a run, several blocks of columns, so many
 # (columns, class) pairs that one CTA each will do
-@pytest.mark.parametrize("n_out,k,batch", [(2 * 2048, 2, 200), (2 * 1984, 2, 200), (3 * 3001, 3, 333), (20000, 1, 130), (30000, 10, 1900)])
+@pytest.mark.parametrize("n_out,k,batch", [(2 * 2048, 2, 200), (2 * 1984, 2, 200), (3 * 3001, 3, 333), (20000, 1, 130), (30000, 10, 1900), (2 * 10000, 2, 256)])
 def test_head(n_out, k, batch):
     g = torch.Generator().manual_seed(n_out)
     n_in, tau = 50, 20.0
@@ -28,3 +28,8 @@ def test_head(n_out, k, batch):
         assert abs(loss.item() - loss_ref.item()) <= 1e-5 * max(1.0, ref.abs().max().item())
         if k > 1:
             assert_grad_close(grad_classes.t() * tau, ref.grad, "grad")
+    if batch % 128 == 0:    # the order of the additions does not depend on how many CTAs share them: 19 blocks of columns more
+        wide = torch.cat([x] + [torch.rand(n_in, 128 * 19, generator=g)] * 4, 1)
+        fill = torch.zeros(wide.shape[1] - batch, dtype=torch.int64)
+        _, more, _, _ = ops.logic_forward_head(wide.cuda(), a.cuda(), b.cuda(), w.cuda(), torch.cat([target, fill]).cuda(), k, tau)
+        assert torch.equal(more[:batch], scores)
