@@ -54,6 +54,8 @@ SIGNATURES = {
     "dl_groupbitsum": (_int, [_ptr, _ptr, _i64, _i64, _i64, _i64, _int, _ptr]),
     "dl_eval_groupbitsum_applicable": (_int, [_ptr, _i64, _i64, _i64, _int, _i64]),
     "dl_eval_groupbitsum": (_int, [_ptr, _ptr, _ptr, _ptr, _ptr, _i64, _i64, _i64, _i64, _i64, _int, _ptr]),
+    "dl_eval_groupbitsum_parts_applicable": (_int, [_ptr, _i64, _i64, _i64, _int, _i64]),
+    "dl_eval_groupbitsum_parts": (_int, [_ptr, _ptr, _ptr, _ptr, _ptr, _i64, _i64, _i64, _i64, _i64, _int, _ptr]),
     "dl_groupsum_workspace_bytes": (ctypes.c_size_t, [_i64, _i64, _i64]),
     "dl_groupsum_f32": (_int, [_ptr, _ptr, _ptr, _i64, _i64, _i64, _f32, _ptr]),
     "dl_groupsum_backward_f32": (_int, [_ptr, _ptr, _i64, _i64, _i64, _f32, _ptr]),

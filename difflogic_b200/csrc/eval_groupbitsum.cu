@@ -4,8 +4,9 @@
 // Unfused, the last layer writes n_out rows and the group bit-sum reads them back: two passes over the largest
 // array of the network.  Here a thread-block CLUSTER of S CTAs owns one work unit = (column block of up to 2 KB, class):
 // CTA q of the cluster takes the q-th share of the class's neurons.  A CTA has three kinds of warps:
-//   * two PRODUCER warps stage the two gathered input rows of 8 neurons at a time in shared memory (one 2 KB bulk
-//     copy per row, ring of 3 stages) together with the neurons' gate masks;
+//   * two PRODUCER warps stage the two gathered input rows of 8 neurons at a time in shared memory (one bulk copy of up to
+//     2 KB per row; a ring of 96 KB: 3 stages, more where the rows are shorter, because a stage takes its 1.2 us whatever
+//     the length of its rows) together with the neurons' gate masks;
 //   * 256 CONSUMER threads own one 64-bit word column each, apply the gate and feed the result to a bit-sliced
 //     counter in registers; at the end of a unit they drop the counter's planes into shared memory and go straight
 //     on to the next unit;
@@ -18,6 +19,9 @@
 // The cluster is also what keeps the gathers in L2: all CTAs of a cluster read the same 2 KB column block of x, the
 // clusters that are resident together cover classes first (unit = column block * k + class), so only a handful
 // of column blocks (n_in * 2 KB each) are live at a time and the second reader of an input row hits L2.
+//
+// A class of more neurons than the counters of 8 CTAs hold (8 x 255) is cut into parts, each a work unit like a class of its own,
+// whose counts are added to a zeroed `out` by atomics (integers: any order gives the same).
 //
 // Synchronisation inside the cluster uses two mbarriers per CTA with remote arrivals (one per warp and peer):
 // red_full -- every consumer warp of every CTA has published its planes of the unit; red_free -- every reducer warp
@@ -38,7 +42,7 @@ namespace cg = cooperative_groups;
 namespace dl {
 
 constexpr int kFgRows = 8;            // neurons per stage
-constexpr int kFgStages = 3;
+constexpr int kFgStages = 5;          // at most; as many as fit kFgRing, 3 for rows of 2 KB (two CTAs have to fit an SM)
 constexpr int kFgChunk = 2048;        // bytes of a row per unit: 256 words of 64 bits
 constexpr int kFgWords = kFgChunk / 8;
 constexpr int kFgProducers = 2;       // producer warps; stage i of the CTA is issued by warp i % kFgProducers
@@ -48,7 +52,7 @@ constexpr int kFgThreads = 32 * kFgProducers + kFgConsumers + 32 * kFgReducers;
 constexpr int kFgRedPlanes = 8;       // planes a CTA publishes: its share of a class is at most 255 neurons
 constexpr int kFgMaxShare = (1 << kFgRedPlanes) - 1;
 constexpr int kFgSumPlanes = kFgRedPlanes + 3;  // the sum over at most 8 CTAs
-constexpr size_t kFgStageBytes = (size_t)2 * kFgRows * kFgChunk;
+constexpr size_t kFgRing = (size_t)3 * 2 * kFgRows * kFgChunk;  // bytes of the ring of stages
 
 __device__ int g_fg_async_error = 0;
 
@@ -104,12 +108,14 @@ struct FgUnit {
     uint32_t bytes;  // bytes per row segment
 };
 
-__device__ __forceinline__ FgUnit fg_unit(int64_t u, int64_t row_bytes, int block_bytes, int k, int m, int q, int nq) {
+__device__ __forceinline__ FgUnit fg_unit(int64_t u, int64_t row_bytes, int block_bytes, int k, int m, int parts, int q, int nq) {
     FgUnit g;
-    g.cls = (int)(u % k);
-    g.col0 = (u / k) * block_bytes;
+    const int unit = (int)(u % ((int64_t)k * parts)), part = unit % parts;
+    g.cls = unit / parts;
+    g.col0 = (u / ((int64_t)k * parts)) * block_bytes;
     g.bytes = (uint32_t)min((int64_t)block_bytes, row_bytes - g.col0);
-    const int64_t r0 = ((int64_t)m * q) / nq, r1 = ((int64_t)m * (q + 1)) / nq;
+    const int64_t first = (int64_t)m * part / parts, rows = (int64_t)m * (part + 1) / parts - first;
+    const int64_t r0 = first + rows * q / nq, r1 = first + rows * (q + 1) / nq;
     g.row0 = (int64_t)g.cls * m + r0;
     g.rows = (int)(r1 - r0);
     return g;
@@ -121,28 +127,28 @@ struct FgCursor {
     int r;          // first row of the stage within the share
     FgUnit g;
     bool valid;
-    __device__ __forceinline__ void seek(int64_t nclusters, int64_t nunits, int64_t row_bytes, int block_bytes, int k, int m, int q, int nq) {
+    __device__ __forceinline__ void seek(int64_t nclusters, int64_t nunits, int64_t row_bytes, int block_bytes, int k, int m, int parts, int q, int nq) {
         // first unit from u on whose share has rows
         for (valid = false; u < nunits; u += nclusters) {
-            g = fg_unit(u, row_bytes, block_bytes, k, m, q, nq);
+            g = fg_unit(u, row_bytes, block_bytes, k, m, parts, q, nq);
             if (g.rows > 0) { valid = true; break; }
         }
     }
     __device__ __forceinline__ void start(int64_t cluster_id, int64_t nclusters, int64_t nunits, int64_t row_bytes, int block_bytes, int k,
-                                          int m, int q, int nq) {
+                                          int m, int parts, int q, int nq) {
         u = cluster_id;
         it = 0;
         r = 0;
-        seek(nclusters, nunits, row_bytes, block_bytes, k, m, q, nq);
+        seek(nclusters, nunits, row_bytes, block_bytes, k, m, parts, q, nq);
     }
-    __device__ __forceinline__ void next(int64_t nclusters, int64_t nunits, int64_t row_bytes, int block_bytes, int k, int m, int q, int nq) {
+    __device__ __forceinline__ void next(int64_t nclusters, int64_t nunits, int64_t row_bytes, int block_bytes, int k, int m, int parts, int q, int nq) {
         if (!valid) return;
         ++it;
         r += kFgRows;
         if (r >= g.rows) {
             u += nclusters;
             r = 0;
-            seek(nclusters, nunits, row_bytes, block_bytes, k, m, q, nq);
+            seek(nclusters, nunits, row_bytes, block_bytes, k, m, parts, q, nq);
         }
     }
 };
@@ -204,22 +210,23 @@ template <int S>
 __global__ void __launch_bounds__(kFgThreads, 2)
 eval_groupbitsum_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict__ a, const int64_t *__restrict__ b,
                         const uint8_t *__restrict__ gate, int32_t *__restrict__ out, int64_t row_bytes, int block_bytes,
-                        int64_t batch, int k, int m, int nplanes, int64_t nunits) {
+                        int64_t batch, int k, int m, int parts, int nplanes, int64_t nunits, int stages) {
     extern __shared__ __align__(128) uint8_t smem[];
-    unsigned long long *red = reinterpret_cast<unsigned long long *>(smem + kFgStages * kFgStageBytes);  // [planes][words]
+    unsigned long long *red = reinterpret_cast<unsigned long long *>(smem + kFgRing);  // [planes][words]
     uint4 *meta = reinterpret_cast<uint4 *>(red + kFgRedPlanes * kFgWords);                               // [stages][rows]
     uint64_t *full = reinterpret_cast<uint64_t *>(meta + kFgStages * kFgRows);
     uint64_t *empty = full + kFgStages;
     uint64_t *red_full = empty + kFgStages;  // every CTA of the cluster has published its planes of the current unit
     uint64_t *red_free = red_full + 1;       // every CTA of the cluster has read this CTA's planes of the current unit
     __shared__ int s_abort;
+    const size_t stage_bytes = (size_t)2 * kFgRows * block_bytes;
 
     cg::cluster_group cluster = cg::this_cluster();
     const int q = (int)cluster.block_rank();
     const int64_t cluster_id = blockIdx.x / S, nclusters = gridDim.x / S;
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     if (tid == 0) {
-        for (int s = 0; s < kFgStages; ++s) {
+        for (int s = 0; s < stages; ++s) {
             mbar_init(full + s, 1);
             mbar_init(empty + s, kFgConsumers / 32);
         }
@@ -241,8 +248,8 @@ eval_groupbitsum_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict
         int64_t last = -1;  // latest stage this warp filled
         bool ok = true;
         FgCursor cur;
-        cur.start(cluster_id, nclusters, nunits, row_bytes, block_bytes, k, m, q, S);
-        for (int i = 0; i < warp; ++i) cur.next(nclusters, nunits, row_bytes, block_bytes, k, m, q, S);
+        cur.start(cluster_id, nclusters, nunits, row_bytes, block_bytes, k, m, parts, q, S);
+        for (int i = 0; i < warp; ++i) cur.next(nclusters, nunits, row_bytes, block_bytes, k, m, parts, q, S);
         int64_t idx = 0;
         uint32_t op = 0;
         if (cur.valid && copier && r_in < cur.g.rows - cur.r) {
@@ -251,7 +258,7 @@ eval_groupbitsum_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict
         }
         while (cur.valid) {
             FgCursor nxt = cur;
-            for (int i = 0; i < kFgProducers; ++i) nxt.next(nclusters, nunits, row_bytes, block_bytes, k, m, q, S);
+            for (int i = 0; i < kFgProducers; ++i) nxt.next(nclusters, nunits, row_bytes, block_bytes, k, m, parts, q, S);
             int64_t idx_next = 0;
             uint32_t op_next = 0;
             if (nxt.valid && copier && r_in < nxt.g.rows - nxt.r) {
@@ -260,8 +267,8 @@ eval_groupbitsum_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict
             }
             const int nr = min(kFgRows, cur.g.rows - cur.r);
             const bool valid = copier && r_in < nr;
-            const int s = (int)(cur.it % kFgStages);
-            const uint32_t use = (uint32_t)(cur.it / kFgStages);
+            const int s = (int)((uint32_t)cur.it % (uint32_t)stages);
+            const uint32_t use = (uint32_t)cur.it / (uint32_t)stages;
             if (!fg_wait(empty + s, (use & 1u) ^ 1u, abort_flag)) { ok = false; break; }
             if (valid && which == 0) {
                 const GateMasks gm = gate_masks((int)op);
@@ -274,7 +281,7 @@ eval_groupbitsum_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict
             if (lane == 0) mbar_arrive_expect_tx(full + s, copies * cur.g.bytes);
             __syncwarp();
             if (needed)
-                bulk_load(smem + s * kFgStageBytes + (size_t)(which * kFgRows + r_in) * kFgChunk, x + idx * row_bytes + cur.g.col0,
+                bulk_load(smem + s * stage_bytes + (size_t)(which * kFgRows + r_in) * block_bytes, x + idx * row_bytes + cur.g.col0,
                           cur.g.bytes, full + s);
             last = cur.it;
             cur = nxt;
@@ -288,24 +295,30 @@ eval_groupbitsum_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict
                 s_abort = 1;
             }
             __syncwarp();
-            if (last >= 0) mbar_wait(full + (last % kFgStages), (uint32_t)(last / kFgStages) & 1u);
+            if (last >= 0) mbar_wait(full + (last % stages), (uint32_t)(last / stages) & 1u);
         }
     } else if (warp < kFgProducers + kFgConsumers / 32) {
         // ---------------- consumers: one 64-bit word column per thread ----------------
         const int ct = tid - 32 * kFgProducers;
         uint32_t remote_full = 0;  // lane p < S: the red_full barrier of rank p
         if (lane < S) remote_full = map_to_rank(smem_addr(red_full), (uint32_t)lane);
-        int64_t it = 0;
+        int s = 0;          // stage of the ring, and how often it has been used
+        uint32_t use = 0;
+        const int row_words = block_bytes / 8;
         uint32_t n = 0;  // units done
         for (int64_t u = cluster_id; u < nunits; u += nclusters, ++n) {
-            const FgUnit g = fg_unit(u, row_bytes, block_bytes, k, m, q, S);
+            const FgUnit g = fg_unit(u, row_bytes, block_bytes, k, m, parts, q, S);
             const bool mine = (uint32_t)ct * 8u < g.bytes;
             BitCounterT<kFgRedPlanes - 3> cn;  // a share is at most 255 neurons
             cn.clear();
-            for (int r = 0; r < g.rows; r += kFgRows, ++it) {
-                const int s = (int)(it % kFgStages);
-                const uint32_t use = (uint32_t)(it / kFgStages);
-                if (!fg_wait(full + s, use & 1u, abort_flag)) {
+            for (int r = 0; r < g.rows; r += kFgRows) {
+                const int at = s;
+                const uint32_t parity = use & 1u;
+                if (++s == stages) {
+                    s = 0;
+                    ++use;
+                }
+                if (!fg_wait(full + at, parity, abort_flag)) {
                     g_fg_async_error = 1;
                     s_abort = 1;
                     continue;  // keep the iteration counts; nothing is waited for any more
@@ -315,22 +328,22 @@ eval_groupbitsum_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict
                 // not held while the adder tree runs
                 unsigned long long v[kFgRows];
                 if (mine) {
-                    const uint2 *col_a = reinterpret_cast<const uint2 *>(smem + s * kFgStageBytes) + ct;
-                    const uint2 *col_b = col_a + kFgRows * kFgWords;
-                    const uint4 *mk = meta + s * kFgRows;
+                    const uint2 *col_a = reinterpret_cast<const uint2 *>(smem + at * stage_bytes) + ct;
+                    const uint2 *col_b = col_a + kFgRows * row_words;
+                    const uint4 *mk = meta + at * kFgRows;
                     // rows past the end of the share count as zero words
 #pragma unroll
                     for (int i = 0; i < kFgRows; ++i) {
                         v[i] = 0ull;
                         if (i < nr) {
-                            const uint2 va = col_a[i * kFgWords], vb = col_b[i * kFgWords];
+                            const uint2 va = col_a[i * row_words], vb = col_b[i * row_words];
                             const uint4 mm = mk[i];
                             v[i] = ((unsigned long long)gate_from_masks(va.y, vb.y, mm) << 32) | gate_from_masks(va.x, vb.x, mm);
                         }
                     }
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(empty + s);
+                if (lane == 0) mbar_arrive(empty + at);
                 if (mine) cn.add8(v);
             }
 
@@ -359,7 +372,7 @@ eval_groupbitsum_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict
         const int sum_planes = min(kFgSumPlanes, nplanes + (S == 8 ? 3 : S == 4 ? 2 : 1));
         uint32_t n = 0;
         for (int64_t u = cluster_id; u < nunits; u += nclusters, ++n) {
-            const FgUnit g = fg_unit(u, row_bytes, block_bytes, k, m, q, S);
+            const FgUnit g = fg_unit(u, row_bytes, block_bytes, k, m, parts, q, S);
             if (!fg_wait_cluster(red_full, n & 1u, abort_flag)) {
                 g_fg_async_error = 1;
                 s_abort = 1;
@@ -413,7 +426,11 @@ eval_groupbitsum_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict
                         for (int i = 0; i < 8; ++i) {
                             int32_t cnt = (int32_t)((lo_bytes[j] >> (8 * i)) & 0xFFull);
                             if (wide) cnt |= (int32_t)((hi_bytes[j] >> (8 * i)) & 0xFFull) << 8;
-                            if (s0 + 8 * j + i < batch) dst[(int64_t)(8 * j + i) * k] = cnt;
+                            if (s0 + 8 * j + i < batch) {
+                                int32_t *at = dst + (int64_t)(8 * j + i) * k;
+                                if (parts == 1) *at = cnt;
+                                else if (cnt != 0) atomicAdd(at, cnt);
+                            }
                         }
                     }
                 }
@@ -433,7 +450,7 @@ int eval_groupbitsum_async_error() {
 }
 
 static size_t fg_shared_bytes() {
-    return kFgStages * kFgStageBytes + (size_t)kFgRedPlanes * kFgWords * 8 + (size_t)kFgStages * kFgRows * sizeof(uint4) +
+    return kFgRing + (size_t)kFgRedPlanes * kFgWords * 8 + (size_t)kFgStages * kFgRows * sizeof(uint4) +
            (2 * kFgStages + 2) * sizeof(uint64_t);
 }
 
@@ -450,13 +467,10 @@ static int fg_cluster_size(int64_t m) {
 
 template <int S>
 static int launch_fg(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, int32_t *out, int64_t row_bytes,
-                     int64_t batch, int64_t k, int64_t m, cudaStream_t st) {
+                     int64_t batch, int64_t k, int64_t m, bool in_parts, cudaStream_t st) {
     const size_t smem = fg_shared_bytes();
     if (cudaFuncSetAttribute(eval_groupbitsum_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return launch_status("dl_eval_groupbitsum (shared memory opt-in)");
-    int nplanes = 1;
-    while (nplanes < kFgRedPlanes && ((int64_t)1 << nplanes) <= ceil_div(m, S)) ++nplanes;
-
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -481,12 +495,29 @@ static int launch_fg(const void *x, const int64_t *a, const int64_t *b, const ui
     // sharing the last round's units among all clusters stage by stage, with the parts' counts added to a zeroed out
     // by atomics: 300 against 288 us for 8000 gates x 2^20 samples, 70 against 64 us for 2^17 samples.
     const int block_bytes = (int)(row_bytes < kFgChunk ? row_bytes : kFgChunk);
-    const int64_t nunits = ceil_div(row_bytes, block_bytes) * k;
+    const int fit = (int)(kFgRing / ((size_t)2 * kFgRows * block_bytes)), stages = fit < kFgStages ? fit : kFgStages;
+    // parts: the number, from the fewest that the counters allow, that leaves the busiest cluster the fewest neurons
+    int64_t parts = 1;
+    if (in_parts) {
+        const int64_t fewest = ceil_div(m, (int64_t)S * kFgMaxShare);
+        int64_t least = 0;
+        for (int64_t p = fewest; p <= 4 * fewest; ++p) {
+            const int64_t rows = ceil_div(ceil_div(row_bytes, block_bytes) * k * p, resident) * (ceil_div(m, p) + 64);  // 64: a unit's fixed cost
+            if (p == fewest || rows < least) {
+                least = rows;
+                parts = p;
+            }
+        }
+        if (cudaMemsetAsync(out, 0, (size_t)batch * k * sizeof(int32_t), st) != cudaSuccess) return launch_status("dl_eval_groupbitsum (clear)");
+    }
+    int nplanes = 1;
+    while (nplanes < kFgRedPlanes && ((int64_t)1 << nplanes) <= ceil_div(ceil_div(m, parts), S)) ++nplanes;
+    const int64_t nunits = ceil_div(row_bytes, block_bytes) * k * parts;
     const int64_t nclusters = nunits < resident ? nunits : resident;
     cfg.gridDim = dim3((unsigned)(nclusters * S));
     const uint8_t *xb = reinterpret_cast<const uint8_t *>(x);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, eval_groupbitsum_kernel<S>, xb, a, b, gate, out, row_bytes, block_bytes, batch, (int)k,
-                                             (int)m, nplanes, nunits);
+                                             (int)m, (int)parts, nplanes, nunits, stages);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(DL_ERR_CUDA, "dl_eval_groupbitsum: %s", cudaGetErrorString(e));
@@ -498,16 +529,26 @@ static int launch_fg(const void *x, const int64_t *a, const int64_t *b, const ui
 
 using namespace dl;
 
+static bool fg_sizes(const void *x, int64_t n_in, int64_t n_out, int64_t words, int bit_count, int64_t k) {
+    if (!(bit_count == 8 || bit_count == 16 || bit_count == 32 || bit_count == 64 || bit_count == 128)) return false;
+    if (n_in <= 0 || n_out <= 0 || n_out > INT32_MAX || k <= 0 || words <= 0 || n_out % k != 0) return false;
+    const int64_t row_bytes = words * (bit_count / 8);
+    return row_bytes % 16 == 0 && row_bytes >= 512 && aligned_to(x, 16) && n_out / k >= 32 && k <= 65535;
+}
+
 // 1 when dl_eval_groupbitsum accepts these sizes and pointers, else 0 (the caller then runs dl_eval_packed and
 // dl_groupbitsum one after the other).
 extern "C" DL_API int dl_eval_groupbitsum_applicable(const void *x, int64_t n_in, int64_t n_out, int64_t words, int bit_count,
                                                      int64_t k) {
-    if (!(bit_count == 8 || bit_count == 16 || bit_count == 32 || bit_count == 64 || bit_count == 128)) return 0;
-    if (n_in <= 0 || n_out <= 0 || k <= 0 || words <= 0 || n_out % k != 0) return 0;
-    const int64_t row_bytes = words * (bit_count / 8), m = n_out / k;
-    if (row_bytes % 16 != 0 || row_bytes < 512 || !aligned_to(x, 16)) return 0;
-    if (m < 32 || ceil_div(m, fg_cluster_size(m)) > kFgMaxShare || k > 65535) return 0;
-    return 1;
+    if (!fg_sizes(x, n_in, n_out, words, bit_count, k)) return 0;
+    const int64_t m = n_out / k;
+    return ceil_div(m, fg_cluster_size(m)) <= kFgMaxShare ? 1 : 0;
+}
+
+// 1 when dl_eval_groupbitsum_parts does: the same with classes longer than one cluster's counters hold.
+extern "C" DL_API int dl_eval_groupbitsum_parts_applicable(const void *x, int64_t n_in, int64_t n_out, int64_t words, int bit_count,
+                                                           int64_t k) {
+    return fg_sizes(x, n_in, n_out, words, bit_count, k) && ceil_div(n_out / k, 8) > kFgMaxShare ? 1 : 0;
 }
 
 extern "C" DL_API int dl_eval_groupbitsum(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, int32_t *out,
@@ -521,8 +562,20 @@ extern "C" DL_API int dl_eval_groupbitsum(const void *x, const int64_t *a, const
     const int64_t row_bytes = words * (bit_count / 8), m = n_out / k, batch = words * bit_count - pad_len;
     cudaStream_t st = as_stream(stream);
     switch (fg_cluster_size(m)) {
-        case 8: return launch_fg<8>(x, a, b, gate, out, row_bytes, batch, k, m, st);
-        case 4: return launch_fg<4>(x, a, b, gate, out, row_bytes, batch, k, m, st);
-        default: return launch_fg<2>(x, a, b, gate, out, row_bytes, batch, k, m, st);
+        case 8: return launch_fg<8>(x, a, b, gate, out, row_bytes, batch, k, m, false, st);
+        case 4: return launch_fg<4>(x, a, b, gate, out, row_bytes, batch, k, m, false, st);
+        default: return launch_fg<2>(x, a, b, gate, out, row_bytes, batch, k, m, false, st);
     }
+}
+
+extern "C" DL_API int dl_eval_groupbitsum_parts(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, int32_t *out,
+                                                int64_t n_in, int64_t n_out, int64_t words, int64_t pad_len, int64_t k, int bit_count,
+                                                void *stream) {
+    DL_REQUIRE(dl_eval_groupbitsum_parts_applicable(x, n_in, n_out, words, bit_count, k) == 1, DL_ERR_INVALID_ARG,
+               "dl_eval_groupbitsum_parts: sizes outside the kernel's range (ask dl_eval_groupbitsum_parts_applicable first)");
+    DL_REQUIRE(pad_len >= 0 && pad_len < bit_count, DL_ERR_INVALID_ARG, "dl_eval_groupbitsum_parts: pad_len %lld out of range",
+               (long long)pad_len);
+    DL_REQUIRE(x && a && b && gate && out, DL_ERR_INVALID_ARG, "dl_eval_groupbitsum_parts: null pointer");
+    const int64_t row_bytes = words * (bit_count / 8);
+    return launch_fg<8>(x, a, b, gate, out, row_bytes, words * bit_count - pad_len, k, n_out / k, true, as_stream(stream));
 }

@@ -466,8 +466,17 @@ def eval_groupbitsum_applicable(x, n_out, k):
     return N.lib().dl_eval_groupbitsum_applicable(x.data_ptr(), n_in, int(n_out), words, bits_of(x), int(k)) == 1
 
 
-def eval_groupbitsum(x, a, b, gate, pad_len, k):
-    """groupbitsum(eval_packed(x, a, b, gate), pad_len, k) in one kernel; the layer's output is never stored."""
+def eval_groupbitsum_parts_applicable(x, n_out, k):
+    """The same for classes longer than that kernel's counters (eval_groupbitsum(..., parts=True))."""
+    if not (x.is_cuda and x.dim() == 2 and x.is_contiguous()):
+        return False
+    n_in, words = x.shape
+    return N.lib().dl_eval_groupbitsum_parts_applicable(x.data_ptr(), n_in, int(n_out), words, bits_of(x), int(k)) == 1
+
+
+def eval_groupbitsum(x, a, b, gate, pad_len, k, parts=False):
+    """groupbitsum(eval_packed(x, a, b, gate), pad_len, k) in one kernel; the layer's output is never stored.  parts: classes
+    of more than 2040 gates, counted in parts."""
     N.require_cuda(x, a, b, gate)
     _need(x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D tensor")
     _need(a.dtype == torch.int64 and b.dtype == torch.int64 and gate.dtype == torch.uint8, "a, b int64 and gate uint8")
@@ -481,8 +490,9 @@ def eval_groupbitsum(x, a, b, gate, pad_len, k):
     _need(batch >= 0, "pad_len exceeds the packed batch")
     out = torch.empty((batch, k), dtype=torch.int32, device=x.device)
     with torch.cuda.device(x.device):
-        N.check(N.lib().dl_eval_groupbitsum(x.data_ptr(), a.data_ptr(), b.data_ptr(), gate.data_ptr(), out.data_ptr(), n_in, n_out,
-                                            words, int(pad_len), k, bits, N.stream_of(x)))
+        run = N.lib().dl_eval_groupbitsum_parts if parts else N.lib().dl_eval_groupbitsum
+        N.check(run(x.data_ptr(), a.data_ptr(), b.data_ptr(), gate.data_ptr(), out.data_ptr(), n_in, n_out, words, int(pad_len), k, bits,
+                    N.stream_of(x)))
     return out
 
 

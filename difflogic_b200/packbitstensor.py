@@ -132,9 +132,10 @@ class PackBitsTensor:
             (layer, gate) = self._pending.pop()
             self._materialize()
             self._pending.append((layer, gate))  # still pending: `.t` would run it as a kernel of its own
-            if ops.eval_groupbitsum_applicable(self._t, layer.out_dim, k):
+            parts = ops.eval_groupbitsum_parts_applicable(self._t, layer.out_dim, k)
+            if parts or ops.eval_groupbitsum_applicable(self._t, layer.out_dim, k):
                 a, b = layer.indices
-                return ops.eval_groupbitsum(self._t, a, b, gate, pad_len, k)
+                return ops.eval_groupbitsum(self._t, a, b, gate, pad_len, k, parts=parts)
         self._materialize()
         return ops.groupbitsum(self._t, pad_len, k)
 

@@ -275,6 +275,12 @@ DL_API int dl_eval_groupbitsum_applicable(const void *x, int64_t n_in, int64_t n
 DL_API int dl_eval_groupbitsum(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, int32_t *out,
                                int64_t n_in, int64_t n_out, int64_t words, int64_t pad_len, int64_t k, int bit_count,
                                void *stream);
+/* The same for classes of more than 8 * 255 neurons, which are counted in parts: out is cleared and added to. */
+DL_API int dl_eval_groupbitsum_parts_applicable(const void *x, int64_t n_in, int64_t n_out, int64_t words, int bit_count,
+                                                int64_t k);
+DL_API int dl_eval_groupbitsum_parts(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, int32_t *out,
+                                     int64_t n_in, int64_t n_out, int64_t words, int64_t pad_len, int64_t k, int bit_count,
+                                     void *stream);
 
 /* ------------------------------------------------------------------------------------------
  * Float GroupSum, forward and backward, on the feature-major activation of the last layer.
