@@ -28,6 +28,9 @@ namespace dl {
 //                              2^20 samples: 784 -> 8000 221 us against 288 us, 4000 -> 8000 254 against 327,
 //                              but 6000 -> 8000 391 against 346).  Also used when the 16 x 2 shape would give a
 //                              CTA fewer than 64 tiles (8000 -> 8000 on 2^17 samples: 48 us against 53 us).
+//    8 x 5 and 8 x 8         -- the second shape for rows too short to fill its stages (chunks of at most 1376 and 860
+//                              bytes): as many stages as two CTAs per SM have room for, since it is the copies in
+//                              flight that count.
 constexpr int kProducers = 2;       // producer warps; tile i is issued by warp i % kProducers
 constexpr int kConsumerWarps = 8;
 constexpr int kTmaThreads = 32 * (kProducers + kConsumerWarps);
@@ -219,7 +222,12 @@ int launch_eval_tma(const void *x, const int64_t *a, const int64_t *b, const uin
     const int force = tuning(DL_TUNE_EVAL_SHAPE);
     const int64_t chunk = row_bytes < kMaxChunk ? row_bytes : kMaxChunk;
     const bool few_tiles = ceil_div(row_bytes, chunk) * ceil_div(n_out, 16) < (int64_t)64 * sm_count();
-    const bool wide = force == 1 ? true : force == 2 ? false : (n_out >= 2 * n_in || few_tiles);
+    constexpr int64_t kFiveStages = 1376, kEightStages = 860;  // bytes of a row for which 5 and 8 stages take 108 KB
+    const bool wide = force == 1 ? true : force == 2 ? false : (n_out >= 2 * n_in || few_tiles || chunk <= kFiveStages);
+    if (wide && chunk <= kEightStages)
+        return launch_eval_tma_shape<8, 8>(x, a, b, gate, y, n_out, row_bytes, 2, st, x_pitch, y_pitch);
+    if (wide && chunk <= kFiveStages)
+        return launch_eval_tma_shape<8, 5>(x, a, b, gate, y, n_out, row_bytes, 2, st, x_pitch, y_pitch);
     if (wide) return launch_eval_tma_shape<8, 3>(x, a, b, gate, y, n_out, row_bytes, 2, st, x_pitch, y_pitch);
     return launch_eval_tma_shape<16, 2>(x, a, b, gate, y, n_out, row_bytes, 1, st, x_pitch, y_pitch);
 }
