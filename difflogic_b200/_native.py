@@ -171,7 +171,26 @@ def check(status):
 
 
 def stream_of(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    """Handle of the current stream of t's device."""
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
+
+
+class _AlreadyThere:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_ALREADY_THERE = _AlreadyThere()
+
+
+def on_device(t):
+    """Context in which t's device is the current one.  Nothing is entered when it is already: entering and leaving
+    torch.cuda.device costs the host more than the rest of a small launch."""
+    index = t.get_device()
+    return _ALREADY_THERE if index == torch._C._cuda_getDevice() else torch.cuda.device(index)
 
 
 def ptr(t):

@@ -14,7 +14,7 @@ class _CrossEntropyFunction(torch.autograd.Function):
         batch, k = logits.shape
         loss = torch.empty((), dtype=torch.float32, device=logits.device)
         probs = torch.empty_like(logits)
-        with torch.cuda.device(logits.device):
+        with N.on_device(logits):
             N.check(N.lib().dl_cross_entropy_f32(logits.data_ptr(), target.data_ptr(), loss.data_ptr(), probs.data_ptr(),
                                                  batch, k, N.stream_of(logits)))
         ctx.save_for_backward(probs, target)
@@ -26,7 +26,7 @@ class _CrossEntropyFunction(torch.autograd.Function):
         batch, k = probs.shape
         grad = torch.empty_like(probs)
         grad_loss = grad_loss.contiguous().to(torch.float32)
-        with torch.cuda.device(probs.device):
+        with N.on_device(probs):
             N.check(N.lib().dl_cross_entropy_backward_f32(probs.data_ptr(), target.data_ptr(), grad_loss.data_ptr(),
                                                           grad.data_ptr(), batch, k, N.stream_of(probs)))
         return grad, None
@@ -44,7 +44,7 @@ class _GroupSumCrossEntropyFunction(torch.autograd.Function):
         batch = scores.shape[0]
         loss = torch.empty((), dtype=torch.float32, device=x.device)
         probs = torch.empty_like(scores)
-        with torch.cuda.device(x.device):
+        with N.on_device(x):
             N.check(N.lib().dl_cross_entropy_f32(scores.data_ptr(), target.data_ptr(), loss.data_ptr(), probs.data_ptr(),
                                                  batch, k, N.stream_of(x)))
         ctx.save_for_backward(probs, target)
@@ -61,7 +61,7 @@ class _GroupSumCrossEntropyFunction(torch.autograd.Function):
         batch = probs.shape[0]
         gx = torch.empty((ctx.n, batch), dtype=torch.float32, device=probs.device)
         grad_loss = grad_loss.contiguous().to(torch.float32)
-        with torch.cuda.device(probs.device):
+        with N.on_device(probs):
             N.check(N.lib().dl_groupsum_cross_entropy_backward_f32(probs.data_ptr(), target.data_ptr(), grad_loss.data_ptr(),
                                                                    gx.data_ptr(), ctx.n, batch, ctx.k, float(ctx.tau),
                                                                    N.stream_of(probs)))

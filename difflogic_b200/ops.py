@@ -23,12 +23,16 @@ def _need(cond, msg):
 
 
 def _f32_matrix(t, name):
+    if t.is_cuda and t.dtype is torch.float32 and t.dim() == 2 and t.is_contiguous():
+        return
     N.require_cuda(t)
     _need(t.dtype == torch.float32, "%s must be float32, got %s (the CUDA path computes in fp32)" % (name, t.dtype))
     _need(t.dim() == 2 and t.is_contiguous(), "%s must be a contiguous 2-D tensor" % name)
 
 
 def _index(t, name, n=None):
+    if t.is_cuda and t.dtype is torch.int64 and t.dim() == 1 and t.is_contiguous() and (n is None or t.numel() == n):
+        return
     N.require_cuda(t)
     _need(t.dtype == torch.int64 and t.dim() == 1 and t.is_contiguous(), "%s must be a contiguous int64 vector" % name)
     if n is not None:
@@ -51,9 +55,9 @@ def logic_forward(x, a, b, w, w_mode=W_LOGITS, want_coef=False, overlap=False):
     _need(w.shape[1] == 16, "w must be [n_out, 16]")
     _index(a, "a", n_out)
     _index(b, "b", n_out)
-    y = torch.empty((n_out, batch), dtype=torch.float32, device=x.device)
-    coef = torch.empty((n_out, 4), dtype=torch.float32, device=x.device) if want_coef else None
-    with torch.cuda.device(x.device):
+    y = x.new_empty((n_out, batch))
+    coef = x.new_empty((n_out, 4)) if want_coef else None
+    with N.on_device(x):
         N.check(N.lib().dl_forward_f32(x.data_ptr(), a.data_ptr(), b.data_ptr(), w.data_ptr(), w_mode, y.data_ptr(),
                                        N.ptr(coef), n_in, n_out, batch, int(overlap), N.stream_of(x)))
     return y, coef
@@ -63,7 +67,7 @@ def logic_coefs(w, w_mode=W_LOGITS):
     _f32_matrix(w, "w")
     _need(w.shape[1] == 16, "w must be [n_out, 16]")
     coef = torch.empty((w.shape[0], 4), dtype=torch.float32, device=w.device)
-    with torch.cuda.device(w.device):
+    with N.on_device(w):
         N.check(N.lib().dl_coefs_f32(w.data_ptr(), w_mode, coef.data_ptr(), w.shape[0], N.stream_of(w)))
     return coef
 
@@ -71,8 +75,8 @@ def logic_coefs(w, w_mode=W_LOGITS):
 def transpose(x):
     """[rows, cols] float32 -> its transpose as a new contiguous tensor (dl_transpose_f32)."""
     _f32_matrix(x, "x")
-    y = torch.empty((x.shape[1], x.shape[0]), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+    y = x.new_empty((x.shape[1], x.shape[0]))
+    with N.on_device(x):
         N.check(N.lib().dl_transpose_f32(x.data_ptr(), y.data_ptr(), x.shape[0], x.shape[1], N.stream_of(x)))
     return y
 
@@ -95,11 +99,11 @@ def logic_backward_w(x, a, b, grad_y, w=None, w_mode=W_PROBS, out=None, overlap=
         _f32_matrix(w, "w")
         _need(tuple(w.shape) == (n_out, 16), "w must be [n_out, 16]")
     if out is None:
-        out = torch.empty((n_out, 16), dtype=torch.float32, device=x.device)
+        out = x.new_empty((n_out, 16))
     else:
         _f32_matrix(out, "out")
         _need(tuple(out.shape) == (n_out, 16), "out must be [n_out, 16]")
-    with torch.cuda.device(x.device):
+    with N.on_device(x):
         if rows_per_class == 1:
             N.check(N.lib().dl_backward_w_f32(x.data_ptr(), a.data_ptr(), b.data_ptr(), grad_y.data_ptr(), N.ptr(w), w_mode,
                                               out.data_ptr(), n_in, n_out, batch, int(overlap), N.stream_of(x)))
@@ -133,7 +137,7 @@ def logic_backward_w_adam(x, a, b, grad_y, w, exp_avg, exp_avg_sq, state, lr, be
     if grad_out is not None:
         _f32_matrix(grad_out, "grad_out")
         _need(tuple(grad_out.shape) == (n_out, 16), "grad_out must be [n_out, 16]")
-    with torch.cuda.device(x.device):
+    with N.on_device(x):
         N.check(N.lib().dl_backward_w_adam_f32(x.data_ptr(), a.data_ptr(), b.data_ptr(), grad_y.data_ptr(), w.data_ptr(),
                                                exp_avg.data_ptr(), exp_avg_sq.data_ptr(), N.ptr(grad_out), n_in, n_out, batch,
                                                rows_per_class, float(lr), float(beta1), float(beta2), float(eps), float(grad_scale),
@@ -159,7 +163,7 @@ def logic_backward_w_announce(x, a, b, grad_y, w, out, rows_per_class, flag_ptrs
     _index(b, "b", n_out)
     for t in (bucket_state, block_ticket, kernel_count):
         _need(t.is_cuda and t.dtype == torch.int32 and t.numel() >= 1, "state words must be int32 CUDA tensors")
-    with torch.cuda.device(x.device):
+    with N.on_device(x):
         N.check(N.lib().dl_backward_w_announce_f32(x.data_ptr(), a.data_ptr(), b.data_ptr(), grad_y.data_ptr(), w.data_ptr(),
                                                    out.data_ptr(), n_in, n_out, batch, rows_per_class, flag_ptrs, rank, world, bucket,
                                                    bucket_state.data_ptr(), block_ticket.data_ptr(), kernel_count.data_ptr(),
@@ -187,7 +191,7 @@ def build_backward_plan(a, b, start, lst):
     _index(start, "start")
     _index(lst, "list", 2 * n_out)
     plan = torch.empty((2 * n_out, 2), dtype=torch.int32, device=a.device)
-    with torch.cuda.device(a.device):
+    with N.on_device(a):
         N.check(N.lib().dl_build_backward_plan(a.data_ptr(), b.data_ptr(), start.data_ptr(), lst.data_ptr(),
                                                plan.data_ptr(), n_in, n_out, N.stream_of(a)))
     return plan
@@ -216,9 +220,9 @@ def logic_forward_walk(x, w, walk, w_mode=W_LOGITS, want_coef=False, overlap=Fal
     n_in, batch = x.shape
     n_out = w.shape[0]
     _need(w.shape[1] == 16, "w must be [n_out, 16]")
-    y = torch.empty((n_out, batch), dtype=torch.float32, device=x.device)
-    coef = torch.empty((n_out, 4), dtype=torch.float32, device=x.device) if want_coef else None
-    with torch.cuda.device(x.device):
+    y = x.new_empty((n_out, batch))
+    coef = x.new_empty((n_out, 4)) if want_coef else None
+    with N.on_device(x):
         N.check(N.lib().dl_forward_walk_f32(x.data_ptr(), w.data_ptr(), w_mode, y.data_ptr(), N.ptr(coef), walk[0].data_ptr(),
                                             walk[0].shape[0], n_in, n_out, batch, int(overlap), N.stream_of(x)))
     return y, coef
@@ -239,12 +243,12 @@ def logic_backward_walk(x, grad_y, coef, w, walk, grad_scale=1.0, want_grad_x=Tr
     _need(tuple(w.shape) == (n_out, 16) and tuple(coef.shape) == (n_out, 4), "w must be [n_out, 16] and coef [n_out, 4]")
     gx = torch.empty_like(x) if want_grad_x else None
     if adam is None and grad_out is None:
-        grad_out = torch.empty((n_out, 16), dtype=torch.float32, device=x.device)
+        grad_out = x.new_empty((n_out, 16))
     if grad_out is not None:
         _f32_matrix(grad_out, "grad_out")
         _need(tuple(grad_out.shape) == (n_out, 16), "grad_out must be [n_out, 16]")
     a = adam or {}
-    with torch.cuda.device(x.device):
+    with N.on_device(x):
         N.check(N.lib().dl_backward_walk_f32(x.data_ptr(), grad_y.data_ptr(), coef.data_ptr(), w.data_ptr(), N.ptr(grad_out), N.ptr(gx),
                                              float(grad_scale), walk[0].data_ptr(), walk[0].shape[0], int(walk[1]), n_in, n_out, batch,
                                              rows_per_class, N.ptr(a.get("exp_avg")), N.ptr(a.get("exp_avg_sq")), float(a.get("lr", 0.0)),
@@ -274,7 +278,7 @@ def logic_backward_w_push(x, a, b, grad_y, w, out, rows_per_class, grad_inbox_pt
     _need(tuple(w.shape) == (n_out, 16) and tuple(out.shape) == (n_out, 16), "w and out must be [n_out, 16]")
     _index(a, "a", n_out)
     _index(b, "b", n_out)
-    with torch.cuda.device(x.device):
+    with N.on_device(x):
         N.check(N.lib().dl_backward_w_push_f32(x.data_ptr(), a.data_ptr(), b.data_ptr(), grad_y.data_ptr(), w.data_ptr(), out.data_ptr(),
                                                n_in, n_out, batch, rows_per_class, grad_inbox_ptrs, int(rank), int(world),
                                                int(bucket_offset), int(bucket_count), int(inbox_offset), int(inbox_stride),
@@ -296,7 +300,7 @@ def check_connections(a, b, n_in, start=None, lst=None, plan=None):
         _need(plan.is_cuda and plan.dtype == torch.int32 and plan.is_contiguous() and tuple(plan.shape) == (2 * n_out, 2),
               "plan must be a contiguous int32 [2*n_out, 2] tensor")
     report = torch.zeros(4, dtype=torch.int64, device=a.device)
-    with torch.cuda.device(a.device):
+    with N.on_device(a):
         N.check(N.lib().dl_check_connections(a.data_ptr(), b.data_ptr(), N.ptr(start), N.ptr(lst), N.ptr(plan), int(n_in), n_out,
                                              report.data_ptr(), N.stream_of(a)))
     code, where, value, limit = report.tolist()
@@ -321,7 +325,7 @@ def logic_backward_x(x, coef, grad_y, start, plan, grad_scale=1.0, overlap=False
     _need(plan.dtype == torch.int32 and plan.is_contiguous() and tuple(plan.shape) == (2 * n_out, 2),
           "plan must be a contiguous int32 [2*n_out, 2] tensor")
     gx = torch.empty_like(x)
-    with torch.cuda.device(x.device):
+    with N.on_device(x):
         if rows_per_class == 1:
             N.check(N.lib().dl_backward_x_f32(x.data_ptr(), coef.data_ptr(), grad_y.data_ptr(), start.data_ptr(),
                                               plan.data_ptr(), float(grad_scale), gx.data_ptr(), n_in, n_out, batch,
@@ -346,7 +350,7 @@ def argmax_gates(w):
     _f32_matrix(w, "w")
     _need(w.shape[1] == 16, "w must be [n_out, 16]")
     g = torch.empty((w.shape[0],), dtype=torch.uint8, device=w.device)
-    with torch.cuda.device(w.device):
+    with N.on_device(w):
         N.check(N.lib().dl_argmax_gate_u8(w.data_ptr(), g.data_ptr(), w.shape[0], N.stream_of(w)))
     return g
 
@@ -366,7 +370,7 @@ def eval_packed(x, a, b, gate, out=None):
         _need(out.dtype == x.dtype and tuple(out.shape) == (n_out, words) and out.is_contiguous() and out.is_cuda,
               "out must be a contiguous [n_out, words] tensor of x's dtype")
         _need(out.data_ptr() != x.data_ptr(), "eval_packed cannot run in place")
-    with torch.cuda.device(x.device):
+    with N.on_device(x):
         N.check(N.lib().dl_eval_packed(x.data_ptr(), a.data_ptr(), b.data_ptr(), gate.data_ptr(), out.data_ptr(),
                                        n_in, n_out, words, bits, N.stream_of(x)))
     return out
@@ -391,7 +395,7 @@ def packbits(t, bit_count):
     n, batch = t.shape
     words = -(-batch // bit_count)
     out = torch.empty((n, words), dtype=_BITS_TO_DTYPE[bit_count], device=t.device)
-    with torch.cuda.device(t.device):
+    with N.on_device(t):
         N.check(N.lib().dl_packbits(t.data_ptr(), out.data_ptr(), n, batch, bit_count, N.stream_of(t)))
     return out, (bit_count - batch % bit_count) % bit_count
 
@@ -407,7 +411,7 @@ def packbits_batch_major(t, bit_count, padded=False):
     batch, n = t.shape
     unit = ROW_UNIT_BITS if padded else bit_count
     out = torch.empty((n, -(-batch // unit) * (unit // bit_count)), dtype=_BITS_TO_DTYPE[bit_count], device=t.device)
-    with torch.cuda.device(t.device):
+    with N.on_device(t):
         N.check(N.lib().dl_packbits_batch_major(t.data_ptr(), out.data_ptr(), n, batch, unit, N.stream_of(t)))
     return out, (bit_count - batch % bit_count) % bit_count
 
@@ -425,7 +429,7 @@ def threshold_packbits_batch_major(t, thresholds, bit_count, padded=False):
     unit = ROW_UNIT_BITS if padded else bit_count
     out = torch.empty((len(thresholds) * n, -(-batch // unit) * (unit // bit_count)), dtype=_BITS_TO_DTYPE[bit_count], device=t.device)
     arr = (ctypes.c_ubyte * len(thresholds))(*thresholds)
-    with torch.cuda.device(t.device):
+    with N.on_device(t):
         N.check(N.lib().dl_threshold_packbits_batch_major(t.data_ptr(), ctypes.addressof(arr), len(thresholds), out.data_ptr(),
                                                           n, batch, unit, N.stream_of(t)))
     return out, (bit_count - batch % bit_count) % bit_count
@@ -453,7 +457,7 @@ def groupbitsum(x, pad_len, k):
     batch = words * bits - int(pad_len)
     _need(batch >= 0, "pad_len exceeds the packed batch")
     out = torch.empty((batch, k), dtype=torch.int32, device=x.device)
-    with torch.cuda.device(x.device):
+    with N.on_device(x):
         N.check(N.lib().dl_groupbitsum(x.data_ptr(), out.data_ptr(), n, words, int(pad_len), k, bits, N.stream_of(x)))
     return out
 
@@ -489,7 +493,7 @@ def eval_groupbitsum(x, a, b, gate, pad_len, k, parts=False):
     batch = words * bits - int(pad_len)
     _need(batch >= 0, "pad_len exceeds the packed batch")
     out = torch.empty((batch, k), dtype=torch.int32, device=x.device)
-    with torch.cuda.device(x.device):
+    with N.on_device(x):
         run = N.lib().dl_eval_groupbitsum_parts if parts else N.lib().dl_eval_groupbitsum
         N.check(run(x.data_ptr(), a.data_ptr(), b.data_ptr(), gate.data_ptr(), out.data_ptr(), n_in, n_out, words, int(pad_len), k, bits,
                     N.stream_of(x)))
@@ -549,13 +553,13 @@ def eval_network(x, network, batch, k=None):
         out = torch.empty((sizes[len(sizes) - 1], words), dtype=x.dtype, device=x.device)
     else:
         out = torch.empty((int(batch), int(k)), dtype=torch.int32, device=x.device)
-    with torch.cuda.device(x.device):
-        stream = torch.cuda.current_stream(x.device)
-        if stream.cuda_stream != network.stream:
-            network.program.record_stream(stream)
+    with N.on_device(x):
+        stream = N.stream_of(x)
+        if stream != network.stream:
+            network.program.record_stream(torch.cuda.current_stream(x.device))
         N.check(N.lib().dl_eval_network(x.data_ptr(), network.program.data_ptr(), sizes, len(sizes) - 1,
                                         0 if k is None else out.data_ptr(), out.data_ptr() if k is None else 0, row_bytes, int(batch),
-                                        1 if k is None else int(k), stream.cuda_stream))
+                                        1 if k is None else int(k), stream))
     return out
 
 
@@ -593,8 +597,8 @@ def groupsum(x, k, tau):
     n, batch = x.shape
     k = int(k)
     _need(k > 0 and n % k == 0, "n (%d) must be divisible by k (%d)" % (n, k))
-    out = torch.empty((batch, k), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+    out = x.new_empty((batch, k))
+    with N.on_device(x):
         stream = N.stream_of(x)
         ws = _groupsum_workspace(x.device, stream, N.lib().dl_groupsum_workspace_bytes(n, batch, k))
         N.check(N.lib().dl_groupsum_f32(x.data_ptr(), out.data_ptr(), ws.data_ptr(), n, batch, k, float(tau), stream))
@@ -619,13 +623,13 @@ def groupsum_cross_entropy(x, target, k, tau):
     _need(target.is_cuda and target.dtype == torch.int64 and target.dim() == 1 and target.is_contiguous()
           and target.shape[0] == batch and target.device == x.device, "target must be a contiguous int64 [batch] CUDA tensor")
     _need(groupsum_cross_entropy_applicable(n, batch, k), "classes of %d rows are outside the fused kernel's range" % (n // k))
-    scores = torch.empty((batch, k), dtype=torch.float32, device=x.device)
+    scores = x.new_empty((batch, k))
     loss = torch.empty((), dtype=torch.float32, device=x.device)
-    grad_classes = torch.empty((k, batch), dtype=torch.float32, device=x.device)
+    grad_classes = x.new_empty((k, batch))
     counter = _HEAD_COUNTERS.get(x.device)
     if counter is None:
         counter = _HEAD_COUNTERS[x.device] = torch.zeros(1, dtype=torch.int32, device=x.device)
-    with torch.cuda.device(x.device):
+    with N.on_device(x):
         N.check(N.lib().dl_groupsum_cross_entropy_f32(x.data_ptr(), target.data_ptr(), scores.data_ptr(), loss.data_ptr(),
                                                       grad_classes.data_ptr(), counter.data_ptr(), n, batch, k, float(tau),
                                                       N.stream_of(x)))
@@ -655,15 +659,15 @@ def logic_forward_head(x, a, b, w, target, k, tau, w_mode=W_LOGITS):
     lib = N.lib()
     rows = lib.dl_forward_class_sums_rows(n_out, batch, k)
     _need(rows > 0, "classes of %d rows are shorter than a forward CTA's run of rows" % (n_out // k))
-    sums = torch.empty((rows, batch), dtype=torch.float32, device=x.device)
-    coef = torch.empty((n_out, 4), dtype=torch.float32, device=x.device)
-    scores = torch.empty((batch, k), dtype=torch.float32, device=x.device)
+    sums = x.new_empty((rows, batch))
+    coef = x.new_empty((n_out, 4))
+    scores = x.new_empty((batch, k))
     loss = torch.empty((), dtype=torch.float32, device=x.device)
-    grad_classes = torch.empty((k, batch), dtype=torch.float32, device=x.device)
+    grad_classes = x.new_empty((k, batch))
     counter = _HEAD_COUNTERS.get(x.device)
     if counter is None:
         counter = _HEAD_COUNTERS[x.device] = torch.zeros(1, dtype=torch.int32, device=x.device)
-    with torch.cuda.device(x.device):
+    with N.on_device(x):
         st = N.stream_of(x)
         N.check(lib.dl_forward_class_sums_f32(x.data_ptr(), a.data_ptr(), b.data_ptr(), w.data_ptr(), w_mode, sums.data_ptr(),
                                               coef.data_ptr(), n_in, n_out, batch, k, N.LAUNCH_OVERLAP_SETUP, st))
@@ -678,7 +682,7 @@ def groupsum_backward(grad_out, n, tau):
     _f32_matrix(grad_out, "grad_out")
     batch, k = grad_out.shape
     gx = torch.empty((n, batch), dtype=torch.float32, device=grad_out.device)
-    with torch.cuda.device(grad_out.device):
+    with N.on_device(grad_out):
         N.check(N.lib().dl_groupsum_backward_f32(grad_out.data_ptr(), gx.data_ptr(), n, batch, k, float(tau),
                                                  N.stream_of(grad_out)))
     return gx

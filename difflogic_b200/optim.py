@@ -305,7 +305,7 @@ class FlatAdam(torch.optim.Optimizer):
         rank, world = self._exchange
         if getattr(self, "_barrier_state", None) is None:
             self._barrier_state = torch.zeros(16, dtype=torch.int32, device=self.flat_param.device)
-        with torch.cuda.device(self.flat_param.device):
+        with N.on_device(self.flat_param):
             N.check(N.lib().dl_rank_barrier(self._peer_ptrs["flags"], rank, world, 31, self._barrier_state.data_ptr(),
                                             self._wait_limit_us, N.stream_of(self.flat_param)))
 
@@ -426,7 +426,7 @@ class FlatAdam(torch.optim.Optimizer):
     def prefetch_state(self):
         """Launches (on the current stream) a kernel that pulls the moments towards L2.  They are touched once per step,
         so a step that begins with a cold L2 otherwise reads them from HBM at the very end, after the last gradient."""
-        with torch.cuda.device(self.flat_param.device):
+        with N.on_device(self.flat_param):
             st = N.stream_of(self.flat_param)
             if getattr(self, "exchange_enabled", False):
                 return   # a rank touches only its slices, and the exchange kernels read them beside their peer loads
@@ -454,8 +454,9 @@ class FlatAdam(torch.optim.Optimizer):
             with torch.enable_grad():
                 loss = closure()
         # a gradient that did not land in the flat buffer (a parameter that is not a LogicLayer weight) is copied in
+        base = self.flat_grad.data_ptr()
         for p in self._params:
-            if p.grad is not None and p.grad.data_ptr() != self.grad_view(p).data_ptr():
+            if p.grad is not None and p.grad.data_ptr() != base + 4 * self._slices[p][0]:
                 self.grad_view(p).copy_(p.grad)
         g = self.param_groups[0]
         beta1, beta2 = g['betas']
@@ -473,7 +474,7 @@ class FlatAdam(torch.optim.Optimizer):
             self._begin_exchange_step()
             self.mark_updated()
             return loss
-        with torch.cuda.device(self.flat_param.device):
+        with N.on_device(self.flat_param):
             N.check(N.lib().dl_adam_step_f32(self.flat_param.data_ptr(), self.flat_grad.data_ptr(), self.exp_avg.data_ptr(),
                                              self.exp_avg_sq.data_ptr(), self.flat_param.numel(), float(g['lr']), float(beta1),
                                              float(beta2), float(g['eps']), float(self.grad_scale), self.state_t.data_ptr(),

@@ -96,12 +96,14 @@ class PackBitsTensor:
         program stays with the last layer until a layer's gates or connections are others.  Not while a CUDA graph is being
         captured: the graph would outlive a program that a change of the weights replaces."""
         layers = [layer.indices + (gate,) for layer, gate in self._pending]
-        sizes = ops.network_sizes(self._t.shape[0], layers)
-        if not ops.eval_network_applicable(self._t, sizes, batch, k) or torch.cuda.is_current_stream_capturing():
-            return None
         last = self._pending[-1][0]
         network = last._network
-        if network is None or not network.matches(layers):
+        if network is not None and not (network.sizes[0] == self._t.shape[0] and network.matches(layers)):
+            network = None
+        sizes = network.sizes if network is not None else ops.network_sizes(self._t.shape[0], layers)
+        if not ops.eval_network_applicable(self._t, sizes, batch, k) or torch.cuda.is_current_stream_capturing():
+            return None
+        if network is None:
             if any(t.device != self._t.device for layer in layers for t in layer):
                 return None
             last._network = None      # given back before the next one is made
