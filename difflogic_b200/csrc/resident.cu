@@ -12,6 +12,9 @@
 // Measured, whole kernel: 784 -> 4 x 8000, 2^20 samples 827 us (1020 with general gates and a full adder tree per count; 1210 layer
 // by layer), of which the busiest unit, the shared-memory pipe, works 65 %; 784 -> 5 x 16000, 10000 samples 43 us (97 layer by layer).
 //
+// CTAs that stay for several blocks and fetch the next one's input while they count were slower (needs more than 64 registers:
+// 16000 wide, 10000 samples 45 -> 51 us, 8000 wide, 2^18 samples 208 -> 212).
+//
 // In-place update: a thread keeps the outputs of its R neurons in registers until every thread has read its inputs, then
 // all store.  That halves the shared memory a layer needs and with it doubles the samples per block.
 //
@@ -353,8 +356,10 @@ struct ResPlan {
     int V, T, R;
 };
 
-// V: the width for which the busiest SM has least to do.  A block of V bytes costs V bytes of row traffic per gate plus what
-// does not depend on V (program words, instructions; about 4 bytes' worth).
+// V: the width for which the busiest SM has least to do.  A block of V bytes costs V bytes of row traffic per gate plus what does
+// not depend on V (program words, instructions; about 8 bytes' worth).  Measured, us with V = 16 / 8 / 4, 784 -> 4 layers: 8000 wide,
+// 100 samples: 19.5 / 18.3 / 18.0, 4000: 20.0 / 19.1 / 17.7, 10000: 20.0 / 24.0 / 28.7, 2^18: 207 / 255 / 399; 10000 wide, 19000: 38 / 48 / 63;
+// 16000 wide, 5 layers, 10000: - / 46 / 54.
 static ResPlan res_plan(const int64_t *n, int layers, int64_t batch, int64_t k) {
     ResPlan best = {0, 0, 0};
     if (layers < 1 || layers > kResLayers || batch < 1 || k < 1) return best;
@@ -373,7 +378,7 @@ static ResPlan res_plan(const int64_t *n, int layers, int64_t batch, int64_t k) 
         if (widest > (int64_t)R * 1024 || k > (1 << 14) || res_shared_bytes((int)most, V, k) > kResMaxShared) continue;
         const int64_t blocks = ceil_div(batch, 8 * V);
         if (blocks >= ((int64_t)1 << 31)) continue;
-        const int64_t cost = ceil_div(blocks, sms) * (V + 4);
+        const int64_t cost = ceil_div(blocks, sms) * (V + 8);
         if (best.V == 0 || cost < least) {
             least = cost;
             // as many threads as there are rows for when an SM has one block at a time anyway, else several smaller CTAs

@@ -19,7 +19,7 @@ CASES = [([5, 3], 1, 1, 4), ([40, 60, 60], 2, 100, 4), ([784] + 4 * [8000], 10, 
          ([64, 16384, 16384], 2, 33, 4), ([50, 640, 320, 640], 64, 7000, 8), ([100, 10241, 10241], 11, 8 * 64 * 148, 8),
          ([16384, 16384], 1, 40000, 8), ([30, 10240, 10240], 10, 128 * 148 - 127, 16), ([33, 2000, 2000, 999], 999, 20, 4),
          ([70] + 32 * [100], 100, 30001, 16), ([117, 5000, 5120], 16, 50000, 16), ([400, 2560, 2561], 13, 40001, 16),
-         ([20, 12, 300], 300, 25000, 8)]
+         ([20, 12, 300], 300, 25000, 16)]
 
 
 def _network(dims, seed):
