@@ -233,25 +233,41 @@ class LogicLayer(torch.nn.Module):
     def __getstate__(self):
         state = self.__dict__.copy()
         state.pop('_network', None)
+        state.pop('_graph_tensors', None)
         state['_walk'] = None
         return state
 
     def train(self, mode=True):
         # Kernels (an optimizer's, a replayed graph's) write the weights without autograd's version counter noticing; what was
         # derived from the weights in eval mode does not outlive a change of mode.
-        self._gate_cache = self._network = None
+        if mode != self.training:
+            self._gate_cache = self._network = None
         return super().train(mode)
+
+    # What kernels in captured graphs read: a graph holds addresses only, so these tensors stay as long as the layer does (one set
+    # per capture with other weights).
+    _graph_tensors = ()
+
+    def _keep_for_graphs(self, tensor):
+        if not any(t is tensor for t in self._graph_tensors):
+            self._graph_tensors = self._graph_tensors + (tensor,)
 
     def _gate_ids(self):
         """uint8 arg-max gate per neuron, cached until the weights change (their version counter moves, which FlatAdam and
-        TrainStep see to for the updates that their kernels make) or the mode is set."""
+        TrainStep see to for the updates that their kernels make) or the mode does.  A graph captured with cached gates keeps
+        working from those; one captured without computes its own, at every replay."""
         w = self.weights
         key = (w.data_ptr(), w._version)
         cached = getattr(self, '_gate_cache', None)
+        capturing = torch.cuda.is_current_stream_capturing()
         if cached is None or cached[0] != key:
             with torch.no_grad():
-                cached = (key, ops.argmax_gates(w.detach().contiguous()))
-            self._gate_cache = cached
+                gates = ops.argmax_gates(w.detach().contiguous())
+            if capturing:
+                return gates
+            self._gate_cache = cached = (key, gates)
+        if capturing:
+            self._keep_for_graphs(cached[1])
         return cached[1]
 
     def extra_repr(self):

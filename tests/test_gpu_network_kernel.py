@@ -115,3 +115,30 @@ def test_a_graph_keeps_its_own_gates():
             counts = model(D.PackBitsTensor(x))
         graph.replay()
     assert torch.equal(counts, want)
+
+
+def test_a_graph_outlives_the_gates_it_was_captured_with():
+    """eval() again, other weights, an eager pass over them and allocations where freed gates would have been: the graph's counts
+    stay those of the gates at its capture."""
+    torch.manual_seed(5)
+    model = torch.nn.Sequential(D.LogicLayer(64, 320), D.LogicLayer(320, 320), D.GroupSum(10)).eval()
+    x = torch.rand(640, 64, device="cuda") < 0.5
+    with torch.no_grad():
+        want = model(D.PackBitsTensor(x)).clone()
+        graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=stream):
+            counts = model(D.PackBitsTensor(x))
+        for change in range(3):
+            if change == 1:
+                model.train()
+            model.eval()
+            if change == 2:
+                for layer in model[:2]:
+                    layer.weights.copy_(layer.weights.flip(1))
+            for _ in range(3):
+                now = model(D.PackBitsTensor(x))
+            over = [torch.full((320,), 7, dtype=torch.uint8, device="cuda") for _ in range(64)]
+            counts.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(counts, want) and torch.equal(now, want) == (change < 2) and len(over) == 64

@@ -1,0 +1,76 @@
+"""What a LogicLayer derives from its weights and connections and keeps (arg-max gates, the walk, the packed network's program),
+with the kernels replaced by stand-ins: when it is made anew, how long it lives, what a captured graph may rely on."""
+import weakref
+
+import pytest
+import torch
+
+import difflogic_b200 as D
+from difflogic_b200 import ops
+
+
+class _Cuda:
+    """Stand-in for the state of torch.cuda that the code under test asks for."""
+    def __init__(self, monkeypatch):
+        self.capturing = False
+        monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: self.capturing)
+        stream = type("Stream", (), {"synchronize": lambda s: None})()
+        monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: stream)
+        monkeypatch.setattr(torch.cuda, "synchronize", lambda device=None: None)
+
+
+@pytest.fixture
+def cuda(monkeypatch):
+    return _Cuda(monkeypatch)
+
+
+def _layer(n_in=8, n_out=8):
+    return D.LogicLayer(n_in, n_out, device="cpu", implementation="cuda").eval()
+
+
+@pytest.fixture
+def argmax(monkeypatch):
+    made = []
+
+    def gates(w):
+        made.append(w.argmax(-1).to(torch.uint8))
+        return made[-1]
+    monkeypatch.setattr(ops, "argmax_gates", gates)
+    return made
+
+
+def test_gates_stay_while_the_mode_stays(cuda, argmax):
+    layer = _layer()
+    kept = weakref.ref(layer._gate_ids())
+    argmax.clear()
+    layer.eval()
+    assert kept() is not None and layer._gate_ids() is kept() and not argmax
+    layer.train()
+    layer.eval()
+    layer._gate_ids()
+    assert len(argmax) == 1
+
+
+def test_gates_that_a_graph_reads_live_as_long_as_the_layer(cuda, argmax):
+    layer = _layer()
+    layer._gate_ids()
+    cuda.capturing = True
+    read = weakref.ref(layer._gate_ids())
+    cuda.capturing = False
+    argmax.clear()
+    layer.train()
+    layer.eval()
+    with torch.no_grad():
+        layer.weights.add_(1.0)
+    assert layer._gate_ids() is not read() and read() is not None
+    del layer
+    argmax.clear()
+    assert read() is None
+
+
+def test_gates_that_only_a_graph_computes_are_not_used_outside_it(cuda, argmax):
+    layer = _layer()
+    cuda.capturing = True
+    inside = layer._gate_ids()
+    cuda.capturing = False
+    assert layer._gate_ids() is not inside
