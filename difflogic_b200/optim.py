@@ -214,6 +214,7 @@ class FlatAdam(torch.optim.Optimizer):
     def _begin_exchange_step(self):
         self._bucket_pending = [len(b[2]) for b in self._buckets]
         self._bucket_launched = [False] * len(self._buckets)
+        self._bucket_ready = [{} for _ in self._buckets]   # per stream that gradients were queued on: the latest one's event
         self._bucket_done = []          # events: the buckets' exchange kernels of this step
         self._bucket_pushes = [0] * len(self._buckets)   # backward_w kernels of this step that pushed their gradients
 
@@ -247,12 +248,17 @@ class FlatAdam(torch.optim.Optimizer):
 
     def gradient_queued(self, p):
         """The kernel that writes p's gradient is in the current stream's queue: launches the exchange of p's bucket once that
-        holds for all of the bucket's parameters."""
+        holds for all of the bucket's parameters.  Their kernels may be on several streams (a layer's backward_w on
+        TrainStep's side stream, the walk kernel that gives both gradients on the stream of the backward pass)."""
         rank, world = self._exchange
         bi = self._bucket_of[p]
         if not self._bucket_launched[bi]:
             self._bucket_pending[bi] -= 1
-            if self._bucket_pending[bi] <= 0:
+            if self._bucket_pending[bi] > 0:
+                stream, queued = torch.cuda.current_stream(self.flat_param.device), torch.cuda.Event()
+                queued.record(stream)
+                self._bucket_ready[bi][stream.cuda_stream] = queued
+            else:
                 last = sum(self._bucket_launched) == len(self._buckets) - 1
                 if not self._forms_fixed:
                     # One pass for the buckets at the END of the backward pass, as many as fit the byte limit: this bucket
@@ -271,6 +277,7 @@ class FlatAdam(torch.optim.Optimizer):
         beta1, beta2 = g['betas']
         dev = self.flat_param.device
         current = torch.cuda.current_stream(dev)
+        elsewhere = [queued for handle, queued in self._bucket_ready[bi].items() if handle != current.cuda_stream]
         if behind_backward_w:
             stream = current     # the kernel's set-up overlaps the end of the backward_w kernel just before it
         else:
@@ -278,7 +285,9 @@ class FlatAdam(torch.optim.Optimizer):
             ready = torch.cuda.Event()
             ready.record(current)
             stream.wait_event(ready)
-        how = N.LAUNCH_OVERLAP_SETUP if behind_backward_w else N.LAUNCH_PLAIN
+        for queued in elsewhere:
+            stream.wait_event(queued)
+        how = N.LAUNCH_OVERLAP_SETUP if behind_backward_w and not elsewhere else N.LAUNCH_PLAIN
         with torch.cuda.device(dev):
             if bi in self._packet_form:
                 N.check(N.lib().dl_exchange_packets_f32(
