@@ -253,11 +253,11 @@ class LogicLayer(torch.nn.Module):
             self._graph_tensors = self._graph_tensors + (tensor,)
 
     def _gate_ids(self):
-        """uint8 arg-max gate per neuron, cached until the weights change (their version counter moves, which FlatAdam and
-        TrainStep see to for the updates that their kernels make) or the mode does.  A graph captured with cached gates keeps
+        """uint8 arg-max gate per neuron, cached until the weights change (their version counter moves, or the count of
+        updates that FlatAdam and TrainStep keep for those that their kernels make) or the mode does.  A graph captured with cached gates keeps
         working from those; one captured without computes its own, at every replay."""
         w = self.weights
-        key = (w.data_ptr(), w._version)
+        key = (w.data_ptr(), w._version, getattr(w, '_dl_updates', 0))
         cached = getattr(self, '_gate_cache', None)
         capturing = torch.cuda.is_current_stream_capturing()
         if cached is None or cached[0] != key:

@@ -27,6 +27,14 @@ def plan_inboxes(bucket_counts, world):
     return offsets, max(slots, 1)
 
 
+def count_update(params):
+    """Notes an update of `params` by kernels that go past autograd's bookkeeping: what is derived from weights and kept
+    (arg-max gates for packed inference) is kept for this count and the version counter.  The version counter itself stays, as a
+    loss that was computed before an update may be differentiated after it."""
+    for p in params:
+        p._dl_updates = getattr(p, '_dl_updates', 0) + 1
+
+
 class ExchangeUnavailable(RuntimeError):
     """enable_exchange could not map a peer's buffers; raised on EVERY rank of the group, with the optimizer untouched."""
 
@@ -443,9 +451,8 @@ class FlatAdam(torch.optim.Optimizer):
                 N.check(N.lib().dl_prefetch_l2(t.data_ptr(), t.numel() * 4, st))
 
     def mark_updated(self):
-        """Moves the version counters of the parameters: the kernels that update them go past autograd's bookkeeping, and
-        what others have derived from the weights (arg-max gates for packed inference) is kept by version."""
-        torch.autograd.graph.increment_version(self._params)
+        """Tells whoever has derived something from the weights that kernels have updated them (count_update)."""
+        count_update(self._params)
 
     def grad_view(self, p):
         off, n = self._slices[p]

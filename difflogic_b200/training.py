@@ -17,6 +17,8 @@ launch on torch's current stream, allocate nothing themselves and never synchron
 import torch
 import torch.distributed as dist
 
+from .optim import count_update
+
 
 class TrainStep:
     def __init__(self, model, optimizer, loss_fn=None, process_group=None, world_size=None, buckets=2, fuse_head=True,
@@ -229,8 +231,8 @@ class TrainStep:
         return self._static_loss
 
     def _mark_updated(self):
-        """A replayed graph has updated the parameters: their version counters move as they would in an eager step."""
-        torch.autograd.graph.increment_version(self.params)
+        """A replayed graph has updated the parameters."""
+        count_update(self.params)
 
     def capture(self, x, y, warmup=3):
         """Captures the step in a CUDA graph.  `x`, `y` give the shapes; their contents are used for

@@ -52,3 +52,25 @@ def test_gates_follow_the_optimizer(way):
             step(x, y)
     after = _counts(model, xb)
     assert not torch.equal(before, after)
+
+
+@pytest.mark.parametrize("way", ["loop", "captured"])
+def test_an_update_leaves_earlier_graphs_usable(way):
+    """The optimizer's kernels change the weights in place without autograd's version counters: a loss computed before a step can
+    be differentiated after it."""
+    torch.manual_seed(1)
+    model = torch.nn.Sequential(D.LogicLayer(64, 200), D.LogicLayer(200, 200), D.GroupSum(10, 3.0))
+    opt = FlatAdam(model.parameters(), lr=0.01)
+    x, y = (torch.rand(40, 64, device="cuda") < 0.4).float(), torch.randint(0, 10, (40,), device="cuda")
+    step = TrainStep(model, opt).capture(x, y) if way == "captured" else None
+    versions = [p._version for p in model.parameters()]
+    loss = torch.nn.functional.cross_entropy(model(x), y)
+    if way == "loop":
+        loss.backward(retain_graph=True)
+        opt.step()
+    else:
+        step.replay()
+    opt.zero_grad()
+    loss.backward()
+    assert all(p.grad is not None and bool(torch.isfinite(p.grad).all()) for p in model.parameters())
+    assert versions == [p._version for p in model.parameters()]

@@ -74,3 +74,13 @@ def test_gates_that_only_a_graph_computes_are_not_used_outside_it(cuda, argmax):
     inside = layer._gate_ids()
     cuda.capturing = False
     assert layer._gate_ids() is not inside
+
+
+def test_gates_follow_updates_that_autograd_does_not_see(cuda, argmax):
+    from difflogic_b200.optim import count_update
+    layer = _layer()
+    layer._gate_ids()
+    version = layer.weights._version
+    layer.weights.data.copy_(layer.weights.data.flip(1))     # as a kernel does: past the version counter
+    count_update([layer.weights])
+    assert torch.equal(layer._gate_ids(), layer.weights.argmax(-1).to(torch.uint8)) and layer.weights._version == version
