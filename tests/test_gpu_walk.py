@@ -87,3 +87,43 @@ def test_walk_kernels_match_the_layer(case, batch):
 def test_a_bad_connection_gives_no_walk():
     a = torch.tensor([0, 1, 5]).cuda()
     assert ops.build_walk(a, a, 5) is None
+
+
+@pytest.mark.parametrize("batch", [1, 31, 64, 75, 128, 131, 1024, 1027])
+@pytest.mark.parametrize("case", CASES)
+def test_both_routes_give_the_same_bits(case, batch):
+    """A layer may take the walk or the gather kernels from one call to the next: outputs and coefficients are the same to the bit,
+    also where rows hold infinities and NaN.  (The gradients' terms are added in another order.)"""
+    kind, n_in, n_out = case
+    a, b = (t.cuda() for t in _connections(*case))
+    g = torch.Generator().manual_seed(batch + 1)
+    x = torch.rand(n_in, batch, generator=g).cuda()
+    w = torch.randn(n_out, 16, generator=g).cuda()
+    walk = ops.build_walk(a, b, n_in)
+    for special in (None, float("inf"), float("nan")):
+        if special is not None:
+            x[::5, ::3] = special
+        for mode in (ops.W_LOGITS, ops.W_ARGMAX):
+            y, coef = ops.logic_forward_walk(x, w, walk, mode, want_coef=True)
+            y_gather, coef_gather = ops.logic_forward(x, a, b, w, mode, want_coef=True)
+            assert torch.equal(coef, coef_gather) and torch.allclose(y, y_gather, rtol=0, atol=0, equal_nan=True)
+
+
+@pytest.mark.parametrize("batch", [75, 128, 1024])
+def test_weight_gradients_are_as_accurate_along_the_walk(batch):
+    """Their error against 64 bits is not larger than that of the gather kernel's sums (both are a few roundings; 1.5 allows for
+    the difference between two samples of them)."""
+    n = 4000
+    a, b = _square(n, 11)
+    g = torch.Generator().manual_seed(batch)
+    x, w, gy = torch.rand(n, batch, generator=g), torch.randn(n, 16, generator=g), torch.randn(n, batch, generator=g)
+    want = _reference(x, a, b, w, gy, 1.0)[2]
+    xd, wd, gyd, ad, bd = x.cuda(), w.cuda(), gy.cuda(), a.cuda(), b.cuda()
+    walk = ops.build_walk(ad, bd, n)
+    coef = ops.logic_coefs(wd, ops.W_LOGITS)
+
+    def error(got):
+        return float((got.cpu().double() - want).norm() / want.norm())
+    along = error(ops.logic_backward_walk(xd, gyd, coef, wd, walk)[1])
+    gathered = error(ops.logic_backward_w(xd, ad, bd, gyd, wd, ops.W_LOGITS))
+    assert along <= 1.5 * gathered, (along, gathered)
