@@ -137,12 +137,22 @@ class LogicLayer(torch.nn.Module):
         133 / 192; 64000 wide, batch 32: 108 / 128, 64 (two columns of 16 lanes): 133 / 130, 512: 491 / 781."""
         if self.out_dim < 12000 or self.out_dim * batch < 2000000 or 32 < batch <= 64:
             return None
-        walk = getattr(self, '_walk', None)
-        if walk is None and not torch.cuda.is_current_stream_capturing():
-            walk = ops.build_walk(self.indices[0], self.indices[1], self.in_dim) or (None, False)
-            torch.cuda.current_stream(self.indices[0].device).synchronize()    # read ahead of the preceding kernel, as the indices
-            self._walk = walk
-        return walk if walk is not None and walk[0] is not None else None
+        a, b = self.indices
+        kept = old = getattr(self, '_walk', None)
+        if kept is not None and not (kept[0] is a and kept[1] is b and kept[2] == (a._version, b._version)):
+            kept = None      # other connections than those it was built from
+        capturing = torch.cuda.is_current_stream_capturing()
+        if kept is None and not capturing:
+            walk = ops.build_walk(a, b, self.in_dim)
+            torch.cuda.current_stream(a.device).synchronize()    # read ahead of the preceding kernel, as the indices
+            if old is not None:
+                torch.cuda.synchronize(a.device)                 # kernels on other streams may still read the old one
+            self._walk = kept = (a, b, (a._version, b._version), walk)
+        if kept is None or kept[3] is None:
+            return None
+        if capturing:
+            self._keep_for_graphs(kept[3][0])
+        return kept[3]
 
     def set_connections(self, a, b):
         """Replaces the connection indices (e.g. to copy them from another model) and rebuilds the inverse index."""

@@ -127,3 +127,25 @@ def test_weight_gradients_are_as_accurate_along_the_walk(batch):
     along = error(ops.logic_backward_walk(xd, gyd, coef, wd, walk)[1])
     gathered = error(ops.logic_backward_w(xd, ad, bd, gyd, wd, ops.W_LOGITS))
     assert along <= 1.5 * gathered, (along, gathered)
+
+
+def test_edited_connections_are_followed_at_every_batch_size():
+    """In-place writes and assignments of `indices`: the walk (large batches) and the gather kernels (small ones) use the same."""
+    import difflogic_b200 as D
+    torch.manual_seed(2)
+    n = 12000
+    layer = D.LogicLayer(n, n).eval()
+    x = (torch.rand(200, n, device="cuda") < 0.5).float()
+
+    def check():
+        want = ops.logic_forward(x.t().contiguous(), *layer.indices, layer.weights.detach(), ops.W_ARGMAX)[0].t()
+        with torch.no_grad():
+            for _ in range(3):
+                assert torch.equal(layer(x), want) and torch.equal(layer(x[:10]), want[:10])
+    check()
+    layer.indices[0].copy_(layer.indices[0].flip(0))
+    check()
+    layer.indices = (layer.indices[0], layer.indices[1].flip(0).contiguous())
+    check()
+    layer.set_connections(layer.indices[1].clone(), layer.indices[0].clone())
+    check()

@@ -84,3 +84,50 @@ def test_gates_follow_updates_that_autograd_does_not_see(cuda, argmax):
     layer.weights.data.copy_(layer.weights.data.flip(1))     # as a kernel does: past the version counter
     count_update([layer.weights])
     assert torch.equal(layer._gate_ids(), layer.weights.argmax(-1).to(torch.uint8)) and layer.weights._version == version
+
+
+@pytest.fixture
+def walks(monkeypatch):
+    """build_walk keeps what it was built from in place of the entries."""
+    made = []
+
+    def build(a, b, n_in):
+        made.append((torch.stack([a, b]), True))
+        return made[-1]
+    monkeypatch.setattr(ops, "build_walk", build)
+    return made
+
+
+def test_a_walk_is_that_of_the_connections(cuda, walks):
+    layer = _layer(12000, 12000).train()
+
+    def check():
+        assert torch.equal(layer._walk_for(1000)[0], torch.stack(layer.indices))
+    check()
+    check()
+    assert len(walks) == 1
+    layer.indices[0].copy_(layer.indices[0].flip(0))
+    check()
+    layer.indices = (layer.indices[0], layer.indices[1].flip(0))
+    check()
+    layer.indices = tuple(i.clone() for i in layer.indices)
+    check()
+    assert len(walks) == 4
+    layer.set_connections(layer.indices[1], layer.indices[0])
+    check()
+
+
+def test_a_capture_takes_no_walk_of_other_connections(cuda, walks):
+    layer = _layer(12000, 12000).train()
+    cuda.capturing = True
+    assert layer._walk_for(1000) is None          # none yet, and none is built
+    cuda.capturing = False
+    layer._walk_for(1000)
+    cuda.capturing = True
+    walks.clear()
+    entries = weakref.ref(layer._walk_for(1000)[0])
+    layer.indices[0].copy_(layer.indices[0].flip(0))
+    assert layer._walk_for(1000) is None
+    cuda.capturing = False
+    layer._walk_for(1000)
+    assert entries() is not None                  # the graph reads it
