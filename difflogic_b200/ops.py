@@ -7,6 +7,8 @@ library raises (see _native.lib()).
 Layouts: float activations are feature-major `[features, batch]` contiguous; packed
 activations are `[features, words]`; indices are int64, as LogicLayer stores them.
 """
+import collections
+
 import torch
 
 from . import _native as N
@@ -197,11 +199,18 @@ def build_backward_plan(a, b, start, lst):
     return plan
 
 
+class Walk(collections.namedtuple("Walk", "entries complete n_in n_out")):
+    """Walk of a layer's connection graph: entries int32 [n, 2] on the device; complete: it gives grad_x; the layer's rows."""
+    __slots__ = ()
+
+
 def build_walk(a, b, n_in):
-    """Walk of a layer's connection graph for logic_forward_walk / logic_backward_walk: (entries int32 [n, 2] on a's device,
-    complete), or None for sizes or indices it does not take.  Built on the host (dl_build_walk)."""
+    """Walk of a layer's connection graph for logic_forward_walk / logic_backward_walk, or None for sizes or indices it does
+    not take.  Built on the host (dl_build_walk)."""
     import ctypes
     n_out = a.numel()
+    _index(a, "a")
+    _index(b, "b", n_out)
     if n_out == 0 or n_in == 0:
         return None
     ah, bh = a.cpu().contiguous(), b.cpu().contiguous()
@@ -210,7 +219,13 @@ def build_walk(a, b, n_in):
     if N.lib().dl_build_walk(ah.data_ptr(), bh.data_ptr(), int(n_in), n_out, out.data_ptr(), ctypes.addressof(entries),
                              ctypes.addressof(complete)) != N.DL_OK:
         return None
-    return out[:entries.value].to(a.device), bool(complete.value)
+    return Walk(out[:entries.value].to(a.device), bool(complete.value), int(n_in), n_out)
+
+
+def _check_walk(walk, n_in, n_out):
+    """The walk's entries are row numbers: of x and of everything that has a row per neuron."""
+    _need(n_in == walk.n_in, "x has %d rows, the walk's layer reads %d" % (n_in, walk.n_in))
+    _need(n_out == walk.n_out, "w has %d rows, expected %d" % (n_out, walk.n_out))
 
 
 def logic_forward_walk(x, w, walk, w_mode=W_LOGITS, want_coef=False, overlap=False):
@@ -220,6 +235,7 @@ def logic_forward_walk(x, w, walk, w_mode=W_LOGITS, want_coef=False, overlap=Fal
     n_in, batch = x.shape
     n_out = w.shape[0]
     _need(w.shape[1] == 16, "w must be [n_out, 16]")
+    _check_walk(walk, n_in, n_out)
     y = x.new_empty((n_out, batch))
     coef = x.new_empty((n_out, 4)) if want_coef else None
     with N.on_device(x):
@@ -239,6 +255,7 @@ def logic_backward_walk(x, grad_y, coef, w, walk, grad_scale=1.0, want_grad_x=Tr
     n_in, batch = x.shape
     n_out = w.shape[0]
     rows_per_class = int(rows_per_class)
+    _check_walk(walk, n_in, n_out)
     _need(tuple(grad_y.shape) == (n_out // max(rows_per_class, 1), batch), "grad_y does not fit x and w")
     _need(tuple(w.shape) == (n_out, 16) and tuple(coef.shape) == (n_out, 4), "w must be [n_out, 16] and coef [n_out, 4]")
     gx = torch.empty_like(x) if want_grad_x else None

@@ -131,3 +131,49 @@ def test_a_capture_takes_no_walk_of_other_connections(cuda, walks):
     cuda.capturing = False
     layer._walk_for(1000)
     assert entries() is not None                  # the graph reads it
+
+
+class _OnCuda:
+    """What the checks of ops ask of a CUDA tensor, and nothing that could be launched."""
+    is_cuda = True
+
+    def __init__(self, rows, columns, dtype=torch.float32):
+        self.shape, self.dtype = (rows, columns), dtype
+
+    def dim(self):
+        return 2
+
+    def is_contiguous(self):
+        return True
+
+
+def test_walks_are_refused_for_other_rows(monkeypatch):
+    """A walk's entries are row numbers; the gather kernels' index vectors are refused when they do not fit the weights."""
+    from difflogic_b200 import _native
+
+    def launched(*a):
+        raise AssertionError("went on to launch")
+    monkeypatch.setattr(_native, "on_device", launched)
+    monkeypatch.setattr(_OnCuda, "new_empty", lambda self, shape: launched(), raising=False)
+    walk = ops.Walk(None, True, 20, 30)
+    for n_in, n_out in ((20, 29), (20, 31), (19, 30)):
+        x, w, gy, coef = _OnCuda(n_in, 8), _OnCuda(n_out, 16), _OnCuda(n_out, 8), _OnCuda(n_out, 4)
+        with pytest.raises(RuntimeError, match="rows"):
+            ops.logic_forward_walk(x, w, walk)
+        with pytest.raises(RuntimeError, match="rows"):
+            ops.logic_backward_walk(x, gy, coef, w, walk, want_grad_x=False)
+
+
+def test_a_walk_is_built_of_int64_vectors_only():
+    """dl_build_walk reads host copies of them as int64."""
+    class Index(_OnCuda):
+        def dim(self):
+            return 1
+
+        def numel(self):
+            return 4
+
+        def cpu(self):
+            raise AssertionError("went on to build")
+    with pytest.raises(RuntimeError, match="int64"):
+        ops.build_walk(Index(4, 1, torch.int32), Index(4, 1, torch.int32), 4)
