@@ -45,6 +45,9 @@ def _is_cuda_device(device):
         return False
 
 
+_WANTED = object()    # in place of a walk that one call in eval mode has wanted and that is not built yet
+
+
 class LogicLayer(torch.nn.Module):
     """A layer of `out_dim` two-input logic gates, each a learned mix of the 16 possible gates."""
 
@@ -129,7 +132,10 @@ class LogicLayer(torch.nn.Module):
 
     def _walk_for(self, batch):
         """The order in which the walk kernels take the neurons (ops.build_walk), or None where the gather kernels are to be
-        used.  Built on the host by the first call that wants it (not while a graph is being captured: it synchronises).
+        used.  Built on the host (0.2 ms for 16000 neurons, 4 ms for 128000, and copies) by the first training call that wants
+        it, in eval mode by the second -- a model that scores one batch does not wait for it -- and not while a graph is being
+        captured, as it synchronises: a capture without a pass before it records the gather kernels.  Both routes give the
+        same outputs to the bit.
 
         A CTA of the walk kernels takes 64 neurons through the whole batch: narrow layers leave SMs idle, and with few columns
         the walk's longer chain from load to store shows.  Captured step, four layers, walk against gather kernels: 8000 wide,
@@ -138,21 +144,22 @@ class LogicLayer(torch.nn.Module):
         if self.out_dim < 12000 or self.out_dim * batch < 2000000 or 32 < batch <= 64:
             return None
         a, b = self.indices
-        kept = old = getattr(self, '_walk', None)
+        kept = getattr(self, '_walk', None)
         if kept is not None and not (kept[0] is a and kept[1] is b and kept[2] == (a._version, b._version)):
-            kept = None      # other connections than those it was built from
+            kept = None          # other connections than those it was built from
         capturing = torch.cuda.is_current_stream_capturing()
-        if kept is None and not capturing:
-            walk = ops.build_walk(a, b, self.in_dim)
-            torch.cuda.current_stream(a.device).synchronize()    # read ahead of the preceding kernel, as the indices
-            if old is not None:
-                torch.cuda.synchronize(a.device)                 # kernels on other streams may still read the old one
+        if (kept is None or kept[3] is _WANTED) and not capturing:
+            if kept is None and getattr(self, '_walk', None) is not None:
+                torch.cuda.synchronize(a.device)                     # kernels on other streams may still read the old one
+            walk = _WANTED
+            if self.training or kept is not None:
+                walk = ops.build_walk(a, b, self.in_dim)
+                torch.cuda.current_stream(a.device).synchronize()    # read ahead of the preceding kernel, as the indices
             self._walk = kept = (a, b, (a._version, b._version), walk)
-        if kept is None or kept[3] is None:
-            return None
-        if capturing:
-            self._keep_for_graphs(kept[3][0])
-        return kept[3]
+        walk = kept[3] if kept is not None and kept[3] is not _WANTED else None
+        if capturing and walk is not None:
+            self._keep_for_graphs(walk[0])
+        return walk
 
     def set_connections(self, a, b):
         """Replaces the connection indices (e.g. to copy them from another model) and rebuilds the inverse index."""

@@ -177,3 +177,14 @@ def test_a_walk_is_built_of_int64_vectors_only():
             raise AssertionError("went on to build")
     with pytest.raises(RuntimeError, match="int64"):
         ops.build_walk(Index(4, 1, torch.int32), Index(4, 1, torch.int32), 4)
+
+
+def test_one_pass_in_eval_mode_builds_no_walk(cuda, walks):
+    layer = _layer(12000, 12000)
+    assert layer._walk_for(1000) is None and not walks
+    assert layer._walk_for(1000) is not None and len(walks) == 1
+    layer.indices[0].copy_(layer.indices[0].flip(0))         # other connections: from the start again
+    assert layer._walk_for(1000) is None and len(walks) == 1
+    assert layer.train()._walk_for(1000) is not None and len(walks) == 2
+    assert layer.eval()._walk_for(1000) is not None and len(walks) == 2
+    assert layer._walk_for(10) is None
