@@ -309,9 +309,9 @@ void apply_logic_gate_net(bool const *inp, int *out, size_t len) {
             words = ops.eval_packed(words, a, b, gate)
         a, b, gate = self._cuda_plan[-1]
         if ops.eval_groupbitsum_applicable(words, a.numel(), self.num_classes):
-            out = ops.eval_groupbitsum(words, a, b, gate, pad_len, self.num_classes)
+            out = ops.eval_groupbitsum(words, a, b, gate, pad_len, self.num_classes, padded=True)
         else:
-            out = ops.groupbitsum(ops.eval_packed(words, a, b, gate), pad_len, self.num_classes)
+            out = ops.groupbitsum(ops.eval_packed(words, a, b, gate), pad_len, self.num_classes, padded=True)
         return out if on_gpu else out.cpu()
 
     @staticmethod

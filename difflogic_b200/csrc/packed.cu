@@ -300,7 +300,7 @@ using namespace dl;
 // 128: rows counted in units of 16 bytes, whatever the width of the caller's words (rows padded to whole units)
 static int check_bits(const char *who, int bit_count) {
     if (bit_count == 8 || bit_count == 16 || bit_count == 32 || bit_count == 64 || bit_count == 128) return DL_OK;
-    return fail(DL_ERR_BAD_BIT_COUNT, "%s: `bit_count` has to be in { 8, 16, 32, 64 }, got %d", who, bit_count);
+    return fail(DL_ERR_BAD_BIT_COUNT, "%s: `bit_count` has to be in { 8, 16, 32, 64, 128 }, got %d", who, bit_count);
 }
 
 extern "C" DL_API int dl_eval_packed(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, void *y, int64_t n_in,

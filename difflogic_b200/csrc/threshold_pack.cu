@@ -69,7 +69,7 @@ using namespace dl;
 extern "C" DL_API int dl_threshold_packbits_batch_major(const uint8_t *t, const uint8_t *thresholds, int n_thresholds, void *out,
                                                         int64_t n, int64_t batch, int bit_count, void *stream) {
     DL_REQUIRE(bit_count == 8 || bit_count == 16 || bit_count == 32 || bit_count == 64 || bit_count == 128, DL_ERR_BAD_BIT_COUNT,
-               "dl_threshold_packbits_batch_major: `bit_count` has to be in { 8, 16, 32, 64 }, got %d", bit_count);
+               "dl_threshold_packbits_batch_major: `bit_count` has to be in { 8, 16, 32, 64, 128 }, got %d", bit_count);
     DL_REQUIRE(n >= 0 && batch >= 0, DL_ERR_INVALID_ARG, "dl_threshold_packbits_batch_major: negative size");
     DL_REQUIRE(thresholds != nullptr && n_thresholds >= 1 && n_thresholds <= kMaxThresholds, DL_ERR_INVALID_ARG,
                "dl_threshold_packbits_batch_major: between 1 and %d thresholds (a host array)", kMaxThresholds);

@@ -452,21 +452,21 @@ def threshold_packbits_batch_major(t, thresholds, bit_count, padded=False):
     return out, (bit_count - batch % bit_count) % bit_count
 
 
-def _row_units(x, pad_len):
-    """(units, bits per unit) of the rows of x for a count that leaves out their last pad_len samples: its words, or, when
-    whole words are left out (rows padded to 16 bytes), units of 16 bytes."""
+def _row_units(x, padded):
+    """(units, bits per unit) of the rows of x for a count: its words, or units of 16 bytes (rows padded to those)."""
     bits = bits_of(x)
     words = x.shape[1]
-    if pad_len >= bits and words * bits % ROW_UNIT_BITS == 0:
+    if padded and words * bits % ROW_UNIT_BITS == 0:
         return words * bits // ROW_UNIT_BITS, ROW_UNIT_BITS
     return words, bits
 
 
-def groupbitsum(x, pad_len, k):
-    """words [n, W] -> int32 [W*bits - pad_len, k] class counts."""
+def groupbitsum(x, pad_len, k, padded=False):
+    """words [n, W] -> int32 [W*bits - pad_len, k] class counts.  pad_len: samples of the last word that are left out; of the last
+    16 bytes with `padded`."""
     N.require_cuda(x)
     _need(x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D tensor")
-    words, bits = _row_units(x, int(pad_len))
+    words, bits = _row_units(x, padded)
     n = x.shape[0]
     k = int(k)
     if k <= 0 or n % k != 0:
@@ -495,14 +495,14 @@ def eval_groupbitsum_parts_applicable(x, n_out, k):
     return N.lib().dl_eval_groupbitsum_parts_applicable(x.data_ptr(), n_in, int(n_out), words, bits_of(x), int(k)) == 1
 
 
-def eval_groupbitsum(x, a, b, gate, pad_len, k, parts=False):
-    """groupbitsum(eval_packed(x, a, b, gate), pad_len, k) in one kernel; the layer's output is never stored.  parts: classes
-    of more than 2040 gates, counted in parts."""
+def eval_groupbitsum(x, a, b, gate, pad_len, k, parts=False, padded=False):
+    """groupbitsum(eval_packed(x, a, b, gate), pad_len, k, padded) in one kernel; the layer's output is never stored.  parts:
+    classes of more than 2040 gates, counted in parts."""
     N.require_cuda(x, a, b, gate)
     _need(x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D tensor")
     _need(a.dtype == torch.int64 and b.dtype == torch.int64 and gate.dtype == torch.uint8, "a, b int64 and gate uint8")
     _need(a.numel() == b.numel() == gate.numel(), "a, b and gate must have one entry per gate")
-    words, bits = _row_units(x, int(pad_len))
+    words, bits = _row_units(x, padded)
     n_in = x.shape[0]
     n_out, k = a.numel(), int(k)
     if k <= 0 or n_out % k != 0:

@@ -124,6 +124,8 @@ class PackBitsTensor:
 
     def group_sum(self, k):
         assert torch.device(self.device).type == 'cuda', self.device
+        if not 0 <= self.pad_len < self.bit_count:
+            raise RuntimeError('difflogic_b200: pad_len %d out of range' % self.pad_len)
         pad_len = self.pad_len + (self._t.shape[1] - self._words) * self.bit_count
         if self._pending and FUSED_LAST_LAYER:
             batch = self._t.shape[1] * self.bit_count - pad_len
@@ -137,9 +139,9 @@ class PackBitsTensor:
             parts = ops.eval_groupbitsum_parts_applicable(self._t, layer.out_dim, k)
             if parts or ops.eval_groupbitsum_applicable(self._t, layer.out_dim, k):
                 a, b = layer.indices
-                return ops.eval_groupbitsum(self._t, a, b, gate, pad_len, k, parts=parts)
+                return ops.eval_groupbitsum(self._t, a, b, gate, pad_len, k, parts=parts, padded=True)
         self._materialize()
-        return ops.groupbitsum(self._t, pad_len, k)
+        return ops.groupbitsum(self._t, pad_len, k, padded=True)
 
     def flatten(self, start_dim=0, end_dim=-1, **kwargs):
         """Returns the object itself so that torch.nn.Flatten passes it through; arguments are ignored."""
