@@ -196,15 +196,19 @@ bool eval_tma_applicable(const void *x, const void *y, int64_t row_bytes, int64_
     return n_out < ((int64_t)1 << 31) && ceil_div(row_bytes, chunk) * ceil_div(n_out, kMinTileRows) < ((int64_t)1 << 31) - 4096;
 }
 
-template <int ROWS, int STAGES>
+// The kernel's limit of shared memory is set for rows of MAX_CHUNK bytes, the longest that this shape is used for, whatever this
+// launch needs: other threads launch the kernel with other rows.
+template <int ROWS, int STAGES, int MAX_CHUNK>
 static int launch_eval_tma_shape(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, void *y, int64_t n_out,
                                  int64_t row_bytes, int ctas_per_sm, cudaStream_t st, int64_t x_pitch, int64_t y_pitch) {
     const int chunk = (int)(row_bytes < kMaxChunk ? row_bytes : kMaxChunk);
     const int64_t col_chunks = ceil_div(row_bytes, chunk);
     const int64_t row_blocks = ceil_div(n_out, ROWS);
     const int64_t ntiles = col_chunks * row_blocks;
-    const size_t smem = (size_t)STAGES * 2 * ROWS * chunk + 2 * STAGES * sizeof(uint64_t) + STAGES * ROWS;
-    if (cudaFuncSetAttribute(eval_tma_kernel<ROWS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    constexpr size_t kFixed = 2 * STAGES * sizeof(uint64_t) + STAGES * ROWS, kPerByte = (size_t)STAGES * 2 * ROWS;
+    const size_t smem = kPerByte * chunk + kFixed;
+    if (cudaFuncSetAttribute(eval_tma_kernel<ROWS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kPerByte * MAX_CHUNK + kFixed)) !=
+        cudaSuccess)
         return launch_status("dl_eval_packed (shared memory opt-in)");
     const int64_t slots = (int64_t)sm_count() * ctas_per_sm;
     const unsigned grid = (unsigned)(ntiles < slots ? ntiles : slots);
@@ -225,11 +229,11 @@ int launch_eval_tma(const void *x, const int64_t *a, const int64_t *b, const uin
     constexpr int64_t kFiveStages = 1376, kEightStages = 860;  // bytes of a row for which 5 and 8 stages take 108 KB
     const bool wide = force == 1 ? true : force == 2 ? false : (n_out >= 2 * n_in || few_tiles || chunk <= kFiveStages);
     if (wide && chunk <= kEightStages)
-        return launch_eval_tma_shape<8, 8>(x, a, b, gate, y, n_out, row_bytes, 2, st, x_pitch, y_pitch);
+        return launch_eval_tma_shape<8, 8, kEightStages>(x, a, b, gate, y, n_out, row_bytes, 2, st, x_pitch, y_pitch);
     if (wide && chunk <= kFiveStages)
-        return launch_eval_tma_shape<8, 5>(x, a, b, gate, y, n_out, row_bytes, 2, st, x_pitch, y_pitch);
-    if (wide) return launch_eval_tma_shape<8, 3>(x, a, b, gate, y, n_out, row_bytes, 2, st, x_pitch, y_pitch);
-    return launch_eval_tma_shape<16, 2>(x, a, b, gate, y, n_out, row_bytes, 1, st, x_pitch, y_pitch);
+        return launch_eval_tma_shape<8, 5, kFiveStages>(x, a, b, gate, y, n_out, row_bytes, 2, st, x_pitch, y_pitch);
+    if (wide) return launch_eval_tma_shape<8, 3, kMaxChunk>(x, a, b, gate, y, n_out, row_bytes, 2, st, x_pitch, y_pitch);
+    return launch_eval_tma_shape<16, 2, kMaxChunk>(x, a, b, gate, y, n_out, row_bytes, 1, st, x_pitch, y_pitch);
 }
 
 }  // namespace dl

@@ -183,8 +183,9 @@ int launch_forward_tma(bool overlap, const float *x, const int64_t *a, const int
     const int chunk = (int)(row_bytes < kFwMaxChunk ? row_bytes : kFwMaxChunk);
     const int64_t row_blocks = ceil_div(n_out, kFwRows);
     const int64_t ntiles = ceil_div(row_bytes, chunk) * row_blocks;
-    const size_t smem = (size_t)kFwStages * 2 * kFwRows * chunk + 2 * kFwStages * sizeof(uint64_t);
-    if (cudaFuncSetAttribute(forward_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    const auto shared_bytes = [](int row) { return (size_t)kFwStages * 2 * kFwRows * row + 2 * kFwStages * sizeof(uint64_t); };
+    const size_t smem = shared_bytes(chunk);
+    if (cudaFuncSetAttribute(forward_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared_bytes(kFwMaxChunk)) != cudaSuccess)
         return launch_status("dl_forward_f32 (shared memory opt-in)");
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

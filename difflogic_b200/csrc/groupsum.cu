@@ -653,12 +653,14 @@ extern "C" DL_API int dl_class_sums_cross_entropy_f32(const float *class_sums, c
     const int64_t colblocks = ceil_div(batch, kGsCols);
     DL_REQUIRE(colblocks <= INT32_MAX && k <= 65535, DL_ERR_TOO_LARGE, "dl_class_sums_cross_entropy_f32: batch or k too large");
     constexpr int kSmallClasses = 16, kSmallPieces = 2;
-    const size_t small_smem = (size_t)k * kCsGroups * kGsCols * sizeof(float);
+    constexpr size_t kPerClass = kCsGroups * kGsCols * sizeof(float);
+    const size_t small_smem = (size_t)k * kPerClass;
     const int64_t pieces = ceil_div(n / k, rows_per_run) + 1;  // runs that can hold rows of one class
     if (colblocks == 1 && k <= kSmallClasses && pieces <= kSmallPieces * kCsGroups * kCsCluster) {
         // one cluster does it all, nothing but the results touches global memory
         auto kernel = class_sums_ce_cluster_kernel<kSmallClasses, kSmallPieces>;
-        if (small_smem > 32 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem) != cudaSuccess)
+        if (small_smem > 32 * 1024 &&
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmallClasses * kPerClass)) != cudaSuccess)
             return launch_status("dl_class_sums_cross_entropy_f32 (shared memory opt-in)");
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kCsCluster);

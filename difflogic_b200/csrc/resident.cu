@@ -395,7 +395,8 @@ static int launch_resident(const void *x, int64_t row_bytes, const uint32_t *pro
                            int64_t batch, int64_t k, int row_slots, cudaStream_t st) {
     constexpr int V = 4 * WORDS;
     const size_t smem = res_shared_bytes(row_slots, V, k);
-    if (cudaFuncSetAttribute(resident_kernel<WORDS, T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    // the most there may be, not this launch's bytes: the limit is the kernel's, and other threads launch it for other networks
+    if (cudaFuncSetAttribute(resident_kernel<WORDS, T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResMaxShared) != cudaSuccess)
         return launch_status("dl_eval_network (shared memory opt-in)");
     resident_kernel<WORDS, T, R><<<(unsigned)ceil_div(batch, 8 * V), T, smem, st>>>(
         reinterpret_cast<const uint8_t *>(x), row_bytes, prog, sz, out, rows_out, batch, (int)k, (int)(sz.n[sz.layers] / k), row_slots);
@@ -444,7 +445,7 @@ extern "C" DL_API int dl_network_program(const int64_t *const *a, const int64_t 
     }
     uint32_t *at = program, *order = program + (total - n[layers]), *scratch = program + total;
     auto kernel = res_classes(n, layers) == 8 ? resident_program_kernel<8> : resident_program_kernel<16>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(widest * sizeof(uint2))) != cudaSuccess)
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kResRows * sizeof(uint2))) != cudaSuccess)
         return launch_status("dl_network_program (shared memory opt-in)");
     for (int l = 1; l <= layers; ++l) {
         const uint32_t *slot_in = l == 1 ? nullptr : scratch + (int64_t)(l % 2) * widest;

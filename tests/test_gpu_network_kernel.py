@@ -104,6 +104,33 @@ def test_programs_follow_the_network():
     check(first)
 
 
+def test_two_threads_with_networks_of_different_size():
+    """Launches of one kernel with little and with much shared memory, from two threads at once: the limit that a launch sets is
+    enough for the other's."""
+    import threading
+    failures = []
+
+    def work(dims, k, batch):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                layers = [tuple(t.cuda() for t in layer) for layer in _network(dims, batch)]
+                x = torch.randint(-2 ** 63, 2 ** 63 - 1, (dims[0], 2), generator=torch.Generator().manual_seed(1)).cuda()
+                network = ops.NetworkProgram(dims[0], layers)
+                want = ops.eval_network(x, network, batch, k)
+                for i in range(3000):
+                    got = ops.eval_network(x, network, batch, k)
+                    if i % 100 == 0:
+                        assert torch.equal(got, want) and ops.NetworkProgram(dims[0], layers).program.numel() > 0
+        except Exception as e:
+            failures.append(e)
+    threads = [threading.Thread(target=work, args=args) for args in (([64, 16384, 16384], 2, 33), ([40, 60, 60], 2, 100))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
+
+
 def test_a_graph_keeps_its_own_gates():
     torch.manual_seed(4)
     model = torch.nn.Sequential(D.LogicLayer(64, 320), D.LogicLayer(320, 320), D.GroupSum(10)).eval()
