@@ -144,8 +144,11 @@ class LogicLayer(torch.nn.Module):
         if self.out_dim < 12000 or self.out_dim * batch < 2000000 or 32 < batch <= 64:
             return None
         a, b = self.indices
+        versions = ops.versions(a, b)
+        if versions is None:
+            return None
         kept = getattr(self, '_walk', None)
-        if kept is not None and not (kept[0] is a and kept[1] is b and kept[2] == (a._version, b._version)):
+        if kept is not None and not (kept[0] is a and kept[1] is b and kept[2] == versions):
             kept = None          # other connections than those it was built from
         capturing = torch.cuda.is_current_stream_capturing()
         if (kept is None or kept[3] is _WANTED) and not capturing:
@@ -155,7 +158,7 @@ class LogicLayer(torch.nn.Module):
             if self.training or kept is not None:
                 walk = ops.build_walk(a, b, self.in_dim)
                 torch.cuda.current_stream(a.device).synchronize()    # read ahead of the preceding kernel, as the indices
-            self._walk = kept = (a, b, (a._version, b._version), walk)
+            self._walk = kept = (a, b, versions, walk)
         walk = kept[3] if kept is not None and kept[3] is not _WANTED else None
         if capturing and walk is not None:
             self._keep_for_graphs(walk[0])

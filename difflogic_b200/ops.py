@@ -199,6 +199,12 @@ def build_backward_plan(a, b, start, lst):
     return plan
 
 
+def versions(*tensors):
+    """Version counters of tensors that something is derived from and kept, or None when one of them has none (tensors made in
+    inference mode): in-place writes to them go unnoticed, and nothing may be kept."""
+    return None if any(t.is_inference() for t in tensors) else tuple(t._version for t in tensors)
+
+
 class Walk(collections.namedtuple("Walk", "entries complete n_in n_out")):
     """Walk of a layer's connection graph: entries int32 [n, 2] on the device; complete: it gives grad_x; the layer's rows."""
     __slots__ = ()
@@ -524,7 +530,7 @@ class NetworkProgram:
 
     def __init__(self, n_in, layers):
         import ctypes
-        self.layers = [(a, b, gate, a._version, b._version) for a, b, gate in layers]
+        self.layers = [(a, b, gate, versions(a, b)) for a, b, gate in layers]
         count = len(layers)
         self.sizes = network_sizes(n_in, layers)
         device = layers[0][2].device
@@ -543,7 +549,7 @@ class NetworkProgram:
 
     def matches(self, layers):
         return len(layers) == len(self.layers) and all(
-            a is p[0] and b is p[1] and gate is p[2] and a._version == p[3] and b._version == p[4]
+            a is p[0] and b is p[1] and gate is p[2] and None is not versions(a, b) == p[3]
             for (a, b, gate), p in zip(layers, self.layers))
 
 

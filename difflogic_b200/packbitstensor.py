@@ -104,7 +104,7 @@ class PackBitsTensor:
         if not ops.eval_network_applicable(self._t, sizes, batch, k) or torch.cuda.is_current_stream_capturing():
             return None
         if network is None:
-            if any(t.device != self._t.device for layer in layers for t in layer):
+            if any(t.device != self._t.device for layer in layers for t in layer) or any(ops.versions(a, b) is None for a, b, _ in layers):
                 return None
             last._network = None      # given back before the next one is made
             network = last._network = ops.NetworkProgram(self._t.shape[0], layers)

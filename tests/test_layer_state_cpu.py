@@ -188,3 +188,21 @@ def test_one_pass_in_eval_mode_builds_no_walk(cuda, walks):
     assert layer.train()._walk_for(1000) is not None and len(walks) == 2
     assert layer.eval()._walk_for(1000) is not None and len(walks) == 2
     assert layer._walk_for(10) is None
+
+
+def test_connections_made_in_inference_mode(cuda, walks, argmax, monkeypatch):
+    """They have no version counter, so that nothing is kept for them: a layer of such connections (a model moved to the GPU in
+    inference mode) runs the kernels that read them on every call."""
+    with torch.inference_mode():
+        layer = _layer(12000, 12000)
+        layer.indices = tuple(i.clone() for i in layer.indices)
+    for mode in (layer.eval, layer.train, layer.eval):
+        mode()
+        for _ in range(3):
+            assert layer._walk_for(1000) is None and not walks
+    monkeypatch.setattr(ops, "eval_network_applicable", lambda x, sizes, batch, k: True)
+    monkeypatch.setattr(ops, "eval_packed", lambda x, a, b, gate: x[a] & x[b])
+    for _ in range(3):
+        packed = D.PackBitsTensor.from_packed(torch.ones(12000, 2, dtype=torch.int32), 0)
+        packed._pending = [(layer, torch.zeros(12000, dtype=torch.uint8))] * 2
+        assert packed.t.shape == (12000, 2)
