@@ -21,6 +21,7 @@
 // before it (the carried gradient term) it recomputes from that step's operands: two extra row loads per chunk.
 #include <stdlib.h>
 
+#include <new>
 #include <vector>
 
 #include "adam_math.cuh"
@@ -436,8 +437,7 @@ using namespace dl;
 // neurons, so that the walk passes every input row exactly once (grad_x can be formed along it).
 extern "C" DL_API int64_t dl_walk_capacity(int64_t n_in, int64_t n_out) { return n_in + 3 * n_out + 1; }
 
-extern "C" DL_API int dl_build_walk(const int64_t *a, const int64_t *b, int64_t n_in, int64_t n_out, int32_t *out, int64_t *entries,
-                                    int *complete) {
+static int build_walk(const int64_t *a, const int64_t *b, int64_t n_in, int64_t n_out, int32_t *out, int64_t *entries, int *complete) {
     DL_REQUIRE(n_in > 0 && n_out > 0 && a && b && out && entries && complete, DL_ERR_INVALID_ARG, "dl_build_walk: null pointer or size");
     DL_REQUIRE(n_in < ((int64_t)1 << 30) && n_out < ((int64_t)1 << 28), DL_ERR_TOO_LARGE, "dl_build_walk: too many rows");
     struct Ends {
@@ -537,6 +537,15 @@ extern "C" DL_API int dl_build_walk(const int64_t *a, const int64_t *b, int64_t 
     *entries = n;
     *complete = 0;
     return DL_OK;
+}
+
+extern "C" DL_API int dl_build_walk(const int64_t *a, const int64_t *b, int64_t n_in, int64_t n_out, int32_t *out, int64_t *entries,
+                                    int *complete) {
+    try {
+        return build_walk(a, b, n_in, n_out, out, entries, complete);
+    } catch (const std::bad_alloc &) {  // callers are C
+        return fail(DL_ERR_TOO_LARGE, "dl_build_walk: no host memory for %lld inputs and %lld neurons", (long long)n_in, (long long)n_out);
+    }
 }
 
 static int walk_checks(const char *who, const int32_t *walk, int64_t entries, int64_t n_in, int64_t n_out, int64_t batch) {

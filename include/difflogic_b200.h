@@ -166,7 +166,7 @@ DL_API int dl_build_backward_plan(const int64_t *a, const int64_t *b, const int6
  * int32; *entries of them are written: {node << 1 | store, neuron << 2 | flip << 1 | emit} or {node << 1 | store, -1}.
  * *complete = 1 when no input feeds more than two neurons (square layers with random connections): the walk then passes
  * every input row once and grad_x can be formed along it.
- * An index outside its range is refused (DL_ERR_INVALID_ARG).
+ * An index outside its range is refused (DL_ERR_INVALID_ARG); DL_ERR_TOO_LARGE also when host memory runs out.
  * ---------------------------------------------------------------------------------------- */
 DL_API int64_t dl_walk_capacity(int64_t n_in, int64_t n_out);
 DL_API int dl_build_walk(const int64_t *a, const int64_t *b, int64_t n_in, int64_t n_out, int32_t *out, int64_t *entries, int *complete);

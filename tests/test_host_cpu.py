@@ -163,3 +163,20 @@ def test_packet_inbox_plan_gives_every_bucket_its_own_slots():
             assert len(seen) == len(range(0, n4, max(1, n4 // 97)))
         assert stride >= end
     assert plan_inboxes([], 4) == ([], 1)
+
+
+def test_the_walk_builder_reports_that_memory_ran_out(lib):
+    """An exception must not leave a C entry: 2^30 - 1 inputs want 4 GB of host memory, in a process that may have less."""
+    import subprocess
+    import sys
+    code = """
+import ctypes, resource, sys
+lib = ctypes.CDLL(sys.argv[1])
+lib.dl_last_error_string.restype = ctypes.c_char_p
+resource.setrlimit(resource.RLIMIT_AS, (2 << 30, 2 << 30))
+index, out, entries, complete = (ctypes.c_int64 * 1)(0), (ctypes.c_int32 * 16)(), ctypes.c_int64(), ctypes.c_int()
+status = lib.dl_build_walk(index, index, ctypes.c_int64((1 << 30) - 1), ctypes.c_int64(1), out, ctypes.byref(entries), ctypes.byref(complete))
+assert status == %d and b"memory" in lib.dl_last_error_string(), status
+""" % _native.DL_ERR_TOO_LARGE
+    done = subprocess.run([sys.executable, "-c", code, _native.library_path()], capture_output=True, text=True)
+    assert done.returncode == 0, done.stderr
