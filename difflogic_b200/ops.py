@@ -526,26 +526,39 @@ def eval_groupbitsum(x, a, b, gate, pad_len, k, parts=False, padded=False):
 class NetworkProgram:
     """What dl_eval_network needs of a network: its row counts and its program (dl_network_program), built from the layers'
     connections and arg-max gates.  `layers`: (a, b, gate) of every layer, in order; they are kept, so that `matches` can
-    tell a network by its tensors."""
+    tell a network by its tensors.  build=False leaves the program to a later build()."""
 
-    def __init__(self, n_in, layers):
-        import ctypes
+    def __init__(self, n_in, layers, build=True):
         self.layers = [(a, b, gate, versions(a, b)) for a, b, gate in layers]
-        count = len(layers)
         self.sizes = network_sizes(n_in, layers)
-        device = layers[0][2].device
+        self.program = None
         for a, b, gate in layers:
             _index(a, "a", gate.numel())
             _index(b, "b", gate.numel())
-        self.program = torch.empty(N.lib().dl_network_program_words(self.sizes, count), dtype=torch.int32, device=device)
-        pointers = [(ctypes.c_void_p * count)(*[t.data_ptr() for t in column]) for column in zip(*layers)]
+        if build:
+            self.build()
+        else:   # the gates are in this stream's queue; build() may be called on another one
+            with N.on_device(layers[0][2]):
+                self.gates_ready = torch.cuda.current_stream().record_event()
+
+    gates_ready = None
+
+    def build(self):
+        import ctypes
+        count = len(self.layers)
+        device = self.layers[0][2].device
+        program = torch.empty(N.lib().dl_network_program_words(self.sizes, count), dtype=torch.int32, device=device)
+        pointers = [(ctypes.c_void_p * count)(*[layer[i].data_ptr() for layer in self.layers]) for i in range(3)]
         with torch.cuda.device(device):
             stream = torch.cuda.current_stream(device)
-            N.check(N.lib().dl_network_program(pointers[0], pointers[1], pointers[2], self.sizes, count, self.program.data_ptr(),
+            if self.gates_ready is not None:
+                stream.wait_event(self.gates_ready)
+            N.check(N.lib().dl_network_program(pointers[0], pointers[1], pointers[2], self.sizes, count, program.data_ptr(),
                                                stream.cuda_stream))
             # other threads and streams may take it from here on
             stream.synchronize()
-        self.stream = stream.cuda_stream
+        program._dl_stream = stream.cuda_stream
+        self.program = program
 
     def matches(self, layers):
         return len(layers) == len(self.layers) and all(
@@ -569,8 +582,8 @@ def eval_network(x, network, batch, k=None):
     """All layers of a NetworkProgram on packed words x in one kernel: int32 [batch, k] class counts, or without k the last
     layer's rows as packed words."""
     _need(x.is_cuda and x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D CUDA tensor")
-    sizes, words = network.sizes, x.shape[1]
-    _need(x.shape[0] == sizes[0] and x.device == network.program.device, "x does not fit the network")
+    sizes, program, words = network.sizes, network.program, x.shape[1]     # another thread may build the same program once more
+    _need(x.shape[0] == sizes[0] and x.device == program.device, "x does not fit the network")
     row_bytes = words * (bits_of(x) // 8)
     if k is None:
         out = torch.empty((sizes[len(sizes) - 1], words), dtype=x.dtype, device=x.device)
@@ -578,9 +591,9 @@ def eval_network(x, network, batch, k=None):
         out = torch.empty((int(batch), int(k)), dtype=torch.int32, device=x.device)
     with N.on_device(x):
         stream = N.stream_of(x)
-        if stream != network.stream:
-            network.program.record_stream(torch.cuda.current_stream(x.device))
-        N.check(N.lib().dl_eval_network(x.data_ptr(), network.program.data_ptr(), sizes, len(sizes) - 1,
+        if stream != program._dl_stream:
+            program.record_stream(torch.cuda.current_stream(x.device))
+        N.check(N.lib().dl_eval_network(x.data_ptr(), program.data_ptr(), sizes, len(sizes) - 1,
                                         0 if k is None else out.data_ptr(), out.data_ptr() if k is None else 0, row_bytes, int(batch),
                                         1 if k is None else int(k), stream))
     return out

@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 def _counts(model, xb):
     model.eval()
     with torch.no_grad():
-        counts = model(D.PackBitsTensor(xb, bit_count=32))
+        counts = model(D.PackBitsTensor(xb, bit_count=32))                            # by single layers
+        assert torch.equal(model(D.PackBitsTensor(xb, bit_count=32)), counts)         # in one kernel
     # the same network from scratch: nothing remembered
     fresh = [(l.weights.detach().argmax(1), l.indices) for l in model if isinstance(l, D.LogicLayer)]
     h = xb

@@ -80,6 +80,7 @@ def test_programs_follow_the_network():
         h = x.cpu().numpy()
         with torch.no_grad():
             counts = model(D.PackBitsTensor(x))
+            assert torch.equal(model(D.PackBitsTensor(x)), counts)
             packed = D.PackBitsTensor(x)
             for layer in layers:
                 packed = layer(packed)

@@ -14,7 +14,7 @@ class _Cuda:
     def __init__(self, monkeypatch):
         self.capturing = False
         monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: self.capturing)
-        stream = type("Stream", (), {"synchronize": lambda s: None})()
+        stream = type("Stream", (), {"synchronize": lambda s: None, "record_event": lambda s: "event"})()
         monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: stream)
         monkeypatch.setattr(torch.cuda, "synchronize", lambda device=None: None)
 
@@ -206,3 +206,52 @@ def test_connections_made_in_inference_mode(cuda, walks, argmax, monkeypatch):
         packed = D.PackBitsTensor.from_packed(torch.ones(12000, 2, dtype=torch.int32), 0)
         packed._pending = [(layer, torch.zeros(12000, dtype=torch.uint8))] * 2
         assert packed.t.shape == (12000, 2)
+
+
+def test_a_program_is_built_for_the_second_pass(cuda, argmax, monkeypatch):
+    """A batch by single layers takes less time than building the program: one pass over a set of weights builds none."""
+    built, single = [], []
+
+    def build(network):
+        built.append(network)
+        assert network.gates_ready == "event"
+        network.program = torch.zeros(1)
+    monkeypatch.setattr(ops, "_index", lambda t, name, n=None: None)
+    monkeypatch.setattr(ops.N, "on_device", lambda t: ops.N._ALREADY_THERE)
+    monkeypatch.setattr(ops.NetworkProgram, "build", build)
+    monkeypatch.setattr(ops, "eval_network_applicable", lambda x, sizes, batch, k: True)
+    monkeypatch.setattr(ops, "eval_network", lambda x, network, batch, k=None: x if k is None else "counts")
+    monkeypatch.setattr(ops, "eval_groupbitsum_parts_applicable", lambda x, n_out, k: False)
+    monkeypatch.setattr(ops, "eval_groupbitsum_applicable", lambda x, n_out, k: False)
+    monkeypatch.setattr(ops, "groupbitsum", lambda x, pad_len, k, padded: "counts")
+
+    def eval_packed(x, a, b, gate):
+        single.append(gate)
+        return x
+    monkeypatch.setattr(ops, "eval_packed", eval_packed)
+    layers = [_layer() for _ in range(4)]
+
+    def passes(model, *, rows=False):
+        """(layers run one by one, programs built) in one pass."""
+        del built[:], single[:]
+        packed = D.PackBitsTensor.from_packed(torch.ones(8, 2, dtype=torch.int32), 0)
+        for layer in model:
+            packed._push_layer(layer)
+        assert packed.t is not None if rows else packed.group_sum(2) == "counts"
+        return len(single), len(built)
+
+    for rows in (False, True):
+        for layer in layers:
+            layer.train()
+            layer.eval()
+        assert [passes(layers, rows=rows) for _ in range(3)] == [(4, 0), (0, 1), (0, 0)]
+        with torch.no_grad():
+            layers[1].weights.add_(1.0)
+        assert [passes(layers, rows=rows) for _ in range(3)] == [(4, 0), (0, 1), (0, 0)]
+        layers[2].indices[0].copy_(layers[2].indices[0].flip(0))
+        assert [passes(layers, rows=rows) for _ in range(3)] == [(4, 0), (0, 1), (0, 0)]
+        cuda.capturing = True
+        assert passes(layers, rows=rows) == (4, 0)
+        cuda.capturing = False
+        assert passes(layers, rows=rows) == (0, 0)
+    assert layers[2]._network is None                     # nothing is noted for a part of the network
