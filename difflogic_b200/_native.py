@@ -147,7 +147,7 @@ class tuning:
 
 
 def check_status(status):
-    """check() for entry points that launch nothing."""
+    """check() for entry points that launch nothing, or nothing that a pass repeats (the program of a network)."""
     global _launches
     check(status)
     _launches -= 1

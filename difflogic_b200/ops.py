@@ -529,7 +529,7 @@ class NetworkProgram:
     tell a network by its tensors.  build=False leaves the program to a later build()."""
 
     def __init__(self, n_in, layers, build=True):
-        self.layers = [(a, b, gate, versions(a, b)) for a, b, gate in layers]
+        self.layers = [(a, b, gate) + (versions(a, b) or (None, None)) for a, b, gate in layers]
         self.sizes = network_sizes(n_in, layers)
         self.program = None
         for a, b, gate in layers:
@@ -553,8 +553,8 @@ class NetworkProgram:
             stream = torch.cuda.current_stream(device)
             if self.gates_ready is not None:
                 stream.wait_event(self.gates_ready)
-            N.check(N.lib().dl_network_program(pointers[0], pointers[1], pointers[2], self.sizes, count, program.data_ptr(),
-                                               stream.cuda_stream))
+            N.check_status(N.lib().dl_network_program(pointers[0], pointers[1], pointers[2], self.sizes, count, program.data_ptr(),
+                                                      stream.cuda_stream))
             # other threads and streams may take it from here on
             stream.synchronize()
         program._dl_stream = stream.cuda_stream
@@ -562,7 +562,7 @@ class NetworkProgram:
 
     def matches(self, layers):
         return len(layers) == len(self.layers) and all(
-            a is p[0] and b is p[1] and gate is p[2] and None is not versions(a, b) == p[3]
+            a is p[0] and b is p[1] and gate is p[2] and p[3] is not None and a._version == p[3] and b._version == p[4]
             for (a, b, gate), p in zip(layers, self.layers))
 
 
