@@ -412,7 +412,8 @@ walk_backward_kernel(const float *__restrict__ x, const float *__restrict__ gy, 
 // ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
-// Lanes per row, warps side by side over the columns, column blocks of 4 * G.  As many warps as there are column blocks
+// Lanes per row (16 lanes, for the rows of 33 .. 64 columns that layers leave to the gather kernels, are not built), warps side by side
+// over the columns, column blocks of 4 * G.  As many warps as there are column blocks
 // (a power of two, at most 8) share a chunk unless that leaves more than a quarter of them idle.
 struct WalkShape {
     int G, wc, ncb;
@@ -420,7 +421,7 @@ struct WalkShape {
 static WalkShape walk_shape(int64_t batch) {
     const int64_t lanes = ceil_div(batch, 4);
     WalkShape s;
-    s.G = lanes <= 8 ? 8 : lanes <= 16 ? 16 : 32;
+    s.G = lanes <= 8 ? 8 : 32;
     s.ncb = (int)ceil_div(batch, 4 * s.G);
     s.wc = kWalkWarps;
     while (s.wc > 1 && ceil_div(s.ncb, s.wc) * s.wc * 4 > (int64_t)s.ncb * 5) s.wc /= 2;
@@ -574,7 +575,7 @@ extern "C" DL_API int dl_forward_walk_f32(const float *x, const float *w, int w_
         else launch_dependent(overlap, walk_forward_kernel<GG, false>, grid, dim3(kThreads), 0, as_stream(stream), x, w, w_mode, y, c4,    \
                               wk, (int)entries, batch, s.wc, s.ncb);                                                                  \
         break;
-    switch (s.G) { DL_WF(8) DL_WF(16) DL_WF(32) }
+    switch (s.G) { DL_WF(8) DL_WF(32) }
 #undef DL_WF
     return launch_status("dl_forward_walk_f32");
 }
@@ -608,7 +609,7 @@ extern "C" DL_API int dl_backward_walk_f32(const float *x, const float *grad_y, 
         if (grad_x != nullptr) vec ? launch(walk_backward_kernel<GG, true, true>) : launch(walk_backward_kernel<GG, false, true>); \
         else vec ? launch(walk_backward_kernel<GG, true, false>) : launch(walk_backward_kernel<GG, false, false>);       \
         break;
-    switch (s.G) { DL_WB(8) DL_WB(16) DL_WB(32) }
+    switch (s.G) { DL_WB(8) DL_WB(32) }
 #undef DL_WB
     return launch_status(who);
 }
