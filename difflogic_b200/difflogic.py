@@ -45,6 +45,33 @@ def _is_cuda_device(device):
         return False
 
 
+def _walk_pays(width, batch, training):
+    """Whether a layer of `width` neurons takes less time by the walk kernels than by the gather kernels.
+
+    A CTA of the walk kernels takes 64 neurons (256 where rows have up to 32 columns) through the whole batch, and 296 CTAs of the
+    backward kernel run at a time: narrow layers leave SMs idle, and so does a second round of few CTAs.  Rows of 65 to 96 columns
+    leave lanes idle, which the gather kernels spread more finely, and with few columns the walk's longer chain from load to store
+    shows.  Rows that are not whole 16-byte units are read value by value by the gather kernels, 1.15 to 2.4 times as slow.
+
+    Measured with four layers, walk / gather kernels, us.  Captured training step: 8000 wide, 256 columns: 80 / 73, 2048: 396 / 391;
+    16000, 64: 77 / 65, 128: 77 / 80, 512: 167 / 218; 64000, 64: 149 / 151, 80: 205 / 199, 96: 207 / 207, 100: 212 / 230; 128000, 68:
+    359 / 364; second round (18945 neurons on): 19000, 128: 104 / 94, 192: 142 / 135, 256: 141 / 139; 22500, 128: 112 / 107, 192: 153 / 156;
+    28000, 128: 116 / 118; up to 32 columns (75777 neurons on): 64000, 32: 120 / 124; 78000, 32: 175 / 156; 112000, 24: 191 / 178, 32: 194 /
+    195; 128000, 24: 201 / 200, 28: 206 / 215.  Forward passes: 12000, 1000: 84 / 88, 1280: 121 / 104, 4096: 318 / 304; 14000, 1200: 131 / 121;
+    16000, 1280: 135 / 134, 2048: 189 / 207; 128000, 16: 39 / 37, 20: 41 / 47."""
+    if width < 12000 or width * batch < 2000000 or 32 < batch <= 64:
+        return False
+    if batch % 4 != 0:
+        return True
+    if not training:
+        return batch >= 20 and (batch <= 1024 or width >= 16000)
+    if batch <= 32:
+        return batch >= 28 and not 75776 < width < 112000
+    if batch <= 96:
+        return width >= 96000
+    return batch > 192 or not 18944 < width < (28000 if batch <= 128 else 22500)
+
+
 _WANTED = object()    # in place of a walk that one call in eval mode has wanted and that is not built yet
 
 
@@ -135,13 +162,8 @@ class LogicLayer(torch.nn.Module):
         used.  Built on the host (0.2 ms for 16000 neurons, 4 ms for 128000, and copies) by the first training call that wants
         it, in eval mode by the second -- a model that scores one batch does not wait for it -- and not while a graph is being
         captured, as it synchronises: a capture without a pass before it records the gather kernels.  Both routes give the
-        same outputs to the bit.
-
-        A CTA of the walk kernels takes 64 neurons through the whole batch: narrow layers leave SMs idle, and with few columns
-        the walk's longer chain from load to store shows.  Captured step, four layers, walk against gather kernels: 8000 wide,
-        batch 256: 68 / 64 us, 2048: 338 / 340; 4000 wide, batch 2048: 279 / 175; 16000 wide, batch 64: 67 / 56, 128: 65 / 67, 512:
-        133 / 192; 64000 wide, batch 32: 108 / 128, 64 (two columns of 16 lanes): 133 / 130, 512: 491 / 781."""
-        if self.out_dim < 12000 or self.out_dim * batch < 2000000 or 32 < batch <= 64:
+        same outputs to the bit."""
+        if not _walk_pays(self.out_dim, batch, self.training):
             return None
         a, b = self.indices
         versions = ops.versions(a, b)

@@ -255,3 +255,21 @@ def test_a_program_is_built_for_the_second_pass(cuda, argmax, monkeypatch):
         cuda.capturing = False
         assert passes(layers, rows=rows) == (0, 0)
     assert layers[2]._network is None                     # nothing is noted for a part of the network
+
+
+@pytest.mark.parametrize("width,batch,training,evaluating", [
+    (11999, 4096, False, False), (12000, 164, False, False), (12000, 168, True, True), (16000, 124, False, False), (16000, 128, True, True),
+    (64000, 33, False, False), (64000, 64, False, False), (12000, 1024, True, True), (12000, 1028, True, False), (15999, 4096, True, False),
+    (16000, 1028, True, True), (12000, 1027, True, True), (128000, 16, False, False), (128000, 17, True, True), (128000, 20, False, True),
+    (128000, 28, True, True), (75776, 32, True, True), (75777, 32, False, True), (111999, 32, False, True), (112000, 32, True, True),
+    (95999, 96, False, True), (96000, 68, True, True), (95999, 67, True, True), (40000, 100, True, True), (18944, 128, True, True),
+    (18945, 128, False, True), (27999, 100, False, True), (28000, 128, True, True), (22499, 192, False, True), (22500, 192, True, True),
+    (22499, 196, True, True), (20000, 129, True, True)])
+def test_which_layers_take_the_walk(cuda, walks, width, batch, training, evaluating):
+    """Both sides of every line at which the faster kernels change (a layer of few neurons stands in for one of many)."""
+    layer = _layer()
+    layer.out_dim = width
+    assert (layer.train()._walk_for(batch) is not None) == training
+    layer._walk = None
+    layer.eval()
+    assert [layer._walk_for(batch) is not None for _ in range(2)] == [False, evaluating]
