@@ -1,5 +1,6 @@
 """The one-kernel evaluation of a packed network against the oracle and the layer-by-layer kernels: counts and rows."""
 import copy
+import ctypes
 
 import numpy as np
 import pytest
@@ -105,26 +106,29 @@ def test_programs_follow_the_network():
     check(first)
 
 
-def test_two_threads_with_networks_of_different_size():
-    """Launches of one kernel with little and with much shared memory, from two threads at once: the limit that a launch sets is
-    enough for the other's."""
+def test_threads_with_networks_of_different_size():
+    """Launches of one kernel with little and with much shared memory, from several threads at once: the limit that a launch sets is
+    enough for the others'.  The entry point is called as directly as can be, so that calls of two threads overlap."""
     import threading
     failures = []
+    start = threading.Barrier(4)
 
     def work(dims, k, batch):
-        try:
-            with torch.cuda.stream(torch.cuda.Stream()):
-                layers = [tuple(t.cuda() for t in layer) for layer in _network(dims, batch)]
-                x = torch.randint(-2 ** 63, 2 ** 63 - 1, (dims[0], 2), generator=torch.Generator().manual_seed(1)).cuda()
-                network = ops.NetworkProgram(dims[0], layers)
-                want = ops.eval_network(x, network, batch, k)
-                for i in range(3000):
-                    got = ops.eval_network(x, network, batch, k)
-                    if i % 100 == 0:
-                        assert torch.equal(got, want) and ops.NetworkProgram(dims[0], layers).program.numel() > 0
-        except Exception as e:
-            failures.append(e)
-    threads = [threading.Thread(target=work, args=args) for args in (([64, 16384, 16384], 2, 33), ([40, 60, 60], 2, 100))]
+        with torch.cuda.stream(torch.cuda.Stream()) as _:
+            layers = [tuple(t.cuda() for t in layer) for layer in _network(dims, batch)]
+            x = torch.randint(-2 ** 63, 2 ** 63 - 1, (dims[0], 2), generator=torch.Generator().manual_seed(1)).cuda()
+            network = ops.NetworkProgram(dims[0], layers)
+            want = ops.eval_network(x, network, batch, k)
+            got = torch.empty_like(want)
+            run = N.lib().dl_eval_network
+            args = tuple(t(v) for t, v in zip(run.argtypes, (x.data_ptr(), network.program.data_ptr(), ctypes.addressof(network.sizes),
+                                                             len(layers), got.data_ptr(), 0, 16, batch, k, N.stream_of(x))))
+            start.wait()
+            statuses = [run(*args) for _ in range(8000)]
+            torch.cuda.current_stream().synchronize()
+            if any(statuses) or not torch.equal(got, want):
+                failures.append((dims, sum(map(bool, statuses))))
+    threads = [threading.Thread(target=work, args=args) for args in 2 * [([64, 16384, 16384], 2, 33), ([40, 60, 60], 2, 100)]]
     for t in threads:
         t.start()
     for t in threads:
