@@ -114,8 +114,9 @@ def test_deep_tabular_net_trains_and_packs():
 
 
 def test_packed_inference_at_the_benchmark_size_is_bit_exact():
-    """784 -> 4 x 8000 -> GroupSum(10) on 2^20 samples in int64 words (the packed benchmark, staged kernels, last layer
-    fused with the class count): every one of the 2^20 x 10 counts equals the C oracle's."""
+    """784 -> 4 x 8000 -> GroupSum(10) on 2^20 samples in int64 words (the packed benchmark): every one of the 2^20 x 10
+    counts equals the C oracle's, in the first pass (staged kernels, last layer fused with the class count) and in the
+    second (all layers in one kernel)."""
     import difflogic_b200 as D
     from tests.helpers import build_model
     torch.manual_seed(0)
@@ -128,19 +129,22 @@ def test_packed_inference_at_the_benchmark_size_is_bit_exact():
     x = torch.empty(samples, dims[0], dtype=torch.bool)
     for s in range(0, samples, 1 << 16):
         x[s:s + (1 << 16)] = torch.rand(1 << 16, dims[0], generator=g) < 0.19
-    with torch.no_grad():
-        counts = model(D.PackBitsTensor(x.cuda(), bit_count=64))
-    ref = O.c_packed_net_counts(x.numpy(), net.idx_a, net.idx_b, net.gate_ids(), k, threads=torch.get_num_threads())
-    assert counts.shape == (samples, k)
-    assert np.array_equal(counts.cpu().numpy(), np.asarray(ref))
+    ref = np.asarray(O.c_packed_net_counts(x.numpy(), net.idx_a, net.idx_b, net.gate_ids(), k, threads=torch.get_num_threads()))
+    for program in (False, True):
+        with torch.no_grad():
+            counts = model(D.PackBitsTensor(x.cuda(), bit_count=64))
+        assert counts.shape == (samples, k) and (model[-2]._network.program is not None) == program
+        assert np.array_equal(counts.cpu().numpy(), ref)
     from difflogic_b200 import _native as N
     assert N.lib().dl_async_error() == 0
 
 
-def test_captured_training_step_at_the_benchmark_size_against_oracle():
+@pytest.mark.parametrize("walk", [False, True])
+def test_captured_training_step_at_the_benchmark_size_against_oracle(walk, monkeypatch):
     """784 -> 5 x 16000 -> GroupSum(10, tau=30), batch 128, through a CUDA-graph-captured TrainStep (fused head, Adam
-    inside backward_w): loss, weight gradients (read back from Adam's first moments of the first step) and updated
-    weights against the oracle's step."""
+    inside the kernels of the backward pass): loss, weight gradients (read back from Adam's first moments of the first
+    step) and updated weights against the oracle's step.  Once by the gather kernels, once along the layers' walks, which
+    are there before the capture as they are after a warm-up step."""
     from difflogic_b200.optim import FlatAdam
     from difflogic_b200.training import TrainStep
     from tests.helpers import build_model, logic_layers
@@ -154,7 +158,14 @@ def test_captured_training_step_at_the_benchmark_size_against_oracle():
     y = torch.randint(0, k, (batch,), generator=g)
     opt = FlatAdam(model.parameters(), lr=lr)
     step = TrainStep(model, opt, torch.nn.CrossEntropyLoss())
+    along = []
+    backward_walk = ops.logic_backward_walk
+    monkeypatch.setattr(ops, "logic_backward_walk", lambda *a, **kw: along.append(kw["want_grad_x"]) or backward_walk(*a, **kw))
+    if walk:
+        for layer in logic_layers(model):
+            assert layer._walk_for(batch) is not None
     step.capture(x.cuda(), y.cuda(), warmup=0)          # nothing runs before the first replay
+    assert along == ([True] * 4 + [False] if walk else [])
     loss = step(x.cuda(), y.cuda())
     torch.cuda.synchronize()
     start = [w.detach().clone() for w in net.weights]

@@ -1,4 +1,4 @@
-"""Both tiles of the packers (a thread per 8 and per 64 samples) against torch: features and batches around the tiles' edges, rows
+"""Both tiles of the packers (a thread takes 8 or 32 samples) against torch: features and batches around the tiles' edges, rows
 and sources at every alignment."""
 import pytest
 import torch
@@ -7,9 +7,10 @@ from difflogic_b200 import ops
 
 pytestmark = pytest.mark.gpu
 
-# (features, batch): the first group is small enough for the 8-sample tile, the second large enough for the 64-sample one
+# (features, batch): the first group is small enough for the tile of 256 features x 64 samples, the second large enough for the one of
+# 64 x 1024: 592 such tiles for up to 128 features, 2368 for more (several blocks of features, whole and ragged, aligned and not)
 SIZES = [(1, 1), (7, 63), (8, 64), (9, 65), (63, 7), (64, 128), (65, 129), (255, 2047), (256, 2048), (257, 2049), (784, 100), (785, 1000),
-         (9, 1300001), (64, 1212416), (70, 620003), (1000, 75800), (1003, 76001), (2048, 38000)]
+         (9, 1300001), (64, 1212416), (70, 620003), (1000, 152000), (1003, 152001), (2048, 76000)]
 
 
 def _pack(bits, word_bits):

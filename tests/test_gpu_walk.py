@@ -73,15 +73,19 @@ def test_walk_kernels_match_the_layer(case, batch):
     # Adam in the epilogue: the same update as the gather kernel's epilogue, given gradients that differ by rounding only.
     # A first step moves every weight by lr * g / (|g| + eps): where |g| is large beside its error (1e-4 of the largest) the
     # two moves agree to lr * 1e-4 * max|g| / |g|.
-    state = torch.zeros(2, dtype=torch.int32, device="cuda")
-    w2, m, v = wd.clone(), torch.zeros(n_out * 16, device="cuda"), torch.zeros(n_out * 16, device="cuda")
-    ops.logic_backward_walk(xd, gyc.cuda(), coef, w2, walk, want_grad_x=False, rows_per_class=n_out // classes,
-                            adam=dict(exp_avg=m, exp_avg_sq=v, state=state, lr=0.01, beta1=0.9, beta2=0.999, eps=1e-8, grad_scale=1.0))
-    assert state.tolist() == [1, 0]
-    assert_grad_close(m.view(n_out, 16) * 10, gw_ref, "first moment")
-    big = gw_ref.abs() > 1e-2 * gw_ref.abs().max()
-    moved = (wd - w2).cpu().double() / 0.01
-    assert bool(((moved - gw_ref.sign()).abs()[big] <= 2e-2).all())
+    for want_x in {False, walk[1]}:                 # with grad_x: what a hidden layer's training step runs
+        state = torch.zeros(2, dtype=torch.int32, device="cuda")
+        w2, m, v = wd.clone(), torch.zeros(n_out * 16, device="cuda"), torch.zeros(n_out * 16, device="cuda")
+        gx, _ = ops.logic_backward_walk(xd, gyc.cuda(), coef, w2, walk, 1.5, want_grad_x=want_x, rows_per_class=n_out // classes,
+                                        adam=dict(exp_avg=m, exp_avg_sq=v, state=state, lr=0.01, beta1=0.9, beta2=0.999, eps=1e-8,
+                                                  grad_scale=1.0))
+        assert state.tolist() == [1, 0]
+        if want_x:
+            assert_grad_close(gx, gx_ref, "grad_x beside Adam")
+        assert_grad_close(m.view(n_out, 16) * 10, gw_ref, "first moment")
+        big = gw_ref.abs() > 1e-2 * gw_ref.abs().max()
+        moved = (wd - w2).cpu().double() / 0.01
+        assert bool(((moved - gw_ref.sign()).abs()[big] <= 2e-2).all())
 
 
 def test_a_bad_connection_gives_no_walk():
