@@ -133,15 +133,23 @@ class ClockSampler:
                 "samples": len(s)}
 
 
-def train_bytes_per_step(dims, batch, k):
+def train_bytes_per_step(dims, batch, k, walks=None):
     """Algorithmic HBM bytes of one training step: per layer every distinct input read once and every output
     written once (forward X+Y+P+I, backward_w X+Y+I+P, backward_x 2X+Y+P+I+C, not for the first layer), parameter
-    work 12 P (softmax 2P+3P, Adam 7P), float GroupSum forward+backward 2 (Y_last + 4 B k)."""
+    work 12 P (softmax 2P+3P, Adam 7P), float GroupSum forward+backward 2 (Y_last + 4 B k).
+    walks[i]: layer i runs along its walk, both gradients in one kernel that reads X and Y once and writes X (not for the
+    first layer); 8 bytes per entry of the walk, one per neuron, in place of the indices, and 16 of coefficients.  The last
+    layer's forward gathers (it adds up its classes)."""
     total = 0
     per_kernel = {}
     for li, (n_in, n_out) in enumerate(zip(dims[:-1], dims[1:])):
         X, Y, P, I = 4 * batch * n_in, 4 * batch * n_out, 64 * n_out, 16 * n_out
         C = 8 * (n_in + 1) + 16 * n_out
+        if walks is not None and walks[li]:
+            W = 8 * n_out
+            total += X + Y + P + (I if li == len(dims) - 2 else W)
+            total += X + Y + P + W + 16 * n_out + (X if li > 0 else 0) + 12 * P
+            continue
         total += (X + Y + P + I) + (X + Y + I + P) + 12 * P
         if li > 0:
             total += 2 * X + Y + P + I + C
@@ -418,7 +426,9 @@ def bench_train(name, args, rank, world, headline):
     # time stamps the exchange kernels took on the device during the last timed step (peer exchange only)
     exchange_timing = opt.exchange_timing() if peer else None
 
-    bytes_step, per_kernel = train_bytes_per_step(dims, batch, k)
+    per_kernel = train_bytes_per_step(dims, batch, k)[1]
+    walks = [layer._walk_for(batch) for layer in model if hasattr(layer, "_walk_for")]
+    bytes_step = train_bytes_per_step(dims, batch, k, [w is not None and (w.complete or i == 0) for i, w in enumerate(walks)])[0]
     peak, peak_kind = measured_peak_gbs()
     out = {
         "value": world * batch * K / t_dev,
@@ -565,11 +575,11 @@ def bench_packed(args, rank, world):
     # two ping-pong activation buffers, allocated once (the API call allocates per layer)
     bufs = [torch.empty(EVAL_DIMS[1], W, dtype=torch.int64, device=dev) for _ in range(2)]
 
-    # the plan PackBitsTensor.group_sum runs: all layers but the last one kernel each, then the last layer and the
-    # group bit-sum in one kernel when its sizes are in that kernel's range
+    # for comparison: all layers but the last one kernel each, then the last layer and the group bit-sum in one kernel when its
+    # sizes are in that kernel's range (what a network's first pass and wider layers run)
     fused_tail = D.packbitstensor.FUSED_LAST_LAYER and ops.eval_groupbitsum_applicable(bufs[0], EVAL_DIMS[-1], EVAL_K)
 
-    def run_resident():
+    def run_layer_by_layer():
         cur = words0
         last = len(layers) - 1
         for i, l in enumerate(layers):
@@ -578,9 +588,16 @@ def bench_packed(args, rank, world):
             cur = ops.eval_packed(cur, l.indices[0], l.indices[1], gates[i], out=bufs[i % 2])
         return ops.groupbitsum(cur, pad, EVAL_K)
 
+    def run_resident():
+        with torch.no_grad():
+            return model(D.PackBitsTensor.from_packed(words0, pad))
+
     K, Wm = max(args.steps, 50), 3
     for _ in range(Wm):
         counts = run_resident()
+    one_kernel = layers[-1]._network is not None and layers[-1]._network.program is not None
+    if not torch.equal(run_layer_by_layer(), counts):
+        raise RuntimeError("bench: packed inference layer by layer differs")
     # ---- bit-exact check of what is being timed: the first 2^17 samples of this run's input through the C oracle
     check = None
     if rank == 0 and not args.skip_cpu:
@@ -606,6 +623,7 @@ def bench_packed(args, rank, world):
         barrier(world)
     launches = _native.launch_count() - before
     t_dev = all_max(s.elapsed_time(e) * 1e-3, world)
+    ms_by_layer = time_launches(run_layer_by_layer) * 1e-3
 
     # end to end through the public API: bool matrix in pinned host memory -> class counts on the host
     out_host = torch.empty(local, EVAL_K, dtype=torch.int32).pin_memory()
@@ -631,8 +649,10 @@ def bench_packed(args, rank, world):
         "workload": "784 -> 4 x 8000 -> GroupSum(10), eval mode, 2^20 samples in int64 words, sharded by batch",
         "metric": "packed-bit inference samples/s", "unit": UNIT,
         "value": EVAL_SAMPLES * K / t_dev, "ms_per_pass": t_dev / K * 1e3, "passes": K, "samples_per_gpu": local,
-        "bytes_per_sample": eval_bytes_per_sample(EVAL_DIMS, EVAL_K, fused_tail),
-        "bytes_per_sample_layer_by_layer": eval_bytes_per_sample(EVAL_DIMS, EVAL_K), "fused_last_layer": bool(fused_tail),
+        "bytes_per_sample": EVAL_DIMS[0] / 8.0 + 4 * EVAL_K if one_kernel else eval_bytes_per_sample(EVAL_DIMS, EVAL_K, fused_tail),
+        "one_kernel": bool(one_kernel),
+        "layer_by_layer": {"ms_per_pass": ms_by_layer, "bytes_per_sample": eval_bytes_per_sample(EVAL_DIMS, EVAL_K, fused_tail),
+                           "fused_last_layer": bool(fused_tail)},
         "e2e": {"value": EVAL_SAMPLES * Ke / t_e2e, "unit": UNIT, "h2d_bytes_per_step": host_bool.numel(),
                 "d2h_bytes_per_step": out_host.numel() * 4, "iterations": Ke},
         "gpu_launches": launches, "clocks": sampler.summary(),

@@ -31,6 +31,24 @@ def test_algorithmic_bytes_of_the_baseline_configurations():
     assert bench.eval_bytes_per_sample(c5["dims"], c5["k"], False) == 192_040
 
 
+def test_bytes_of_a_step_along_the_walks():
+    """Beside the gather kernels a layer saves one read of its gradients and outputs, one pass over its weights and most of the
+    index arrays."""
+    bench = _bench()
+    for c in (bench.CONFIGS["c4"], bench.CONFIGS["c5"]):
+        dims, batch = c["dims"], c["batch"]
+        none = [False] * (len(dims) - 1)
+        gathered = bench.train_bytes_per_step(dims, batch, c["k"])[0]
+        assert bench.train_bytes_per_step(dims, batch, c["k"], none)[0] == gathered
+        for li, (n_in, n_out) in enumerate(zip(dims[:-1], dims[1:])):
+            one = bench.train_bytes_per_step(dims, batch, c["k"], [i == li for i in range(len(none))])[0]
+            saved = 8 * n_out if li < len(none) - 1 else 0                                     # forward: entries for indices
+            saved += 8 * n_out - 16 * n_out                                                    # gradients: as well, and coefficients
+            if li > 0:
+                saved += 4 * batch * (n_in + n_out) + 64 * n_out + 16 * n_out + 8 * (n_in + 1) + 16 * n_out
+            assert gathered - one == saved
+
+
 def test_both_bench_arms_name_the_same_configuration():
     bench = _bench()
     assert bench.train_config(4) == bench.train_config(4) and bench.train_config(1)["global_batch"] == 128
