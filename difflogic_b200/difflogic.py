@@ -294,23 +294,27 @@ class LogicLayer(torch.nn.Module):
         if not any(t is tensor for t in self._graph_tensors):
             self._graph_tensors = self._graph_tensors + (tensor,)
 
-    def _gate_ids(self):
+    def _gates(self):
         """uint8 arg-max gate per neuron, cached until the weights change (their version counter moves, or the count of
-        updates that FlatAdam and TrainStep keep for those that their kernels make) or the mode does.  A graph captured with cached gates keeps
-        working from those; one captured without computes its own, at every replay."""
+        updates that FlatAdam and TrainStep keep for those that their kernels make) or the mode does."""
         w = self.weights
         key = (w.data_ptr(), w._version, getattr(w, '_dl_updates', 0))
         cached = getattr(self, '_gate_cache', None)
-        capturing = torch.cuda.is_current_stream_capturing()
         if cached is None or cached[0] != key:
             with torch.no_grad():
                 gates = ops.argmax_gates(w.detach().contiguous())
-            if capturing:
+            if torch.cuda.is_current_stream_capturing():
                 return gates
             self._gate_cache = cached = (key, gates)
-        if capturing:
-            self._keep_for_graphs(cached[1])
         return cached[1]
+
+    def _gate_ids(self):
+        """The gates, for kernels that are launched next.  A graph captured with cached gates keeps working from those; one
+        captured without computes its own, at every replay."""
+        gates = self._gates()
+        if torch.cuda.is_current_stream_capturing():
+            self._keep_for_graphs(gates)
+        return gates
 
     def extra_repr(self):
         return '{}, {}, {}'.format(self.in_dim, self.out_dim, 'train' if self.training else 'eval')

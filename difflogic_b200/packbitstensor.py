@@ -91,7 +91,16 @@ class PackBitsTensor:
         """Called by LogicLayer.forward_cuda_eval: remember the layer (its connections and current arg-max gates)."""
         rows = self._pending[-1][0].out_dim if self._pending else self._t.shape[0]
         assert rows == layer.in_dim, ((rows,), layer.in_dim)
-        self._pending.append((layer, layer._gate_ids()))
+        self._pending.append((layer, layer._gates()))
+
+    def _capturing(self):
+        """Whether the pending layers, which are about to run, are being captured in a CUDA graph; their gates, from whenever they
+        were applied, then stay with the layers."""
+        if not torch.cuda.is_current_stream_capturing():
+            return False
+        for layer, gate in self._pending:
+            layer._keep_for_graphs(gate)
+        return True
 
     def _network(self, batch, k):
         """The pending layers as a program for the one-kernel evaluation, None when that kernel does not take them, False when it
@@ -105,7 +114,7 @@ class PackBitsTensor:
         if network is not None and not (network.sizes[0] == self._t.shape[0] and network.matches(layers)):
             network = None
         sizes = network.sizes if network is not None else ops.network_sizes(self._t.shape[0], layers)
-        if not ops.eval_network_applicable(self._t, sizes, batch, k) or torch.cuda.is_current_stream_capturing():
+        if not ops.eval_network_applicable(self._t, sizes, batch, k):
             return None
         if network is None:
             if any(t.device != self._t.device for layer in layers for t in layer) or any(ops.versions(a, b) is None for a, b, _ in layers):
@@ -117,6 +126,8 @@ class PackBitsTensor:
         return network
 
     def _materialize(self, in_one=True):
+        if self._pending and self._capturing():
+            in_one = False
         if in_one and len(self._pending) > 1:
             batch = self._t.shape[1] * self.bit_count
             network = self._network(batch, 1)
@@ -135,7 +146,7 @@ class PackBitsTensor:
         pad_len = self.pad_len + (self._t.shape[1] - self._words) * self.bit_count
         if self._pending and FUSED_LAST_LAYER:
             batch = self._t.shape[1] * self.bit_count - pad_len
-            network = self._network(batch, k)
+            network = None if self._capturing() else self._network(batch, k)
             if network:
                 return ops.eval_network(self._t, network, batch, k)   # all layers are still pending
             # all layers but the last run now; the last one is counted as it is computed, its output never stored

@@ -68,6 +68,29 @@ def test_gates_that_a_graph_reads_live_as_long_as_the_layer(cuda, argmax):
     assert read() is None
 
 
+@pytest.mark.parametrize("rows", [False, True])
+def test_layers_applied_before_a_capture_that_runs_them(cuda, argmax, monkeypatch, rows):
+    """A packed layer runs when its output is wanted: a capture may begin in between, and its graph reads the gates."""
+    monkeypatch.setattr(ops, "eval_network_applicable", lambda x, sizes, batch, k: True)
+    monkeypatch.setattr(ops, "eval_packed", lambda x, a, b, gate: x)
+    monkeypatch.setattr(ops, "eval_groupbitsum_parts_applicable", lambda x, n_out, k: False)
+    monkeypatch.setattr(ops, "eval_groupbitsum_applicable", lambda x, n_out, k: False)
+    monkeypatch.setattr(ops, "groupbitsum", lambda x, pad_len, k, padded: "counts")
+    layers = [_layer(), _layer()]
+    packed = D.PackBitsTensor.from_packed(torch.ones(8, 2, dtype=torch.int32), 0)
+    for layer in layers:
+        packed._push_layer(layer)
+    read = [weakref.ref(gate) for _, gate in packed._pending]
+    cuda.capturing = True
+    assert packed.t is not None if rows else packed.group_sum(2) == "counts"
+    cuda.capturing = False
+    del packed
+    argmax.clear()
+    for layer in layers:
+        layer.train()
+    assert all(gate() is not None for gate in read) and all(layer._network is None for layer in layers)
+
+
 def test_gates_that_only_a_graph_computes_are_not_used_outside_it(cuda, argmax):
     layer = _layer()
     cuda.capturing = True
