@@ -10,9 +10,9 @@ at a time by the kernels for long rows; `.t` shows the words of the batch only.
 Evaluation is lazy.  A LogicLayer in eval mode does not compute at once; it appends itself to the
 tensor's list of pending layers.  Layers of up to 16384 rows run in ONE kernel that keeps the activations
 in shared memory (ops.eval_network): `group_sum(k)` -- what GroupSum calls -- gets the class counts from it,
-reading `.t` the last layer's rows.  That kernel works from a program of the network, which takes longer to
-build than one batch takes without it; a network's first pass, and the first after its gates or connections
-have changed, therefore runs one kernel per layer.  So do wider layers, exactly as the reference does, and
+reading `.t` the last layer's rows.  That kernel works from a program of the network, which mostly takes longer
+to build than one batch takes without it; a network's first pass, and the first after its gates or connections
+have changed, then runs one kernel per layer.  So do wider layers, exactly as the reference does, and
 `group_sum(k)` then hands the last layer together with the bit-sum to one kernel that never stores the
 layer's output (ops.eval_groupbitsum) when the sizes are in that kernel's range.  The counts are
 identical either way; the in-place semantics of the reference (the layer returns the same object, `.t`
@@ -28,6 +28,14 @@ from . import ops
 
 # Module switch, read from the environment once at import (set the attribute to change it afterwards).
 FUSED_LAST_LAYER = os.environ.get("DL_FUSED_LAST_LAYER", "1") != "0"   # last layer + bit-sum in one kernel
+
+
+# A network's first pass builds its program when no layer is wider, or the batch as large.  First pass with the program / by single
+# layers, us, host and build included: 784 -> 2 x 2000: 2^10 samples 101 / 113, 2^17 111 / 118; 256 -> 12 x 4000: 2^13 267 / 261, 2^16 306 /
+# 269; 784 -> 4 x 8000: 2^13 162 / 147, 2^17 256 / 267, 2^18 361 / 422; 784 -> 5 x 16000: 2^13 311 / 189, 2^17 573 / 532, 2^18 848 / 904;
+# 784 -> 12 x 12000: 2^13 520 / 277, 2^18 1384 / 1722.
+PROGRAM_AT_ONCE_ROWS = 2000
+PROGRAM_AT_ONCE_SAMPLES = 1 << 18
 
 
 class PackBitsTensor:
@@ -104,9 +112,8 @@ class PackBitsTensor:
 
     def _network(self, batch, k):
         """The pending layers as a program for the one-kernel evaluation, None when that kernel does not take them, False when it
-        is not their turn yet: the program is built when the same gates and connections are met a second time, as building it
-        takes longer than a batch by the kernels for single layers (784 -> 5 x 16000, 10000 samples: 200 us beside 122, and 43
-        with the program).  It stays with the last layer until a layer's gates or connections are others.  Not while a CUDA
+        is not their turn yet: where building the program takes longer than it saves one batch (PROGRAM_AT_ONCE_ROWS), it is built
+        when the same gates and connections are met a second time.  It stays with the last layer until a layer's gates or connections are others.  Not while a CUDA
         graph is being captured: the graph would outlive a program that a change of the weights replaces."""
         layers = [layer.indices + (gate,) for layer, gate in self._pending]
         last = self._pending[-1][0]
@@ -119,8 +126,9 @@ class PackBitsTensor:
         if network is None:
             if any(t.device != self._t.device for layer in layers for t in layer) or any(ops.versions(a, b) is None for a, b, _ in layers):
                 return None
-            last._network = ops.NetworkProgram(self._t.shape[0], layers, build=False)
-            return False
+            network = last._network = ops.NetworkProgram(self._t.shape[0], layers, build=False)
+            if max(network.sizes[1:]) > PROGRAM_AT_ONCE_ROWS and self._t.shape[1] * self.bit_count < PROGRAM_AT_ONCE_SAMPLES:
+                return False
         if network.program is None:
             network.build()
         return network

@@ -12,8 +12,8 @@ pytestmark = pytest.mark.gpu
 def _counts(model, xb):
     model.eval()
     with torch.no_grad():
-        counts = model(D.PackBitsTensor(xb, bit_count=32))                            # by single layers
-        assert torch.equal(model(D.PackBitsTensor(xb, bit_count=32)), counts)         # in one kernel
+        counts = model(D.PackBitsTensor(xb, bit_count=32))
+        assert torch.equal(model(D.PackBitsTensor(xb, bit_count=32)), counts)         # the second pass, by whichever kernels
     # the same network from scratch: nothing remembered
     fresh = [(l.weights.detach().argmax(1), l.indices) for l in model if isinstance(l, D.LogicLayer)]
     h = xb

@@ -113,10 +113,10 @@ def test_deep_tabular_net_trains_and_packs():
     assert torch.equal(torch.round(fl * 20.0).to(torch.int32), counts)
 
 
-def test_packed_inference_at_the_benchmark_size_is_bit_exact():
+def test_packed_inference_at_the_benchmark_size_is_bit_exact(monkeypatch):
     """784 -> 4 x 8000 -> GroupSum(10) on 2^20 samples in int64 words (the packed benchmark): every one of the 2^20 x 10
-    counts equals the C oracle's, in the first pass (staged kernels, last layer fused with the class count) and in the
-    second (all layers in one kernel)."""
+    counts equals the C oracle's, by staged kernels with the last layer fused with the class count (what a smaller batch's
+    first pass runs) and with all layers in one kernel."""
     import difflogic_b200 as D
     from tests.helpers import build_model
     torch.manual_seed(0)
@@ -130,6 +130,7 @@ def test_packed_inference_at_the_benchmark_size_is_bit_exact():
     for s in range(0, samples, 1 << 16):
         x[s:s + (1 << 16)] = torch.rand(1 << 16, dims[0], generator=g) < 0.19
     ref = np.asarray(O.c_packed_net_counts(x.numpy(), net.idx_a, net.idx_b, net.gate_ids(), k, threads=torch.get_num_threads()))
+    monkeypatch.setattr(D.packbitstensor, "PROGRAM_AT_ONCE_SAMPLES", 1 << 40)
     for program in (False, True):
         with torch.no_grad():
             counts = model(D.PackBitsTensor(x.cuda(), bit_count=64))

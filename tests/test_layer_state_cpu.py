@@ -252,6 +252,7 @@ def test_a_program_is_built_for_the_second_pass(cuda, argmax, monkeypatch):
         single.append(gate)
         return x
     monkeypatch.setattr(ops, "eval_packed", eval_packed)
+    monkeypatch.setattr(D.packbitstensor, "PROGRAM_AT_ONCE_ROWS", 7)
     layers = [_layer() for _ in range(4)]
 
     def passes(model, *, rows=False):
@@ -278,6 +279,13 @@ def test_a_program_is_built_for_the_second_pass(cuda, argmax, monkeypatch):
         cuda.capturing = False
         assert passes(layers, rows=rows) == (0, 0)
     assert layers[2]._network is None                     # nothing is noted for a part of the network
+    for limit, value in (("ROWS", 8), ("SAMPLES", 64)):   # a narrow network, a large batch: the first pass builds it
+        monkeypatch.setattr(D.packbitstensor, "PROGRAM_AT_ONCE_ROWS", 7)
+        monkeypatch.setattr(D.packbitstensor, "PROGRAM_AT_ONCE_" + limit, value)
+        for layer in layers:
+            layer.train()
+            layer.eval()
+        assert [passes(layers) for _ in range(2)] == [(0, 1), (0, 0)]
 
 
 @pytest.mark.parametrize("width,batch,training,evaluating", [
