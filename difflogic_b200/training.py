@@ -236,7 +236,8 @@ class TrainStep:
 
     def capture(self, x, y, warmup=3):
         """Captures the step in a CUDA graph.  `x`, `y` give the shapes; their contents are used for
-        `warmup` eager steps (they DO update the weights) that run before the capture."""
+        `warmup` eager steps (they DO update the weights) that run before the capture.  With warmup=0 the graph has the kernels
+        that need no preparation: the walks of wide layers (LogicLayer._walk_for) are built by a step outside a capture."""
         self._static_x = x.clone()
         self._static_y = y.clone()
         side = torch.cuda.Stream()
