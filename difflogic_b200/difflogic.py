@@ -49,13 +49,13 @@ def _walk_pays(width, batch, training):
     """Whether a layer of `width` neurons takes less time by the walk kernels than by the gather kernels.
 
     A CTA of the walk kernels takes 64 neurons (256 where rows have up to 32 columns) through the whole batch, and 296 CTAs of the
-    backward kernel run at a time: narrow layers leave SMs idle, and so does a second round of few CTAs.  Rows of 65 to 96 columns
+    backward kernel run at a time: narrow layers leave SMs idle, and so does a second wave of few CTAs.  Rows of 65 to 96 columns
     leave lanes idle, which the gather kernels spread more finely, and with few columns the walk's longer chain from load to store
     shows.  Rows that are not whole 16-byte units are read value by value by the gather kernels, 1.15 to 2.4 times as slow.
 
     Measured with four layers, walk / gather kernels, us.  Captured training step: 8000 wide, 256 columns: 80 / 73, 2048: 396 / 391;
     16000, 64: 77 / 65, 128: 77 / 80, 512: 167 / 218; 64000, 64: 149 / 151, 80: 205 / 199, 96: 207 / 207, 100: 212 / 230; 128000, 68:
-    359 / 364; second round (18945 neurons on): 19000, 128: 104 / 94, 192: 142 / 135, 256: 141 / 139; 22500, 128: 112 / 107, 192: 153 / 156;
+    359 / 364; second wave (18945 neurons on): 19000, 128: 104 / 94, 192: 142 / 135, 256: 141 / 139; 22500, 128: 112 / 107, 192: 153 / 156;
     28000, 128: 116 / 118; up to 32 columns (75777 neurons on): 64000, 32: 120 / 124; 78000, 32: 175 / 156; 112000, 24: 191 / 178, 32: 194 /
     195; 128000, 24: 201 / 200, 28: 206 / 215.  Forward passes: 12000, 1000: 84 / 88, 1280: 121 / 104, 4096: 318 / 304; 14000, 1200: 131 / 121;
     16000, 1280: 135 / 134, 2048: 189 / 207; 128000, 16: 39 / 37, 20: 41 / 47."""
