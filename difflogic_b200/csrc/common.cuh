@@ -24,6 +24,16 @@ static inline int pow2_at_least(int64_t v, int cap) {
     return g;
 }
 
+// Packed rows that lie in two buffers: row i < split in x, the others in more (row i - split).  One buffer: split_rows(x).
+struct SplitRows {
+    const uint8_t *x, *more;
+    int64_t split;
+#ifdef __CUDACC__
+    __device__ __forceinline__ const uint8_t *row(int64_t i, int64_t pitch) const { return i < split ? x + i * pitch : more + (i - split) * pitch; }
+#endif
+};
+static inline SplitRows split_rows(const void *x) { return {reinterpret_cast<const uint8_t *>(x), nullptr, INT64_MAX}; }
+
 }  // namespace dl
 
 #define DL_REQUIRE(cond, code, ...)                       \

@@ -208,7 +208,7 @@ __device__ __forceinline__ void planes_to_bytes(const unsigned long long (&P)[8]
 
 template <int S>
 __global__ void __launch_bounds__(kFgThreads, 2)
-eval_groupbitsum_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict__ a, const int64_t *__restrict__ b,
+eval_groupbitsum_kernel(const SplitRows x, const int64_t *__restrict__ a, const int64_t *__restrict__ b,
                         const uint8_t *__restrict__ gate, int32_t *__restrict__ out, int64_t row_bytes, int block_bytes,
                         int64_t batch, int k, int m, int parts, int nplanes, int64_t nunits, int stages) {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -281,7 +281,7 @@ eval_groupbitsum_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict
             if (lane == 0) mbar_arrive_expect_tx(full + s, copies * cur.g.bytes);
             __syncwarp();
             if (needed)
-                bulk_load(smem + s * stage_bytes + (size_t)(which * kFgRows + r_in) * block_bytes, x + idx * row_bytes + cur.g.col0,
+                bulk_load(smem + s * stage_bytes + (size_t)(which * kFgRows + r_in) * block_bytes, x.row(idx, row_bytes) + cur.g.col0,
                           cur.g.bytes, full + s);
             last = cur.it;
             cur = nxt;
@@ -466,7 +466,7 @@ static int fg_cluster_size(int64_t m) {
 }
 
 template <int S>
-static int launch_fg(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, int32_t *out, int64_t row_bytes,
+static int launch_fg(const SplitRows &x, const int64_t *a, const int64_t *b, const uint8_t *gate, int32_t *out, int64_t row_bytes,
                      int64_t batch, int64_t k, int64_t m, bool in_parts, cudaStream_t st) {
     const size_t smem = fg_shared_bytes();
     if (cudaFuncSetAttribute(eval_groupbitsum_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -515,14 +515,23 @@ static int launch_fg(const void *x, const int64_t *a, const int64_t *b, const ui
     const int64_t nunits = ceil_div(row_bytes, block_bytes) * k * parts;
     const int64_t nclusters = nunits < resident ? nunits : resident;
     cfg.gridDim = dim3((unsigned)(nclusters * S));
-    const uint8_t *xb = reinterpret_cast<const uint8_t *>(x);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, eval_groupbitsum_kernel<S>, xb, a, b, gate, out, row_bytes, block_bytes, batch, (int)k,
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, eval_groupbitsum_kernel<S>, x, a, b, gate, out, row_bytes, block_bytes, batch, (int)k,
                                              (int)m, (int)parts, nplanes, nunits, stages);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(DL_ERR_CUDA, "dl_eval_groupbitsum: %s", cudaGetErrorString(e));
     }
     return launch_status("dl_eval_groupbitsum");
+}
+
+int eval_class_counts(const SplitRows &x, const int64_t *a, const int64_t *b, const uint8_t *gate, int32_t *out, int64_t row_bytes,
+                      int64_t batch, int64_t k, int64_t m, bool in_parts, cudaStream_t st) {
+    if (in_parts) return launch_fg<8>(x, a, b, gate, out, row_bytes, batch, k, m, true, st);
+    switch (fg_cluster_size(m)) {
+        case 8: return launch_fg<8>(x, a, b, gate, out, row_bytes, batch, k, m, false, st);
+        case 4: return launch_fg<4>(x, a, b, gate, out, row_bytes, batch, k, m, false, st);
+        default: return launch_fg<2>(x, a, b, gate, out, row_bytes, batch, k, m, false, st);
+    }
 }
 
 }  // namespace dl
@@ -561,11 +570,7 @@ extern "C" DL_API int dl_eval_groupbitsum(const void *x, const int64_t *a, const
     DL_REQUIRE(x && a && b && gate && out, DL_ERR_INVALID_ARG, "dl_eval_groupbitsum: null pointer");
     const int64_t row_bytes = words * (bit_count / 8), m = n_out / k, batch = words * bit_count - pad_len;
     cudaStream_t st = as_stream(stream);
-    switch (fg_cluster_size(m)) {
-        case 8: return launch_fg<8>(x, a, b, gate, out, row_bytes, batch, k, m, false, st);
-        case 4: return launch_fg<4>(x, a, b, gate, out, row_bytes, batch, k, m, false, st);
-        default: return launch_fg<2>(x, a, b, gate, out, row_bytes, batch, k, m, false, st);
-    }
+    return eval_class_counts(split_rows(x), a, b, gate, out, row_bytes, batch, k, m, false, st);
 }
 
 extern "C" DL_API int dl_eval_groupbitsum_parts(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, int32_t *out,
@@ -577,5 +582,5 @@ extern "C" DL_API int dl_eval_groupbitsum_parts(const void *x, const int64_t *a,
                (long long)pad_len);
     DL_REQUIRE(x && a && b && gate && out, DL_ERR_INVALID_ARG, "dl_eval_groupbitsum_parts: null pointer");
     const int64_t row_bytes = words * (bit_count / 8);
-    return launch_fg<8>(x, a, b, gate, out, row_bytes, words * bit_count - pad_len, k, n_out / k, true, as_stream(stream));
+    return eval_class_counts(split_rows(x), a, b, gate, out, row_bytes, words * bit_count - pad_len, k, n_out / k, true, as_stream(stream));
 }

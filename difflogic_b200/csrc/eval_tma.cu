@@ -48,7 +48,7 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, vo
 
 template <int kTileRows, int kStages>
 __global__ void __launch_bounds__(kTmaThreads)
-eval_tma_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict__ a, const int64_t *__restrict__ b,
+eval_tma_kernel(const SplitRows x, const int64_t *__restrict__ a, const int64_t *__restrict__ b,
                 const uint8_t *__restrict__ gate, uint8_t *__restrict__ y, uint32_t n_out, int64_t row_bytes, int chunk,
                 uint32_t row_blocks, uint32_t ntiles, int64_t x_pitch, int64_t y_pitch) {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -116,7 +116,7 @@ eval_tma_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict__ a, co
             if (lane == 0) mbar_arrive_expect_tx(full + s, copies * bytes);
             __syncwarp();
             if (needed)
-                bulk_load(smem + s * stage_bytes + (size_t)(which * kTileRows + r) * chunk, x + idx * x_pitch + col0, bytes,
+                bulk_load(smem + s * stage_bytes + (size_t)(which * kTileRows + r) * chunk, x.row(idx, x_pitch) + col0, bytes,
                           full + s);
             ++issued;
             idx = idx_next;
@@ -199,7 +199,7 @@ bool eval_tma_applicable(const void *x, const void *y, int64_t row_bytes, int64_
 // The kernel's limit of shared memory is set for rows of MAX_CHUNK bytes, the longest that this shape is used for, whatever this
 // launch needs: other threads launch the kernel with other rows.
 template <int ROWS, int STAGES, int MAX_CHUNK>
-static int launch_eval_tma_shape(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, void *y, int64_t n_out,
+static int launch_eval_tma_shape(const SplitRows &x, const int64_t *a, const int64_t *b, const uint8_t *gate, void *y, int64_t n_out,
                                  int64_t row_bytes, int ctas_per_sm, cudaStream_t st, int64_t x_pitch, int64_t y_pitch) {
     const int chunk = (int)(row_bytes < kMaxChunk ? row_bytes : kMaxChunk);
     const int64_t col_chunks = ceil_div(row_bytes, chunk);
@@ -212,15 +212,14 @@ static int launch_eval_tma_shape(const void *x, const int64_t *a, const int64_t 
         return launch_status("dl_eval_packed (shared memory opt-in)");
     const int64_t slots = (int64_t)sm_count() * ctas_per_sm;
     const unsigned grid = (unsigned)(ntiles < slots ? ntiles : slots);
-    eval_tma_kernel<ROWS, STAGES><<<grid, kTmaThreads, smem, st>>>(reinterpret_cast<const uint8_t *>(x), a, b, gate,
-                                                                  reinterpret_cast<uint8_t *>(y), (uint32_t)n_out, row_bytes, chunk,
-                                                                  (uint32_t)row_blocks, (uint32_t)ntiles, x_pitch, y_pitch);
+    eval_tma_kernel<ROWS, STAGES><<<grid, kTmaThreads, smem, st>>>(x, a, b, gate, reinterpret_cast<uint8_t *>(y), (uint32_t)n_out, row_bytes,
+                                                                  chunk, (uint32_t)row_blocks, (uint32_t)ntiles, x_pitch, y_pitch);
     return launch_status("dl_eval_packed");
 }
 
 // x_pitch / y_pitch: bytes from one row of x / y to the next (row_bytes for contiguous matrices; larger when the rows
 // are a column slice of wider rows).  Multiples of 16.
-int launch_eval_tma(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, void *y, int64_t n_in, int64_t n_out,
+int launch_eval_tma(const SplitRows &x, const int64_t *a, const int64_t *b, const uint8_t *gate, void *y, int64_t n_in, int64_t n_out,
                     int64_t row_bytes, cudaStream_t st, int64_t x_pitch, int64_t y_pitch) {
     // fan-out of an input row: 2 * n_out / n_in.  DL_TUNE_EVAL_SHAPE = 1 (wide) | 2 (square) overrides the choice.
     const int force = tuning(DL_TUNE_EVAL_SHAPE);

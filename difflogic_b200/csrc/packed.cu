@@ -17,7 +17,7 @@ namespace dl {
 
 // packed_tma.cu: the same eval with the gathered rows staged in shared memory by bulk copies
 bool eval_tma_applicable(const void *x, const void *y, int64_t row_bytes, int64_t n_out);
-int launch_eval_tma(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, void *y, int64_t n_in, int64_t n_out,
+int launch_eval_tma(const SplitRows &x, const int64_t *a, const int64_t *b, const uint8_t *gate, void *y, int64_t n_in, int64_t n_out,
                     int64_t row_bytes, cudaStream_t st, int64_t x_pitch, int64_t y_pitch);
 // groupbitsum_tma.cu: the group bit-sum with rows staged the same way
 bool groupbitsum_tma_applicable(const void *x, int64_t n, int64_t row_bytes, int64_t k);
@@ -41,9 +41,9 @@ __device__ __forceinline__ uint32_t gate_apply(uint32_t a, uint32_t b, const Gat
 __device__ __forceinline__ uint16_t gate_apply(uint16_t a, uint16_t b, const GateMasks &g) { return (uint16_t)gate32(a, b, g); }
 __device__ __forceinline__ uint8_t gate_apply(uint8_t a, uint8_t b, const GateMasks &g) { return (uint8_t)gate32(a, b, g); }
 
-template <typename V, int G, int U>
+template <typename V, int G, int U, bool SPLIT>
 __global__ void __launch_bounds__(kThreads)
-eval_kernel(const V *__restrict__ x, const int64_t *__restrict__ a, const int64_t *__restrict__ b,
+eval_kernel(const SplitRows x, const int64_t *__restrict__ a, const int64_t *__restrict__ b,
             const uint8_t *__restrict__ gate, V *__restrict__ y, int64_t n_out, int64_t ncols, int64_t nslabs) {
     constexpr int R = kThreads / G;
     const int tid = threadIdx.x;
@@ -57,8 +57,9 @@ eval_kernel(const V *__restrict__ x, const int64_t *__restrict__ a, const int64_
     for (int u = 0; u < U; ++u) {
         const int64_t j = j0 + u * R;
         if (j < n_out) {
-            xa[u] = x + __ldg(a + j) * ncols;
-            xb[u] = x + __ldg(b + j) * ncols;
+            const int64_t ia = __ldg(a + j), ib = __ldg(b + j);
+            xa[u] = reinterpret_cast<const V *>(SPLIT && ia >= x.split ? x.more : x.x) + (SPLIT && ia >= x.split ? ia - x.split : ia) * ncols;
+            xb[u] = reinterpret_cast<const V *>(SPLIT && ib >= x.split ? x.more : x.x) + (SPLIT && ib >= x.split ? ib - x.split : ib) * ncols;
             gm[u] = gate_masks(__ldg(gate + j));
         }
     }
@@ -79,24 +80,39 @@ eval_kernel(const V *__restrict__ x, const int64_t *__restrict__ a, const int64_
 }
 
 template <typename V>
-static int launch_eval(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, void *y, int64_t n_out,
+static int launch_eval(const SplitRows &x, const int64_t *a, const int64_t *b, const uint8_t *gate, void *y, int64_t n_out,
                        int64_t row_bytes, cudaStream_t st) {
     constexpr int U = 4;
     const int64_t ncols = row_bytes / (int64_t)sizeof(V);
     const int G = pow2_at_least(ncols, 32);
     const int64_t nslabs = ceil_div(ncols, G);
     const dim3 grid((unsigned)ceil_div(n_out, (kThreads / G) * U), (unsigned)(nslabs < 65535 ? nslabs : 65535));
-    const V *xv = reinterpret_cast<const V *>(x);
     V *yv = reinterpret_cast<V *>(y);
 #define DL_EV(GG)                                                                                   \
     case GG:                                                                                        \
-        eval_kernel<V, GG, U><<<grid, kThreads, 0, st>>>(xv, a, b, gate, yv, n_out, ncols, nslabs); \
+        if (x.more != nullptr) eval_kernel<V, GG, U, true><<<grid, kThreads, 0, st>>>(x, a, b, gate, yv, n_out, ncols, nslabs); \
+        else eval_kernel<V, GG, U, false><<<grid, kThreads, 0, st>>>(x, a, b, gate, yv, n_out, ncols, nslabs); \
         break;
     switch (G) {
         DL_EV(1) DL_EV(2) DL_EV(4) DL_EV(8) DL_EV(16) DL_EV(32)
     }
 #undef DL_EV
     return launch_status("dl_eval_packed");
+}
+
+// One layer of packed gates: staged where its rows are long enough, else in the widest unit that rows and pointers allow.
+int eval_rows(const SplitRows &x, const int64_t *a, const int64_t *b, const uint8_t *gate, void *y, int64_t n_in, int64_t n_out,
+              int64_t row_bytes, cudaStream_t st) {
+    auto fits = [&](int64_t sz) { return row_bytes % sz == 0 && aligned_to(x.x, sz) && aligned_to(x.more, sz) && aligned_to(y, sz); };
+    // DL_TUNE_EVAL_KERNEL = 1 forces the register-staged kernel (for A/B measurements)
+    const bool plain_only = tuning(DL_TUNE_EVAL_KERNEL) == 1;
+    if (!plain_only && eval_tma_applicable(x.x, y, row_bytes, n_out) && aligned_to(x.more, 16))
+        return launch_eval_tma(x, a, b, gate, y, n_in, n_out, row_bytes, st, row_bytes, row_bytes);
+    if (fits(16)) return launch_eval<uint4>(x, a, b, gate, y, n_out, row_bytes, st);
+    if (fits(8)) return launch_eval<unsigned long long>(x, a, b, gate, y, n_out, row_bytes, st);
+    if (fits(4)) return launch_eval<uint32_t>(x, a, b, gate, y, n_out, row_bytes, st);
+    if (fits(2)) return launch_eval<uint16_t>(x, a, b, gate, y, n_out, row_bytes, st);
+    return launch_eval<uint8_t>(x, a, b, gate, y, n_out, row_bytes, st);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -310,17 +326,7 @@ extern "C" DL_API int dl_eval_packed(const void *x, const int64_t *a, const int6
     if (n_out == 0 || words == 0) return DL_OK;
     DL_REQUIRE(x && a && b && gate && y, DL_ERR_INVALID_ARG, "dl_eval_packed: null pointer");
     DL_REQUIRE(n_in > 0, DL_ERR_INVALID_ARG, "dl_eval_packed: n_in is 0 but n_out is %lld", (long long)n_out);
-    const int64_t row_bytes = words * (bit_count / 8);
-    cudaStream_t st = as_stream(stream);
-    auto fits = [&](int64_t sz) { return row_bytes % sz == 0 && aligned_to(x, sz) && aligned_to(y, sz); };
-    // DL_TUNE_EVAL_KERNEL = 1 forces the register-staged kernel (for A/B measurements)
-    const bool plain_only = tuning(DL_TUNE_EVAL_KERNEL) == 1;
-    if (!plain_only && eval_tma_applicable(x, y, row_bytes, n_out)) return launch_eval_tma(x, a, b, gate, y, n_in, n_out, row_bytes, st, row_bytes, row_bytes);
-    if (fits(16)) return launch_eval<uint4>(x, a, b, gate, y, n_out, row_bytes, st);
-    if (fits(8)) return launch_eval<unsigned long long>(x, a, b, gate, y, n_out, row_bytes, st);
-    if (fits(4)) return launch_eval<uint32_t>(x, a, b, gate, y, n_out, row_bytes, st);
-    if (fits(2)) return launch_eval<uint16_t>(x, a, b, gate, y, n_out, row_bytes, st);
-    return launch_eval<uint8_t>(x, a, b, gate, y, n_out, row_bytes, st);
+    return eval_rows(split_rows(x), a, b, gate, y, n_in, n_out, words * (bit_count / 8), as_stream(stream));
 }
 
 // dl_eval_packed on column slices: the rows of x and y are `row_bytes` long but lie x_pitch / y_pitch bytes apart (a column
@@ -334,7 +340,7 @@ extern "C" DL_API int dl_eval_packed_pitched(const void *x, int64_t x_pitch, con
                "dl_eval_packed_pitched: pitches must be multiples of 16 and at least row_bytes");
     DL_REQUIRE(eval_tma_applicable(x, y, row_bytes, n_out), DL_ERR_INVALID_ARG,
                "dl_eval_packed_pitched: rows must be at least 512 bytes, a multiple of 16 and 16-byte aligned");
-    return launch_eval_tma(x, a, b, gate, y, n_in, n_out, row_bytes, as_stream(stream), x_pitch, y_pitch);
+    return launch_eval_tma(split_rows(x), a, b, gate, y, n_in, n_out, row_bytes, as_stream(stream), x_pitch, y_pitch);
 }
 
 extern "C" DL_API int dl_packbits(const uint8_t *t, void *out, int64_t n, int64_t batch, int bit_count, void *stream) {

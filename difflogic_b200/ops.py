@@ -542,28 +542,99 @@ class NetworkProgram:
                 self.gates_ready = torch.cuda.current_stream().record_event()
 
     gates_ready = None
+    counted = None      # number of classes to make a table for along with the program
 
     def build(self):
+        count = len(self.layers)
+        program = torch.empty(N.lib().dl_network_program_words(self.sizes, count), dtype=torch.int32, device=self.layers[0][2].device)
+        self._launch(N.lib().dl_network_program, program)
+        program._dl_tables = {}     # by number of classes; another thread may build the program once more, with other slots
+        if self.counted is not None:
+            self._make_table(program, self.counted)
+        # other threads and streams may take program and table from here on: this waits for them
+        program._dl_needs = tuple(program[:2].tolist())
+        self.program = program
+
+    def _launch(self, build, program):
+        """build(connections, gates, sizes, layers, program, stream)."""
         import ctypes
         count = len(self.layers)
-        device = self.layers[0][2].device
-        program = torch.empty(N.lib().dl_network_program_words(self.sizes, count), dtype=torch.int32, device=device)
         pointers = [(ctypes.c_void_p * count)(*[layer[i].data_ptr() for layer in self.layers]) for i in range(3)]
-        with torch.cuda.device(device):
-            stream = torch.cuda.current_stream(device)
+        with torch.cuda.device(program.device):
+            stream = torch.cuda.current_stream(program.device)
             if self.gates_ready is not None:
                 stream.wait_event(self.gates_ready)
-            N.check_status(N.lib().dl_network_program(pointers[0], pointers[1], pointers[2], self.sizes, count, program.data_ptr(),
-                                                      stream.cuda_stream))
-            # other threads and streams may take it from here on
-            stream.synchronize()
+            N.check_status(build(pointers[0], pointers[1], pointers[2], self.sizes, count, program.data_ptr(), stream.cuda_stream))
         program._dl_stream = stream.cuda_stream
-        self.program = program
+
+    def _make_table(self, program, k):
+        layers = len(self.layers)
+        table = torch.empty(N.lib().dl_network_table_words(self.sizes, layers, k), dtype=torch.int32, device=program.device)
+        with N.on_device(program):
+            stream = N.stream_of(program)
+            N.check_status(N.lib().dl_network_table(program.data_ptr(), self.sizes, layers, k, table.data_ptr(), stream))
+        table._dl_stream = stream
+        if len(program._dl_tables) >= 4:
+            program._dl_tables = {}
+        program._dl_tables[k] = table
+        return table
+
+    def table(self, program, k):
+        """The class table of a program for k classes; made, and waited for, when k is met first."""
+        table = program._dl_tables.get(k)
+        if table is None:
+            table = self._make_table(program, k)
+            torch.cuda.current_stream(table.device).synchronize()
+        return table
+
+    def serves(self, x, k):
+        """Whether the program is there, has counted k classes before, and takes the rows of x: all that has to be asked of a
+        pass that is like an earlier one.  (What the classes' counts need depends on k alone, not on the batch.)"""
+        program = self.program
+        return (program is not None and k in getattr(program, '_dl_tables', ()) and x.shape[1] * x.element_size() % 16 == 0
+                and x.data_ptr() % 16 == 0 and x.is_contiguous() and x.numel() > 0)
 
     def matches(self, layers):
         return len(layers) == len(self.layers) and all(
             a is p[0] and b is p[1] and gate is p[2] and p[3] is not None and a._version == p[3] and b._version == p[4]
             for (a, b, gate), p in zip(layers, self.layers))
+
+
+FOLDED_LAYERS = 32     # layers of a network that can be folded
+
+
+class FoldedLayers(NetworkProgram):
+    """The same for networks of any width (dl_fold_layers): the gates that are left of every layer, and how many they are."""
+
+    def __init__(self, n_in, layers, build=True):
+        self.layers = [(a, b, gate) + (versions(a, b) or (None, None)) for a, b, gate in layers]
+        self.sizes = network_sizes(n_in, layers)
+        self.program = None
+        self.stream = N.stream_of(layers[0][2])     # the gates are in its queue
+        if build:
+            self.build()
+
+    def build(self):
+        import ctypes
+        count = len(self.layers)
+        for a, b, gate, _, _ in self.layers:
+            _index(a, "a", gate.numel())
+            _index(b, "b", gate.numel())
+        device = self.layers[0][2].device
+        if N.stream_of(self.layers[0][2]) != self.stream:
+            torch.cuda.synchronize(device)
+        program = torch.empty(N.lib().dl_fold_layers_bytes(self.sizes, count), dtype=torch.uint8, device=device)
+        self._launch(N.lib().dl_fold_layers, program)
+        # other threads and streams may take the program from here on: this waits for it
+        left = program[:4 * count].view(torch.int32).tolist()
+        program._dl_left = (ctypes.c_int32 * count)(*left)
+        self.rows = sum(left[1:])
+        self.program = program
+
+    def pays(self):
+        """Whether this takes less than whole layers: fewer rows to compute, and at most half as much memory again as two
+        activations of the widest layer."""
+        return self.rows * 10 <= 9 * sum(self.sizes[1:-1]) and self.rows <= 3 * max(self.sizes[1:])
 
 
 def network_sizes(n_in, layers):
@@ -590,12 +661,42 @@ def eval_network(x, network, batch, k=None):
     else:
         out = torch.empty((int(batch), int(k)), dtype=torch.int32, device=x.device)
     with N.on_device(x):
+        table = None if k is None else network.table(program, int(k))
+        stream = N.stream_of(x)
+        for t in (program, table):
+            if t is not None and stream != t._dl_stream:
+                t.record_stream(torch.cuda.current_stream(x.device))
+        N.check(N.lib().dl_eval_network_sized(x.data_ptr(), program.data_ptr(), sizes, len(sizes) - 1, *program._dl_needs,
+                                              N.ptr(table), 0 if k is None else out.data_ptr(), out.data_ptr() if k is None else 0, row_bytes,
+                                              int(batch), 1 if k is None else int(k), stream))
+    return out
+
+
+def eval_folded_applicable(x, sizes):
+    """True when a network of these sizes on packed words x can be folded: more than one layer, and the sizes of dl_fold_layers."""
+    return (x.is_cuda and x.dim() == 2 and x.is_contiguous() and x.dtype in _DTYPE_TO_BITS and x.shape[0] == sizes[0] and x.shape[1] > 0
+            and 2 < len(sizes) <= FOLDED_LAYERS + 1 and min(sizes) > 0 and sum(sizes) < 1 << 27)
+
+
+def eval_folded(x, network, batch, k=None):
+    """All layers of a FoldedLayers on packed words x: int32 [batch, k] class counts, or without k the last layer's rows as
+    packed words."""
+    _need(x.is_cuda and x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D CUDA tensor")
+    sizes, program, words = network.sizes, network.program, x.shape[1]
+    _need(x.shape[0] == sizes[0] and x.device == program.device, "x does not fit the network")
+    row_bytes = words * (bits_of(x) // 8)
+    pool = torch.empty((sum(program._dl_left[1:]), words), dtype=x.dtype, device=x.device)
+    if k is None:
+        out = torch.empty((sizes[len(sizes) - 1], words), dtype=x.dtype, device=x.device)
+    else:
+        out = torch.empty((int(batch), int(k)), dtype=torch.int32, device=x.device)
+    with N.on_device(x):
         stream = N.stream_of(x)
         if stream != program._dl_stream:
             program.record_stream(torch.cuda.current_stream(x.device))
-        N.check(N.lib().dl_eval_network(x.data_ptr(), program.data_ptr(), sizes, len(sizes) - 1,
-                                        0 if k is None else out.data_ptr(), out.data_ptr() if k is None else 0, row_bytes, int(batch),
-                                        1 if k is None else int(k), stream))
+        N.check(N.lib().dl_eval_folded(x.data_ptr(), program.data_ptr(), sizes, program._dl_left, len(sizes) - 1, pool.data_ptr(),
+                                       0 if k is None else out.data_ptr(), out.data_ptr() if k is None else 0, row_bytes, int(batch),
+                                       1 if k is None else int(k), stream))
     return out
 
 

@@ -14,7 +14,9 @@ reading `.t` the last layer's rows.  That kernel works from a program of the net
 to build than one batch takes without it; a network's first pass, and the first after its gates or connections
 have changed, then runs one kernel per layer.  So do wider layers, exactly as the reference does, and
 `group_sum(k)` then hands the last layer together with the bit-sum to one kernel that never stores the
-layer's output (ops.eval_groupbitsum) when the sizes are in that kernel's range.  The counts are
+layer's output (ops.eval_groupbitsum) when the sizes are in that kernel's range.  From the second pass on the wider
+networks, too, run folded (ops.eval_folded): over the gates that are left when neurons that hand on a row or a constant,
+and rows that nothing reads, are taken out.  The counts are
 identical either way; the in-place semantics of the reference (the layer returns the same object, `.t`
 then holds the layer's output) are kept.
 """
@@ -30,12 +32,17 @@ from . import ops
 FUSED_LAST_LAYER = os.environ.get("DL_FUSED_LAST_LAYER", "1") != "0"   # last layer + bit-sum in one kernel
 
 
-# A network's first pass builds its program when no layer is wider, or the batch as large.  First pass with the program / by single
-# layers, us, host and build included: 784 -> 2 x 2000: 2^10 samples 101 / 113, 2^17 111 / 118; 256 -> 12 x 4000: 2^13 267 / 261, 2^16 306 /
-# 269; 784 -> 4 x 8000: 2^13 162 / 147, 2^17 256 / 267, 2^18 361 / 422; 784 -> 5 x 16000: 2^13 311 / 189, 2^17 573 / 532, 2^18 848 / 904;
-# 784 -> 12 x 12000: 2^13 520 / 277, 2^18 1384 / 1722.
-PROGRAM_AT_ONCE_ROWS = 2000
+# A network's first pass builds its program when the batch is as large, or no layer wider (none is: a program takes 26 launches and a
+# synchronisation for four layers).  First pass with the program / by single layers, us, host and build included: 784 -> 4 x 2000: 2^10
+# samples 283 / 185; 784 -> 4 x 8000: 2^13 246 / 161, 2^17 310 / 281, 2^18 366 / 428; 784 -> 5 x 16000: 2^15 312 / 224, 2^17 452 / 530; 784 ->
+# 12 x 12000: 2^13 471 / 293, 2^16 520 / 575, 2^18 777 / 1753.
+PROGRAM_AT_ONCE_ROWS = 0
 PROGRAM_AT_ONCE_SAMPLES = 1 << 18
+
+# Wider networks are folded in the first pass when their hidden rows take up this much memory.  The same figures: 784 -> 2 x 20000: 2^17
+# samples (330 MB) 305 / 257; 9216 -> 4 x 128000: 10000 (490 MB) 369 / 363, 2^15 601 / 797; 256 -> 12 x 64000: 1000 (90 MB) 478 / 353, 10000
+# (890 MB) 481 / 554, 2^17 1511 / 4509.
+FOLD_AT_ONCE_BYTES = 5 << 27
 
 
 class PackBitsTensor:
@@ -110,7 +117,7 @@ class PackBitsTensor:
             layer._keep_for_graphs(gate)
         return True
 
-    def _network(self, batch, k):
+    def _network(self, batch, k, counts=True):
         """The pending layers as a program for the one-kernel evaluation, None when that kernel does not take them, False when it
         is not their turn yet: where building the program takes longer than it saves one batch (PROGRAM_AT_ONCE_ROWS), it is built
         when the same gates and connections are met a second time.  It stays with the last layer until a layer's gates or connections are others.  Not while a CUDA
@@ -120,27 +127,49 @@ class PackBitsTensor:
         network = last._network
         if network is not None and not (network.sizes[0] == self._t.shape[0] and network.matches(layers)):
             network = None
+        if network is not None and network.serves(self._t, k):
+            return network
         sizes = network.sizes if network is not None else ops.network_sizes(self._t.shape[0], layers)
-        if not ops.eval_network_applicable(self._t, sizes, batch, k):
+        folded = not ops.eval_network_applicable(self._t, sizes, batch, k)
+        if folded and not ops.eval_folded_applicable(self._t, sizes):
             return None
-        if network is None:
-            if any(t.device != self._t.device for layer in layers for t in layer) or any(ops.versions(a, b) is None for a, b, _ in layers):
+        kind = ops.FoldedLayers if folded else ops.NetworkProgram
+        if type(network) is not kind:
+            device = self._t.get_device()
+            if any(t.get_device() != device for layer in layers for t in layer) or any(ops.versions(a, b) is None for a, b, _ in layers):
                 return None
-            network = last._network = ops.NetworkProgram(self._t.shape[0], layers, build=False)
-            if max(network.sizes[1:]) > PROGRAM_AT_ONCE_ROWS and self._t.shape[1] * self.bit_count < PROGRAM_AT_ONCE_SAMPLES:
+            network = last._network = kind(self._t.shape[0], layers, build=False)
+            if folded:
+                at_once = sum(sizes[1:-1]) * self._t.shape[1] * self.bit_count >= 8 * FOLD_AT_ONCE_BYTES
+            else:
+                at_once = max(sizes[1:]) <= PROGRAM_AT_ONCE_ROWS or self._t.shape[1] * self.bit_count >= PROGRAM_AT_ONCE_SAMPLES
+            if not at_once:
                 return False
         if network.program is None:
+            if counts and not folded:
+                network.counted = k
             network.build()
-        return network
+        return False if folded and not network.pays() else network
+
+    def _run(self, network, batch, k=None):
+        """The class counts of the pending layers, without k the last one's rows; None where there is no memory for the rows of
+        a folded network (single layers need less)."""
+        if not isinstance(network, ops.FoldedLayers):
+            return ops.eval_network(self._t, network, batch, k)
+        try:
+            return ops.eval_folded(self._t, network, batch, k)
+        except torch.cuda.OutOfMemoryError:
+            return None
 
     def _materialize(self, in_one=True):
         if self._pending and self._capturing():
             in_one = False
         if in_one and len(self._pending) > 1:
             batch = self._t.shape[1] * self.bit_count
-            network = self._network(batch, 1)
-            if network:
-                self._t, self._pending = ops.eval_network(self._t, network, batch), []
+            network = self._network(batch, 1, counts=False)
+            rows = self._run(network, batch) if network else None
+            if rows is not None:
+                self._t, self._pending = rows, []
                 return
         pending, self._pending = self._pending, []
         for layer, gate in pending:
@@ -154,19 +183,29 @@ class PackBitsTensor:
         pad_len = self.pad_len + (self._t.shape[1] - self._words) * self.bit_count
         if self._pending and FUSED_LAST_LAYER:
             batch = self._t.shape[1] * self.bit_count - pad_len
-            network = None if self._capturing() else self._network(batch, k)
-            if network:
-                return ops.eval_network(self._t, network, batch, k)   # all layers are still pending
+            network = None if self._capturing() else self._network(batch, k)   # all layers are still pending
+            if network and isinstance(network, ops.FoldedLayers) and not self._counts_with_last_layer(self._pending[-1][0].out_dim, k):
+                self._materialize()
+                return ops.groupbitsum(self._t, pad_len, k, padded=True)
+            counts = self._run(network, batch, k) if network else None
+            if counts is not None:
+                return counts
             # all layers but the last run now; the last one is counted as it is computed, its output never stored
             (layer, gate) = self._pending.pop()
             self._materialize(in_one=network is None)
             self._pending.append((layer, gate))  # still pending: `.t` would run it as a kernel of its own
-            parts = ops.eval_groupbitsum_parts_applicable(self._t, layer.out_dim, k)
-            if parts or ops.eval_groupbitsum_applicable(self._t, layer.out_dim, k):
+            how = self._counts_with_last_layer(layer.out_dim, k)
+            if how:
                 a, b = layer.indices
-                return ops.eval_groupbitsum(self._t, a, b, gate, pad_len, k, parts=parts, padded=True)
+                return ops.eval_groupbitsum(self._t, a, b, gate, pad_len, k, parts=how == 'parts', padded=True)
         self._materialize()
         return ops.groupbitsum(self._t, pad_len, k, padded=True)
+
+    def _counts_with_last_layer(self, n_out, k):
+        """Whether one kernel takes a last layer of n_out neurons together with the class counts: 'parts', 'whole' or None."""
+        if ops.eval_groupbitsum_parts_applicable(self._t, n_out, k):
+            return 'parts'
+        return 'whole' if ops.eval_groupbitsum_applicable(self._t, n_out, k) else None
 
     def flatten(self, start_dim=0, end_dim=-1, **kwargs):
         """Returns the object itself so that torch.nn.Flatten passes it through; arguments are ignored."""

@@ -214,10 +214,15 @@ DL_API int dl_eval_packed_pitched(const void *x, int64_t x_pitch, const int64_t 
  *                               rows of whole 16 bytes, 16-byte aligned, n[layers] divisible by k, and the widest layer plus
  *                               the counts of a block within shared memory.
  *   dl_network_program          order of evaluation and gate masks from every layer's connections and gate ids (HOST arrays of
- *                               device pointers) into dl_network_program_words() 32-bit words.  Connections outside the
- *                               layer's input read row 0.
+ *                               device pointers) into dl_network_program_words() 32-bit words, 16-byte aligned.  Connections
+ *                               outside the layer's input read row 0.  The first two words then say how many row slots the
+ *                               program uses and how many gates of a layer are left at most.
  *   dl_eval_network             x [n[0]][row_bytes] -> out [batch][k] class counts, or the last layer's rows
  *                               rows_out [n[layers]][row_bytes]; one of the two is null.
+ *   dl_network_table            order in which the program's last rows are counted in k classes, into dl_network_table_words()
+ *                               32-bit words, 16-byte aligned
+ *   dl_eval_network_sized       the same for a caller that has read the program's first two words (less shared memory, and with it
+ *                               wider blocks or more of them per SM) and, for counts, has a table for this k or null
  * The counts and rows are those of dl_eval_packed per layer followed by dl_groupbitsum. */
 DL_API int dl_eval_network_applicable(const void *x, const int64_t *n, int layers, int64_t row_bytes, int64_t batch, int64_t k);
 DL_API int64_t dl_network_program_words(const int64_t *n, int layers);
@@ -225,6 +230,26 @@ DL_API int dl_network_program(const int64_t *const *a, const int64_t *const *b, 
                               int layers, uint32_t *program, void *stream);
 DL_API int dl_eval_network(const void *x, const uint32_t *program, const int64_t *n, int layers, int32_t *out, void *rows_out,
                            int64_t row_bytes, int64_t batch, int64_t k, void *stream);
+DL_API int64_t dl_network_table_words(const int64_t *n, int layers, int64_t k);
+DL_API int dl_network_table(const uint32_t *program, const int64_t *n, int layers, int64_t k, uint32_t *table, void *stream);
+DL_API int dl_eval_network_sized(const void *x, const uint32_t *program, const int64_t *n, int layers, int64_t slots, int64_t gates,
+                                 const uint32_t *table, int32_t *out, void *rows_out, int64_t row_bytes, int64_t batch, int64_t k,
+                                 void *stream);
+
+/* A packed network of any width, layer by layer, over the gates that are left when neurons that hand on a row, its inverse or a
+ * constant, and neurons that nothing reads, are taken out (fold.cu, folded_layers.cu).  n as above; 1 .. 32 layers.
+ *   dl_fold_layers_bytes        bytes of `work` (16-byte aligned), 0 for sizes outside the range
+ *   dl_fold_layers              fills work from every layer's connections and gate ids (HOST arrays of device pointers); its first
+ *                               words, int32, then say how many gates of layer l = 1 .. layers - 1 are left (word l).
+ *   dl_eval_folded              x [n[0]][row_bytes] -> out [batch][k] class counts, in the range of dl_eval_groupbitsum or
+ *                               dl_eval_groupbitsum_parts, or the last layer's rows rows_out [n[layers]][row_bytes]; one of the two
+ *                               is null.  left: those words, on the HOST.  pool: room for their sum in rows of row_bytes.
+ * The counts and rows are those of dl_eval_packed per layer followed by dl_groupbitsum. */
+DL_API int64_t dl_fold_layers_bytes(const int64_t *n, int layers);
+DL_API int dl_fold_layers(const int64_t *const *a, const int64_t *const *b, const uint8_t *const *gate, const int64_t *n, int layers,
+                          void *work, void *stream);
+DL_API int dl_eval_folded(const void *x, const void *work, const int64_t *n, const int32_t *left, int layers, void *pool, int32_t *out,
+                          void *rows_out, int64_t row_bytes, int64_t batch, int64_t k, void *stream);
 
 /* argmax over the 16 gate weights -> uint8 gate id, first maximum on ties
  * (weights.argmax(-1).to(uint8), difflogic/difflogic.py:146). */

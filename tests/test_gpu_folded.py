@@ -1,0 +1,87 @@
+"""Folded packed networks (gates that hand on a row or a constant, and rows that nothing reads, taken out) against the oracle and
+the layer-by-layer kernels: counts and rows."""
+import numpy as np
+import pytest
+import torch
+
+import difflogic_b200 as D
+from difflogic_b200 import ops
+from oracle import logic_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+ALL = tuple(range(16))
+# (rows of the input and of every layer, k, bytes of a row, word bits, gates): one gate kernel CTA and several, a remainder of the
+# list's CTAs (256 neurons), layers of one row, rows for each unit of the plain kernel (1, 2, 4, 8, 16 bytes), for the staged
+# kernel (512 on) and a remainder of its column blocks (2048); classes counted with the last layer, in parts and apart; layers of
+# which nothing is left, everything is, and of copies only (a value read many layers on)
+CASES = [([5, 3, 4], 2, 16, 32, ALL), ([1, 1, 1, 1], 1, 3, 8, ALL), ([40, 257, 255, 256], 2, 6, 16, ALL), ([9, 70, 70], 7, 12, 32, ALL),
+         ([300, 1001, 1001, 1001], 7, 24, 64, ALL), ([64, 3000, 500, 700], 1, 48, 64, ALL), ([64, 640, 640], 10, 512, 64, ALL),
+         ([200, 4100, 4200], 2, 2064, 64, ALL), ([200] + 31 * [2050], 50, 528, 32, ALL), ([30, 400, 400, 400], 4, 1040, 64, (0, 15)),
+         ([30, 400, 400, 400], 4, 1040, 64, (3, 5, 10, 12)), ([100, 900, 900, 900], 9, 640, 64, (1, 2, 4, 6, 7, 8, 9, 11, 13, 14))]
+
+
+@pytest.mark.parametrize("dims,k,row_bytes,bits,gates", CASES)
+def test_counts_and_rows(dims, k, row_bytes, bits, gates):
+    g = torch.Generator().manual_seed(row_bytes)
+    layers = []
+    for n_in, n_out in zip(dims[:-1], dims[1:]):
+        a, b = torch.randint(0, n_in, (2, n_out), generator=g)
+        b[:: 17] = a[:: 17]                                     # neurons that read one row twice
+        layers.append((a, b, torch.tensor(gates, dtype=torch.uint8)[torch.randint(0, len(gates), (n_out,), generator=g)]))
+    data = torch.randint(0, 256, (dims[0], row_bytes), generator=g, dtype=torch.uint8).numpy()
+    x = torch.from_numpy(data.view("int%d" % bits))
+    device_layers, xd = [tuple(t.cuda() for t in layer) for layer in layers], x.cuda()
+    network = ops.FoldedLayers(dims[0], device_layers)
+    left = network.program._dl_left
+    assert len(left) == len(layers) and all(0 <= gates <= n for gates, n in zip(left[1:], dims[1:]))
+    assert not network.rows if set(gates) <= {0, 3, 5, 10, 12, 15} else network.rows <= sum(dims[1:-1])
+    rows = x.numpy()
+    for a, b, gate in layers:
+        rows = O.eval_packed(rows, a.numpy(), b.numpy(), gate.numpy())
+    assert np.array_equal(ops.eval_folded(xd, network, row_bytes * 8).cpu().numpy(), rows)
+    batch = row_bytes * 8 - 5
+    one_by_one = xd
+    for a, b, gate in device_layers:
+        one_by_one = ops.eval_packed(one_by_one, a, b, gate)
+    want = ops.groupbitsum(one_by_one, 5, k)
+    packed = D.PackBitsTensor.from_packed(xd, 5)
+    if packed._counts_with_last_layer(dims[-1], k):
+        assert torch.equal(ops.eval_folded(xd, network, batch, k), want)
+
+
+def test_a_wide_network_is_folded(monkeypatch):
+    """Through the modules: first pass, second pass, a pass with the output's rows, and one that finds no memory."""
+    torch.manual_seed(6)
+    model = torch.nn.Sequential(D.LogicLayer(70, 17000), D.LogicLayer(17000, 17000), D.LogicLayer(17000, 17000), D.GroupSum(10)).eval()
+    layers = [m for m in model if isinstance(m, D.LogicLayer)]
+    x = torch.rand(5001, 70, device="cuda") < 0.5
+    want = O.packed_net_counts(x.cpu().numpy(), [l.indices[0].cpu() for l in layers], [l.indices[1].cpu() for l in layers],
+                               [l.weights.detach().argmax(1).cpu().numpy().astype(np.uint8) for l in layers], 10, 32)
+    folded = []
+    run = ops.eval_folded
+    monkeypatch.setattr(ops, "eval_folded", lambda *a: folded.append(a) or run(*a))
+
+    def counts():
+        with torch.no_grad():
+            return model(D.PackBitsTensor(x)).cpu().numpy()
+    assert np.array_equal(counts(), want) and not folded
+    assert np.array_equal(counts(), want) and len(folded) == 1
+    few = D.PackBitsTensor(x[:200])             # rows too short for the counting kernel
+    assert np.array_equal(model[3](model[2](model[1](model[0](few)))).cpu().numpy(), want[:200]) and len(folded) == 2
+    packed = D.PackBitsTensor(x)
+    for layer in layers:
+        packed = layer(packed)
+    assert np.array_equal(ops.groupbitsum(packed.t, packed.pad_len, 10).cpu().numpy(), want) and len(folded) == 3
+
+    def no_memory(*a):
+        raise torch.cuda.OutOfMemoryError
+    monkeypatch.setattr(ops, "eval_folded", no_memory)
+    assert np.array_equal(counts(), want)
+    with torch.no_grad():                       # nothing to fold: whole layers
+        for layer in layers:
+            layer.weights.zero_()
+            layer.weights[:, 6] = 1.0
+    monkeypatch.setattr(ops, "eval_folded", lambda *a: folded.append(a) or run(*a))
+    first, again = counts(), counts()
+    assert np.array_equal(first, again) and len(folded) == 3
