@@ -2,8 +2,12 @@
 // (packed.cu) and the thermometer packer (threshold_pack.cu).
 //
 // A thread owns eight adjacent features and reads eight samples of them at a time, eight bytes each.  No bit is moved on its
-// own: a predicate turns the 8 bytes of a load into 8 bits (two multiplies and a shift), and the 8 x 8 bit matrix of eight
-// samples is transposed in registers by three delta swaps: byte f then holds the 8 samples' bits of feature f.
+// own: every byte is compared with its threshold in place (bytes_above, four at a time), which leaves the answer in its top bit, and
+// the answers of successive samples are shifted down the bytes: after eight samples byte f holds the samples' bits of feature f,
+// which is the transposed order that is wanted.  Five instructions for four bytes.  (Squeezing a sample's answers together and
+// transposing 8 x 8 bits afterwards took three times as many instructions; the packer waited for those and for the loads in turn.)
+// Bound by memory: bool 784 x 2^20 226 -> 156 us (5.9 TB/s), uint8 3072 x 10000 with three thresholds 20.2 -> 13.1 us, 1021 x 2^18
+// 260 -> 116 us.
 //
 // A CTA of 256 threads takes 8 * WF features x 8 * K * (256 / WF) samples: WF threads side by side over the features, each going
 // through 8 * K samples.  The bytes meet in shared memory, so that a feature's samples leave as one run of K * 256 / WF bytes.
@@ -20,24 +24,18 @@
 
 namespace dl {
 
-// 0x01 in every selected byte of lo / hi -> 8 bits (byte 0 of lo to bit 0): the two products put the bytes' low bits
-// next to each other in bits 24..31 and overlap nowhere, so the sum cannot carry
-__device__ __forceinline__ uint32_t squeeze8_ones(uint32_t lo_ones, uint32_t hi_ones) {
-    return (lo_ones * 0x01020408u + hi_ones * 0x10204080u) >> 24;
+// Threshold t for bytes_above: what a byte's low seven bits need to reach bit 7, in every byte, and all ones for t < 128.
+struct ByteThreshold {
+    uint32_t add, either;
+};
+__host__ __device__ __forceinline__ ByteThreshold byte_threshold(int t) {
+    return {(uint32_t)(127 - (t & 127)) * 0x01010101u, t < 128 ? 0xffffffffu : 0u};
 }
-// 0x01 in every non-zero byte
-__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t v) { return ((((v & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | v) >> 7) & 0x01010101u; }
-
-// 8 x 8 bit matrix in a 64-bit word, byte = row: transposed (byte = column)
-__device__ __forceinline__ unsigned long long transpose_bits_8x8(unsigned long long x) {
-    unsigned long long t;
-    t = (x ^ (x >> 7)) & 0x00AA00AA00AA00AAull;
-    x ^= t ^ (t << 7);
-    t = (x ^ (x >> 14)) & 0x0000CCCC0000CCCCull;
-    x ^= t ^ (t << 14);
-    t = (x ^ (x >> 28)) & 0x00000000F0F0F0F0ull;
-    x ^= t ^ (t << 28);
-    return x;
+// Top bit of every byte of v: whether the byte is above the threshold.  The low seven bits decide alone or, for t < 128, together with
+// the top bit, which is enough then; for t >= 128 the top bit is needed as well.  Other bits: undefined.
+__device__ __forceinline__ uint32_t bytes_above(uint32_t v, const ByteThreshold &t) {
+    const uint32_t low = (v & 0x7f7f7f7fu) + t.add;
+    return (low & v) | ((low | v) & t.either);
 }
 
 // r[i] byte j  <-  v[j] byte i   for four 32-bit values
@@ -65,26 +63,27 @@ __device__ __forceinline__ uint2 load_features(const uint8_t *__restrict__ p, in
     return make_uint2(__funnelshift_r(w0, w1, 8 * off), __funnelshift_r(w1, w2, 8 * off));
 }
 
-// Eight samples from src on, `live` of which exist: out[i] byte f = their bits of feature f for output i.  MASK: functor (lo, hi:
-// the 8 bytes of one load; i: which of the NT outputs) -> 8 bits, bit f set when feature f is selected for output i.
-template <int NT, bool ALIGNED, typename MASK>
-__device__ __forceinline__ void pack_eight(const uint8_t *__restrict__ src, int64_t n, int features, int live, MASK mask,
-                                           unsigned long long (&out)[NT]) {
-    uint2 v[8];
+// Eight samples from src on, `live` of which exist; the others count as zeros, which are above no threshold.
+template <bool ALIGNED>
+__device__ __forceinline__ void load_eight(const uint8_t *__restrict__ src, int64_t n, int features, int live, uint2 (&v)[8]) {
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         v[r] = make_uint2(0u, 0u);
         if (r < live) v[r] = load_features<ALIGNED>(src + (int64_t)r * n, features);
     }
+}
+// out[i] byte f = the eight samples' bits of feature f for threshold i.
+template <int NT>
+__device__ __forceinline__ void pack_eight(const uint2 (&v)[8], const ByteThreshold (&thr)[NT], unsigned long long (&out)[NT]) {
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
-        uint32_t lo = 0u, hi = 0u;  // byte r = the mask of sample r
+        uint32_t lo = 0u, hi = 0u;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            lo |= (r < live ? mask(v[r].x, v[r].y, i) : 0u) << (8 * r);
-            hi |= (4 + r < live ? mask(v[4 + r].x, v[4 + r].y, i) : 0u) << (8 * r);
+        for (int r = 0; r < 8; ++r) {
+            lo = lo >> 1 | (bytes_above(v[r].x, thr[i]) & 0x80808080u);
+            hi = hi >> 1 | (bytes_above(v[r].y, thr[i]) & 0x80808080u);
         }
-        out[i] = transpose_bits_8x8((unsigned long long)lo | ((unsigned long long)hi << 32));
+        out[i] = (unsigned long long)lo | ((unsigned long long)hi << 32);
     }
 }
 
@@ -98,9 +97,9 @@ struct PackTile {
 
 // Output i goes to the rows starting at dst + i * out_stride (row_bytes bytes per feature row).  Samples beyond the batch give
 // zero bits.  fblk, sblk: which tile.
-template <int NT, int WF, int K, bool ALIGNED, typename MASK>
+template <int NT, int WF, int K, bool ALIGNED>
 __device__ __forceinline__ void pack_tile(const uint8_t *__restrict__ t, uint8_t *__restrict__ dst, int64_t out_stride, const PackShape &sh,
-                                          int64_t fblk, int64_t sblk, uint8_t *s_bytes, MASK mask) {
+                                          int64_t fblk, int64_t sblk, uint8_t *s_bytes, const ByteThreshold (&thr)[NT]) {
     using Tile = PackTile<WF, K>;
     static_assert(K == 1 || K == 4, "a thread's bytes are written one or four at a time");
     const int group = threadIdx.x / WF, octet = threadIdx.x % WF;
@@ -108,8 +107,27 @@ __device__ __forceinline__ void pack_tile(const uint8_t *__restrict__ t, uint8_t
     const int live = f < sh.n ? (int)max((int64_t)0, min((int64_t)(8 * K), sh.batch - s0)) : 0;
     const int features = (int)min((int64_t)8, sh.n - f);
     unsigned long long bits[K][NT];  // per round of 8 samples and output: byte f = the samples' bits of feature f
+    const uint8_t *src = t + s0 * sh.n + f;
+    if (live == 8 * K) {  // the next eight samples are on their way while eight are packed
+        uint2 v[8];
+        load_eight<ALIGNED>(src, sh.n, features, 8, v);
 #pragma unroll
-    for (int g = 0; g < K; ++g) pack_eight<NT, ALIGNED>(t + (s0 + g * 8) * sh.n + f, sh.n, features, live - g * 8, mask, bits[g]);
+        for (int g = 0; g < K; ++g) {
+            uint2 next[8];
+            if (g + 1 < K) load_eight<ALIGNED>(src + (int64_t)(g + 1) * 8 * sh.n, sh.n, features, 8, next);
+            pack_eight<NT>(v, thr, bits[g]);
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                if (g + 1 < K) v[r] = next[r];
+        }
+    } else {
+#pragma unroll
+        for (int g = 0; g < K; ++g) {
+            uint2 v[8];
+            load_eight<ALIGNED>(src + (int64_t)g * 8 * sh.n, sh.n, features, live - g * 8, v);
+            pack_eight<NT>(v, thr, bits[g]);
+        }
+    }
     constexpr int kPiece = Tile::kRun >= 16 ? 16 : 8, kPieces = Tile::kRun / kPiece;
     const bool wide = sh.row_bytes % kPiece == 0 && (reinterpret_cast<uintptr_t>(dst) % kPiece) == 0 && out_stride % kPiece == 0;
 #pragma unroll
@@ -156,8 +174,10 @@ struct PackGrid {
     int kind;
     dim3 grid;
 };
-// Measured (us, 64 x 1024 tile / 256 x 64 tile; n x batch): 784 x 10000: 6.4 / 4.1; 784 x 100000: 23.9 / 22.9; 784 x 2^20: 227 / 232;
-// 783 x 2^20: 344 / 464; 30 x 2^20: 24 / 73; 117 x 10000: 10.8 / 4.0; 9216 x 10000: 29 / 22.
+// The 64 x 1024 tile once there are two of them per SM.  Measured (us, 64 x 1024 / 256 x 64; bool n x batch, in brackets the tiles):
+// 784 x 1000 (13): 4.1 / 2.3; 784 x 10000 (130): 4.3 / 4.2; 783 x 10000 (130): 7.8 / 5.3; 256 x 2^17 (512): 6.0 / 8.0; 117 x 2^18 (512): 12.3 /
+// 19.5; 1001 x 60000 (944): 18.6 / 18.0; 784 x 100000 (1274): 14.1 / 18.5; 784 x 2^20: 156 / 189; 30 x 2^20 (1024): 19 / 64; three
+// thresholds: 1021 x 10000 (160): 11.0 / 9.0; 3072 x 10000 (480): 13.1 / 16.4.
 static inline PackGrid pack_grid(const PackShape &sh) {
     auto grid = [&](int64_t features, int64_t bytes) {
         const int64_t sb = ceil_div(sh.row_bytes, bytes);
@@ -165,7 +185,7 @@ static inline PackGrid pack_grid(const PackShape &sh) {
     };
     const PackGrid small = {0, grid(256, 8)}, large = {1, grid(64, 128)};
     const int64_t tiles = (int64_t)large.grid.x * large.grid.y;
-    return tiles >= 16 * 148 || (sh.n <= 128 && tiles >= 4 * 148) ? large : small;
+    return tiles >= 2 * 148 ? large : small;
 }
 
 }  // namespace dl

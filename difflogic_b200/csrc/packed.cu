@@ -148,20 +148,15 @@ packbits_kernel(const uint8_t *__restrict__ t, uint8_t *__restrict__ out, int64_
     }
 }
 
-// packbits from the batch-major matrix t[batch][n]: transpose and pack in one pass, bits moved eight by eight (pack_tile.cuh).
-struct MaskNonZero {
-    __device__ __forceinline__ uint32_t operator()(uint32_t lo, uint32_t hi, int) const {
-        return squeeze8_ones(nonzero_bytes(lo), nonzero_bytes(hi));
-    }
-};
-
+// packbits from the batch-major matrix t[batch][n]: transpose and pack in one pass (pack_tile.cuh).  Non-zero: above 0.
 template <int KIND, bool ALIGNED>
 __global__ void __launch_bounds__(kThreads)
 packbits_bm_kernel(const uint8_t *__restrict__ t, uint8_t *__restrict__ out, PackShape sh) {
     using Tile = PackTileOf<KIND>;
     __shared__ __align__(16) uint8_t s_bytes[Tile::kShared];
+    const ByteThreshold above[1] = {byte_threshold(0)};
     for (int64_t sblk = blockIdx.y; sblk * Tile::kRun < sh.row_bytes; sblk += gridDim.y)
-        pack_tile<1, Tile::kFeatures / 8, KIND == 0 ? 1 : 4, ALIGNED>(t, out, 0, sh, blockIdx.x, sblk, s_bytes, MaskNonZero());
+        pack_tile<1, Tile::kFeatures / 8, KIND == 0 ? 1 : 4, ALIGNED>(t, out, 0, sh, blockIdx.x, sblk, s_bytes, above);
 }
 
 template <bool ALIGNED>

@@ -20,25 +20,17 @@ struct Thresholds {
 // NT thresholds per pass over the source: the pixels are read once for up to kThresholdsPerPass of them.
 constexpr int kThresholdsPerPass = 4;
 
-template <int NT>
-struct MaskAbove {
-    uint32_t th4[NT];  // the threshold in every byte
-    __device__ __forceinline__ uint32_t operator()(uint32_t lo, uint32_t hi, int i) const {
-        return squeeze8_ones(__vcmpgtu4(lo, th4[i]) & 0x01010101u, __vcmpgtu4(hi, th4[i]) & 0x01010101u);
-    }
-};
-
 template <int NT, int KIND, bool ALIGNED>
 __global__ void __launch_bounds__(kThreads, 2)
 threshold_pack_kernel(const uint8_t *__restrict__ t, Thresholds thr, int first, uint8_t *__restrict__ out, PackShape sh) {
     using Tile = PackTileOf<KIND>;
     __shared__ __align__(16) uint8_t s_bytes[Tile::kShared];
-    MaskAbove<NT> mask;
+    ByteThreshold above[NT];
 #pragma unroll
-    for (int i = 0; i < NT; ++i) mask.th4[i] = (uint32_t)thr.v[first + i] * 0x01010101u;
+    for (int i = 0; i < NT; ++i) above[i] = byte_threshold(thr.v[first + i]);
     uint8_t *dst = out + (int64_t)first * sh.n * sh.row_bytes;
     for (int64_t sblk = blockIdx.y; sblk * Tile::kRun < sh.row_bytes; sblk += gridDim.y)
-        pack_tile<NT, Tile::kFeatures / 8, KIND == 0 ? 1 : 4, ALIGNED>(t, dst, sh.n * sh.row_bytes, sh, blockIdx.x, sblk, s_bytes, mask);
+        pack_tile<NT, Tile::kFeatures / 8, KIND == 0 ? 1 : 4, ALIGNED>(t, dst, sh.n * sh.row_bytes, sh, blockIdx.x, sblk, s_bytes, above);
 }
 
 template <int NT, bool ALIGNED>
