@@ -103,12 +103,14 @@ SIGNATURES = {
 }
 
 _lib = None
+_nodes = None
 _launches = 0
 
 
 def launch_count():
-    """Number of kernel launches issued through check() so far (every checked entry point launches one kernel)."""
-    return _launches
+    """Number of kernel launches issued through check() or by the native autograd nodes so far (every checked entry point launches
+    one kernel)."""
+    return _launches + (_nodes.launches() if _nodes is not None else 0)
 
 
 class NativeLibraryMissing(RuntimeError):
@@ -135,6 +137,26 @@ def lib():
             fn.argtypes = args
         _lib = handle
     return _lib
+
+
+def nodes():
+    """The module of the native autograd nodes (csrc/autograd_nodes.cpp), built beside the library; raises NativeLibraryMissing when
+    it has not been."""
+    global _nodes
+    if _nodes is None:
+        lib()
+        import importlib.util
+        spec = importlib.util.spec_from_file_location("dl_autograd", _build.NODES_PATH)
+        try:
+            module = importlib.util.module_from_spec(spec)
+        except ImportError as e:
+            raise NativeLibraryMissing("difflogic_b200: %s. Build it with `python -m difflogic_b200.build` (needs nvcc and g++); there is "
+                                       "no fallback implementation of the CUDA path." % e) from e
+        spec.loader.exec_module(module)
+        from . import difflogic
+        module.connect(vars(difflogic))
+        _nodes = module
+    return _nodes
 
 
 class tuning:

@@ -4,7 +4,8 @@
 
 compiles difflogic_b200/csrc/*.cu with nvcc into difflogic_b200/_lib/libdifflogic_b200.so.
 The library has a plain C ABI (include/difflogic_b200.h) and links the CUDA runtime statically,
-so it depends on nothing but the driver.
+so it depends on nothing but the driver.  The training path's autograd nodes (csrc/autograd_nodes.cpp) are a Python
+module of their own beside it, _lib/dl_autograd.so: host code that calls the library and links PyTorch.
 """
 import os
 import shutil
@@ -16,6 +17,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "_lib")
 LIB_PATH = os.path.join(LIB_DIR, "libdifflogic_b200.so")
+NODES_PATH = os.path.join(LIB_DIR, "dl_autograd.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -36,10 +38,25 @@ def sources():
     return sorted(os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cu"))
 
 
+def nodes_command():
+    """Compiles and links the module of the autograd nodes against the library and the PyTorch that runs this."""
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(find_nvcc())))
+    include = [os.path.join(ROOT, "include"), os.path.join(cuda, "include"), os.path.join(root, "include"),
+               os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"]]
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
+            *[flag for path in include for flag in ("-I", path)], os.path.join(CSRC, "autograd_nodes.cpp"), "-o", NODES_PATH,
+            "-L", os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda",
+            "-L", LIB_DIR, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN"]
+
+
 def is_stale():
-    if not os.path.exists(LIB_PATH):
+    if not (os.path.exists(LIB_PATH) and os.path.exists(NODES_PATH)):
         return True
-    built = os.path.getmtime(LIB_PATH)
+    built = min(os.path.getmtime(LIB_PATH), os.path.getmtime(NODES_PATH))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(ROOT, "include", "difflogic_b200.h")]
     return any(os.path.getmtime(d) > built for d in deps)
 
@@ -68,10 +85,11 @@ def build(verbose=False, force=False):
             raise RuntimeError("nvcc failed: " + " ".join(cmd))
     link = [nvcc, "-shared", "-cudart", "static", "-gencode", "arch=compute_100a,code=sm_100a",
             "-Xcompiler", "-fPIC", "-o", LIB_PATH, *objs]
-    r = subprocess.run(link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
-    if r.returncode != 0:
-        sys.stderr.write(r.stdout)
-        raise RuntimeError("link failed")
+    for cmd, what in ((link, "link"), (nodes_command(), "g++")):
+        r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(r.stdout)
+            raise RuntimeError(what + " failed")
     return LIB_PATH
 
 

@@ -12,8 +12,11 @@ layer runs on the library declared in include/difflogic_b200.h:
 
 `implementation='python'` is the pure-torch definition of the same layer and runs anywhere.
 """
+import types
+
 import torch
 
+from . import _native as N
 from . import ops
 from .functional import GradFactor, bin_op_s, get_unique_connections
 from .packbitstensor import PackBitsTensor
@@ -236,6 +239,16 @@ class LogicLayer(torch.nn.Module):
 
     def forward_cuda(self, x):
         if self.training:
+            if x.is_cuda and x.dim() == 2 and self._plan is not None:
+                # the native node; None for a call that is not of the ordinary form
+                a, b = self.indices
+                weights, walk = self.weights, self._walk_for(x.shape[0])
+                fits = walk is None or (walk.n_in == x.shape[1] and walk.n_out == weights.shape[0])   # else ops says what is wrong
+                y = N.nodes().layer(x, weights, a, b, self.given_x_indices_of_y_start, self._plan, float(self.grad_factor),
+                                    getattr(weights, '_dl_grad_out', None), None if walk is None else walk.entries,
+                                    walk is not None and bool(walk.complete)) if fits else None
+                if y is not None:
+                    return y
             assert x.device.type == 'cuda', x.device
         assert x.ndim == 2, x.ndim
 
@@ -343,7 +356,10 @@ class GroupSum(torch.nn.Module):
 
         assert x.shape[-1] % self.k == 0, (x.shape, self.k)
         if x.is_cuda and x.dtype == torch.float32 and x.dim() == 2 and x.shape[0] > 0:
-            return GroupSumFunction.apply(x, self.k, float(self.tau))
+            with N.on_device(x):
+                workspace = ops.groupsum_workspace(x, self.k)
+            out = N.nodes().group_sum(x, workspace, self.k, float(self.tau)) if type(self.k) is int else None
+            return out if out is not None else GroupSumFunction.apply(x, self.k, float(self.tau))
         return x.reshape(*x.shape[:-1], self.k, x.shape[-1] // self.k).sum(-1) / self.tau
 
     def extra_repr(self):
@@ -410,6 +426,17 @@ def _run_backward(ctx, x, weights, a, b, start, plan, coef, grad_y, rows_per_cla
         # the gradient stays inside the flat bucket
         grad_w = grad_w.view(grad_w.shape)
     return grad_x, grad_w
+
+
+def _backward_of_node(x, weights, a, b, start, plan, coef, grad_y, grad_factor, grad_out, walk, want_x, want_w):
+    """What the native node of a layer calls when an optimizer, an exchange or a stream for backward_w has a say in the weights'
+    gradient."""
+    ctx = types.SimpleNamespace(needs_input_grad=(want_x, want_w), walk=_walk_of(walk, x, weights), grad_factor=grad_factor, grad_out=grad_out)
+    return _run_backward(ctx, x, weights, a, b, start, plan, coef, grad_y)
+
+
+def _walk_of(walk, x, weights):
+    return None if walk is None else ops.Walk(walk[0], walk[1], x.shape[0], weights.shape[0])
 
 
 class LogicLayerFunction(torch.autograd.Function):

@@ -728,6 +728,11 @@ def _groupsum_workspace(device, stream, nbytes):
     return ws
 
 
+def groupsum_workspace(x, k):
+    """Scratch for the sums of x [batch, n] in k classes, by a call on the current stream."""
+    return _groupsum_workspace(x.device, N.stream_of(x), N.lib().dl_groupsum_workspace_bytes(x.shape[1], x.shape[0], k))
+
+
 def groupsum(x, k, tau):
     """feature-major x [n, batch] -> [batch, k] = per-class row sums / tau."""
     _f32_matrix(x, "x")
