@@ -20,7 +20,7 @@ DL_OK, DL_ERR_INVALID_ARG, DL_ERR_BAD_BIT_COUNT, DL_ERR_NOT_DIVISIBLE, DL_ERR_CU
 W_LOGITS, W_PROBS, W_ARGMAX = 0, 1, 2
 LAUNCH_PLAIN, LAUNCH_OVERLAP_SETUP = 0, 1
 (TUNE_NO_PDL, TUNE_EVAL_KERNEL, TUNE_EVAL_SHAPE, TUNE_GROUPBITSUM_KERNEL, TUNE_GROUPSUM_KERNEL, TUNE_FUSED_CLUSTER,
- TUNE_FORWARD_KERNEL) = range(7)
+ TUNE_FORWARD_KERNEL, TUNE_WALK_KERNEL) = range(8)
 
 # name -> (restype, argtypes); mirrors include/difflogic_b200.h one to one
 SIGNATURES = {

@@ -39,6 +39,7 @@ static const bool g_tuning_loaded = [] {
     g_tuning[DL_TUNE_GROUPSUM_KERNEL] = env_choice("DL_GROUPSUM_KERNEL", "t", gs, 1);
     g_tuning[DL_TUNE_FUSED_CLUSTER] = env_choice("DL_FUSED_CLUSTER", "248", fc, 3);
     g_tuning[DL_TUNE_FORWARD_KERNEL] = env_choice("DL_FORWARD_KERNEL", "ps", fk, 2);
+    g_tuning[DL_TUNE_WALK_KERNEL] = env_choice("DL_WALK_KERNEL", "ps", fk, 2);
     return true;
 }();
 

@@ -65,7 +65,7 @@ DL_API const char *dl_last_error_string(void);
 /* Kernel-choice switches for A/B measurements; 0 = the library chooses (the default).  Process-wide.  Their initial
  * values come from the environment once, when the library is loaded (DL_PDL=0, DL_EVAL_KERNEL=plain,
  * DL_EVAL_SHAPE=wide|square, DL_GROUPBITSUM_KERNEL=plain|staged, DL_GROUPSUM_KERNEL=ticket, DL_FUSED_CLUSTER=2|4|8,
- * DL_FORWARD_KERNEL=plain|staged); no entry point reads the environment afterwards.  No counterpart in the reference. */
+ * DL_FORWARD_KERNEL=plain|staged, DL_WALK_KERNEL=plain|staged); no entry point reads the environment afterwards.  No counterpart in the reference. */
 enum {
     DL_TUNE_NO_PDL = 0,             /* 1: never launch with programmatic stream serialisation                    */
     DL_TUNE_EVAL_KERNEL = 1,        /* 1: dl_eval_packed always takes the register-staged kernel                 */
@@ -74,7 +74,8 @@ enum {
     DL_TUNE_GROUPSUM_KERNEL = 4,    /* 1: dl_groupsum_f32 always takes the workspace (ticket) kernel             */
     DL_TUNE_FUSED_CLUSTER = 5,      /* dl_eval_groupbitsum: CTAs per class, 2, 4 or 8                            */
     DL_TUNE_FORWARD_KERNEL = 6,     /* dl_forward_f32: 1 = register kernel, 2 = staged (bulk-copy) kernel        */
-    DL_TUNE_COUNT = 7
+    DL_TUNE_WALK_KERNEL = 7,        /* dl_backward_walk_f32: 1 = register kernel, 2 = staged kernel where it can  */
+    DL_TUNE_COUNT = 8
 };
 DL_API int dl_set_tuning(int key, int value);
 DL_API int dl_get_tuning(int key);
