@@ -46,11 +46,11 @@ def nodes_command():
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(find_nvcc())))
     include = [os.path.join(ROOT, "include"), os.path.join(cuda, "include"), os.path.join(root, "include"),
                os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"]]
-    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-ffunction-sections", "-fdata-sections",
             "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
             *[flag for path in include for flag in ("-I", path)], os.path.join(CSRC, "autograd_nodes.cpp"), "-o", NODES_PATH,
             "-L", os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda",
-            "-L", LIB_DIR, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN"]
+            "-L", LIB_DIR, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN", "-Wl,--gc-sections"]
 
 
 def is_stale():

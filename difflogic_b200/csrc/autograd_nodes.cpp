@@ -35,6 +35,15 @@ using at::Tensor;
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
+struct WithGil {  // for the engine's threads
+    PyGILState_STATE state = PyGILState_Ensure();
+    ~WithGil() { PyGILState_Release(state); }
+};
+struct WithoutGil {
+    PyThreadState *state = PyEval_SaveThread();
+    ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+
 std::atomic<long long> g_launches{0};  // kernels launched from here, as _native.launch_count() counts
 PyObject *g_module_dict = nullptr;     // difflogic.py's: `_backward_w_stream` and `_backward_of_node`
 
@@ -156,7 +165,7 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
         if (!gy.is_contiguous()) gy = gy.contiguous();
         variable_list out(3);
         {
-            pybind11::gil_scoped_acquire gil;
+            const WithGil gil;
             if (managed(weights)) {
                 out = in_python(ctx, saved, gy, grad_out, walk, want_x, want_w);
                 if (out[0].defined()) out[0] = out[0].t();
@@ -254,7 +263,7 @@ PyObject *layer(PyObject *, PyObject *const *args, Py_ssize_t count) {
     l.transposed = !x.t().is_contiguous() && x.is_contiguous();
     Tensor y;
     {
-        pybind11::gil_scoped_release nogil;
+        const WithoutGil nogil;
         const c10::cuda::CUDAGuard guard(device);
         y = LayerNode::apply(x, w, l);
     }
@@ -277,7 +286,7 @@ PyObject *group_sum(PyObject *, PyObject *const *args, Py_ssize_t count) {
     if (!plain(x, at::kFloat, 2, x.device()) || x.numel() == 0 || k <= 0 || x.size(1) % k != 0 || observed() || x._fw_grad(0).defined()) Py_RETURN_NONE;
     Tensor y;
     {
-        pybind11::gil_scoped_release nogil;
+        const WithoutGil nogil;
         const c10::cuda::CUDAGuard guard(x.device());
         y = GroupSumNode::apply(x, workspace, (int64_t)k, tau);
     }

@@ -606,9 +606,11 @@ FOLDED_LAYERS = 32     # layers of a network that can be folded
 class FoldedLayers(NetworkProgram):
     """The same for networks of any width (dl_fold_layers): the gates that are left of every layer, and how many they are."""
 
-    def __init__(self, n_in, layers, build=True):
-        self.layers = [(a, b, gate) + (versions(a, b) or (None, None)) for a, b, gate in layers]
-        self.sizes = network_sizes(n_in, layers)
+    def __init__(self, n_in, layers, build=True, counters=None, sizes=None):
+        """counters, sizes: versions() of every layer's connections and network_sizes(), if the caller has them."""
+        counters = counters or [versions(a, b) or (None, None) for a, b, _ in layers]
+        self.layers = [layer + counter for layer, counter in zip(layers, counters)]
+        self.sizes = sizes or network_sizes(n_in, layers)
         self.program = None
         self.stream = N.stream_of(layers[0][2])     # the gates are in its queue
         if build:
@@ -675,7 +677,7 @@ def eval_network(x, network, batch, k=None):
 def eval_folded_applicable(x, sizes):
     """True when a network of these sizes on packed words x can be folded: more than one layer, and the sizes of dl_fold_layers."""
     return (x.is_cuda and x.dim() == 2 and x.is_contiguous() and x.dtype in _DTYPE_TO_BITS and x.shape[0] == sizes[0] and x.shape[1] > 0
-            and 2 < len(sizes) <= FOLDED_LAYERS + 1 and min(sizes) > 0 and sum(sizes) < 1 << 27)
+            and 2 < len(sizes) <= FOLDED_LAYERS + 1 and 0 < min(sizes) and sum(sizes) < 1 << 27)
 
 
 def eval_folded(x, network, batch, k=None):

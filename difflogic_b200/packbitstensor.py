@@ -136,12 +136,14 @@ class PackBitsTensor:
         kind = ops.FoldedLayers if folded else ops.NetworkProgram
         if type(network) is not kind:
             device = self._t.get_device()
-            if any(t.get_device() != device for layer in layers for t in layer) or any(ops.versions(a, b) is None for a, b, _ in layers):
+            counters = [ops.versions(a, b) for a, b, _ in layers]
+            if None in counters or any(t.get_device() != device for layer in layers for t in layer):
                 return None
-            network = last._network = kind(self._t.shape[0], layers, build=False)
             if folded:
+                network = last._network = kind(self._t.shape[0], layers, False, counters, sizes)
                 at_once = sum(sizes[1:-1]) * self._t.shape[1] * self.bit_count >= 8 * FOLD_AT_ONCE_BYTES
             else:
+                network = last._network = kind(self._t.shape[0], layers, build=False)
                 at_once = max(sizes[1:]) <= PROGRAM_AT_ONCE_ROWS or self._t.shape[1] * self.bit_count >= PROGRAM_AT_ONCE_SAMPLES
             if not at_once:
                 return False
