@@ -52,7 +52,9 @@ SIGNATURES = {
     "dl_eval_network_sized": (_int, [_ptr, _ptr, _ptr, _int, _i64, _i64, _ptr, _ptr, _ptr, _i64, _i64, _i64, _ptr]),
     "dl_fold_layers_bytes": (_i64, [_ptr, _int]),
     "dl_fold_layers": (_int, [_ptr, _ptr, _ptr, _ptr, _int, _ptr, _ptr]),
-    "dl_eval_folded": (_int, [_ptr, _ptr, _ptr, _ptr, _int, _ptr, _ptr, _ptr, _i64, _i64, _i64, _ptr]),
+    "dl_fold_tail_bytes": (_i64, [_ptr, _int, _i64]),
+    "dl_fold_tail": (_int, [_ptr, _ptr, _int, _i64, _ptr, _ptr]),
+    "dl_eval_folded": (_int, [_ptr, _ptr, _ptr, _ptr, _int, _ptr, _ptr, _i64, _ptr, _ptr, _i64, _i64, _i64, _ptr]),
     "dl_argmax_gate_u8": (_int, [_ptr, _ptr, _i64, _ptr]),
     "dl_packbits": (_int, [_ptr, _ptr, _i64, _i64, _int, _ptr]),
     "dl_packbits_batch_major": (_int, [_ptr, _ptr, _i64, _i64, _int, _ptr]),

@@ -32,6 +32,12 @@ struct SplitRows {
     __device__ __forceinline__ const uint8_t *row(int64_t i, int64_t pitch) const { return i < split ? x + i * pitch : more + (i - split) * pitch; }
 #endif
 };
+// Neurons of a last layer by class: those of class c are start[c] .. start[c + 1] - 1 (start null: m each), and ones[c] of them (null:
+// none) that are always true are not in the list.  m: the longest class.
+struct ClassRows {
+    const int32_t *start, *ones;
+    int m;
+};
 static inline SplitRows split_rows(const void *x) { return {reinterpret_cast<const uint8_t *>(x), nullptr, INT64_MAX}; }
 
 }  // namespace dl

@@ -104,19 +104,26 @@ struct FgUnit {
     int64_t col0;    // first byte of the column block within a row
     int64_t row0;    // first neuron of this CTA's share
     int rows;        // neurons in the share
-    int cls;
+    int cls, part;
     uint32_t bytes;  // bytes per row segment
 };
 
-__device__ __forceinline__ FgUnit fg_unit(int64_t u, int64_t row_bytes, int block_bytes, int k, int m, int parts, int q, int nq) {
+__device__ __forceinline__ FgUnit fg_unit(int64_t u, int64_t row_bytes, int block_bytes, int k, const ClassRows &classes, int parts, int q, int nq) {
     FgUnit g;
-    const int unit = (int)(u % ((int64_t)k * parts)), part = unit % parts;
+    const int unit = (int)(u % ((int64_t)k * parts));
+    g.part = unit % parts;
     g.cls = unit / parts;
     g.col0 = (u / ((int64_t)k * parts)) * block_bytes;
     g.bytes = (uint32_t)min((int64_t)block_bytes, row_bytes - g.col0);
-    const int64_t first = (int64_t)m * part / parts, rows = (int64_t)m * (part + 1) / parts - first;
+    int64_t begin = (int64_t)g.cls * classes.m;
+    int m = classes.m;
+    if (classes.start != nullptr) {
+        begin = __ldg(classes.start + g.cls);
+        m = __ldg(classes.start + g.cls + 1) - (int)begin;
+    }
+    const int64_t first = (int64_t)m * g.part / parts, rows = (int64_t)m * (g.part + 1) / parts - first;
     const int64_t r0 = first + rows * q / nq, r1 = first + rows * (q + 1) / nq;
-    g.row0 = (int64_t)g.cls * m + r0;
+    g.row0 = begin + r0;
     g.rows = (int)(r1 - r0);
     return g;
 }
@@ -127,28 +134,28 @@ struct FgCursor {
     int r;          // first row of the stage within the share
     FgUnit g;
     bool valid;
-    __device__ __forceinline__ void seek(int64_t nclusters, int64_t nunits, int64_t row_bytes, int block_bytes, int k, int m, int parts, int q, int nq) {
+    __device__ __forceinline__ void seek(int64_t nclusters, int64_t nunits, int64_t row_bytes, int block_bytes, int k, const ClassRows &classes, int parts, int q, int nq) {
         // first unit from u on whose share has rows
         for (valid = false; u < nunits; u += nclusters) {
-            g = fg_unit(u, row_bytes, block_bytes, k, m, parts, q, nq);
+            g = fg_unit(u, row_bytes, block_bytes, k, classes, parts, q, nq);
             if (g.rows > 0) { valid = true; break; }
         }
     }
     __device__ __forceinline__ void start(int64_t cluster_id, int64_t nclusters, int64_t nunits, int64_t row_bytes, int block_bytes, int k,
-                                          int m, int parts, int q, int nq) {
+                                          const ClassRows &classes, int parts, int q, int nq) {
         u = cluster_id;
         it = 0;
         r = 0;
-        seek(nclusters, nunits, row_bytes, block_bytes, k, m, parts, q, nq);
+        seek(nclusters, nunits, row_bytes, block_bytes, k, classes, parts, q, nq);
     }
-    __device__ __forceinline__ void next(int64_t nclusters, int64_t nunits, int64_t row_bytes, int block_bytes, int k, int m, int parts, int q, int nq) {
+    __device__ __forceinline__ void next(int64_t nclusters, int64_t nunits, int64_t row_bytes, int block_bytes, int k, const ClassRows &classes, int parts, int q, int nq) {
         if (!valid) return;
         ++it;
         r += kFgRows;
         if (r >= g.rows) {
             u += nclusters;
             r = 0;
-            seek(nclusters, nunits, row_bytes, block_bytes, k, m, parts, q, nq);
+            seek(nclusters, nunits, row_bytes, block_bytes, k, classes, parts, q, nq);
         }
     }
 };
@@ -210,7 +217,7 @@ template <int S>
 __global__ void __launch_bounds__(kFgThreads, 2)
 eval_groupbitsum_kernel(const SplitRows x, const int64_t *__restrict__ a, const int64_t *__restrict__ b,
                         const uint8_t *__restrict__ gate, int32_t *__restrict__ out, int64_t row_bytes, int block_bytes,
-                        int64_t batch, int k, int m, int parts, int nplanes, int64_t nunits, int stages) {
+                        int64_t batch, int k, const ClassRows classes, int parts, int nplanes, int64_t nunits, int stages) {
     extern __shared__ __align__(128) uint8_t smem[];
     unsigned long long *red = reinterpret_cast<unsigned long long *>(smem + kFgRing);  // [planes][words]
     uint4 *meta = reinterpret_cast<uint4 *>(red + kFgRedPlanes * kFgWords);                               // [stages][rows]
@@ -248,8 +255,8 @@ eval_groupbitsum_kernel(const SplitRows x, const int64_t *__restrict__ a, const 
         int64_t last = -1;  // latest stage this warp filled
         bool ok = true;
         FgCursor cur;
-        cur.start(cluster_id, nclusters, nunits, row_bytes, block_bytes, k, m, parts, q, S);
-        for (int i = 0; i < warp; ++i) cur.next(nclusters, nunits, row_bytes, block_bytes, k, m, parts, q, S);
+        cur.start(cluster_id, nclusters, nunits, row_bytes, block_bytes, k, classes, parts, q, S);
+        for (int i = 0; i < warp; ++i) cur.next(nclusters, nunits, row_bytes, block_bytes, k, classes, parts, q, S);
         int64_t idx = 0;
         uint32_t op = 0;
         if (cur.valid && copier && r_in < cur.g.rows - cur.r) {
@@ -258,7 +265,7 @@ eval_groupbitsum_kernel(const SplitRows x, const int64_t *__restrict__ a, const 
         }
         while (cur.valid) {
             FgCursor nxt = cur;
-            for (int i = 0; i < kFgProducers; ++i) nxt.next(nclusters, nunits, row_bytes, block_bytes, k, m, parts, q, S);
+            for (int i = 0; i < kFgProducers; ++i) nxt.next(nclusters, nunits, row_bytes, block_bytes, k, classes, parts, q, S);
             int64_t idx_next = 0;
             uint32_t op_next = 0;
             if (nxt.valid && copier && r_in < nxt.g.rows - nxt.r) {
@@ -307,7 +314,7 @@ eval_groupbitsum_kernel(const SplitRows x, const int64_t *__restrict__ a, const 
         const int row_words = block_bytes / 8;
         uint32_t n = 0;  // units done
         for (int64_t u = cluster_id; u < nunits; u += nclusters, ++n) {
-            const FgUnit g = fg_unit(u, row_bytes, block_bytes, k, m, parts, q, S);
+            const FgUnit g = fg_unit(u, row_bytes, block_bytes, k, classes, parts, q, S);
             const bool mine = (uint32_t)ct * 8u < g.bytes;
             BitCounterT<kFgRedPlanes - 3> cn;  // a share is at most 255 neurons
             cn.clear();
@@ -372,7 +379,7 @@ eval_groupbitsum_kernel(const SplitRows x, const int64_t *__restrict__ a, const 
         const int sum_planes = min(kFgSumPlanes, nplanes + (S == 8 ? 3 : S == 4 ? 2 : 1));
         uint32_t n = 0;
         for (int64_t u = cluster_id; u < nunits; u += nclusters, ++n) {
-            const FgUnit g = fg_unit(u, row_bytes, block_bytes, k, m, parts, q, S);
+            const FgUnit g = fg_unit(u, row_bytes, block_bytes, k, classes, parts, q, S);
             if (!fg_wait_cluster(red_full, n & 1u, abort_flag)) {
                 g_fg_async_error = 1;
                 s_abort = 1;
@@ -420,12 +427,13 @@ eval_groupbitsum_kernel(const SplitRows x, const int64_t *__restrict__ a, const 
                     if (wide) planes_to_bytes(hi_planes, hi_bytes);
                     const int64_t s0 = (g.col0 + (int64_t)w * 8) * 8;  // first sample of the word
                     int32_t *dst = out + s0 * k + g.cls;
+                    const int ones = classes.ones != nullptr && g.part == 0 ? __ldg(classes.ones + g.cls) : 0;
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
-                            int32_t cnt = (int32_t)((lo_bytes[j] >> (8 * i)) & 0xFFull);
-                            if (wide) cnt |= (int32_t)((hi_bytes[j] >> (8 * i)) & 0xFFull) << 8;
+                            int32_t cnt = (int32_t)((lo_bytes[j] >> (8 * i)) & 0xFFull) + ones;
+                            if (wide) cnt += (int32_t)((hi_bytes[j] >> (8 * i)) & 0xFFull) << 8;
                             if (s0 + 8 * j + i < batch) {
                                 int32_t *at = dst + (int64_t)(8 * j + i) * k;
                                 if (parts == 1) *at = cnt;
@@ -467,7 +475,8 @@ static int fg_cluster_size(int64_t m) {
 
 template <int S>
 static int launch_fg(const SplitRows &x, const int64_t *a, const int64_t *b, const uint8_t *gate, int32_t *out, int64_t row_bytes,
-                     int64_t batch, int64_t k, int64_t m, bool in_parts, cudaStream_t st) {
+                     int64_t batch, int64_t k, const ClassRows &classes, bool in_parts, cudaStream_t st) {
+    const int64_t m = classes.m;
     const size_t smem = fg_shared_bytes();
     if (cudaFuncSetAttribute(eval_groupbitsum_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return launch_status("dl_eval_groupbitsum (shared memory opt-in)");
@@ -516,7 +525,7 @@ static int launch_fg(const SplitRows &x, const int64_t *a, const int64_t *b, con
     const int64_t nclusters = nunits < resident ? nunits : resident;
     cfg.gridDim = dim3((unsigned)(nclusters * S));
     const cudaError_t e = cudaLaunchKernelEx(&cfg, eval_groupbitsum_kernel<S>, x, a, b, gate, out, row_bytes, block_bytes, batch, (int)k,
-                                             (int)m, (int)parts, nplanes, nunits, stages);
+                                             classes, (int)parts, nplanes, nunits, stages);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(DL_ERR_CUDA, "dl_eval_groupbitsum: %s", cudaGetErrorString(e));
@@ -525,14 +534,16 @@ static int launch_fg(const SplitRows &x, const int64_t *a, const int64_t *b, con
 }
 
 int eval_class_counts(const SplitRows &x, const int64_t *a, const int64_t *b, const uint8_t *gate, int32_t *out, int64_t row_bytes,
-                      int64_t batch, int64_t k, int64_t m, bool in_parts, cudaStream_t st) {
-    if (in_parts) return launch_fg<8>(x, a, b, gate, out, row_bytes, batch, k, m, true, st);
-    switch (fg_cluster_size(m)) {
-        case 8: return launch_fg<8>(x, a, b, gate, out, row_bytes, batch, k, m, false, st);
-        case 4: return launch_fg<4>(x, a, b, gate, out, row_bytes, batch, k, m, false, st);
-        default: return launch_fg<2>(x, a, b, gate, out, row_bytes, batch, k, m, false, st);
+                      int64_t batch, int64_t k, const ClassRows &classes, bool in_parts, cudaStream_t st) {
+    if (in_parts) return launch_fg<8>(x, a, b, gate, out, row_bytes, batch, k, classes, true, st);
+    switch (fg_cluster_size(classes.m)) {
+        case 8: return launch_fg<8>(x, a, b, gate, out, row_bytes, batch, k, classes, false, st);
+        case 4: return launch_fg<4>(x, a, b, gate, out, row_bytes, batch, k, classes, false, st);
+        default: return launch_fg<2>(x, a, b, gate, out, row_bytes, batch, k, classes, false, st);
     }
 }
+// Whether classes of up to m neurons are longer than one cluster's counters hold.
+bool class_counts_in_parts(int64_t m) { return ceil_div(m, fg_cluster_size(m)) > kFgMaxShare; }
 
 }  // namespace dl
 
@@ -570,7 +581,7 @@ extern "C" DL_API int dl_eval_groupbitsum(const void *x, const int64_t *a, const
     DL_REQUIRE(x && a && b && gate && out, DL_ERR_INVALID_ARG, "dl_eval_groupbitsum: null pointer");
     const int64_t row_bytes = words * (bit_count / 8), m = n_out / k, batch = words * bit_count - pad_len;
     cudaStream_t st = as_stream(stream);
-    return eval_class_counts(split_rows(x), a, b, gate, out, row_bytes, batch, k, m, false, st);
+    return eval_class_counts(split_rows(x), a, b, gate, out, row_bytes, batch, k, {nullptr, nullptr, (int)m}, false, st);
 }
 
 extern "C" DL_API int dl_eval_groupbitsum_parts(const void *x, const int64_t *a, const int64_t *b, const uint8_t *gate, int32_t *out,
@@ -582,5 +593,6 @@ extern "C" DL_API int dl_eval_groupbitsum_parts(const void *x, const int64_t *a,
                (long long)pad_len);
     DL_REQUIRE(x && a && b && gate && out, DL_ERR_INVALID_ARG, "dl_eval_groupbitsum_parts: null pointer");
     const int64_t row_bytes = words * (bit_count / 8);
-    return eval_class_counts(split_rows(x), a, b, gate, out, row_bytes, words * bit_count - pad_len, k, n_out / k, true, as_stream(stream));
+    return eval_class_counts(split_rows(x), a, b, gate, out, row_bytes, words * bit_count - pad_len, k,
+                             {nullptr, nullptr, (int)(n_out / k)}, true, as_stream(stream));
 }

@@ -3,7 +3,9 @@
 // Every gate that is left has a row in one POOL, layers one after the other; a gate reads rows of the pool or of the packed
 // input, from whichever layer its inputs come, so rows that a layer only hands on are neither moved nor stored.  The kernels are
 // those for whole layers (eval_rows), over shorter lists; the last layer keeps all of its neurons, in order, because its rows or
-// class counts are wanted, with the gates in terms of pool rows: constants read nothing and copies one row.
+// class counts are wanted, with the gates in terms of pool rows: constants read nothing and copies one row.  Where the counts are
+// wanted, a table by class (one per number of classes) leaves the constants out: what the counting kernel takes goes by its
+// neurons, whatever they read.
 //
 // Bound by memory as before, with fewer rows: 256 -> 12 x 64000, 2^17 samples 4340 -> 1190 us (12 x 64000 neurons of which 139000 are
 // left as gates); 9216 -> 4 x 128000, 10000 samples, with the packing 289 -> 195 us.
@@ -15,7 +17,8 @@ namespace dl {
 int eval_rows(const SplitRows &x, const int64_t *a, const int64_t *b, const uint8_t *gate, void *y, int64_t n_in, int64_t n_out,
               int64_t row_bytes, cudaStream_t st);                                                   // packed.cu
 int eval_class_counts(const SplitRows &x, const int64_t *a, const int64_t *b, const uint8_t *gate, int32_t *out, int64_t row_bytes,
-                      int64_t batch, int64_t k, int64_t m, bool in_parts, cudaStream_t st);          // eval_groupbitsum.cu
+                      int64_t batch, int64_t k, const ClassRows &classes, bool in_parts, cudaStream_t st);  // eval_groupbitsum.cu
+bool class_counts_in_parts(int64_t m);
 
 // The lists: gates that are left by place, then the last layer's neurons.
 struct GateList {
@@ -64,6 +67,93 @@ static GateList gate_list(const FoldShape &sh, void *work) {
     return l;
 }
 
+// Neurons of the last layer by class, without constants.
+struct TailTable {
+    GateList list;
+    int32_t *start, *longest, *ones, *count, *rank;  // [k + 1], [1], [k], [k], by neuron
+};
+static int64_t tail_table(int64_t n, int64_t k, TailTable *t, void *at) {
+    t->list.a = reinterpret_cast<int64_t *>(at);
+    t->list.b = t->list.a + n;
+    t->longest = reinterpret_cast<int32_t *>(t->list.b + n);  // at byte 16 n, as the header says
+    t->start = t->longest + 1;
+    t->ones = t->start + k + 1;
+    t->count = t->ones + k;
+    t->rank = t->count + k;
+    t->list.gate = reinterpret_cast<uint8_t *>(t->rank + n);
+    return 21 * n + 4 * (3 * k + 2);
+}
+
+__global__ void __launch_bounds__(kThreads)
+tail_count_kernel(TailTable t, int n, int rows_per_class, const uint8_t *__restrict__ gate) {
+    grid_dependents_launch();
+    const int j = blockIdx.x * kThreads + threadIdx.x;
+    const int op = j < n ? gate[j] : 0, c = j < n ? j / rows_per_class : 0;
+    // a warp's neurons are mostly of one class: one addition for all
+    const bool one = __all_sync(0xffffffffu, c == __shfl_sync(0xffffffffu, c, 0) || j >= n);
+    const bool counts = op != 0 && op != 15;
+    const unsigned listed = __ballot_sync(0xffffffffu, counts), lane = threadIdx.x % 32;
+    if (one) {
+        const unsigned always = __ballot_sync(0xffffffffu, op == 15);
+        int base = 0;
+        if (lane == 0) {
+            if (listed) base = atomicAdd(t.count + c, __popc(listed));
+            if (always) atomicAdd(t.ones + c, __popc(always));
+        }
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (counts) t.rank[j] = base + __popc(listed & ((1u << lane) - 1u));
+    } else if (counts) {
+        t.rank[j] = atomicAdd(t.count + c, 1);
+    } else if (op == 15) {
+        atomicAdd(t.ones + c, 1);
+    }
+}
+
+__global__ void __launch_bounds__(1024)
+tail_start_kernel(TailTable t, int k) {
+    __shared__ int s_sum[1024], s_most;
+    grid_dependency_wait();
+    grid_dependents_launch();
+    const int tid = threadIdx.x, each = (k + 1023) / 1024;
+    if (tid == 0) s_most = 0;
+    int mine = 0, most = 0;
+    for (int c = tid * each; c < min(k, (tid + 1) * each); ++c) {
+        mine += __ldcg(t.count + c);
+        most = max(most, __ldcg(t.count + c));
+    }
+    s_sum[tid] = mine;
+    __syncthreads();
+    atomicMax(&s_most, most);
+    for (int d = 1; d < 1024; d <<= 1) {
+        const int v = tid >= d ? s_sum[tid - d] : 0;
+        __syncthreads();
+        s_sum[tid] += v;
+        __syncthreads();
+    }
+    int at = s_sum[tid] - mine;
+    for (int c = tid * each; c < min(k, (tid + 1) * each); ++c) {
+        t.start[c] = at;
+        at += __ldcg(t.count + c);
+    }
+    if (tid == 1023) {
+        t.start[k] = s_sum[tid];
+        *t.longest = s_most;
+    }
+}
+
+__global__ void __launch_bounds__(kThreads)
+tail_place_kernel(TailTable t, int n, int rows_per_class, GateList from) {
+    grid_dependency_wait();
+    const int j = blockIdx.x * kThreads + threadIdx.x;
+    if (j >= n) return;
+    const int op = from.gate[j];
+    if (op == 0 || op == 15) return;
+    const int at = __ldcg(t.start + j / rows_per_class) + t.rank[j];
+    t.list.a[at] = from.a[j];
+    t.list.b[at] = from.b[j];
+    t.list.gate[at] = (uint8_t)op;
+}
+
 }  // namespace dl
 
 using namespace dl;
@@ -88,8 +178,36 @@ extern "C" DL_API int dl_fold_layers(const int64_t *const *a, const int64_t *con
     return launch_status("dl_fold_layers");
 }
 
+extern "C" DL_API int64_t dl_fold_tail_bytes(const int64_t *n, int layers, int64_t k) {
+    FoldShape sh;
+    TailTable t;
+    if (!fold_shape(n, layers, &sh) || k < 1 || n[layers] % k != 0) return 0;
+    return tail_table(n[layers], k, &t, nullptr);
+}
+extern "C" DL_API int dl_fold_tail(const void *work, const int64_t *n, int layers, int64_t k, void *table, void *stream) {
+    FoldShape sh;
+    TailTable t;
+    DL_REQUIRE(work && n && table && aligned_to(work, 16) && aligned_to(table, 16), DL_ERR_INVALID_ARG, "dl_fold_tail: null or unaligned pointer");
+    DL_REQUIRE(fold_shape(n, layers, &sh) && k >= 1 && n[layers] % k == 0, DL_ERR_INVALID_ARG, "dl_fold_tail: bad sizes");
+    const int rows = sh.n[layers], rows_per_class = (int)(rows / k);
+    tail_table(rows, k, &t, table);
+    GateList list = gate_list(sh, const_cast<void *>(work));
+    const int64_t tail = sh.first[layers] - sh.n[0];
+    list.a += tail;
+    list.b += tail;
+    list.gate += tail;
+    cudaStream_t st = as_stream(stream);
+    if (cudaMemsetAsync(t.ones, 0, (size_t)(2 * k) * sizeof(int32_t), st) != cudaSuccess) return launch_status("dl_fold_tail (clear)");
+    const dim3 grid((unsigned)ceil_div(rows, kThreads));
+    launch_dependent(false, tail_count_kernel, grid, dim3(kThreads), 0, st, t, rows, rows_per_class, (const uint8_t *)list.gate);
+    launch_dependent(true, tail_start_kernel, dim3(1), dim3(1024), 0, st, t, (int)k);
+    launch_dependent(true, tail_place_kernel, grid, dim3(kThreads), 0, st, t, rows, rows_per_class, list);
+    return launch_status("dl_fold_tail");
+}
+
 extern "C" DL_API int dl_eval_folded(const void *x, const void *work, const int64_t *n, const int32_t *left, int layers, void *pool,
-                                     int32_t *out, void *rows_out, int64_t row_bytes, int64_t batch, int64_t k, void *stream) {
+                                     const void *table, int64_t longest, int32_t *out, void *rows_out, int64_t row_bytes, int64_t batch,
+                                     int64_t k, void *stream) {
     const char *who = "dl_eval_folded";
     FoldShape sh;
     DL_REQUIRE(x && work && n && left && (out != nullptr) != (rows_out != nullptr) && aligned_to(work, 16), DL_ERR_INVALID_ARG, "%s: null pointer", who);
@@ -102,8 +220,9 @@ extern "C" DL_API int dl_eval_folded(const void *x, const void *work, const int6
     }
     DL_REQUIRE(pool != nullptr || rows == 0, DL_ERR_INVALID_ARG, "%s: null pointer", who);
     const int64_t m = n[layers] / k;
-    const bool whole = dl_eval_groupbitsum_applicable(x, n[0], n[layers], row_bytes, 8, k) == 1;
-    DL_REQUIRE(out == nullptr || (aligned_to(pool, 16) && (whole || dl_eval_groupbitsum_parts_applicable(x, n[0], n[layers], row_bytes, 8, k) == 1)),
+    DL_REQUIRE(out == nullptr || (table && aligned_to(table, 16) && longest >= 0 && longest <= m), DL_ERR_INVALID_ARG, "%s: counts need a table", who);
+    DL_REQUIRE(out == nullptr || (aligned_to(pool, 16) && (dl_eval_groupbitsum_applicable(x, n[0], n[layers], row_bytes, 8, k) == 1 ||
+                                                           dl_eval_groupbitsum_parts_applicable(x, n[0], n[layers], row_bytes, 8, k) == 1)),
                DL_ERR_INVALID_ARG, "%s: counts outside the range of dl_eval_groupbitsum and dl_eval_groupbitsum_parts", who);
     const GateList list = gate_list(sh, const_cast<void *>(work));
     const SplitRows src = {reinterpret_cast<const uint8_t *>(x), reinterpret_cast<const uint8_t *>(pool), n[0]};
@@ -116,7 +235,12 @@ extern "C" DL_API int dl_eval_folded(const void *x, const void *work, const int6
             return e;
     }
     const int64_t tail = sh.first[layers] - sh.n[0];
-    if (out != nullptr)
-        return eval_class_counts(src, list.a + tail, list.b + tail, list.gate + tail, out, row_bytes, batch, k, m, !whole, as_stream(stream));
+    if (out != nullptr) {
+        TailTable t;
+        tail_table(n[layers], k, &t, const_cast<void *>(table));
+        const ClassRows classes = {t.start, t.ones, longest > 0 ? (int)longest : 1};
+        return eval_class_counts(src, t.list.a, t.list.b, t.list.gate, out, row_bytes, batch, k, classes, class_counts_in_parts(classes.m),
+                                 as_stream(stream));
+    }
     return eval_rows(src, list.a + tail, list.b + tail, list.gate + tail, rows_out, n[layers - 1], n[layers], row_bytes, as_stream(stream));
 }

@@ -567,12 +567,16 @@ class NetworkProgram:
             N.check_status(build(pointers[0], pointers[1], pointers[2], self.sizes, count, program.data_ptr(), stream.cuda_stream))
         program._dl_stream = stream.cuda_stream
 
-    def _make_table(self, program, k):
+    def _table_of(self, program, k, stream):
         layers = len(self.layers)
         table = torch.empty(N.lib().dl_network_table_words(self.sizes, layers, k), dtype=torch.int32, device=program.device)
+        N.check_status(N.lib().dl_network_table(program.data_ptr(), self.sizes, layers, k, table.data_ptr(), stream))
+        return table
+
+    def _make_table(self, program, k):
         with N.on_device(program):
             stream = N.stream_of(program)
-            N.check_status(N.lib().dl_network_table(program.data_ptr(), self.sizes, layers, k, table.data_ptr(), stream))
+            table = self._table_of(program, k, stream)
         table._dl_stream = stream
         if len(program._dl_tables) >= 4:
             program._dl_tables = {}
@@ -627,16 +631,27 @@ class FoldedLayers(NetworkProgram):
             torch.cuda.synchronize(device)
         program = torch.empty(N.lib().dl_fold_layers_bytes(self.sizes, count), dtype=torch.uint8, device=device)
         self._launch(N.lib().dl_fold_layers, program)
-        # other threads and streams may take the program from here on: this waits for it
+        program._dl_tables = {}
+        if self.counted is not None:
+            self._make_table(program, self.counted)
+        # other threads and streams may take program and table from here on: this waits for them
         left = program[:4 * count].view(torch.int32).tolist()
         program._dl_left = (ctypes.c_int32 * count)(*left)
         self.rows = sum(left[1:])
+        # fewer rows to compute than by whole layers, and at most half as much memory again as two activations of the widest layer
+        self.pays = self.rows * 10 <= 9 * sum(self.sizes[1:-1]) and self.rows <= 3 * max(self.sizes[1:])
         self.program = program
 
-    def pays(self):
-        """Whether this takes less than whole layers: fewer rows to compute, and at most half as much memory again as two
-        activations of the widest layer."""
-        return self.rows * 10 <= 9 * sum(self.sizes[1:-1]) and self.rows <= 3 * max(self.sizes[1:])
+    def _table_of(self, program, k, stream):
+        layers = len(self.layers)
+        table = torch.empty(N.lib().dl_fold_tail_bytes(self.sizes, layers, k), dtype=torch.uint8, device=program.device)
+        N.check_status(N.lib().dl_fold_tail(program.data_ptr(), self.sizes, layers, k, table.data_ptr(), stream))
+        at = 16 * self.sizes[layers]
+        table._dl_longest = int(table[at:at + 4].view(torch.int32))
+        return table
+
+    def serves(self, x, k):
+        return super().serves(x, k) and self.pays
 
 
 def network_sizes(n_in, layers):
@@ -693,11 +708,13 @@ def eval_folded(x, network, batch, k=None):
     else:
         out = torch.empty((int(batch), int(k)), dtype=torch.int32, device=x.device)
     with N.on_device(x):
+        table = None if k is None else network.table(program, int(k))
         stream = N.stream_of(x)
-        if stream != program._dl_stream:
-            program.record_stream(torch.cuda.current_stream(x.device))
+        for t in (program, table):
+            if t is not None and stream != t._dl_stream:
+                t.record_stream(torch.cuda.current_stream(x.device))
         N.check(N.lib().dl_eval_folded(x.data_ptr(), program.data_ptr(), sizes, program._dl_left, len(sizes) - 1, pool.data_ptr(),
-                                       0 if k is None else out.data_ptr(), out.data_ptr() if k is None else 0, row_bytes, int(batch),
+                                       N.ptr(table), 0 if k is None else table._dl_longest, 0 if k is None else out.data_ptr(), out.data_ptr() if k is None else 0, row_bytes, int(batch),
                                        1 if k is None else int(k), stream))
     return out
 

@@ -148,10 +148,10 @@ class PackBitsTensor:
             if not at_once:
                 return False
         if network.program is None:
-            if counts and not folded:
+            if counts and (not folded or self._counts_with_last_layer(self._pending[-1][0].out_dim, k)):
                 network.counted = k
             network.build()
-        return False if folded and not network.pays() else network
+        return False if folded and not network.pays else network
 
     def _run(self, network, batch, k=None):
         """The class counts of the pending layers, without k the last one's rows; None where there is no memory for the rows of

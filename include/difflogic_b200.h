@@ -242,15 +242,20 @@ DL_API int dl_eval_network_sized(const void *x, const uint32_t *program, const i
  *   dl_fold_layers_bytes        bytes of `work` (16-byte aligned), 0 for sizes outside the range
  *   dl_fold_layers              fills work from every layer's connections and gate ids (HOST arrays of device pointers); its first
  *                               words, int32, then say how many gates of layer l = 1 .. layers - 1 are left (word l).
+ *   dl_fold_tail                table for counting the last layer's rows in k classes, dl_fold_tail_bytes() of them, 16-byte aligned;
+ *                               at byte 16 * n[layers] it then says, int32, how many neurons the longest class has.
  *   dl_eval_folded              x [n[0]][row_bytes] -> out [batch][k] class counts, in the range of dl_eval_groupbitsum or
  *                               dl_eval_groupbitsum_parts, or the last layer's rows rows_out [n[layers]][row_bytes]; one of the two
- *                               is null.  left: those words, on the HOST.  pool: room for their sum in rows of row_bytes.
+ *                               is null.  left: those words, on the HOST.  pool: room for their sum in rows of row_bytes.  For counts:
+ *                               the table for k and that number.
  * The counts and rows are those of dl_eval_packed per layer followed by dl_groupbitsum. */
 DL_API int64_t dl_fold_layers_bytes(const int64_t *n, int layers);
 DL_API int dl_fold_layers(const int64_t *const *a, const int64_t *const *b, const uint8_t *const *gate, const int64_t *n, int layers,
                           void *work, void *stream);
-DL_API int dl_eval_folded(const void *x, const void *work, const int64_t *n, const int32_t *left, int layers, void *pool, int32_t *out,
-                          void *rows_out, int64_t row_bytes, int64_t batch, int64_t k, void *stream);
+DL_API int64_t dl_fold_tail_bytes(const int64_t *n, int layers, int64_t k);
+DL_API int dl_fold_tail(const void *work, const int64_t *n, int layers, int64_t k, void *table, void *stream);
+DL_API int dl_eval_folded(const void *x, const void *work, const int64_t *n, const int32_t *left, int layers, void *pool, const void *table,
+                          int64_t longest, int32_t *out, void *rows_out, int64_t row_bytes, int64_t batch, int64_t k, void *stream);
 
 /* argmax over the 16 gate weights -> uint8 gate id, first maximum on ties
  * (weights.argmax(-1).to(uint8), difflogic/difflogic.py:146). */
