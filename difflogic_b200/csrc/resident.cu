@@ -375,7 +375,7 @@ template <int WORDS, int T, int R>
 __global__ void __launch_bounds__(T, 1024 / T)
 resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t *__restrict__ prog, ResidentSizes sz,
                 const uint32_t *__restrict__ table, int32_t *__restrict__ out, uint8_t *__restrict__ rows_out, int64_t batch, int k,
-                int rows_per_class, int row_slots) {
+                int rows_per_class, int row_slots, int ahead) {
     using Row = typename ResRow<WORDS>::type;
     constexpr int V = 4 * WORDS, W = T / 32;
     static_assert(R % 2 == 0, "gates are taken in pairs");
@@ -384,21 +384,36 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
     int *counts = reinterpret_cast<int *>(res_smem + (size_t)row_slots * V);  // [k][WORDS][33]: a word's samples, and no two words' in a bank
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
 
+    // The input's rows, four per thread at a time; what else a block needs to begin with is fetched while the first four are on
+    // their way (one after the other the loads took 2500 of a block's 36000 cycles more).
     const uint8_t *src = x + (int64_t)blockIdx.x * V;
-    for (int i = tid; i < sz.n[0]; i += T) rows[i] = __ldg(reinterpret_cast<const Row *>(src + (int64_t)i * row_bytes));
+    const uint32_t *level = prog + kResHeader;
+    int and_end = (int)__ldg(level), n = (int)__ldg(level + 1);
     const int zero_row = (int)__ldg(prog);
-    // the rows to be counted, by class: those of a table, or all in their own order
+    constexpr int kBatch = 4;
+    Row in[kBatch];
+    auto load = [&](int i) {
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+            if (i + u * T < sz.n[0]) in[u] = __ldg(reinterpret_cast<const Row *>(src + (int64_t)(i + u * T) * row_bytes));
+    };
+    auto store = [&](int i) {
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+            if (i + u * T < sz.n[0]) rows[i + u * T] = in[u];
+    };
+    load(tid);
+    // the rows to be counted, by class: those of a table, or all in their own order; behind their beginnings the constants
     const uint32_t *start_of = table != nullptr ? table + (sz.n[sz.layers] + (int64_t)k * 8 * kResClasses + 7) / 8 * 4 : nullptr;
     constexpr int kPitch = kResPitch * WORDS;
-    int *starts = counts + kPitch * k;  // [k + 1]
+    int *starts = counts + kPitch * k, *ones = starts + k + 1;
     if (rows_out == nullptr) {
-        for (int t = tid; t <= k; t += T) starts[t] = start_of != nullptr ? (int)__ldg(start_of + t) : t * rows_per_class;
-        for (int t = tid; t < kPitch * k; t += T) counts[t] = start_of != nullptr ? (int)__ldg(start_of + k + 1 + t / kPitch) : 0;
+        for (int t = tid; t < 2 * k + 1; t += T) starts[t] = start_of != nullptr ? (int)__ldg(start_of + t) : t <= k ? t * rows_per_class : 0;
+        for (int t = tid; t < kPitch * k; t += T) counts[t] = 0;
     }
 
     // layer l: `level`; its output slots are fetched before its gates are evaluated, the gates of the next one behind the last use of
     // the slots (held at the same time they do not fit the registers) and, so that this is short, into L1 before
-    const uint32_t *level = prog + kResHeader;
     uint2 w[R / 2];
     uint32_t o[R / 2];
     auto fetch_gates = [&](const uint32_t *at, int gates) {
@@ -408,8 +423,15 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
             w[r] = chunk * 64 < gates ? __ldg(reinterpret_cast<const uint2 *>(at + kResHeader) + chunk * 32 + lane) : make_uint2(0u, 0u);
         }
     };
-    int and_end = (int)__ldg(level), n = (int)__ldg(level + 1);
     fetch_gates(level, n);
+    store(tid);
+    for (int i = tid + kBatch * T; i < sz.n[0]; i += kBatch * T) {
+        load(i);
+        store(i);
+    }
+    // the block that will run here next finds its input in L2
+    if ((int64_t)blockIdx.x + ahead < gridDim.x)
+        for (int i = tid; i < sz.n[0]; i += T) prefetch_l2(src + (int64_t)ahead * V + (int64_t)i * row_bytes);
     __syncthreads();
     for (int l = 1; l <= sz.layers; ++l) {
         const uint32_t *outs = level + kResHeader + res_whole(sz.n[l]);
@@ -419,9 +441,12 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
             o[r] = chunk * 64 < n ? __ldg(outs + chunk * 32 + lane) : 0u;
         }
         if (l < sz.layers) {
-            const uint32_t *ahead = level + res_layer_words(sz.n[l]);
+            const uint32_t *following = level + res_layer_words(sz.n[l]);
             for (int t = tid * 32; t < kResHeader + (int)sz.n[l + 1]; t += T * 32)
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(ahead + t));
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(following + t));
+        } else if (start_of != nullptr && rows_out == nullptr) {
+            for (int t = tid * 64; t < starts[k]; t += T * 64)
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const uint16_t *>(table) + t));
         }
         Row y[R];
 #pragma unroll
@@ -579,7 +604,8 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
     const float per_sample = 1.f / (float)k;
     for (int t = tid; t < live; t += T) {
         const int sample = (int)(((float)t + 0.5f) * per_sample);  // t / k: t < 2^21, so the error stays below the half
-        out[s0 * k + t] = counts[(t - sample * k) * kPitch + sample / 32 * kResPitch + sample % 32];
+        const int c = t - sample * k;
+        out[s0 * k + t] = counts[c * kPitch + sample / 32 * kResPitch + sample % 32] + ones[c];
     }
 }
 
@@ -589,7 +615,7 @@ static int res_sms() {
     return n;
 }
 static size_t res_shared_bytes(int64_t row_slots, int V, int64_t k) {
-    return (size_t)row_slots * V + ((size_t)kResPitch * (V / 4) * k + k + 1) * sizeof(int);
+    return (size_t)row_slots * V + ((size_t)kResPitch * (V / 4) * k + 2 * k + 1) * sizeof(int);
 }
 
 constexpr size_t kResMaxShared = 227 * 1024;
@@ -648,8 +674,10 @@ static int launch_resident(const void *x, int64_t row_bytes, const uint32_t *pro
     // the most there may be, not this launch's bytes: the limit is the kernel's, and other threads launch it for other networks
     if (cudaFuncSetAttribute(resident_kernel<WORDS, T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResMaxShared) != cudaSuccess)
         return launch_status("dl_eval_network (shared memory opt-in)");
+    const int at_a_time = (int)(kResMaxShared / (smem + 1024)), per_sm = at_a_time < 1024 / T ? (at_a_time < 1 ? 1 : at_a_time) : 1024 / T;
     resident_kernel<WORDS, T, R><<<(unsigned)ceil_div(batch, 8 * V), T, smem, st>>>(
-        reinterpret_cast<const uint8_t *>(x), row_bytes, prog, sz, table, out, rows_out, batch, (int)k, (int)(sz.n[sz.layers] / k), row_slots);
+        reinterpret_cast<const uint8_t *>(x), row_bytes, prog, sz, table, out, rows_out, batch, (int)k, (int)(sz.n[sz.layers] / k), row_slots,
+        res_sms() * per_sm);
     return launch_status("dl_eval_network");
 }
 
