@@ -154,6 +154,156 @@ tail_place_kernel(TailTable t, int n, int rows_per_class, GateList from) {
     t.list.gate[at] = (uint8_t)op;
 }
 
+// ---------------------------------------------------------------------------------------------
+// class counts of a folded last layer
+// ---------------------------------------------------------------------------------------------
+// A CTA takes (512 bytes of the rows, class, part of its neurons), a warp an eighth of those: lane l holds 16 bytes of the columns and
+// adds the gates' outputs up bit by bit (carry-save, eight neurons at a time); the sixteen loads of eight neurons are in flight at
+// once, straight into registers.  What a warp needs to know of 32 neurons lies in shared memory.  At the end the eight warps' sums meet
+// there, as planes, and become integers that are stored, or added where a class has several parts.
+//
+// eval_groupbitsum_kernel stages rows in shared memory for eight neurons at a time and takes its 1.2 us for them whatever the length of
+// the rows, from 512 bytes on; its 2 KB pieces suit long rows.  Whole folded passes, us, that kernel / this one: 9216 -> 4 x 128000, rows of
+// 576 bytes 135 / 108, 1264 158 / 138, 4096 364 / 352; 256 -> 12 x 64000, 4096 277 / 273, 16384 1027 / 1028; 784 -> 2 x 20000, 1264 42 / 29, 16384
+// 130 / 142; 784 -> 5 x 32000 in 100 classes, 1264 70 / 61, 16384 423 / 453.
+constexpr int64_t kTailLongest = 4096;  // bytes of a row
+constexpr int kTailWarps = kThreads / 32, kTailPlanes = 10, kTailShare = (1 << kTailPlanes) - 1;  // neurons of a warp at most
+constexpr int kTailSum = kTailPlanes + 3;                                                          // planes of a CTA's sums
+constexpr uint32_t kTailMore = 1u << 31;  // of an offset: in the second buffer
+
+#define DL_TAIL_CSA(h, l, a, b, c)     \
+    {                                  \
+        const uint32_t u_ = (a) ^ (b); \
+        const uint32_t c_ = (c);       \
+        h = ((a) & (b)) | (u_ & c_);   \
+        l = u_ ^ c_;                   \
+    }
+
+__global__ void __launch_bounds__(kThreads, 2)
+tail_counts_kernel(const SplitRows x, const int64_t *__restrict__ a, const int64_t *__restrict__ b, const uint8_t *__restrict__ gate,
+                   const int32_t *__restrict__ start, const int32_t *__restrict__ ones, int32_t *__restrict__ out, int64_t row_bytes,
+                   int64_t batch, int k, int parts) {
+    __shared__ uint4 s_mask[kTailWarps][32];
+    __shared__ uint2 s_row[kTailWarps][32];                 // offsets of both inputs, in 16-byte units
+    __shared__ uint32_t s_plane[kTailWarps][kTailPlanes][128];
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    const int c = blockIdx.x % k, part = blockIdx.x / k;
+    const int64_t col = (int64_t)blockIdx.y * 512 + lane * 16;
+    const bool live = col < row_bytes;
+    const int begin = __ldg(start + c), len = __ldg(start + c + 1) - begin;
+    const int from = begin + (int)((int64_t)len * part / parts), to = begin + (int)((int64_t)len * (part + 1) / parts);
+    const int mine = from + (int)((int64_t)(to - from) * warp / kTailWarps), end = from + (int)((int64_t)(to - from) * (warp + 1) / kTailWarps);
+    const int64_t units = row_bytes / 16;
+    const uint4 *base = reinterpret_cast<const uint4 *>(x.x + col), *more = reinterpret_cast<const uint4 *>(x.more + col);
+
+    uint32_t p[4][kTailPlanes];
+#pragma unroll
+    for (int w = 0; w < 4; ++w)
+#pragma unroll
+        for (int i = 0; i < kTailPlanes; ++i) p[w][i] = 0u;
+    for (int j0 = mine; j0 < end; j0 += 32) {
+        {
+            const int j = j0 + lane;
+            uint2 rows = make_uint2(0u, 0u);
+            GateMasks m = {0u, 0u, 0u, 0u};
+            if (j < end) {
+                const int64_t ia = __ldg(a + j), ib = __ldg(b + j);
+                rows.x = ia < x.split ? (uint32_t)(ia * units) : (uint32_t)((ia - x.split) * units) | kTailMore;
+                rows.y = ib < x.split ? (uint32_t)(ib * units) : (uint32_t)((ib - x.split) * units) | kTailMore;
+                m = gate_masks(__ldg(gate + j));
+            }
+            __syncwarp();
+            s_row[warp][lane] = rows;
+            s_mask[warp][lane] = make_uint4(m.m0, m.ma, m.mb, m.mab);
+            __syncwarp();
+        }
+        const int here = min(32, end - j0);
+        for (int g = 0; g < here; g += 8) {
+            uint4 va[8], vb[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint2 r = s_row[warp][g + i];
+                const uint4 m = s_mask[warp][g + i];
+                va[i] = vb[i] = make_uint4(0u, 0u, 0u, 0u);
+                if ((m.y | m.w) != 0u && live) va[i] = __ldg((r.x & kTailMore ? more : base) + (r.x & ~kTailMore));
+                if ((m.z | m.w) != 0u && live) vb[i] = __ldg((r.y & kTailMore ? more : base) + (r.y & ~kTailMore));
+            }
+            uint32_t two[4], four[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint4 m0 = s_mask[warp][g + 2 * q], m1 = s_mask[warp][g + 2 * q + 1];
+                const uint32_t a0[4] = {va[2 * q].x, va[2 * q].y, va[2 * q].z, va[2 * q].w}, b0[4] = {vb[2 * q].x, vb[2 * q].y, vb[2 * q].z, vb[2 * q].w};
+                const uint32_t a1[4] = {va[2 * q + 1].x, va[2 * q + 1].y, va[2 * q + 1].z, va[2 * q + 1].w},
+                               b1[4] = {vb[2 * q + 1].x, vb[2 * q + 1].y, vb[2 * q + 1].z, vb[2 * q + 1].w};
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    const uint32_t v0 = gate32(a0[w], b0[w], {m0.x, m0.y, m0.z, m0.w}), v1 = gate32(a1[w], b1[w], {m1.x, m1.y, m1.z, m1.w});
+                    uint32_t t, f;
+                    DL_TAIL_CSA(t, p[w][0], p[w][0], v0, v1);
+                    if (q % 2 == 0) {
+                        two[w] = t;
+                    } else {
+                        DL_TAIL_CSA(f, p[w][1], p[w][1], two[w], t);
+                        if (q == 1) {
+                            four[w] = f;
+                        } else {
+                            uint32_t carry;
+                            DL_TAIL_CSA(carry, p[w][2], p[w][2], four[w], f);
+#pragma unroll
+                            for (int i = 3; i < kTailPlanes; ++i) {
+                                const uint32_t n = p[w][i] & carry;
+                                p[w][i] ^= carry;
+                                carry = n;
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    }
+    // ---- the warps' sums meet; a thread adds up those of one word of 32 samples and takes half of the samples on ----
+#pragma unroll
+    for (int i = 0; i < kTailPlanes; ++i) *reinterpret_cast<uint4 *>(&s_plane[warp][i][lane * 4]) = make_uint4(p[0][i], p[1][i], p[2][i], p[3][i]);
+    __syncthreads();
+    const int word = tid % 128, first = tid / 128 * 16;
+    const int64_t s0 = ((int64_t)blockIdx.y * 512 + word * 4) * 8 + first;
+    if (s0 >= batch) return;
+    uint32_t sum[kTailSum];
+#pragma unroll
+    for (int i = 0; i < kTailSum; ++i) sum[i] = 0u;
+#pragma unroll
+    for (int r = 0; r < kTailWarps; ++r) {
+        uint32_t carry = 0u;
+#pragma unroll
+        for (int i = 0; i < kTailSum; ++i) {
+            uint32_t h, l;
+            DL_TAIL_CSA(h, l, sum[i], i < kTailPlanes ? s_plane[r][i][word] : 0u, carry);
+            sum[i] = l;
+            carry = h;
+        }
+    }
+    const int always = part == 0 ? __ldg(ones + c) : 0;
+    int32_t *dst = out + s0 * k + c;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // four samples: a nibble of each plane -> a bit in each of four bytes
+        uint32_t low = 0u, high = 0u;
+#pragma unroll
+        for (int i = 0; i < kTailSum; ++i) {
+            const uint32_t bits = (((sum[i] >> (first + 4 * q)) & 15u) * 0x00204081u) & 0x01010101u;
+            if (i < 8) low |= bits << i;
+            else high |= bits << (i - 8);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int count = (int)((low >> (8 * i)) & 255u) + ((int)((high >> (8 * i)) & 255u) << 8) + always;
+            if (s0 + 4 * q + i < batch) {
+                if (parts == 1) dst[(int64_t)(4 * q + i) * k] = count;
+                else if (count != 0) atomicAdd(dst + (int64_t)(4 * q + i) * k, count);
+            }
+        }
+    }
+}
+
 }  // namespace dl
 
 using namespace dl;
@@ -221,9 +371,12 @@ extern "C" DL_API int dl_eval_folded(const void *x, const void *work, const int6
     DL_REQUIRE(pool != nullptr || rows == 0, DL_ERR_INVALID_ARG, "%s: null pointer", who);
     const int64_t m = n[layers] / k;
     DL_REQUIRE(out == nullptr || (table && aligned_to(table, 16) && longest >= 0 && longest <= m), DL_ERR_INVALID_ARG, "%s: counts need a table", who);
-    DL_REQUIRE(out == nullptr || (aligned_to(pool, 16) && (dl_eval_groupbitsum_applicable(x, n[0], n[layers], row_bytes, 8, k) == 1 ||
-                                                           dl_eval_groupbitsum_parts_applicable(x, n[0], n[layers], row_bytes, 8, k) == 1)),
-               DL_ERR_INVALID_ARG, "%s: counts outside the range of dl_eval_groupbitsum and dl_eval_groupbitsum_parts", who);
+    const bool staged = aligned_to(pool, 16) && (dl_eval_groupbitsum_applicable(x, n[0], n[layers], row_bytes, 8, k) == 1 ||
+                                                 dl_eval_groupbitsum_parts_applicable(x, n[0], n[layers], row_bytes, 8, k) == 1);
+    const int64_t most_rows = rows > n[0] ? rows : n[0];
+    const bool direct = row_bytes % 16 == 0 && aligned_to(x, 16) && aligned_to(pool, 16) && most_rows * (row_bytes / 16) <= INT32_MAX &&
+                        ceil_div(row_bytes, 512) <= 65535 && k * (ceil_div(m, 64) + 1) <= INT32_MAX;
+    DL_REQUIRE(out == nullptr || staged || direct, DL_ERR_INVALID_ARG, "%s: rows whose classes no kernel counts", who);
     const GateList list = gate_list(sh, const_cast<void *>(work));
     const SplitRows src = {reinterpret_cast<const uint8_t *>(x), reinterpret_cast<const uint8_t *>(pool), n[0]};
     int64_t at = rows;  // the first layer's gates come last
@@ -239,6 +392,24 @@ extern "C" DL_API int dl_eval_folded(const void *x, const void *work, const int6
         TailTable t;
         tail_table(n[layers], k, &t, const_cast<void *>(table));
         const ClassRows classes = {t.start, t.ones, longest > 0 ? (int)longest : 1};
+        if (direct && (!staged || row_bytes <= kTailLongest)) {
+            // parts: as many as leave the busiest of the CTAs that run at a time (two per SM) the fewest neurons; 200: what a part costs besides
+            const int64_t blocks = ceil_div(row_bytes, 512), slots = 2 * 148, fewest = ceil_div(classes.m, kTailShare * kTailWarps);
+            int64_t parts = fewest, least = 0;
+            for (int64_t p = fewest; p <= fewest + 64 && (p == fewest || p <= classes.m / 64); ++p) {
+                const int64_t cost = ceil_div(blocks * k * p, slots) * (ceil_div(classes.m, p) + 200);
+                if (least == 0 || cost < least) {
+                    least = cost;
+                    parts = p;
+                }
+            }
+            cudaStream_t st = as_stream(stream);
+            if (parts > 1 && cudaMemsetAsync(out, 0, (size_t)batch * k * sizeof(int32_t), st) != cudaSuccess)
+                return launch_status("dl_eval_folded (clear)");
+            tail_counts_kernel<<<dim3((unsigned)(k * parts), (unsigned)blocks), kThreads, 0, st>>>(
+                src, t.list.a, t.list.b, t.list.gate, t.start, t.ones, out, row_bytes, batch, (int)k, (int)parts);
+            return launch_status("dl_eval_folded");
+        }
         return eval_class_counts(src, t.list.a, t.list.b, t.list.gate, out, row_bytes, batch, k, classes, class_counts_in_parts(classes.m),
                                  as_stream(stream));
     }

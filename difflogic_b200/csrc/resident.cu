@@ -250,7 +250,9 @@ res_outputs_kernel(ResBuild p, int n, const int32_t *__restrict__ ref, const uin
 // ---------------------------------------------------------------------------------------------
 // By class: constants that are true (they are counted once and for all), and the rows, dealt out over the bank classes as above.
 // A class begins with a whole group of 8 NC entries.  A lane of the counting loop loads eight entries at a time, so the entries
-// of a group lie lane by lane: entry q at (q mod NC) * 8 + q / NC.  What a class does not fill reads the row of zeros.
+// of a group lie lane by lane: entry q at (q mod NC) * 8 + q / NC.  Short classes, of which groups would be mostly empty, take whole
+// eights instead, in order.  What a class does not fill reads the row of zeros.
+constexpr int kResShort = 256;  // rows of a class
 struct ResTable {
     uint32_t *start;    // [k + 1] first entry, by class
     uint32_t *ones;     // [k]
@@ -288,11 +290,11 @@ res_table_count_kernel(ResTable t, int n, int rows_per_class, const uint32_t *__
 }
 
 __global__ void __launch_bounds__(1024)
-res_table_start_kernel(ResTable t, int k, const uint32_t *__restrict__ prog) {
+res_table_start_kernel(ResTable t, int k, int rows_per_class, const uint32_t *__restrict__ prog) {
     __shared__ int s_sum[1024];
     grid_dependency_wait();
     grid_dependents_launch();
-    const int tid = threadIdx.x, each = (k + 1023) / 1024, group = 8 * (int)__ldg(prog + 2);
+    const int tid = threadIdx.x, each = (k + 1023) / 1024, group = rows_per_class < kResShort ? 8 : 8 * (int)__ldg(prog + 2);
     auto entries = [&](int c) {
         int rows = 0;
         for (int i = 0; i < kResClasses; ++i) rows += __ldcg(t.count + (int64_t)c * kResClasses + i);
@@ -331,7 +333,8 @@ res_table_place_kernel(ResTable t, int n, int rows_per_class, const uint32_t *__
         q += min(have, rank) + (i < cls && have > rank ? 1 : 0);
     }
     const int group = 8 * nc;
-    t.entries[__ldcg(t.start + c) + q / group * group + q % nc * 8 + q % group / nc] = (uint16_t)e;
+    if (rows_per_class >= kResShort) q = q / group * group + q % nc * 8 + q % group / nc;
+    t.entries[__ldcg(t.start + c) + q] = (uint16_t)e;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -370,12 +373,167 @@ __device__ __forceinline__ uint32_t res_mask15(uint32_t w) {
         l = u_ ^ c_;                   \
     }
 
+// Rows that a group of lanes counts side by side: all that a warp has lanes for, or fewer where there are more classes than warps.
+template <int WORDS, int T>
+__device__ __forceinline__ int res_side_by_side(int k) {
+    constexpr int kParts = WORDS < 2 ? 1 : WORDS / 2;
+    int subs = 32 / kParts;
+    while (subs > 1 && subs * kParts * k > T) subs /= 2;
+    return subs;
+}
+
+// The counts of many classes: groups of as few lanes as there are classes for (down to the parts of one row) take a class each, and
+// the sums over the lanes, which cost as much as 200 rows, shrink with them.  400 -> 4 x 1000, 100 classes, 2^18 samples: 193 us with a
+// warp per class, 120 so; 400 -> 3 x 8000, 1000 classes, 2^14: 308 and 74.  A function of its own: as part of the kernel it takes
+// registers away from the layers (784 -> 12 x 12000: 189 -> 206 us).
+template <int WORDS, int T>
+__device__ __noinline__ void res_count_many(int row_slots, const uint32_t *__restrict__ table, const uint16_t *__restrict__ outputs,
+                                               int zero_row, int k) {
+    constexpr int V = 4 * WORDS, kPitch = kResPitch * WORDS;
+    extern __shared__ __align__(16) uint8_t res_smem[];
+    int *counts = reinterpret_cast<int *>(res_smem + (size_t)row_slots * V);
+    const int *starts = counts + kPitch * k;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    constexpr int kWords = WORDS < 2 ? 1 : 2, kParts = WORDS / kWords;  // words of a lane, lanes of a row
+    constexpr int kSubs = 32 / kParts;
+    constexpr int kSteps = kSubs == 16 ? 4 : 5;                        // of adding up over the lanes, at most
+    constexpr int kLane = 6, kPlanes = kLane + kSteps;                 // planes of a lane's count, and of the sum
+    constexpr int kLaneRows = 56;                                      // rows of a lane at a time at most
+    using Pair = typename ResRow<kWords>::type;
+    const int subs = res_side_by_side<WORDS, T>(k);
+    const int part = lane % kParts;
+    const uint8_t *mine = res_smem + part * (int)sizeof(Pair);
+    auto fetch = [&](int r, int end) {
+        const uint32_t none = (uint32_t)zero_row << 16 | (uint32_t)zero_row;
+        uint4 e = make_uint4(none, none, none, none);
+        if (table != nullptr) {
+            if (r < end) e = __ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(table) + r));
+        } else {
+            uint32_t *half = &e.x;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (r + 2 * i < end) half[i] = (half[i] & 0xffff0000u) | __ldg(outputs + r + 2 * i);
+                if (r + 2 * i + 1 < end) half[i] = (half[i] & 0xffffu) | (uint32_t)__ldg(outputs + r + 2 * i + 1) << 16;
+            }
+        }
+        return e;
+    };
+    // rows pos .. end - 1 (at most kLaneRows * subs) of class c, which may be none; all groups of a warp together.
+    auto count_rows = [&](int c, int pos, int end) {
+        const int sub = lane / kParts % subs, stride = 8 * subs;
+
+        uint32_t p[kWords][kPlanes];
+#pragma unroll
+        for (int i = 0; i < kPlanes; ++i)
+#pragma unroll
+            for (int h = 0; h < kWords; ++h) p[h][i] = 0u;
+        auto add8 = [&](uint32_t (&q)[kPlanes], const uint32_t (&v)[8]) {
+            uint32_t t2a, t2b, t4a, t4b, carry;
+            DL_CSA32(t2a, q[0], q[0], v[0], v[1]);
+            DL_CSA32(t2b, q[0], q[0], v[2], v[3]);
+            DL_CSA32(t4a, q[1], q[1], t2a, t2b);
+            DL_CSA32(t2a, q[0], q[0], v[4], v[5]);
+            DL_CSA32(t2b, q[0], q[0], v[6], v[7]);
+            DL_CSA32(t4b, q[1], q[1], t2a, t2b);
+            DL_CSA32(carry, q[2], q[2], t4a, t4b);
+#pragma unroll
+            for (int i = 3; i < kLane; ++i) {
+                const uint32_t t = q[i] & carry;
+                q[i] ^= carry;
+                carry = t;
+            }
+        };
+        int r = pos + sub * 8;
+        uint4 e = fetch(r, end);
+        while (__any_sync(0xffffffffu, r < end)) {
+            r += stride;
+            const uint4 next = fetch(r, end);
+            const uint32_t pairs[4] = {e.x, e.y, e.z, e.w};
+            uint32_t v[kWords][8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t one = i % 2 ? pairs[i / 2] >> 16 : pairs[i / 2], m = res_mask15(one);
+                const Pair row = *reinterpret_cast<const Pair *>(mine + (one & ((1u << kResOutput) - 1u)) * V);
+                v[0][i] = *reinterpret_cast<const uint32_t *>(&row) ^ m;
+                if (kWords == 2) v[kWords - 1][i] = (reinterpret_cast<const uint32_t *>(&row))[kWords - 1] ^ m;
+            }
+#pragma unroll
+            for (int h = 0; h < kWords; ++h) add8(p[h], v[h]);
+            e = next;
+        }
+        // four samples' counts, from a nibble of each plane a bit in each of four bytes, are added
+        auto put = [&](const uint32_t (&planes)[kPlanes], int word, int first, int from, int step) {
+            uint32_t low = 0u, high = 0u;
+#pragma unroll
+            for (int pl = 0; pl < kPlanes; ++pl) {
+                const uint32_t bits = (((planes[pl] >> first) & 15u) * 0x00204081u) & 0x01010101u;
+                if (pl < 8) low |= bits << pl;
+                else high |= bits << (pl - 8);
+            }
+            int *at = counts + c * kPitch + word * kResPitch + first;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int count = (int)((low >> (8 * i)) & 255u) | (int)((high >> (8 * i)) & 255u) << 8;
+                if (i % step == from && count) atomicAdd(at + i, count);
+            }
+        };
+        if (subs == 1) {
+#pragma unroll
+            for (int h = 0; h < kWords; ++h)
+#pragma unroll 1
+                for (int nibble = 0; nibble < 8; ++nibble) put(p[h], part * kWords + h, 4 * nibble, 0, 1);
+            return;
+        }
+        // sums over the lanes of a part, a plane more each time; in the first step a lane hands one of its two words over and
+        // keeps the other
+        const bool upper = kWords == 2 && (sub & 1);
+        uint32_t s[kPlanes];
+#pragma unroll
+        for (int i = 0; i < kPlanes; ++i) s[i] = upper ? p[kWords - 1][i] : p[0][i];
+#pragma unroll
+        for (int step = 0; step < kSteps; ++step) {
+            if (1 << step >= subs) break;
+            uint32_t carry = 0u;
+#pragma unroll
+            for (int i = 0; i < kLane + step; ++i) {
+                const uint32_t give = step == 0 && kWords == 2 ? (upper ? p[0][i] : p[kWords - 1][i]) : s[i];
+                const uint32_t o = __shfl_xor_sync(0xffffffffu, give, kParts << step);
+                uint32_t h, l;
+                DL_CSA32(h, l, s[i], o, carry);
+                s[i] = l;
+                carry = h;
+            }
+            s[kLane + step] = carry;
+        }
+        // the lanes that hold one word's sums share its samples, four at a time, or four among two lanes and more
+        const int holders = subs / kWords, holder = sub / kWords, word = part * kWords + (upper ? 1 : 0);
+        if (holders >= 8) {
+            const int share = holders / 8;
+            put(s, word, holder / share * 4, holder % share, share);
+        } else {
+#pragma unroll 1
+            for (int nibble = holder; nibble < 8; nibble += holders) put(s, word, 4 * nibble, 0, 1);
+        }
+    };
+    const int lanes = kParts * subs;
+    for (int c0 = warp * (32 / lanes); c0 < k; c0 += T / lanes) {
+        const int c = min(c0 + lane / lanes, k - 1);
+        int pos = starts[c];
+        const int stop = c0 + lane / lanes < k ? starts[c + 1] : pos;
+        while (__any_sync(0xffffffffu, pos < stop)) {
+            const int end = min(stop, pos + kLaneRows * subs);
+            count_rows(c, pos, end);
+            pos = end;
+        }
+    }
+}
+
 // WORDS: 32-bit words per row of a block (V = 4 * WORDS bytes); T threads; R gates per thread and layer at most.
 template <int WORDS, int T, int R>
 __global__ void __launch_bounds__(T, 1024 / T)
 resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t *__restrict__ prog, ResidentSizes sz,
                 const uint32_t *__restrict__ table, int32_t *__restrict__ out, uint8_t *__restrict__ rows_out, int64_t batch, int k,
-                int rows_per_class, int row_slots, int ahead) {
+                int rows_per_class, int row_slots) {
     using Row = typename ResRow<WORDS>::type;
     constexpr int V = 4 * WORDS, W = T / 32;
     static_assert(R % 2 == 0, "gates are taken in pairs");
@@ -384,36 +542,23 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
     int *counts = reinterpret_cast<int *>(res_smem + (size_t)row_slots * V);  // [k][WORDS][33]: a word's samples, and no two words' in a bank
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
 
-    // The input's rows, four per thread at a time; what else a block needs to begin with is fetched while the first four are on
-    // their way (one after the other the loads took 2500 of a block's 36000 cycles more).
     const uint8_t *src = x + (int64_t)blockIdx.x * V;
-    const uint32_t *level = prog + kResHeader;
-    int and_end = (int)__ldg(level), n = (int)__ldg(level + 1);
+    for (int i = tid; i < sz.n[0]; i += T) rows[i] = __ldg(reinterpret_cast<const Row *>(src + (int64_t)i * row_bytes));
     const int zero_row = (int)__ldg(prog);
-    constexpr int kBatch = 4;
-    Row in[kBatch];
-    auto load = [&](int i) {
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u)
-            if (i + u * T < sz.n[0]) in[u] = __ldg(reinterpret_cast<const Row *>(src + (int64_t)(i + u * T) * row_bytes));
-    };
-    auto store = [&](int i) {
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u)
-            if (i + u * T < sz.n[0]) rows[i + u * T] = in[u];
-    };
-    load(tid);
-    // the rows to be counted, by class: those of a table, or all in their own order; behind their beginnings the constants
+    // the rows to be counted, by class: those of a table, or all in their own order
     const uint32_t *start_of = table != nullptr ? table + (sz.n[sz.layers] + (int64_t)k * 8 * kResClasses + 7) / 8 * 4 : nullptr;
     constexpr int kPitch = kResPitch * WORDS;
-    int *starts = counts + kPitch * k, *ones = starts + k + 1;
+    int *starts = counts + kPitch * k;  // [k + 1]
     if (rows_out == nullptr) {
-        for (int t = tid; t < 2 * k + 1; t += T) starts[t] = start_of != nullptr ? (int)__ldg(start_of + t) : t <= k ? t * rows_per_class : 0;
-        for (int t = tid; t < kPitch * k; t += T) counts[t] = 0;
+        for (int t = tid; t <= k; t += T) starts[t] = start_of != nullptr ? (int)__ldg(start_of + t) : t * rows_per_class;
+        for (int t = tid; t < kPitch * k; t += T) counts[t] = start_of != nullptr ? (int)__ldg(start_of + k + 1 + t / kPitch) : 0;
     }
 
-    // layer l: `level`; its output slots are fetched before its gates are evaluated, the gates of the next one behind the last use of
-    // the slots (held at the same time they do not fit the registers) and, so that this is short, into L1 before
+    // layer l: `level`; its output slots are fetched before its gates are evaluated, the gates of the next one before the rows are
+    // exchanged (rows of 4 bytes) or behind the last use of the slots (wider ones: held at the same time they do not fit the registers)
+    // and, so that this is short, into L1 before
+    constexpr bool kEarly = WORDS == 1;
+    const uint32_t *level = prog + kResHeader;
     uint2 w[R / 2];
     uint32_t o[R / 2];
     auto fetch_gates = [&](const uint32_t *at, int gates) {
@@ -423,15 +568,8 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
             w[r] = chunk * 64 < gates ? __ldg(reinterpret_cast<const uint2 *>(at + kResHeader) + chunk * 32 + lane) : make_uint2(0u, 0u);
         }
     };
+    int and_end = (int)__ldg(level), n = (int)__ldg(level + 1);
     fetch_gates(level, n);
-    store(tid);
-    for (int i = tid + kBatch * T; i < sz.n[0]; i += kBatch * T) {
-        load(i);
-        store(i);
-    }
-    // the block that will run here next finds its input in L2
-    if ((int64_t)blockIdx.x + ahead < gridDim.x)
-        for (int i = tid; i < sz.n[0]; i += T) prefetch_l2(src + (int64_t)ahead * V + (int64_t)i * row_bytes);
     __syncthreads();
     for (int l = 1; l <= sz.layers; ++l) {
         const uint32_t *outs = level + kResHeader + res_whole(sz.n[l]);
@@ -440,13 +578,13 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
             const int chunk = warp + r * W;
             o[r] = chunk * 64 < n ? __ldg(outs + chunk * 32 + lane) : 0u;
         }
+        int next_and_end = 0, next_n = 0;
         if (l < sz.layers) {
-            const uint32_t *following = level + res_layer_words(sz.n[l]);
+            const uint32_t *ahead = level + res_layer_words(sz.n[l]);
+            next_and_end = (int)__ldg(ahead);
+            next_n = (int)__ldg(ahead + 1);
             for (int t = tid * 32; t < kResHeader + (int)sz.n[l + 1]; t += T * 32)
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(following + t));
-        } else if (start_of != nullptr && rows_out == nullptr) {
-            for (int t = tid * 64; t < starts[k]; t += T * 64)
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const uint16_t *>(table) + t));
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(ahead + t));
         }
         Row y[R];
 #pragma unroll
@@ -458,20 +596,19 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
             if (p < and_end) y[r] = res_and(*first, *second, (uint32_t)((int)g >> 31), res_mask15(g));
             else if (p < n) y[r] = res_xor(*first, *second);
         }
+        const int live = n;
+        level += res_layer_words(sz.n[l]);
+        if (kEarly && l < sz.layers) fetch_gates(level, next_n);
+        and_end = next_and_end;
+        n = next_n;
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int p = (warp + r / 2 * W) * 64 + r % 2 * 32 + lane;
-            if (p < n) rows[r % 2 ? o[r / 2] >> 16 : o[r / 2] & 0xffffu] = y[r];
+            if (p < live) rows[r % 2 ? o[r / 2] >> 16 : o[r / 2] & 0xffffu] = y[r];
         }
-        level += res_layer_words(sz.n[l]);
-        if (l < sz.layers) {
-            and_end = (int)__ldg(level);
-            n = (int)__ldg(level + 1);
-            fetch_gates(level, n);
-        } else if (tid == 0) {
-            res_fill(rows[zero_row], 0u);
-        }
+        if (!kEarly && l < sz.layers) fetch_gates(level, n);
+        if (l == sz.layers && tid == 0) res_fill(rows[zero_row], 0u);
         __syncthreads();
     }
     const uint16_t *outputs = reinterpret_cast<const uint16_t *>(level);
@@ -486,8 +623,8 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
         return;
     }
 
-    // ---- class counts: every warp takes its share of the rows, class by class.  A lane adds up eight rows at a time of one row
-    // word, or of two (an instruction that finds a row is paid once for both); lane = (row, part of a row) ----
+    // ---- class counts.  Many classes: see there.  Else every warp takes its share of the rows, class by class.  A lane adds up eight
+    // rows at a time of one row word, or of two (an instruction that finds a row is paid once for both); lane = (row, part of a row) ----
     constexpr int kWords = WORDS < 2 ? 1 : 2, kParts = WORDS / kWords;  // words of a lane, lanes of a row
     constexpr int kSubs = 32 / kParts;
     constexpr int kSteps = kSubs == 16 ? 4 : 5;                        // of adding up over the lanes
@@ -496,7 +633,9 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
     using Pair = typename ResRow<kWords>::type;
     const int part = lane % kParts, sub = lane / kParts;
     const uint8_t *mine = res_smem + part * (int)sizeof(Pair);
-    const int total = starts[k], share = (total / 8 + W) / W * 8;
+    const bool many = res_side_by_side<WORDS, T>(k) < kSubs;
+    if (many) res_count_many<WORDS, T>(row_slots, table, outputs, zero_row, k);
+    const int total = many ? 0 : starts[k], share = (total / 8 + W) / W * 8;
     int pos = min(total, warp * share), c = 0;
     const int stop = min(total, pos + share);
     for (int hi = k; hi - c > 1;) {  // the class of row `pos`
@@ -604,8 +743,7 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
     const float per_sample = 1.f / (float)k;
     for (int t = tid; t < live; t += T) {
         const int sample = (int)(((float)t + 0.5f) * per_sample);  // t / k: t < 2^21, so the error stays below the half
-        const int c = t - sample * k;
-        out[s0 * k + t] = counts[c * kPitch + sample / 32 * kResPitch + sample % 32] + ones[c];
+        out[s0 * k + t] = counts[(t - sample * k) * kPitch + sample / 32 * kResPitch + sample % 32];
     }
 }
 
@@ -615,7 +753,7 @@ static int res_sms() {
     return n;
 }
 static size_t res_shared_bytes(int64_t row_slots, int V, int64_t k) {
-    return (size_t)row_slots * V + ((size_t)kResPitch * (V / 4) * k + 2 * k + 1) * sizeof(int);
+    return (size_t)row_slots * V + ((size_t)kResPitch * (V / 4) * k + k + 1) * sizeof(int);
 }
 
 constexpr size_t kResMaxShared = 227 * 1024;
@@ -674,10 +812,8 @@ static int launch_resident(const void *x, int64_t row_bytes, const uint32_t *pro
     // the most there may be, not this launch's bytes: the limit is the kernel's, and other threads launch it for other networks
     if (cudaFuncSetAttribute(resident_kernel<WORDS, T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResMaxShared) != cudaSuccess)
         return launch_status("dl_eval_network (shared memory opt-in)");
-    const int at_a_time = (int)(kResMaxShared / (smem + 1024)), per_sm = at_a_time < 1024 / T ? (at_a_time < 1 ? 1 : at_a_time) : 1024 / T;
     resident_kernel<WORDS, T, R><<<(unsigned)ceil_div(batch, 8 * V), T, smem, st>>>(
-        reinterpret_cast<const uint8_t *>(x), row_bytes, prog, sz, table, out, rows_out, batch, (int)k, (int)(sz.n[sz.layers] / k), row_slots,
-        res_sms() * per_sm);
+        reinterpret_cast<const uint8_t *>(x), row_bytes, prog, sz, table, out, rows_out, batch, (int)k, (int)(sz.n[sz.layers] / k), row_slots);
     return launch_status("dl_eval_network");
 }
 
@@ -772,7 +908,7 @@ extern "C" DL_API int dl_network_table(const uint32_t *program, const int64_t *n
     const uint16_t *outputs = reinterpret_cast<const uint16_t *>(level);
     const int64_t fill = t.room / 2 > rows ? t.room / 2 : rows;
     launch_dependent(false, res_table_count_kernel, dim3((unsigned)ceil_div(fill, kThreads)), dim3(kThreads), 0, st, t, rows, rows_per_class, program, outputs);
-    launch_dependent(true, res_table_start_kernel, dim3(1), dim3(1024), 0, st, t, (int)k, program);
+    launch_dependent(true, res_table_start_kernel, dim3(1), dim3(1024), 0, st, t, (int)k, rows_per_class, program);
     launch_dependent(true, res_table_place_kernel, dim3((unsigned)ceil_div(rows, kThreads)), dim3(kThreads), 0, st, t, rows, rows_per_class, program, outputs);
     return launch_status("dl_network_table");
 }

@@ -528,9 +528,11 @@ class NetworkProgram:
     connections and arg-max gates.  `layers`: (a, b, gate) of every layer, in order; they are kept, so that `matches` can
     tell a network by its tensors.  build=False leaves the program to a later build()."""
 
-    def __init__(self, n_in, layers, build=True):
-        self.layers = [(a, b, gate) + (versions(a, b) or (None, None)) for a, b, gate in layers]
-        self.sizes = network_sizes(n_in, layers)
+    def __init__(self, n_in, layers, build=True, counters=None, sizes=None):
+        """counters, sizes: versions() of every layer's connections and network_sizes(), if the caller has them."""
+        counters = counters or [versions(a, b) or (None, None) for a, b, _ in layers]
+        self.layers = [layer + counter for layer, counter in zip(layers, counters)]
+        self.sizes = sizes or network_sizes(n_in, layers)
         self.program = None
         for a, b, gate in layers:
             _index(a, "a", gate.numel())
@@ -611,7 +613,6 @@ class FoldedLayers(NetworkProgram):
     """The same for networks of any width (dl_fold_layers): the gates that are left of every layer, and how many they are."""
 
     def __init__(self, n_in, layers, build=True, counters=None, sizes=None):
-        """counters, sizes: versions() of every layer's connections and network_sizes(), if the caller has them."""
         counters = counters or [versions(a, b) or (None, None) for a, b, _ in layers]
         self.layers = [layer + counter for layer, counter in zip(layers, counters)]
         self.sizes = sizes or network_sizes(n_in, layers)
@@ -693,6 +694,13 @@ def eval_folded_applicable(x, sizes):
     """True when a network of these sizes on packed words x can be folded: more than one layer, and the sizes of dl_fold_layers."""
     return (x.is_cuda and x.dim() == 2 and x.is_contiguous() and x.dtype in _DTYPE_TO_BITS and x.shape[0] == sizes[0] and x.shape[1] > 0
             and 2 < len(sizes) <= FOLDED_LAYERS + 1 and 0 < min(sizes) and sum(sizes) < 1 << 27)
+
+
+def eval_folded_counts_applicable(x, sizes, rows, k):
+    """True when eval_folded counts classes of these rows of a network with `rows` gates left: whole units of 16 bytes, whose places
+    in a buffer fit 32 bits."""
+    row_bytes = x.shape[1] * x.element_size()
+    return k > 0 and sizes[len(sizes) - 1] % k == 0 and row_bytes % 16 == 0 and x.data_ptr() % 16 == 0 and max(rows, sizes[0]) * row_bytes < 1 << 35
 
 
 def eval_folded(x, network, batch, k=None):

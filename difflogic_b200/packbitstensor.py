@@ -139,16 +139,15 @@ class PackBitsTensor:
             counters = [ops.versions(a, b) for a, b, _ in layers]
             if None in counters or any(t.get_device() != device for layer in layers for t in layer):
                 return None
+            network = last._network = kind(self._t.shape[0], layers, False, counters, sizes)
             if folded:
-                network = last._network = kind(self._t.shape[0], layers, False, counters, sizes)
                 at_once = sum(sizes[1:-1]) * self._t.shape[1] * self.bit_count >= 8 * FOLD_AT_ONCE_BYTES
             else:
-                network = last._network = kind(self._t.shape[0], layers, build=False)
                 at_once = max(sizes[1:]) <= PROGRAM_AT_ONCE_ROWS or self._t.shape[1] * self.bit_count >= PROGRAM_AT_ONCE_SAMPLES
             if not at_once:
                 return False
         if network.program is None:
-            if counts and (not folded or self._counts_with_last_layer(self._pending[-1][0].out_dim, k)):
+            if counts and (not folded or self._folded_counts(sizes, sum(sizes), k)):
                 network.counted = k
             network.build()
         return False if folded and not network.pays else network
@@ -186,7 +185,7 @@ class PackBitsTensor:
         if self._pending and FUSED_LAST_LAYER:
             batch = self._t.shape[1] * self.bit_count - pad_len
             network = None if self._capturing() else self._network(batch, k)   # all layers are still pending
-            if network and isinstance(network, ops.FoldedLayers) and not self._counts_with_last_layer(self._pending[-1][0].out_dim, k):
+            if network and isinstance(network, ops.FoldedLayers) and not self._folded_counts(network.sizes, network.rows, k):
                 self._materialize()
                 return ops.groupbitsum(self._t, pad_len, k, padded=True)
             counts = self._run(network, batch, k) if network else None
@@ -202,6 +201,9 @@ class PackBitsTensor:
                 return ops.eval_groupbitsum(self._t, a, b, gate, pad_len, k, parts=how == 'parts', padded=True)
         self._materialize()
         return ops.groupbitsum(self._t, pad_len, k, padded=True)
+
+    def _folded_counts(self, sizes, rows, k):
+        return ops.eval_folded_counts_applicable(self._t, sizes, rows, k) or self._counts_with_last_layer(sizes[len(sizes) - 1], k)
 
     def _counts_with_last_layer(self, n_out, k):
         """Whether one kernel takes a last layer of n_out neurons together with the class counts: 'parts', 'whole' or None."""

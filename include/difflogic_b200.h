@@ -244,8 +244,9 @@ DL_API int dl_eval_network_sized(const void *x, const uint32_t *program, const i
  *                               words, int32, then say how many gates of layer l = 1 .. layers - 1 are left (word l).
  *   dl_fold_tail                table for counting the last layer's rows in k classes, dl_fold_tail_bytes() of them, 16-byte aligned;
  *                               at byte 16 * n[layers] it then says, int32, how many neurons the longest class has.
- *   dl_eval_folded              x [n[0]][row_bytes] -> out [batch][k] class counts, in the range of dl_eval_groupbitsum or
- *                               dl_eval_groupbitsum_parts, or the last layer's rows rows_out [n[layers]][row_bytes]; one of the two
+ *   dl_eval_folded              x [n[0]][row_bytes] -> out [batch][k] class counts, for rows of whole 16 bytes, 16-byte aligned, of which
+ *                               neither the input nor the pool has more than 2^31 * 16 bytes, or in the range of dl_eval_groupbitsum or
+ *                               dl_eval_groupbitsum_parts; or the last layer's rows rows_out [n[layers]][row_bytes]; one of the two
  *                               is null.  left: those words, on the HOST.  pool: room for their sum in rows of row_bytes.  For counts:
  *                               the table for k and that number.
  * The counts and rows are those of dl_eval_packed per layer followed by dl_groupbitsum. */

@@ -12,12 +12,13 @@ pytestmark = pytest.mark.gpu
 
 ALL = tuple(range(16))
 # (rows of the input and of every layer, k, bytes of a row, word bits, gates): one gate kernel CTA and several, a remainder of the
-# list's CTAs (256 neurons), layers of one row, rows for each unit of the plain kernel (1, 2, 4, 8, 16 bytes), for the staged
+# list's CTAs (256 neurons), layers of one row, classes of more neurons than a warp counts and classes of one, rows for each unit of the plain kernel (1, 2, 4, 8, 16 bytes), for the staged
 # kernel (512 on) and a remainder of its column blocks (2048); classes counted with the last layer, in parts and apart; layers of
 # which nothing is left, everything is, and of copies only (a value read many layers on)
 CASES = [([5, 3, 4], 2, 16, 32, ALL), ([1, 1, 1, 1], 1, 3, 8, ALL), ([40, 257, 255, 256], 2, 6, 16, ALL), ([9, 70, 70], 7, 12, 32, ALL),
          ([300, 1001, 1001, 1001], 7, 24, 64, ALL), ([64, 3000, 500, 700], 1, 48, 64, ALL), ([64, 640, 640], 10, 512, 64, ALL),
          ([200, 4100, 4200], 2, 2064, 64, ALL), ([200] + 31 * [2050], 50, 528, 32, ALL), ([30, 400, 400, 400], 4, 1040, 64, (0, 15)),
+         ([100, 40000, 40000], 1, 528, 64, ALL), ([64, 2500, 2600], 2, 4112, 64, ALL), ([20, 900, 900], 900, 1040, 64, ALL),
          ([30, 400, 400, 400], 4, 1040, 64, (3, 5, 10, 12)), ([100, 900, 900, 900], 9, 640, 64, (1, 2, 4, 6, 7, 8, 9, 11, 13, 14))]
 
 
@@ -46,7 +47,8 @@ def test_counts_and_rows(dims, k, row_bytes, bits, gates):
         one_by_one = ops.eval_packed(one_by_one, a, b, gate)
     want = ops.groupbitsum(one_by_one, 5, k)
     packed = D.PackBitsTensor.from_packed(xd, 5)
-    if packed._counts_with_last_layer(dims[-1], k):
+    assert packed._folded_counts(network.sizes, network.rows, k) or row_bytes % 16 != 0
+    if row_bytes % 16 == 0:
         assert torch.equal(ops.eval_folded(xd, network, batch, k), want)
 
 
@@ -67,7 +69,7 @@ def test_a_wide_network_is_folded(monkeypatch):
             return model(D.PackBitsTensor(x)).cpu().numpy()
     assert np.array_equal(counts(), want) and not folded
     assert np.array_equal(counts(), want) and len(folded) == 1
-    few = D.PackBitsTensor(x[:200])             # rows too short for the counting kernel
+    few = D.PackBitsTensor(x[:200])             # rows too short for the staged counting kernel
     assert np.array_equal(model[3](model[2](model[1](model[0](few)))).cpu().numpy(), want[:200]) and len(folded) == 2
     packed = D.PackBitsTensor(x)
     for layer in layers:
