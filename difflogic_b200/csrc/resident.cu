@@ -12,10 +12,12 @@
 // The program is that of the FOLDED network (fold.cu): only gates that need both inputs and are read by something, each one
 // AND(a ^ i, b ^ j) or XOR(a, b); a row that later layers only hand on stays in its slot until its last reader has read it.
 //
-// Measured, whole kernel, 2^20 samples: 784 -> 4 x 8000 827 -> 525 us (all neurons in the program, their rows put into class order
-// for the counts; 1210 layer by layer); 10000 samples, 784 -> 5 x 16000 40 -> 30 us.  What is left as gates: 40 % of the neurons with
-// gates drawn evenly, 100 % of a network that needs them all.  Shared-memory pipe 59 %, issue 55 % busy: neither is what
-// bounds it alone; a block goes through load, layers and counts one after the other and two blocks share an SM.
+// Measured, whole kernel, all neurons in the program and their rows put into class order for the counts -> now, us: 784 -> 4 x 8000, 2^20
+// samples 826 -> 492 (1210 layer by layer); 784 -> 5 x 16000, 10000 samples 45 -> 23, 2^18 560 -> 248; 784 -> 12 x 12000, 2^17 451 -> 167;
+// 256 -> 12 x 4000, 2^18 201 -> 85; 784 -> 4 x 8000, 100 samples 14.4 -> 15.7 (four CTAs whose loads wait for one another). What is left as gates:
+// 40 % of the neurons with gates drawn evenly, 100 % of a network that needs them all.  Shared-memory pipe 59 %, issue 55 % busy: neither
+// is what bounds it alone; a block goes through load, layers and counts one after the other and two blocks share an SM.  Loading
+// the input four rows per thread at a time, and fetching the next block's into L2, changed nothing.
 //
 // CTAs that stay for several blocks and fetch the next one's input while they count were slower (needs more than 64 registers:
 // 16000 wide, 10000 samples 45 -> 51 us, 8000 wide, 2^18 samples 208 -> 212).
@@ -589,6 +591,7 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
         Row y[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
+            if ((warp + r / 2 * W) * 64 >= n) break;
             const int p = (warp + r / 2 * W) * 64 + r % 2 * 32 + lane;
             const uint32_t g = r % 2 ? w[r / 2].y : w[r / 2].x;
             const Row *first = reinterpret_cast<const Row *>(res_smem + ((g >> 16) & 0x3fffu) * V);
@@ -604,6 +607,8 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < R; ++r) {
+            // (checked for every pair of gates, rows of 16 bytes are stored later: 784 -> 5 x 16000 248 -> 261 us; never: 784 -> 12 x 12000 167 -> 182)
+            if ((WORDS == 1 || r == R / 2 / 2 * 2) && (warp + r / 2 * W) * 64 >= live) break;
             const int p = (warp + r / 2 * W) * 64 + r % 2 * 32 + lane;
             if (p < live) rows[r % 2 ? o[r / 2] >> 16 : o[r / 2] & 0xffffu] = y[r];
         }
@@ -759,8 +764,8 @@ static size_t res_shared_bytes(int64_t row_slots, int V, int64_t k) {
 constexpr size_t kResMaxShared = 227 * 1024;
 
 // Kernels: bytes of a row per block, threads, gates per thread and layer; in order of preference.  Registers decide: 64 (T a power of
-// two) hold the outputs of 8 gates of 16 bytes, 72 those of 10 (as 68 bytes per thread that went through local memory they cost
-// 15 % of the shared-memory pipe).
+// two) hold the outputs of 8 gates of 16 bytes, 72 those of 10 (in 64, 68 bytes per thread went through local memory and took 15 % of
+// the shared-memory pipe).
 struct ResShape {
     int V, T, R;
 };
