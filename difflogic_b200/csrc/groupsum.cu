@@ -559,20 +559,15 @@ extern "C" DL_API int dl_groupsum_f32(const float *x, float *out, void *workspac
     // Classes of up to 4096 rows: one cluster of 8 CTAs per (class, column block), no scratch needed.
     const int64_t m_rows = n / k;
     if (groupsum_takes_cluster_kernel(n, batch, k)) {
-        // An SM holds four CTAs; where clusters of eight would just not fit all at a time, the last few would take as long again:
-        // 16000 rows, batch 1000, 10 classes (640 CTAs on 148 SMs): 11.7 us with clusters of eight, 9.1 with four
-        // (rows in L2); 8000 rows: 9.9 / 6.8.
-        const int64_t ctas = colblocks * k * kGcCluster, at_a_time = 4 * 148;
-        const unsigned cluster = ctas > at_a_time && ctas <= 2 * at_a_time ? kGcCluster / 2 : kGcCluster;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)colblocks, (unsigned)k, cluster);
+        cfg.gridDim = dim3((unsigned)colblocks, (unsigned)k, kGcCluster);
         cfg.blockDim = dim3(kGcThreads);
         cfg.stream = as_stream(stream);
         cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 1;
         attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = cluster;
+        attr[0].val.clusterDim.z = kGcCluster;
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
         cfg.attrs = attr;
