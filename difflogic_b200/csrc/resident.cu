@@ -14,9 +14,10 @@
 //
 // Measured, whole kernel, all neurons in the program and their rows put into class order for the counts -> now, us: 784 -> 4 x 8000, 2^20
 // samples 826 -> 492 (1210 layer by layer); 784 -> 5 x 16000, 10000 samples 45 -> 23, 2^18 560 -> 248; 784 -> 12 x 12000, 2^17 451 -> 167;
-// 256 -> 12 x 4000, 2^18 201 -> 85; 784 -> 4 x 8000, 100 samples 14.4 -> 15.7 (four CTAs whose loads wait for one another). What is left as gates:
-// 40 % of the neurons with gates drawn evenly, 100 % of a network that needs them all.  Shared-memory pipe 59 %, issue 55 % busy: neither
-// is what bounds it alone; a block goes through load, layers and counts one after the other and two blocks share an SM.  Loading
+// 256 -> 12 x 4000, 2^18 201 -> 85; 784 -> 4 x 8000, 100 samples 14.4 -> 15.7 (four CTAs whose loads wait for one another). What is
+// left as gates: 40 % of the neurons with gates drawn evenly; networks of which three quarters are left run in resident_whole.cu.
+// Shared-memory pipe 59 %, issue 55 % busy: neither is what bounds it alone; a block goes through load, layers and counts one after
+// the other and two blocks share an SM.  Loading
 // the input four rows per thread at a time, and fetching the next block's into L2, changed nothing.
 //
 // CTAs that stay for several blocks and fetch the next one's input while they count were slower (needs more than 64 registers:
@@ -31,6 +32,7 @@
 // 3 V bytes of shared-memory traffic.
 #include "common.cuh"
 #include "fold.cuh"
+#include "resident.cuh"
 #include "gates.cuh"
 
 namespace dl {
@@ -44,7 +46,8 @@ struct ResidentSizes {
     int n[kResLayers + 1];  // rows of the input and of every layer
 };
 
-// A program, in 32-bit words: a header {slots, most gates of a layer}; per layer a header {gates that are ANDs, gates}, the gates'
+// A program, in 32-bit words: a header {slots, most gates of a layer, bank classes, gates in all}; per layer a header {gates that
+// are ANDs, gates}, the gates'
 // words and their output slots (16 bits each); the last layer's rows (16 bits each: slot, above it whether inverted).  A warp takes
 // 64 gates at a time, lane l gates l and l + 32, whose words lie side by side.
 constexpr int kResHeader = 4;
@@ -106,6 +109,7 @@ res_inputs_kernel(ResBuild p, uint32_t *__restrict__ prog) {
         prog[0] = (uint32_t)p.n0;
         prog[1] = 0u;
         prog[2] = (uint32_t)nc;
+        prog[3] = 0u;
     }
     if (i >= p.n0) return;
     p.slot[i] = i;
@@ -199,6 +203,7 @@ res_place_kernel(ResBuild p, int layer, int first, int n, uint32_t *__restrict__
         }
         prog[0] = (uint32_t)slots;
         prog[1] = max(__ldcg(prog + 1), (uint32_t)total);
+        prog[3] = __ldcg(prog + 3) + (uint32_t)total;
     }
     if (j >= n) return;
     const int mark = p.rank[j];
@@ -342,39 +347,6 @@ res_table_place_kernel(ResTable t, int n, int rows_per_class, const uint32_t *__
 // ---------------------------------------------------------------------------------------------
 // evaluation
 // ---------------------------------------------------------------------------------------------
-template <int WORDS> struct ResRow;
-template <> struct ResRow<1> { using type = uint32_t; };
-template <> struct ResRow<2> { using type = uint2; };
-template <> struct ResRow<4> { using type = uint4; };
-
-__device__ __forceinline__ uint32_t res_and(uint32_t a, uint32_t b, uint32_t i, uint32_t j) { return (a ^ i) & (b ^ j); }
-__device__ __forceinline__ uint2 res_and(const uint2 &a, const uint2 &b, uint32_t i, uint32_t j) {
-    return make_uint2(res_and(a.x, b.x, i, j), res_and(a.y, b.y, i, j));
-}
-__device__ __forceinline__ uint4 res_and(const uint4 &a, const uint4 &b, uint32_t i, uint32_t j) {
-    return make_uint4(res_and(a.x, b.x, i, j), res_and(a.y, b.y, i, j), res_and(a.z, b.z, i, j), res_and(a.w, b.w, i, j));
-}
-__device__ __forceinline__ uint32_t res_xor(uint32_t a, uint32_t b) { return a ^ b; }
-__device__ __forceinline__ uint2 res_xor(const uint2 &a, const uint2 &b) { return make_uint2(a.x ^ b.x, a.y ^ b.y); }
-__device__ __forceinline__ uint4 res_xor(const uint4 &a, const uint4 &b) { return make_uint4(a.x ^ b.x, a.y ^ b.y, a.z ^ b.z, a.w ^ b.w); }
-__device__ __forceinline__ void res_fill(uint32_t &v, uint32_t m) { v = m; }
-__device__ __forceinline__ void res_fill(uint2 &v, uint32_t m) { v = make_uint2(m, m); }
-__device__ __forceinline__ void res_fill(uint4 &v, uint32_t m) { v = make_uint4(m, m, m, m); }
-// all ones where bit 15 of w is set
-__device__ __forceinline__ uint32_t res_mask15(uint32_t w) {
-    uint32_t m;
-    asm("prmt.b32 %0, %1, 0, 0x9999;" : "=r"(m) : "r"(w));
-    return m;
-}
-
-#define DL_CSA32(h, l, a, b, c)        \
-    {                                  \
-        const uint32_t u_ = (a) ^ (b); \
-        const uint32_t c_ = (c);       \
-        h = ((a) & (b)) | (u_ & c_);   \
-        l = u_ ^ c_;                   \
-    }
-
 // Rows that a group of lanes counts side by side: all that a warp has lanes for, or fewer where there are more classes than warps.
 template <int WORDS, int T>
 __device__ __forceinline__ int res_side_by_side(int k) {
@@ -752,11 +724,6 @@ resident_kernel(const uint8_t *__restrict__ x, int64_t row_bytes, const uint32_t
     }
 }
 
-static int res_sms() {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
-    return n;
-}
 static size_t res_shared_bytes(int64_t row_slots, int V, int64_t k) {
     return (size_t)row_slots * V + ((size_t)kResPitch * (V / 4) * k + k + 1) * sizeof(int);
 }
@@ -789,7 +756,7 @@ static ResPlan res_plan(const int64_t *n, int layers, int64_t batch, int64_t k, 
     if (n[layers] % k != 0) return best;
     if (slots <= 0 || slots > most) slots = most;
     if (gates < 0 || gates > widest) gates = widest;
-    const int sms = res_sms();
+    const int sms = current_sms();
     int64_t least = 0;
     for (const int V : {16, 8, 4}) {
         const size_t smem = res_shared_bytes(slots + 1, V, k);

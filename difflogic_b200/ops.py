@@ -554,7 +554,14 @@ class NetworkProgram:
         if self.counted is not None:
             self._make_table(program, self.counted)
         # other threads and streams may take program and table from here on: this waits for them
-        program._dl_needs = tuple(program[:2].tolist())
+        slots, gates, _, left = program[:4].tolist()
+        program._dl_needs = (slots, gates)
+        program._dl_whole = None
+        if left * 4 >= 3 * sum(self.sizes[1:]):     # hardly folded: all neurons take less time
+            whole = torch.empty(N.lib().dl_network_whole_words(self.sizes, count), dtype=torch.int32, device=program.device)
+            self._launch(N.lib().dl_network_whole, whole)
+            torch.cuda.current_stream(whole.device).synchronize()
+            program._dl_whole = whole
         self.program = program
 
     def _launch(self, build, program):
@@ -679,11 +686,18 @@ def eval_network(x, network, batch, k=None):
     else:
         out = torch.empty((int(batch), int(k)), dtype=torch.int32, device=x.device)
     with N.on_device(x):
-        table = None if k is None else network.table(program, int(k))
+        whole = program._dl_whole
+        if whole is not None and k is not None:
+            program._dl_tables.setdefault(int(k))       # counts these without a table
+        table = None if k is None or whole is not None else network.table(program, int(k))
         stream = N.stream_of(x)
-        for t in (program, table):
+        for t in (program, table, whole):
             if t is not None and stream != t._dl_stream:
                 t.record_stream(torch.cuda.current_stream(x.device))
+        if whole is not None:
+            N.check(N.lib().dl_eval_whole(x.data_ptr(), whole.data_ptr(), sizes, len(sizes) - 1, 0 if k is None else out.data_ptr(),
+                                          out.data_ptr() if k is None else 0, row_bytes, int(batch), 1 if k is None else int(k), stream))
+            return out
         N.check(N.lib().dl_eval_network_sized(x.data_ptr(), program.data_ptr(), sizes, len(sizes) - 1, *program._dl_needs,
                                               N.ptr(table), 0 if k is None else out.data_ptr(), out.data_ptr() if k is None else 0, row_bytes,
                                               int(batch), 1 if k is None else int(k), stream))
