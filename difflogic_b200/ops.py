@@ -550,11 +550,11 @@ class NetworkProgram:
         count = len(self.layers)
         program = torch.empty(N.lib().dl_network_program_words(self.sizes, count), dtype=torch.int32, device=self.layers[0][2].device)
         self._launch(N.lib().dl_network_program, program)
-        program._dl_tables = {}     # by number of classes; another thread may build the program once more, with other slots
-        if self.counted is not None:
-            self._make_table(program, self.counted)
+        k = self.counted        # once: another thread may count other classes
+        table = None if k is None else self._make_table(program, k)
         # other threads and streams may take program and table from here on: this waits for them
         slots, gates, _, left = program[:4].tolist()
+        program._dl_tables = {} if table is None else {k: table}     # by number of classes, of this program's slots
         program._dl_needs = (slots, gates)
         program._dl_whole = None
         if left * 4 >= 3 * sum(self.sizes[1:]):     # hardly folded: all neurons take less time
@@ -587,17 +587,17 @@ class NetworkProgram:
             stream = N.stream_of(program)
             table = self._table_of(program, k, stream)
         table._dl_stream = stream
-        if len(program._dl_tables) >= 4:
-            program._dl_tables = {}
-        program._dl_tables[k] = table
         return table
 
     def table(self, program, k):
-        """The class table of a program for k classes; made, and waited for, when k is met first."""
+        """The class table of a program for k classes; made, and waited for, when k is met first.  Other threads, whose streams wait
+        for nothing, see it when it is finished."""
         table = program._dl_tables.get(k)
         if table is None:
             table = self._make_table(program, k)
             torch.cuda.current_stream(table.device).synchronize()
+            others = program._dl_tables
+            program._dl_tables = {**(others if len(others) < 4 else {}), k: table}
         return table
 
     def serves(self, x, k):
@@ -639,11 +639,11 @@ class FoldedLayers(NetworkProgram):
             torch.cuda.synchronize(device)
         program = torch.empty(N.lib().dl_fold_layers_bytes(self.sizes, count), dtype=torch.uint8, device=device)
         self._launch(N.lib().dl_fold_layers, program)
-        program._dl_tables = {}
-        if self.counted is not None:
-            self._make_table(program, self.counted)
+        k = self.counted        # once: another thread may count other classes
+        table = None if k is None else self._make_table(program, k)
         # other threads and streams may take program and table from here on: this waits for them
         left = program[:4 * count].view(torch.int32).tolist()
+        program._dl_tables = {} if table is None else {k: table}
         program._dl_left = (ctypes.c_int32 * count)(*left)
         self.rows = sum(left[1:])
         # fewer rows to compute than by whole layers, and at most half as much memory again as two activations of the widest layer

@@ -136,6 +136,37 @@ def test_threads_with_networks_of_different_size():
     assert not failures, failures
 
 
+def test_threads_that_count_other_classes():
+    """Two threads on streams of their own ask one network, whose program is there, for numbers of classes that it has not counted."""
+    import threading
+    dims, ks, batch = [100, 4800, 4800], (1, 2, 3, 4, 5, 6, 8, 10, 12, 15), 5000
+    layers = _network(dims, batch)
+    words = -(-batch // 128) * 2
+    x = torch.randint(-2 ** 63, 2 ** 63 - 1, (dims[0], words), generator=torch.Generator().manual_seed(1))
+    hidden = x.numpy()
+    for a, b, gate in layers:
+        hidden = O.eval_packed(hidden, a.numpy(), b.numpy(), gate.numpy())
+    want = {k: O.group_bit_sum(hidden, 0, k)[:batch] for k in ks}
+    xd, network = x.cuda(), ops.NetworkProgram(dims[0], [tuple(t.cuda() for t in layer) for layer in layers])
+    torch.cuda.synchronize()
+    start, got = threading.Barrier(2), [[], []]
+
+    def work(mine, order):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for k in order:
+                start.wait(60)
+                got[mine].append((k, ops.eval_network(xd, network, batch, k)))
+            torch.cuda.current_stream().synchronize()
+    threads = [threading.Thread(target=work, args=args) for args in ((0, 3 * ks), (1, 3 * (ks[1:] + ks[:1])))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert [len(g) for g in got] == [30, 30]
+    for k, counts in got[0] + got[1]:
+        assert np.array_equal(counts.cpu().numpy(), want[k]), k
+
+
 def test_a_graph_keeps_its_own_gates():
     torch.manual_seed(4)
     model = torch.nn.Sequential(D.LogicLayer(64, 320), D.LogicLayer(320, 320), D.GroupSum(10)).eval()

@@ -288,6 +288,44 @@ def test_a_program_is_built_for_the_second_pass(cuda, argmax, monkeypatch):
         assert [passes(layers) for _ in range(2)] == [(0, 1), (0, 0)]
 
 
+@pytest.mark.parametrize("kind", [ops.NetworkProgram, ops.FoldedLayers])
+def test_tables_are_seen_when_they_are_finished(cuda, monkeypatch, kind):
+    """Threads share a program's class tables, and a thread that finds one launches on a stream that waits for nothing."""
+    monkeypatch.setattr(ops.N, "on_device", lambda t: ops.N._ALREADY_THERE)
+    monkeypatch.setattr(ops.N, "stream_of", lambda t: 7)
+    network, program = kind.__new__(kind), torch.zeros(4, dtype=torch.int32)
+    network.sizes, network.layers, network.counted = (8, 8, 8), [()] * 2, 2
+    program._dl_tables, seen = {}, []
+    monkeypatch.setattr(kind, "_table_of", lambda network, program, k, stream: torch.zeros(1))
+    stream = torch.cuda.current_stream()
+    monkeypatch.setattr(type(stream), "synchronize", lambda stream: seen.append(set(program._dl_tables)))
+    for k in (1, 2, 4, 8, 1):                             # by reading rows first, then counting; by counting with other classes
+        table = network.table(program, k)
+        assert program._dl_tables[k] is table and table._dl_stream == 7
+    assert seen == [set(), {1}, {1, 2}, {1, 2, 4}]
+    network.table(program, 16)                            # a fifth: from the start again
+    assert seen[4:] == [{1, 2, 4, 8}] and set(program._dl_tables) == {16}
+
+
+def test_a_table_is_that_of_the_classes_it_is_kept_under(cuda, monkeypatch):
+    """`counted` is what the latest pass asks for; another thread may change it while one builds."""
+    network = ops.NetworkProgram.__new__(ops.NetworkProgram)
+    network.sizes, network.layers, network.counted, made = (8, 8, 8), [(None, None, torch.zeros(8))] * 2, 2, []
+    words = type("Library", (), {"dl_network_program_words": lambda s, sizes, n: 8, "dl_network_program": None})()
+    monkeypatch.setattr(ops.N, "lib", lambda: words)
+    monkeypatch.setattr(ops.NetworkProgram, "_launch", lambda network, build, program: program.zero_())
+
+    def make(network, program, k):
+        assert network.program is None and not hasattr(program, "_dl_tables")
+        network.counted = 4
+        made.append(torch.tensor(k))
+        return made[-1]
+    monkeypatch.setattr(ops.NetworkProgram, "_make_table", make)
+    network.program = None
+    network.build()
+    assert {k: int(table) for k, table in network.program._dl_tables.items()} == {2: 2}
+
+
 @pytest.mark.parametrize("width,batch,training,evaluating", [
     (11999, 4096, False, False), (12000, 164, False, False), (12000, 168, True, True), (16000, 124, False, False), (16000, 128, True, True),
     (64000, 33, False, False), (64000, 64, False, False), (12000, 1024, True, True), (12000, 1028, True, False), (15999, 4096, True, False),
