@@ -146,12 +146,12 @@ def lib():
 
 def nodes():
     """The module of the native autograd nodes (csrc/autograd_nodes.cpp), built beside the library; raises NativeLibraryMissing when
-    it has not been."""
+    it has not been built for this PyTorch and Python."""
     global _nodes
     if _nodes is None:
         lib()
         import importlib.util
-        spec = importlib.util.spec_from_file_location("dl_autograd", _build.NODES_PATH)
+        spec = importlib.util.spec_from_file_location("dl_autograd", _build.nodes_path())
         try:
             module = importlib.util.module_from_spec(spec)
         except ImportError as e:

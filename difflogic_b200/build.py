@@ -5,19 +5,19 @@
 compiles difflogic_b200/csrc/*.cu with nvcc into difflogic_b200/_lib/libdifflogic_b200.so.
 The library has a plain C ABI (include/difflogic_b200.h) and links the CUDA runtime statically,
 so it depends on nothing but the driver.  The training path's autograd nodes (csrc/autograd_nodes.cpp) are a Python
-module of their own beside it, _lib/dl_autograd.so: host code that calls the library and links PyTorch.
+module of their own beside it, _lib/dl_autograd-<PyTorch>-<Python>.so: host code that calls the library and links PyTorch.
 """
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "_lib")
 LIB_PATH = os.path.join(LIB_DIR, "libdifflogic_b200.so")
-NODES_PATH = os.path.join(LIB_DIR, "dl_autograd.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -38,9 +38,16 @@ def sources():
     return sorted(os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cu"))
 
 
+def nodes_path():
+    """Where the module of the autograd nodes is for the PyTorch and Python that run this.  It has the layouts of their objects
+    compiled in, so that one built for another version is another file, which is neither taken for this one nor loaded."""
+    import torch
+    return os.path.join(LIB_DIR, "dl_autograd-%s-%s-%s.so" % (torch.__version__, (torch.version.git_version or "")[:8],
+                                                             sysconfig.get_config_var("SOABI")))
+
+
 def nodes_command():
     """Compiles and links the module of the autograd nodes against the library and the PyTorch that runs this."""
-    import sysconfig
     import torch
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(find_nvcc())))
@@ -48,23 +55,38 @@ def nodes_command():
                os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"]]
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-ffunction-sections", "-fdata-sections",
             "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
-            *[flag for path in include for flag in ("-I", path)], os.path.join(CSRC, "autograd_nodes.cpp"), "-o", NODES_PATH,
+            *[flag for path in include for flag in ("-I", path)], os.path.join(CSRC, "autograd_nodes.cpp"), "-o", nodes_path(),
             "-L", os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda",
             "-L", LIB_DIR, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN", "-Wl,--gc-sections"]
 
 
-def is_stale():
-    if not (os.path.exists(LIB_PATH) and os.path.exists(NODES_PATH)):
-        return True
-    built = min(os.path.getmtime(LIB_PATH), os.path.getmtime(NODES_PATH))
+def _older_than_sources(path):
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(ROOT, "include", "difflogic_b200.h")]
-    return any(os.path.getmtime(d) > built for d in deps)
+    return not os.path.exists(path) or any(os.path.getmtime(d) > os.path.getmtime(path) for d in deps)
+
+
+def is_stale():
+    return _older_than_sources(LIB_PATH) or _older_than_sources(nodes_path())
+
+
+def _run(cmd, what):
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout)
+        raise RuntimeError(what + " failed")
 
 
 def build(verbose=False, force=False):
-    """Compiles the library if it is missing or older than its sources; returns its path."""
-    if not force and not is_stale():
-        return LIB_PATH
+    """Compiles the library and the module of the autograd nodes, each if it is missing or older than its sources; returns the
+    library's path."""
+    if force or _older_than_sources(LIB_PATH):
+        _build_library(verbose)
+    if force or _older_than_sources(nodes_path()):
+        _run(nodes_command(), "g++")
+    return LIB_PATH
+
+
+def _build_library(verbose):
     os.makedirs(LIB_DIR, exist_ok=True)
     nvcc = find_nvcc()
     objs = []
@@ -85,12 +107,7 @@ def build(verbose=False, force=False):
             raise RuntimeError("nvcc failed: " + " ".join(cmd))
     link = [nvcc, "-shared", "-cudart", "static", "-gencode", "arch=compute_100a,code=sm_100a",
             "-Xcompiler", "-fPIC", "-o", LIB_PATH, *objs]
-    for cmd, what in ((link, "link"), (nodes_command(), "g++")):
-        r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
-        if r.returncode != 0:
-            sys.stderr.write(r.stdout)
-            raise RuntimeError(what + " failed")
-    return LIB_PATH
+    _run(link, "link")
 
 
 if __name__ == "__main__":

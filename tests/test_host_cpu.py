@@ -55,6 +55,25 @@ def test_argument_errors_are_reported_before_any_launch(lib):
     assert lib.dl_groupsum_workspace_bytes(16000, 128, 10) > 4096
 
 
+@pytest.mark.parametrize("where,name,other", [("torch", "__version__", "0.1"), ("torch.version", "git_version", "0" * 40), ("sysconfig", "SOABI", "cp0")])
+def test_nodes_of_another_pytorch_or_python_are_not_loaded(lib, monkeypatch, where, name, other):
+    """The module of the autograd nodes has PyTorch's and Python's object layouts compiled in."""
+    import sysconfig
+    assert not dl_build.is_stale() and os.path.exists(dl_build.nodes_path()) and _native.nodes() is not None
+    if where == "sysconfig":
+        monkeypatch.setattr(sysconfig, "get_config_var", lambda key, get=sysconfig.get_config_var: other if key == name else get(key))
+    else:
+        monkeypatch.setattr(torch if where == "torch" else torch.version, name, other)
+    monkeypatch.setattr(_native, "_nodes", None)
+    with pytest.raises(_native.NativeLibraryMissing, match="difflogic_b200.build"):
+        _native.nodes()
+    assert dl_build.is_stale()
+    made = []
+    monkeypatch.setattr(dl_build, "_run", lambda cmd, what: made.append(cmd))
+    dl_build.build()                       # and what that advice does: the module, for these versions
+    assert len(made) == 1 and made[0][made[0].index("-o") + 1] == dl_build.nodes_path() and other[:8] in dl_build.nodes_path()
+
+
 def test_cuda_path_has_no_cpu_stand_in():
     layer = D.LogicLayer(8, 8, device='cpu', implementation='cuda')
     with pytest.raises((RuntimeError, AssertionError)):
