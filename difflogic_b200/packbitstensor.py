@@ -44,6 +44,14 @@ PROGRAM_AT_ONCE_SAMPLES = 1 << 18
 # (890 MB) 481 / 554, 2^17 1511 / 4509.
 FOLD_AT_ONCE_BYTES = 5 << 27
 
+# Classes of fewer neurons of a folded network than this are counted from the last layer's rows, unless (class, 512 bytes of a row) are at
+# most so many: counting along with the layer takes a CTA for each and its 1.2 us for every CTA, however few neurons it has.  Whole passes
+# of 784 -> 3 x 20000, us, counts with the layer / rows first, in classes of 4, 8, 16, 32, 50, 80 neurons: 2^17 samples 5591 / 3716,
+# 2886 / 2119, 1537 / 1100, 818 / 720, 546 / 592, 393 / 488; 2^15 (8 pieces) 1408 / 925, 733 / 529, 396 / 283, 227 / 186, 165 / 154, 121 /
+# 146; 10000 (3) 471 / 316, 253 / 193, 145 / 116, 89 / 98, 69 / 89, 55 / 84; 1000 (1) 96 / 76, 59 / 76, 52 / 75, 51 / 75.
+FOLDED_COUNTS_NEURONS = 48
+FOLDED_COUNTS_CTAS = 3000
+
 
 class PackBitsTensor:
     def __init__(self, t: torch.BoolTensor, bit_count=32, device='cuda'):
@@ -203,6 +211,10 @@ class PackBitsTensor:
         return ops.groupbitsum(self._t, pad_len, k, padded=True)
 
     def _folded_counts(self, sizes, rows, k):
+        """Whether the classes of a folded network are counted along with its last layer."""
+        pieces = -(-self._t.shape[1] * self._t.element_size() // 512)
+        if k > 0 and sizes[len(sizes) - 1] < FOLDED_COUNTS_NEURONS * k and k * pieces > FOLDED_COUNTS_CTAS:
+            return False
         return ops.eval_folded_counts_applicable(self._t, sizes, rows, k) or self._counts_with_last_layer(sizes[len(sizes) - 1], k)
 
     def _counts_with_last_layer(self, n_out, k):

@@ -326,6 +326,16 @@ def test_a_table_is_that_of_the_classes_it_is_kept_under(cuda, monkeypatch):
     assert {k: int(table) for k, table in network.program._dl_tables.items()} == {2: 2}
 
 
+@pytest.mark.parametrize("rows,k,words,together", [
+    (20000, 5000, 2048, False), (20000, 2500, 64, True), (20000, 3001, 64, False), (20000, 3000, 64, True), (20000, 1250, 192, False),
+    (20000, 1000, 192, True), (20000, 400, 2048, True), (47 * 400, 400, 512, False), (48 * 400, 400, 512, True), (3, 1, 1 << 12, True)])
+def test_which_classes_are_counted_along_with_the_last_layer(monkeypatch, rows, k, words, together):
+    """Both sides of the lines from which on a CTA per class and piece of the rows takes longer than rows and counts one after the other."""
+    monkeypatch.setattr(ops, "eval_folded_counts_applicable", lambda x, sizes, rows, k: True)
+    packed = D.PackBitsTensor.from_packed(torch.ones(8, words, dtype=torch.int64), 0)
+    assert bool(packed._folded_counts((8, 9, rows), 9, k)) == together
+
+
 @pytest.mark.parametrize("width,batch,training,evaluating", [
     (11999, 4096, False, False), (12000, 164, False, False), (12000, 168, True, True), (16000, 124, False, False), (16000, 128, True, True),
     (64000, 33, False, False), (64000, 64, False, False), (12000, 1024, True, True), (12000, 1028, True, False), (15999, 4096, True, False),
