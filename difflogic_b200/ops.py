@@ -662,9 +662,13 @@ class FoldedLayers(NetworkProgram):
         return super().serves(x, k) and self.pays
 
 
-def network_sizes(n_in, layers):
+def row_counts(rows):
     import ctypes
-    return (ctypes.c_int64 * (len(layers) + 1))(n_in, *[gate.numel() for _, _, gate in layers])
+    return (ctypes.c_int64 * len(rows))(*rows)
+
+
+def network_sizes(n_in, layers):
+    return row_counts([n_in] + [gate.numel() for _, _, gate in layers])
 
 
 def eval_network_applicable(x, sizes, batch, k):

@@ -141,6 +141,8 @@ class PackBitsTensor:
         folded = not ops.eval_network_applicable(self._t, sizes, batch, k)
         if folded and not ops.eval_folded_applicable(self._t, sizes):
             return None
+        if folded and k > 1 and ops.eval_network_applicable(self._t, sizes, batch, 1) and not self._folded_counts(sizes, sum(sizes), k):
+            return None                     # the classes are too many for the one kernel, not the layers
         kind = ops.FoldedLayers if folded else ops.NetworkProgram
         if type(network) is not kind:
             device = self._t.get_device()
@@ -158,7 +160,14 @@ class PackBitsTensor:
             if counts and (not folded or self._folded_counts(sizes, sum(sizes), k)):
                 network.counted = k
             network.build()
-        return False if folded and not network.pays else network
+        if folded and not network.pays:
+            # Three hidden layers or more that fit the one kernel run there all the same.  With gates that all need both inputs, us, one by
+            # one / in one kernel: 784 -> 2 x 8000 -> 20000: 10000 samples 75 / 80, 2^17 207 / 245, 2^20 1456 / 1941; 4 x 8000: 102 / 87, 306 /
+            # 278, 2195 / 2111; 12 x 8000: 202 / 109, 714 / 400, 5158 / 2976.  (With gates drawn evenly, folded / in one kernel: 4 x 8000: 62 /
+            # 74, 166 / 284, 1152 / 2221.)
+            hidden = sizes[:-1]
+            return None if len(hidden) > 3 and ops.eval_network_applicable(self._t, ops.row_counts(hidden), batch, 1) else False
+        return network
 
     def _run(self, network, batch, k=None):
         """The class counts of the pending layers, without k the last one's rows; None where there is no memory for the rows of

@@ -87,3 +87,36 @@ def test_a_wide_network_is_folded(monkeypatch):
     monkeypatch.setattr(ops, "eval_folded", lambda *a: folded.append(a) or run(*a))
     first, again = counts(), counts()
     assert np.array_equal(first, again) and len(folded) == 3
+
+
+@pytest.mark.parametrize("dims,k,both,route", [
+    ([30, 600, 600, 16400], 10, False, ["folded"]),                          # the last layer does not fit the one kernel, gates fold
+    ([30, 600, 600, 600, 16400], 10, True, ["one kernel", "with counts"]),   # they do not: the hidden layers go there
+    ([30, 600, 600, 16400], 10, True, ["layer", "layer", "with counts"]),
+    ([30, 17000, 17000, 17000], 10, True, ["layer", "layer", "with counts"]),    # nor do the hidden layers
+    ([30, 2000, 2000, 2000], 2000, False, ["one kernel", "layer"]),          # the classes do not
+    ([30, 2000, 2000, 2000], 2000, True, ["one kernel", "layer"])])
+def test_where_networks_run_that_do_not_fit_the_one_kernel(monkeypatch, dims, k, both, route):
+    """From the third pass on, and the counts of all passes."""
+    torch.manual_seed(len(dims))
+    model = torch.nn.Sequential(*[D.LogicLayer(*d) for d in zip(dims, dims[1:])], D.GroupSum(k)).eval()
+    layers = list(model)[:-1]
+    with torch.no_grad():
+        if both:
+            for layer in layers:
+                kind = torch.tensor([1, 2, 4, 6, 7, 8, 9, 11, 13, 14], device="cuda")[torch.randint(0, 10, (layer.out_dim,), device="cuda")]
+                layer.weights.zero_().scatter_(1, kind[:, None], 1.0)
+                layer.set_connections(layer.indices[0], (layer.indices[0] + 1) % layer.in_dim)
+        x = torch.rand(5001, dims[0], device="cuda") < 0.5
+        want = O.packed_net_counts(x.cpu().numpy(), [l.indices[0].cpu() for l in layers], [l.indices[1].cpu() for l in layers],
+                                   [l.weights.argmax(1).cpu().numpy().astype(np.uint8) for l in layers], k, 32)
+        run = []
+        for name, what in (("eval_folded", "folded"), ("eval_network", "one kernel"), ("eval_packed", "layer"), ("eval_groupbitsum", "with counts")):
+            def spy(*a, kernel=getattr(ops, name), what=what, **kw):
+                run.append(what)
+                return kernel(*a, **kw)
+            monkeypatch.setattr(ops, name, spy)
+        for _ in range(4):
+            del run[:]
+            assert np.array_equal(model(D.PackBitsTensor(x)).cpu().numpy(), want)
+    assert run == route
