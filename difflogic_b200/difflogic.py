@@ -281,13 +281,14 @@ class LogicLayer(torch.nn.Module):
         x._push_layer(self)  # evaluated when x.t is read, or fused with the other layers by GroupSum
         return x
 
-    # Program of the packed network that ends with this layer (PackBitsTensor._network).  It follows from the layers' tensors,
-    # as the walk follows from the connections; both are left out of copies and files.
-    _network = None
+    # Programs of the packed network that ends with this layer (PackBitsTensor._network), for one kernel and for the folded layers.  They
+    # follow from the layers' tensors, as the walk follows from the connections; all are left out of copies and files.
+    _network = _folded_network = None
 
     def __getstate__(self):
         state = self.__dict__.copy()
         state.pop('_network', None)
+        state.pop('_folded_network', None)
         state.pop('_graph_tensors', None)
         state['_walk'] = None
         return state
@@ -296,7 +297,7 @@ class LogicLayer(torch.nn.Module):
         # Kernels (an optimizer's, a replayed graph's) write the weights without autograd's version counter noticing; what was
         # derived from the weights in eval mode does not outlive a change of mode.
         if mode != self.training:
-            self._gate_cache = self._network = None
+            self._gate_cache = self._network = self._folded_network = None
         return super().train(mode)
 
     # What kernels in captured graphs read: a graph holds addresses only, so these tensors stay as long as the layer does (one set

@@ -128,28 +128,31 @@ class PackBitsTensor:
     def _network(self, batch, k, counts=True):
         """The pending layers as a program for the one-kernel evaluation, None when that kernel does not take them, False when it
         is not their turn yet: where building the program takes longer than it saves one batch (PROGRAM_AT_ONCE_ROWS), it is built
-        when the same gates and connections are met a second time.  It stays with the last layer until a layer's gates or connections are others.  Not while a CUDA
+        when the same gates and connections are met a second time.  It stays with the last layer until a layer's gates or connections
+        are others, one of each kind: which one a pass takes goes by its classes and the alignment of its rows, too.  Not while a CUDA
         graph is being captured: the graph would outlive a program that a change of the weights replaces."""
         layers = [layer.indices + (gate,) for layer, gate in self._pending]
         last = self._pending[-1][0]
-        network = last._network
-        if network is not None and not (network.sizes[0] == self._t.shape[0] and network.matches(layers)):
-            network = None
-        if network is not None and network.serves(self._t, k):
-            return network
-        sizes = network.sizes if network is not None else ops.network_sizes(self._t.shape[0], layers)
+        kept = [network if network is not None and network.sizes[0] == self._t.shape[0] and network.matches(layers) else None
+                for network in (last._network, last._folded_network)]
+        for network in kept:
+            if network is not None and network.serves(self._t, k):
+                return network
+        any_kept = kept[0] or kept[1]
+        sizes = any_kept.sizes if any_kept is not None else ops.network_sizes(self._t.shape[0], layers)
         folded = not ops.eval_network_applicable(self._t, sizes, batch, k)
         if folded and not ops.eval_folded_applicable(self._t, sizes):
             return None
         if folded and k > 1 and ops.eval_network_applicable(self._t, sizes, batch, 1) and not self._folded_counts(sizes, sum(sizes), k):
             return None                     # the classes are too many for the one kernel, not the layers
-        kind = ops.FoldedLayers if folded else ops.NetworkProgram
-        if type(network) is not kind:
+        network = kept[folded]
+        if network is None:
             device = self._t.get_device()
             counters = [ops.versions(a, b) for a, b, _ in layers]
             if None in counters or any(t.get_device() != device for layer in layers for t in layer):
                 return None
-            network = last._network = kind(self._t.shape[0], layers, False, counters, sizes)
+            network = kept[folded] = (ops.FoldedLayers if folded else ops.NetworkProgram)(self._t.shape[0], layers, False, counters, sizes)
+            last._network, last._folded_network = kept
             if folded:
                 at_once = sum(sizes[1:-1]) * self._t.shape[1] * self.bit_count >= 8 * FOLD_AT_ONCE_BYTES
             else:

@@ -326,6 +326,51 @@ def test_a_table_is_that_of_the_classes_it_is_kept_under(cuda, monkeypatch):
     assert {k: int(table) for k, table in network.program._dl_tables.items()} == {2: 2}
 
 
+def test_uses_that_take_turns_build_each_program_once(cuda, argmax, monkeypatch):
+    """The same layers counted in few classes (one kernel), in many (folded layers) and read as rows (one kernel)."""
+    built, ran = [], []
+
+    def build(network):
+        built.append(type(network))
+        network.program, network.pays, network.rows = torch.zeros(1), True, 8
+        network.program._dl_tables = {network.counted: None}
+    monkeypatch.setattr(ops, "_index", lambda t, name, n=None: None)
+    monkeypatch.setattr(ops.N, "on_device", lambda t: ops.N._ALREADY_THERE)
+    monkeypatch.setattr(ops.N, "stream_of", lambda t: 7)
+    for kind in (ops.NetworkProgram, ops.FoldedLayers):
+        monkeypatch.setattr(kind, "build", build)
+    monkeypatch.setattr(ops, "eval_network_applicable", lambda x, sizes, batch, k: k < 4)
+    monkeypatch.setattr(ops, "eval_folded_applicable", lambda x, sizes: True)
+    monkeypatch.setattr(ops, "eval_folded_counts_applicable", lambda x, sizes, rows, k: True)
+    monkeypatch.setattr(ops, "eval_groupbitsum_parts_applicable", lambda x, n_out, k: False)
+    monkeypatch.setattr(ops, "eval_groupbitsum_applicable", lambda x, n_out, k: False)
+    monkeypatch.setattr(ops, "groupbitsum", lambda x, pad_len, k, padded: "counts")
+    monkeypatch.setattr(ops, "eval_packed", lambda x, a, b, gate: ran.append("layer") or x)
+    monkeypatch.setattr(ops, "eval_network", lambda x, network, batch, k=None: ran.append("one kernel") or (x if k is None else "counts"))
+    monkeypatch.setattr(ops, "eval_folded", lambda x, network, batch, k=None: ran.append("folded") or (x if k is None else "counts"))
+    layers = [_layer(), _layer()]
+
+    def use(k):
+        del ran[:]
+        packed = D.PackBitsTensor.from_packed(torch.ones(8, 2, dtype=torch.int64), 0)
+        for layer in layers:
+            packed._push_layer(layer)
+        assert packed.t is not None if k is None else packed.group_sum(k) == "counts"
+        return list(ran)
+    uses = (2, 8, None)
+    for k in uses:
+        assert use(k) in (["layer"] * 2, ["one kernel"])
+    for _ in range(3):
+        assert [use(k) for k in uses] == [["one kernel"], ["folded"], ["one kernel"]]
+    assert sorted(kind.__name__ for kind in built) == ["FoldedLayers", "NetworkProgram"]
+    with torch.no_grad():
+        layers[0].weights.add_(1.0)
+    use(8)
+    assert layers[1]._network is None and layers[1]._folded_network is not None     # nothing of other gates stays
+    layers[1].train()
+    assert layers[1]._folded_network is None and not {"_network", "_folded_network"} & set(layers[1].__getstate__())
+
+
 @pytest.mark.parametrize("rows,k,words,together", [
     (20000, 5000, 2048, False), (20000, 2500, 64, True), (20000, 3001, 64, False), (20000, 3000, 64, True), (20000, 1250, 192, False),
     (20000, 1000, 192, True), (20000, 400, 2048, True), (47 * 400, 400, 512, False), (48 * 400, 400, 512, True), (3, 1, 1 << 12, True)])
