@@ -523,6 +523,16 @@ def eval_groupbitsum(x, a, b, gate, pad_len, k, parts=False, padded=False):
     return out
 
 
+# Layers of up to FOLD_ROWS rows are folded for passes of this many neurons x samples; smaller passes evaluate all neurons: that program is
+# four launches for four layers, the folded one 26 and a table, and what its kernel saves does not show where the host takes longer than
+# the GPU.  Second pass, with the build / pass among others, us, all neurons / folded: 784 -> 4 x 2000: 10000 samples 65 / 203, 42 / 41, 2^17
+# 86 / 240, 56 / 56; 4 x 8000: 100 samples 176 / 208, 42 / 42 (the kernel 14.4 / 15.7), 2^15 200 / 217, 43 / 42, 2^16 (225) / 236, 75 / 48;
+# 256 -> 12 x 4000: 10000 274 / 369, 60 / 59, 2^15 287 / 365, 61 / 61, 2^16 (318) / 379, 74 / 59.  Of wider layers the program of all neurons
+# takes longer to build, one CTA per layer: 784 -> 5 x 16000, 100 samples (301) / 236, 10000 (322) / 240, 51 / 43.
+FOLD_WORK = 3 << 29
+FOLD_ROWS = 10240
+
+
 class NetworkProgram:
     """What dl_eval_network needs of a network: its row counts and its program (dl_network_program), built from the layers'
     connections and arg-max gates.  `layers`: (a, b, gate) of every layer, in order; they are kept, so that `matches` can
@@ -545,12 +555,25 @@ class NetworkProgram:
 
     gates_ready = None
     counted = None      # number of classes to make a table for along with the program
+    samples = None      # of the pass that it is built for; None: the form for large batches
+    limit = None        # samples of a pass from which on that form is wanted and not there
+
+    def folds(self, samples):
+        """Whether a pass of so many samples wants the network folded."""
+        return max(self.sizes[1:]) > FOLD_ROWS or sum(self.sizes[1:]) * samples >= FOLD_WORK
 
     def build(self):
+        samples, k = self.samples, self.counted      # once: another thread may want another form, and count other classes
+        if samples is not None and not self.folds(samples):
+            whole = self._whole()
+            program = whole[:4]
+            program._dl_whole, program._dl_tables, program._dl_stream = whole, {}, whole._dl_stream
+            self.limit = -(-FOLD_WORK // sum(self.sizes[1:]))
+            self.program = program
+            return
         count = len(self.layers)
         program = torch.empty(N.lib().dl_network_program_words(self.sizes, count), dtype=torch.int32, device=self.layers[0][2].device)
         self._launch(N.lib().dl_network_program, program)
-        k = self.counted        # once: another thread may count other classes
         table = None if k is None else self._make_table(program, k)
         # other threads and streams may take program and table from here on: this waits for them
         slots, gates, _, left = program[:4].tolist()
@@ -558,11 +581,18 @@ class NetworkProgram:
         program._dl_needs = (slots, gates)
         program._dl_whole = None
         if left * 4 >= 3 * sum(self.sizes[1:]):     # hardly folded: all neurons take less time
-            whole = torch.empty(N.lib().dl_network_whole_words(self.sizes, count), dtype=torch.int32, device=program.device)
-            self._launch(N.lib().dl_network_whole, whole)
-            torch.cuda.current_stream(whole.device).synchronize()
-            program._dl_whole = whole
-        self.program = program
+            program._dl_whole = self._whole()
+        self.program, self.limit = program, None
+
+    def _whole(self):
+        """The program for all neurons, finished."""
+        whole = getattr(self.program, '_dl_whole', None)
+        if whole is not None:
+            return whole
+        whole = torch.empty(N.lib().dl_network_whole_words(self.sizes, len(self.layers)), dtype=torch.int32, device=self.layers[0][2].device)
+        self._launch(N.lib().dl_network_whole, whole)
+        torch.cuda.current_stream(whole.device).synchronize()
+        return whole
 
     def _launch(self, build, program):
         """build(connections, gates, sizes, layers, program, stream)."""
@@ -603,8 +633,8 @@ class NetworkProgram:
     def serves(self, x, k):
         """Whether the program is there, has counted k classes before, and takes the rows of x: all that has to be asked of a
         pass that is like an earlier one.  (What the classes' counts need depends on k alone, not on the batch.)"""
-        program = self.program
-        return (program is not None and k in getattr(program, '_dl_tables', ()) and x.shape[1] * x.element_size() % 16 == 0
+        program, limit = self.program, self.limit
+        return (program is not None and (limit is None or x.shape[1] * x.element_size() * 8 < limit) and k in getattr(program, '_dl_tables', ()) and x.shape[1] * x.element_size() % 16 == 0
                 and x.data_ptr() % 16 == 0 and x.is_contiguous() and x.numel() > 0)
 
     def matches(self, layers):

@@ -32,11 +32,11 @@ from . import ops
 FUSED_LAST_LAYER = os.environ.get("DL_FUSED_LAST_LAYER", "1") != "0"   # last layer + bit-sum in one kernel
 
 
-# A network's first pass builds its program when the batch is as large, or no layer wider (none is: a program takes 26 launches and a
-# synchronisation for four layers).  First pass with the program / by single layers, us, host and build included: 784 -> 4 x 2000: 2^10
-# samples 283 / 185; 784 -> 4 x 8000: 2^13 246 / 161, 2^17 310 / 281, 2^18 366 / 428; 784 -> 5 x 16000: 2^15 312 / 224, 2^17 452 / 530; 784 ->
-# 12 x 12000: 2^13 471 / 293, 2^16 520 / 575, 2^18 777 / 1753.
-PROGRAM_AT_ONCE_ROWS = 0
+# A network's first pass builds its program when the batch is as large, or no layer wider and the program that of all neurons.  First
+# pass with the program / by single layers, us, host and build included, folded: 784 -> 4 x 8000: 2^13 246 / 161, 2^17 310 / 281, 2^18 366 /
+# 428; 784 -> 5 x 16000: 2^15 312 / 224, 2^17 452 / 530; 784 -> 12 x 12000: 2^13 471 / 293, 2^16 520 / 575, 2^18 777 / 1753.  All neurons: 784 ->
+# 2 x 2000: 2^10 samples 101 / 113, 2^17 111 / 118; 256 -> 12 x 4000: 2^13 267 / 261, 2^16 306 / 269.
+PROGRAM_AT_ONCE_ROWS = 2000
 PROGRAM_AT_ONCE_SAMPLES = 1 << 18
 
 # Wider networks are folded in the first pass when their hidden rows take up this much memory.  The same figures: 784 -> 2 x 20000: 2^17
@@ -145,7 +145,7 @@ class PackBitsTensor:
             return None
         if folded and k > 1 and ops.eval_network_applicable(self._t, sizes, batch, 1) and not self._folded_counts(sizes, sum(sizes), k):
             return None                     # the classes are too many for the one kernel, not the layers
-        network = kept[folded]
+        network, samples = kept[folded], self._t.shape[1] * self.bit_count
         if network is None:
             device = self._t.get_device()
             counters = [ops.versions(a, b) for a, b, _ in layers]
@@ -154,12 +154,13 @@ class PackBitsTensor:
             network = kept[folded] = (ops.FoldedLayers if folded else ops.NetworkProgram)(self._t.shape[0], layers, False, counters, sizes)
             last._network, last._folded_network = kept
             if folded:
-                at_once = sum(sizes[1:-1]) * self._t.shape[1] * self.bit_count >= 8 * FOLD_AT_ONCE_BYTES
+                at_once = sum(sizes[1:-1]) * samples >= 8 * FOLD_AT_ONCE_BYTES
             else:
-                at_once = max(sizes[1:]) <= PROGRAM_AT_ONCE_ROWS or self._t.shape[1] * self.bit_count >= PROGRAM_AT_ONCE_SAMPLES
+                at_once = samples >= PROGRAM_AT_ONCE_SAMPLES or (max(sizes[1:]) <= PROGRAM_AT_ONCE_ROWS and not network.folds(samples))
             if not at_once:
                 return False
-        if network.program is None:
+        if network.program is None or (network.limit is not None and samples >= network.limit):
+            network.samples = samples
             if counts and (not folded or self._folded_counts(sizes, sum(sizes), k)):
                 network.counted = k
             network.build()

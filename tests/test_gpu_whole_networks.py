@@ -75,3 +75,27 @@ def test_through_the_layers():
             want = O.packed_net_counts(x.cpu().numpy(), *[[t[i].cpu() for t in net] for i in range(2)], [t[2].cpu().numpy() for t in net], k, 32)
             assert np.array_equal(got.cpu().numpy(), want)
         assert model[1]._network is None or model[1]._network.program is None or model[1]._network.program._dl_whole is not None
+
+
+@pytest.mark.parametrize("fold", [True, False])
+def test_small_passes_before_large_ones(monkeypatch, fold):
+    """A small pass builds the program for all neurons, the first large one the folded network; the large form serves both then."""
+    monkeypatch.setattr(ops, "FOLD_WORK", 2400 * 3000)
+    torch.manual_seed(2)
+    model = torch.nn.Sequential(D.LogicLayer(30, 2400), D.LogicLayer(2400, 2400), D.GroupSum(10)).eval()
+    layers = list(model)[:-1]
+    with torch.no_grad():
+        if not fold:
+            for layer in layers:
+                layer.weights.zero_()
+                layer.weights[:, 6] = 1.0
+                layer.set_connections(layer.indices[0], (layer.indices[0] + 1) % layer.in_dim)
+        x = torch.rand(5000, 30, device="cuda") < 0.5
+        want = O.packed_net_counts(x.cpu().numpy(), [l.indices[0].cpu() for l in layers], [l.indices[1].cpu() for l in layers],
+                                   [l.weights.argmax(1).cpu().numpy().astype(np.uint8) for l in layers], 10, 32)
+        forms = []
+        for n in (100, 100, 1400, 5000, 100, 5000):
+            assert np.array_equal(model(D.PackBitsTensor(x[:n])).cpu().numpy(), want[:n])
+            program = layers[1]._network.program
+            forms.append("none" if program is None else "whole" if program._dl_whole is not None else "folded")
+    assert forms == ["none"] + ["whole"] * 2 + ["folded" if fold else "whole"] * 3

@@ -326,6 +326,36 @@ def test_a_table_is_that_of_the_classes_it_is_kept_under(cuda, monkeypatch):
     assert {k: int(table) for k, table in network.program._dl_tables.items()} == {2: 2}
 
 
+@pytest.mark.parametrize("rows,samples,folds", [(10240, 78644, True), (10240, 78643, False), (8000, 32768, False), (10241, 64, True)])
+def test_small_passes_over_narrow_networks_do_not_fold(cuda, monkeypatch, rows, samples, folds):
+    """Both sides of the lines; a network met by a small pass first is folded by the first one that is large enough."""
+    made = []
+    library = type("Library", (), {"dl_network_program_words": lambda s, sizes, n: 8, "dl_network_whole_words": lambda s, sizes, n: 8,
+                                   "dl_network_program": "folded", "dl_network_whole": "whole"})()
+
+    def launch(network, build, program):
+        made.append(build)
+        program.zero_()._dl_stream = 7
+    monkeypatch.setattr(ops.N, "lib", lambda: library)
+    monkeypatch.setattr(ops.NetworkProgram, "_launch", launch)
+    network = ops.NetworkProgram.__new__(ops.NetworkProgram)
+    network.sizes, network.layers, network.program = (8, rows, rows), [(None, None, torch.zeros(8))] * 2, None
+    network.samples = samples
+    network.build()
+    assert made == ["folded" if folds else "whole"]
+    assert (network.limit is None) == folds and (network.program._dl_whole is None) == folds
+    if not folds:
+        assert not network.folds(network.limit - 1) and network.folds(network.limit)
+        network.program._dl_tables[2] = None                   # two classes have been counted
+
+        def words(samples):
+            return torch.empty(8, samples // 64, dtype=torch.int64)
+        assert network.serves(words(64 * 100), 2) and not network.serves(words(network.limit + 1024), 2)
+        network.samples = network.limit
+        network.build()
+        assert made == ["whole", "folded"] and network.limit is None and network.program._dl_needs == (0, 0)
+
+
 def test_uses_that_take_turns_build_each_program_once(cuda, argmax, monkeypatch):
     """The same layers counted in few classes (one kernel), in many (folded layers) and read as rows (one kernel)."""
     built, ran = [], []
