@@ -46,6 +46,8 @@ SIGNATURES = {
     "dl_eval_network_applicable": (_int, [_ptr, _ptr, _int, _i64, _i64, _i64]),
     "dl_network_program_words": (_i64, [_ptr, _int]),
     "dl_network_program": (_int, [_ptr, _ptr, _ptr, _ptr, _int, _ptr, _ptr]),
+    "dl_network_fold": (_int, [_ptr, _ptr, _ptr, _ptr, _int, _ptr, _ptr]),
+    "dl_network_order": (_int, [_ptr, _int, _ptr, _ptr]),
     "dl_eval_network": (_int, [_ptr, _ptr, _ptr, _int, _ptr, _ptr, _i64, _i64, _i64, _ptr]),
     "dl_network_whole_words": (_i64, [_ptr, _int]),
     "dl_network_whole": (_int, [_ptr, _ptr, _ptr, _ptr, _int, _ptr, _ptr]),

@@ -37,7 +37,7 @@
 
 namespace dl {
 
-constexpr int kResLayers = kFoldLayers;  // layers per network
+constexpr int kResLayers = kFoldLayers;  // layers per network: a lane each
 constexpr int kResRows = 1 << 14;        // rows per layer or input
 constexpr int kResPad = 1 << 14;         // words behind a program that a CTA may read and not use
 
@@ -96,6 +96,14 @@ __device__ __forceinline__ int res_stack_room(const ResBuild &p, int nc) { retur
 __device__ __forceinline__ void res_give_back(const ResBuild &p, int nc, int32_t *state, int slot) {
     const int c = slot & (nc - 1);
     p.stack[(int64_t)c * res_stack_room(p, nc) + atomicAdd(state + c, 1)] = slot;
+}
+
+// Gates in all, for those who want to know before the program is made.
+__global__ void __launch_bounds__(32)
+res_left_kernel(ResBuild p, uint32_t *__restrict__ prog) {
+    grid_dependency_wait();
+    const int left = __reduce_add_sync(0xffffffffu, (int)threadIdx.x < p.layers ? __ldcg(p.fold_header + 1 + threadIdx.x) : 0);
+    if (threadIdx.x == 0) prog[3] = (uint32_t)left;
 }
 
 // The input's rows are in slots 0 ..; those that nothing reads are free from the start.
@@ -823,29 +831,46 @@ extern "C" DL_API int64_t dl_network_program_words(const int64_t *n, int layers)
            (int64_t)(layers + 1) * 2 * kResClasses + most + 2 * kResClasses + kResPad;
 }
 
-extern "C" DL_API int dl_network_program(const int64_t *const *a, const int64_t *const *b, const uint8_t *const *gate, const int64_t *n,
-                                         int layers, uint32_t *program, void *stream) {
-    DL_REQUIRE(a && b && gate && n && program && aligned_to(program, 16), DL_ERR_INVALID_ARG, "dl_network_program: null or unaligned pointer");
-    DL_REQUIRE(layers >= 1 && layers <= kResLayers, DL_ERR_INVALID_ARG, "dl_network_program: 1 .. %d layers", kResLayers);
-    FoldShape sh;
-    DL_REQUIRE(network_shape(n, layers, &sh), DL_ERR_TOO_LARGE, "dl_network_program: layers of 1 .. %d rows", kResRows);
-    for (int l = 0; l < layers; ++l) DL_REQUIRE(a[l] && b[l] && gate[l], DL_ERR_INVALID_ARG, "dl_network_program: null pointer");
-    cudaStream_t st = as_stream(stream);
+// Where a program's scratch is, behind the program proper.
+static FoldScratch program_scratch(const FoldShape &sh, uint32_t *program, ResBuild *p) {
     const int64_t most = most_rows(sh);
     int32_t *work = reinterpret_cast<int32_t *>(program) + program_words(sh);
     const FoldScratch s = fold_scratch(sh, work);
-    ResBuild p = {s.header, s.ref, s.in_a, s.in_b, s.use};
-    p.slot = work + fold_words(sh);
-    p.rank = p.slot + sh.first[layers + 1];
-    p.bucket = p.rank + most;
-    p.state = p.bucket + (int64_t)layers * kResBuckets;
-    p.stack = p.state + (int64_t)(layers + 1) * 2 * kResClasses;
-    p.slots = (int)most;
-    p.layers = layers;
-    p.n0 = sh.n[0];
-    if (int e = fold_network(sh, a, b, gate, s, false, st)) return e;
+    *p = {s.header, s.ref, s.in_a, s.in_b, s.use};
+    p->slot = work + fold_words(sh);
+    p->rank = p->slot + sh.first[sh.layers + 1];
+    p->bucket = p->rank + most;
+    p->state = p->bucket + (int64_t)sh.layers * kResBuckets;
+    p->stack = p->state + (int64_t)(sh.layers + 1) * 2 * kResClasses;
+    p->slots = (int)most;
+    p->layers = sh.layers;
+    p->n0 = sh.n[0];
+    return s;
+}
+
+extern "C" DL_API int dl_network_fold(const int64_t *const *a, const int64_t *const *b, const uint8_t *const *gate, const int64_t *n,
+                                      int layers, uint32_t *program, void *stream) {
+    DL_REQUIRE(a && b && gate && n && program && aligned_to(program, 16), DL_ERR_INVALID_ARG, "dl_network_fold: null or unaligned pointer");
+    DL_REQUIRE(layers >= 1 && layers <= kResLayers, DL_ERR_INVALID_ARG, "dl_network_fold: 1 .. %d layers", kResLayers);
+    FoldShape sh;
+    DL_REQUIRE(network_shape(n, layers, &sh), DL_ERR_TOO_LARGE, "dl_network_fold: layers of 1 .. %d rows", kResRows);
+    for (int l = 0; l < layers; ++l) DL_REQUIRE(a[l] && b[l] && gate[l], DL_ERR_INVALID_ARG, "dl_network_fold: null pointer");
+    ResBuild p;
+    const FoldScratch s = program_scratch(sh, program, &p);
+    if (int e = fold_network(sh, a, b, gate, s, false, as_stream(stream))) return e;
+    launch_dependent(true, res_left_kernel, dim3(1), dim3(32), 0, as_stream(stream), p, program);
+    return launch_status("dl_network_fold");
+}
+
+extern "C" DL_API int dl_network_order(const int64_t *n, int layers, uint32_t *program, void *stream) {
+    FoldShape sh;
+    DL_REQUIRE(program && aligned_to(program, 16), DL_ERR_INVALID_ARG, "dl_network_order: null or unaligned pointer");
+    DL_REQUIRE(network_shape(n, layers, &sh), DL_ERR_TOO_LARGE, "dl_network_order: 1 .. %d layers of 1 .. %d rows", kResLayers, kResRows);
+    cudaStream_t st = as_stream(stream);
+    ResBuild p;
+    const FoldScratch s = program_scratch(sh, program, &p);
     if (cudaMemsetAsync(p.bucket, 0, ((size_t)layers * kResBuckets + (size_t)(layers + 1) * 2 * kResClasses) * sizeof(int32_t), st) != cudaSuccess)
-        return launch_status("dl_network_program (clear)");
+        return launch_status("dl_network_order (clear)");
     auto grid = [](int rows) { return dim3((unsigned)ceil_div(rows, kThreads)); };
     launch_dependent(false, res_inputs_kernel, grid(sh.n[0]), dim3(kThreads), 0, st, p, program);
     uint32_t *level = program + kResHeader;
@@ -856,7 +881,13 @@ extern "C" DL_API int dl_network_program(const int64_t *const *a, const int64_t 
     }
     launch_dependent(true, res_outputs_kernel, grid(sh.n[layers]), dim3(kThreads), 0, st, p, sh.n[layers],
                      (const int32_t *)(s.ref + (sh.first[layers] - sh.n[0])), (const uint32_t *)program, reinterpret_cast<uint16_t *>(level));
-    return launch_status("dl_network_program");
+    return launch_status("dl_network_order");
+}
+
+extern "C" DL_API int dl_network_program(const int64_t *const *a, const int64_t *const *b, const uint8_t *const *gate, const int64_t *n,
+                                         int layers, uint32_t *program, void *stream) {
+    if (int e = dl_network_fold(a, b, gate, n, layers, program, stream)) return e;
+    return dl_network_order(n, layers, program, stream);
 }
 
 extern "C" DL_API int64_t dl_network_table_words(const int64_t *n, int layers, int64_t k) {

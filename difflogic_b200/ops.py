@@ -565,24 +565,39 @@ class NetworkProgram:
     def build(self):
         samples, k = self.samples, self.counted      # once: another thread may want another form, and count other classes
         if samples is not None and not self.folds(samples):
-            whole = self._whole()
-            program = whole[:4]
-            program._dl_whole, program._dl_tables, program._dl_stream = whole, {}, whole._dl_stream
+            self._keep_whole()
             self.limit = -(-FOLD_WORK // sum(self.sizes[1:]))
-            self.program = program
             return
+        program = self._folded()
+        if int(program[3]) * 4 >= 3 * sum(self.sizes[1:]):     # hardly folded: all neurons take less time
+            self._keep_whole(program[:4].clone())
+            self.limit = None
+        else:
+            self.order(program, k)
+
+    def _folded(self):
+        """Room for the folded program, so far with the number of gates left (word 3)."""
         count = len(self.layers)
         program = torch.empty(N.lib().dl_network_program_words(self.sizes, count), dtype=torch.int32, device=self.layers[0][2].device)
-        self._launch(N.lib().dl_network_program, program)
+        self._launch(N.lib().dl_network_fold, program)
+        return program
+
+    def order(self, program, k=None):
+        """The rest of it, and the class table for k."""
+        with N.on_device(program):
+            N.check_status(N.lib().dl_network_order(self.sizes, len(self.layers), program.data_ptr(), N.stream_of(program)))
         table = None if k is None else self._make_table(program, k)
         # other threads and streams may take program and table from here on: this waits for them
-        slots, gates, _, left = program[:4].tolist()
+        program._dl_needs = tuple(program[:2].tolist())     # slots, gates of a layer
         program._dl_tables = {} if table is None else {k: table}     # by number of classes, of this program's slots
-        program._dl_needs = (slots, gates)
         program._dl_whole = None
-        if left * 4 >= 3 * sum(self.sizes[1:]):     # hardly folded: all neurons take less time
-            program._dl_whole = self._whole()
         self.program, self.limit = program, None
+
+    def _keep_whole(self, header=None):
+        whole = self._whole()
+        program = whole[:4] if header is None else header
+        program._dl_whole, program._dl_needs, program._dl_tables, program._dl_stream = whole, None, {}, whole._dl_stream
+        self.program = program
 
     def _whole(self):
         """The program for all neurons, finished."""
@@ -720,6 +735,9 @@ def eval_network(x, network, batch, k=None):
     else:
         out = torch.empty((int(batch), int(k)), dtype=torch.int32, device=x.device)
     with N.on_device(x):
+        if program._dl_whole is None and program._dl_needs is None:
+            network.order(network._folded())
+            program = network.program
         whole = program._dl_whole
         if whole is not None and k is not None:
             program._dl_tables.setdefault(int(k))       # counts these without a table

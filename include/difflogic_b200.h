@@ -218,6 +218,7 @@ DL_API int dl_eval_packed_pitched(const void *x, int64_t x_pitch, const int64_t 
  *                               device pointers) into dl_network_program_words() 32-bit words, 16-byte aligned.  Connections
  *                               outside the layer's input read row 0.  Words 0, 1 and 3 then say how many row slots the program
  *                               uses, how many gates of a layer are left at most, and how many in all.
+ *   dl_network_fold, _order     the same in two steps: word 3, then the rest.  A caller may look at it in between and take dl_eval_whole.
  *   dl_eval_network             x [n[0]][row_bytes] -> out [batch][k] class counts, or the last layer's rows
  *                               rows_out [n[layers]][row_bytes]; one of the two is null.
  *   dl_network_table            order in which the program's last rows are counted in k classes, into dl_network_table_words()
@@ -229,6 +230,9 @@ DL_API int dl_eval_network_applicable(const void *x, const int64_t *n, int layer
 DL_API int64_t dl_network_program_words(const int64_t *n, int layers);
 DL_API int dl_network_program(const int64_t *const *a, const int64_t *const *b, const uint8_t *const *gate, const int64_t *n,
                               int layers, uint32_t *program, void *stream);
+DL_API int dl_network_fold(const int64_t *const *a, const int64_t *const *b, const uint8_t *const *gate, const int64_t *n, int layers,
+                           uint32_t *program, void *stream);
+DL_API int dl_network_order(const int64_t *n, int layers, uint32_t *program, void *stream);
 DL_API int dl_eval_network(const void *x, const uint32_t *program, const int64_t *n, int layers, int32_t *out, void *rows_out,
                            int64_t row_bytes, int64_t batch, int64_t k, void *stream);
 /* The same for networks that are hardly any smaller folded: program and evaluation of all neurons. */

@@ -311,8 +311,10 @@ def test_a_table_is_that_of_the_classes_it_is_kept_under(cuda, monkeypatch):
     """`counted` is what the latest pass asks for; another thread may change it while one builds."""
     network = ops.NetworkProgram.__new__(ops.NetworkProgram)
     network.sizes, network.layers, network.counted, made = (8, 8, 8), [(None, None, torch.zeros(8))] * 2, 2, []
-    words = type("Library", (), {"dl_network_program_words": lambda s, sizes, n: 8, "dl_network_program": None})()
+    words = type("Library", (), {"dl_network_program_words": lambda s, sizes, n: 8, "dl_network_fold": None, "dl_network_order": lambda *a: 0})()
     monkeypatch.setattr(ops.N, "lib", lambda: words)
+    monkeypatch.setattr(ops.N, "on_device", lambda t: ops.N._ALREADY_THERE)
+    monkeypatch.setattr(ops.N, "stream_of", lambda t: 7)
     monkeypatch.setattr(ops.NetworkProgram, "_launch", lambda network, build, program: program.zero_())
 
     def make(network, program, k):
@@ -326,23 +328,39 @@ def test_a_table_is_that_of_the_classes_it_is_kept_under(cuda, monkeypatch):
     assert {k: int(table) for k, table in network.program._dl_tables.items()} == {2: 2}
 
 
-@pytest.mark.parametrize("rows,samples,folds", [(10240, 78644, True), (10240, 78643, False), (8000, 32768, False), (10241, 64, True)])
-def test_small_passes_over_narrow_networks_do_not_fold(cuda, monkeypatch, rows, samples, folds):
-    """Both sides of the lines; a network met by a small pass first is folded by the first one that is large enough."""
+@pytest.fixture
+def programs(cuda, monkeypatch):
+    """Steps of NetworkProgram.build in place of launches; `left`: of 100 neurons, what is left as gates."""
     made = []
-    library = type("Library", (), {"dl_network_program_words": lambda s, sizes, n: 8, "dl_network_whole_words": lambda s, sizes, n: 8,
-                                   "dl_network_program": "folded", "dl_network_whole": "whole"})()
+    library = type("Library", (), {"left": 0, "dl_network_program_words": lambda s, sizes, n: 8, "dl_network_whole_words": lambda s, sizes, n: 8,
+                                   "dl_network_fold": "fold", "dl_network_order": lambda *a: made.append("order") or 0,
+                                   "dl_network_whole": "whole"})()
+    library.made = made
 
     def launch(network, build, program):
         made.append(build)
-        program.zero_()._dl_stream = 7
+        program.fill_(library.left * sum(network.sizes[1:]) // 100)._dl_stream = 7
     monkeypatch.setattr(ops.N, "lib", lambda: library)
+    monkeypatch.setattr(ops.N, "on_device", lambda t: ops.N._ALREADY_THERE)
+    monkeypatch.setattr(ops.N, "stream_of", lambda t: 7)
     monkeypatch.setattr(ops.NetworkProgram, "_launch", launch)
+    monkeypatch.setattr(ops.NetworkProgram, "_make_table", lambda network, program, k: made.append("table"))
+    return library
+
+
+def _unbuilt(rows):
     network = ops.NetworkProgram.__new__(ops.NetworkProgram)
     network.sizes, network.layers, network.program = (8, rows, rows), [(None, None, torch.zeros(8))] * 2, None
+    return network
+
+
+@pytest.mark.parametrize("rows,samples,folds", [(10240, 78644, True), (10240, 78643, False), (8000, 32768, False), (10241, 64, True)])
+def test_small_passes_over_narrow_networks_do_not_fold(programs, rows, samples, folds):
+    """Both sides of the lines; a network met by a small pass first is folded by the first one that is large enough."""
+    network = _unbuilt(rows)
     network.samples = samples
     network.build()
-    assert made == ["folded" if folds else "whole"]
+    assert programs.made == (["fold", "order"] if folds else ["whole"])
     assert (network.limit is None) == folds and (network.program._dl_whole is None) == folds
     if not folds:
         assert not network.folds(network.limit - 1) and network.folds(network.limit)
@@ -353,7 +371,27 @@ def test_small_passes_over_narrow_networks_do_not_fold(cuda, monkeypatch, rows, 
         assert network.serves(words(64 * 100), 2) and not network.serves(words(network.limit + 1024), 2)
         network.samples = network.limit
         network.build()
-        assert made == ["whole", "folded"] and network.limit is None and network.program._dl_needs == (0, 0)
+        assert programs.made == ["whole", "fold", "order"] and network.limit is None and network.program._dl_needs == (0, 0)
+
+
+@pytest.mark.parametrize("small_first", [False, True])
+@pytest.mark.parametrize("left,steps", [(74, ["fold", "order", "table"]), (75, ["fold", "whole"]), (100, ["fold", "whole"])])
+def test_networks_that_do_not_fold_have_one_program(programs, left, steps, small_first):
+    """How many gates are left is known before the rest of the folded program is made, and of what was made for it nothing stays."""
+    programs.left = left
+    network = _unbuilt(1000)
+    network.counted = 2
+    if small_first:
+        network.samples = 64
+        network.build()
+        assert programs.made == ["whole"]
+        del programs.made[:]
+        steps = [step for step in steps if step != "whole"]     # which is there
+    network.samples = 1 << 30
+    network.build()
+    assert programs.made == steps and network.limit is None
+    kept = network.program
+    assert (kept._dl_whole is not None) == (left >= 75) and (left < 75 or kept.untyped_storage().nbytes() == 16)
 
 
 def test_uses_that_take_turns_build_each_program_once(cuda, argmax, monkeypatch):
