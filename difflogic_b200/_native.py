@@ -56,7 +56,8 @@ SIGNATURES = {
     "dl_network_table": (_int, [_ptr, _ptr, _int, _i64, _ptr, _ptr]),
     "dl_eval_network_sized": (_int, [_ptr, _ptr, _ptr, _int, _i64, _i64, _ptr, _ptr, _ptr, _i64, _i64, _i64, _ptr]),
     "dl_fold_layers_bytes": (_i64, [_ptr, _int]),
-    "dl_fold_layers": (_int, [_ptr, _ptr, _ptr, _ptr, _int, _ptr, _ptr]),
+    "dl_fold_scratch_bytes": (_i64, [_ptr, _int]),
+    "dl_fold_layers": (_int, [_ptr, _ptr, _ptr, _ptr, _int, _ptr, _ptr, _ptr]),
     "dl_fold_tail_bytes": (_i64, [_ptr, _int, _i64]),
     "dl_fold_tail": (_int, [_ptr, _ptr, _int, _i64, _ptr, _ptr]),
     "dl_eval_folded": (_int, [_ptr, _ptr, _ptr, _ptr, _int, _ptr, _ptr, _i64, _ptr, _ptr, _i64, _i64, _i64, _ptr]),

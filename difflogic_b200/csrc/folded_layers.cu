@@ -58,10 +58,10 @@ fold_emit_kernel(int n0, int hidden, int tail, const int32_t *__restrict__ ref, 
     list.gate[at] = (uint8_t)op;
 }
 
-static GateList gate_list(const FoldShape &sh, void *work) {
+static GateList gate_list(const FoldShape &sh, void *lists) {
     const int64_t neurons = sh.first[sh.layers + 1] - sh.n[0];
     GateList l;
-    l.a = reinterpret_cast<int64_t *>(reinterpret_cast<int32_t *>(work) + (fold_words(sh) + 3) / 4 * 4);
+    l.a = reinterpret_cast<int64_t *>(lists);
     l.b = l.a + neurons;
     l.gate = reinterpret_cast<uint8_t *>(l.b + neurons);
     return l;
@@ -311,20 +311,25 @@ using namespace dl;
 extern "C" DL_API int64_t dl_fold_layers_bytes(const int64_t *n, int layers) {
     FoldShape sh;
     if (!fold_shape(n, layers, &sh)) return 0;
-    return (fold_words(sh) + 3) / 4 * 16 + 17 * ((int64_t)sh.first[layers + 1] - sh.n[0]);
+    return 17 * ((int64_t)sh.first[layers + 1] - sh.n[0]);
+}
+extern "C" DL_API int64_t dl_fold_scratch_bytes(const int64_t *n, int layers) {
+    FoldShape sh;
+    return fold_shape(n, layers, &sh) ? 4 * fold_words(sh) : 0;
 }
 
 extern "C" DL_API int dl_fold_layers(const int64_t *const *a, const int64_t *const *b, const uint8_t *const *gate, const int64_t *n, int layers,
-                                     void *work, void *stream) {
+                                     void *lists, void *scratch, void *stream) {
     FoldShape sh;
-    DL_REQUIRE(a && b && gate && n && work && aligned_to(work, 16), DL_ERR_INVALID_ARG, "dl_fold_layers: null pointer or unaligned scratch");
+    DL_REQUIRE(a && b && gate && n && lists && scratch && aligned_to(lists, 16) && aligned_to(scratch, 16), DL_ERR_INVALID_ARG,
+               "dl_fold_layers: null or unaligned pointer");
     DL_REQUIRE(fold_shape(n, layers, &sh), DL_ERR_TOO_LARGE, "dl_fold_layers: 1 .. %d layers of fewer than 2^27 rows in all", kFoldLayers);
     for (int l = 0; l < layers; ++l) DL_REQUIRE(a[l] && b[l] && gate[l], DL_ERR_INVALID_ARG, "dl_fold_layers: null pointer");
-    const FoldScratch s = fold_scratch(sh, reinterpret_cast<int32_t *>(work));
+    const FoldScratch s = fold_scratch(sh, reinterpret_cast<int32_t *>(scratch));
     if (int e = fold_network(sh, a, b, gate, s, true, as_stream(stream))) return e;
     const int tail = sh.n[layers], hidden = sh.first[layers + 1] - sh.n[0] - tail;
     fold_emit_kernel<<<(unsigned)ceil_div(hidden + tail, kThreads), kThreads, 0, as_stream(stream)>>>(sh.n[0], hidden, tail, s.ref, s.in_a, s.in_b,
-                                                                                                      s.use, s.row, gate_list(sh, work));
+                                                                                                      s.use, s.row, gate_list(sh, lists));
     return launch_status("dl_fold_layers");
 }
 
@@ -334,14 +339,14 @@ extern "C" DL_API int64_t dl_fold_tail_bytes(const int64_t *n, int layers, int64
     if (!fold_shape(n, layers, &sh) || k < 1 || n[layers] % k != 0) return 0;
     return tail_table(n[layers], k, &t, nullptr);
 }
-extern "C" DL_API int dl_fold_tail(const void *work, const int64_t *n, int layers, int64_t k, void *table, void *stream) {
+extern "C" DL_API int dl_fold_tail(const void *lists, const int64_t *n, int layers, int64_t k, void *table, void *stream) {
     FoldShape sh;
     TailTable t;
-    DL_REQUIRE(work && n && table && aligned_to(work, 16) && aligned_to(table, 16), DL_ERR_INVALID_ARG, "dl_fold_tail: null or unaligned pointer");
+    DL_REQUIRE(lists && n && table && aligned_to(lists, 16) && aligned_to(table, 16), DL_ERR_INVALID_ARG, "dl_fold_tail: null or unaligned pointer");
     DL_REQUIRE(fold_shape(n, layers, &sh) && k >= 1 && n[layers] % k == 0, DL_ERR_INVALID_ARG, "dl_fold_tail: bad sizes");
     const int rows = sh.n[layers], rows_per_class = (int)(rows / k);
     tail_table(rows, k, &t, table);
-    GateList list = gate_list(sh, const_cast<void *>(work));
+    GateList list = gate_list(sh, const_cast<void *>(lists));
     const int64_t tail = sh.first[layers] - sh.n[0];
     list.a += tail;
     list.b += tail;
@@ -355,12 +360,12 @@ extern "C" DL_API int dl_fold_tail(const void *work, const int64_t *n, int layer
     return launch_status("dl_fold_tail");
 }
 
-extern "C" DL_API int dl_eval_folded(const void *x, const void *work, const int64_t *n, const int32_t *left, int layers, void *pool,
+extern "C" DL_API int dl_eval_folded(const void *x, const void *lists, const int64_t *n, const int32_t *left, int layers, void *pool,
                                      const void *table, int64_t longest, int32_t *out, void *rows_out, int64_t row_bytes, int64_t batch,
                                      int64_t k, void *stream) {
     const char *who = "dl_eval_folded";
     FoldShape sh;
-    DL_REQUIRE(x && work && n && left && (out != nullptr) != (rows_out != nullptr) && aligned_to(work, 16), DL_ERR_INVALID_ARG, "%s: null pointer", who);
+    DL_REQUIRE(x && lists && n && left && (out != nullptr) != (rows_out != nullptr) && aligned_to(lists, 16), DL_ERR_INVALID_ARG, "%s: null pointer", who);
     DL_REQUIRE(fold_shape(n, layers, &sh) && row_bytes > 0 && batch > 0 && batch <= row_bytes * 8 && k > 0 && n[layers] % k == 0,
                DL_ERR_INVALID_ARG, "%s: bad sizes", who);
     int64_t rows = 0;
@@ -377,7 +382,7 @@ extern "C" DL_API int dl_eval_folded(const void *x, const void *work, const int6
     const bool direct = row_bytes % 16 == 0 && aligned_to(x, 16) && aligned_to(pool, 16) && most_rows * (row_bytes / 16) <= INT32_MAX &&
                         ceil_div(row_bytes, 512) <= 65535 && k * (ceil_div(m, 64) + 1) <= INT32_MAX;
     DL_REQUIRE(out == nullptr || staged || direct, DL_ERR_INVALID_ARG, "%s: rows whose classes no kernel counts", who);
-    const GateList list = gate_list(sh, const_cast<void *>(work));
+    const GateList list = gate_list(sh, const_cast<void *>(lists));
     const SplitRows src = {reinterpret_cast<const uint8_t *>(x), reinterpret_cast<const uint8_t *>(pool), n[0]};
     int64_t at = rows;  // the first layer's gates come last
     for (int l = 1; l < layers; ++l) {

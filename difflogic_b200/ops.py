@@ -609,8 +609,8 @@ class NetworkProgram:
         torch.cuda.current_stream(whole.device).synchronize()
         return whole
 
-    def _launch(self, build, program):
-        """build(connections, gates, sizes, layers, program, stream)."""
+    def _launch(self, build, program, *scratch):
+        """build(connections, gates, sizes, layers, program, scratch, stream)."""
         import ctypes
         count = len(self.layers)
         pointers = [(ctypes.c_void_p * count)(*[layer[i].data_ptr() for layer in self.layers]) for i in range(3)]
@@ -618,7 +618,7 @@ class NetworkProgram:
             stream = torch.cuda.current_stream(program.device)
             if self.gates_ready is not None:
                 stream.wait_event(self.gates_ready)
-            N.check_status(build(pointers[0], pointers[1], pointers[2], self.sizes, count, program.data_ptr(), stream.cuda_stream))
+            N.check_status(build(*pointers, self.sizes, count, program.data_ptr(), *[t.data_ptr() for t in scratch], stream.cuda_stream))
         program._dl_stream = stream.cuda_stream
 
     def _table_of(self, program, k, stream):
@@ -683,11 +683,12 @@ class FoldedLayers(NetworkProgram):
         if N.stream_of(self.layers[0][2]) != self.stream:
             torch.cuda.synchronize(device)
         program = torch.empty(N.lib().dl_fold_layers_bytes(self.sizes, count), dtype=torch.uint8, device=device)
-        self._launch(N.lib().dl_fold_layers, program)
+        scratch = torch.empty(N.lib().dl_fold_scratch_bytes(self.sizes, count), dtype=torch.uint8, device=device)
+        self._launch(N.lib().dl_fold_layers, program, scratch)
         k = self.counted        # once: another thread may count other classes
         table = None if k is None else self._make_table(program, k)
         # other threads and streams may take program and table from here on: this waits for them
-        left = program[:4 * count].view(torch.int32).tolist()
+        left = scratch[:4 * count].view(torch.int32).tolist()
         program._dl_tables = {} if table is None else {k: table}
         program._dl_left = (ctypes.c_int32 * count)(*left)
         self.rows = sum(left[1:])
@@ -705,6 +706,10 @@ class FoldedLayers(NetworkProgram):
 
     def serves(self, x, k):
         return super().serves(x, k) and self.pays
+
+    def drop(self):
+        """What remains of a network that does not pay: that it does not."""
+        self.program = ()
 
 
 def row_counts(rows):

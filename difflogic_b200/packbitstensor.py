@@ -165,6 +165,7 @@ class PackBitsTensor:
                 network.counted = k
             network.build()
         if folded and not network.pays:
+            network.drop()
             # Three hidden layers or more that fit the one kernel run there all the same.  With gates that all need both inputs, us, one by
             # one / in one kernel: 784 -> 2 x 8000 -> 20000: 10000 samples 75 / 80, 2^17 207 / 245, 2^20 1456 / 1941; 4 x 8000: 102 / 87, 306 /
             # 278, 2195 / 2111; 12 x 8000: 202 / 109, 714 / 400, 5158 / 2976.  (With gates drawn evenly, folded / in one kernel: 4 x 8000: 62 /

@@ -249,9 +249,10 @@ DL_API int dl_eval_network_sized(const void *x, const uint32_t *program, const i
 
 /* A packed network of any width, layer by layer, over the gates that are left when neurons that hand on a row, its inverse or a
  * constant, and neurons that nothing reads, are taken out (fold.cu, folded_layers.cu).  n as above; 1 .. 32 layers.
- *   dl_fold_layers_bytes        bytes of `work` (16-byte aligned), 0 for sizes outside the range
- *   dl_fold_layers              fills work from every layer's connections and gate ids (HOST arrays of device pointers); its first
- *                               words, int32, then say how many gates of layer l = 1 .. layers - 1 are left (word l).
+ *   dl_fold_layers_bytes        bytes of `lists` (16-byte aligned), 0 for sizes outside the range; dl_fold_scratch_bytes: of `scratch`
+ *   dl_fold_layers              fills lists from every layer's connections and gate ids (HOST arrays of device pointers).  The first
+ *                               words of scratch, int32, then say how many gates of layer l = 1 .. layers - 1 are left (word l); it is
+ *                               needed no longer.
  *   dl_fold_tail                table for counting the last layer's rows in k classes, dl_fold_tail_bytes() of them, 16-byte aligned;
  *                               at byte 16 * n[layers] it then says, int32, how many neurons the longest class has.
  *   dl_eval_folded              x [n[0]][row_bytes] -> out [batch][k] class counts, for rows of whole 16 bytes, 16-byte aligned, of which
@@ -262,10 +263,11 @@ DL_API int dl_eval_network_sized(const void *x, const uint32_t *program, const i
  * The counts and rows are those of dl_eval_packed per layer followed by dl_groupbitsum. */
 DL_API int64_t dl_fold_layers_bytes(const int64_t *n, int layers);
 DL_API int dl_fold_layers(const int64_t *const *a, const int64_t *const *b, const uint8_t *const *gate, const int64_t *n, int layers,
-                          void *work, void *stream);
+                          void *lists, void *scratch, void *stream);
+DL_API int64_t dl_fold_scratch_bytes(const int64_t *n, int layers);
 DL_API int64_t dl_fold_tail_bytes(const int64_t *n, int layers, int64_t k);
-DL_API int dl_fold_tail(const void *work, const int64_t *n, int layers, int64_t k, void *table, void *stream);
-DL_API int dl_eval_folded(const void *x, const void *work, const int64_t *n, const int32_t *left, int layers, void *pool, const void *table,
+DL_API int dl_fold_tail(const void *lists, const int64_t *n, int layers, int64_t k, void *table, void *stream);
+DL_API int dl_eval_folded(const void *x, const void *lists, const int64_t *n, const int32_t *left, int layers, void *pool, const void *table,
                           int64_t longest, int32_t *out, void *rows_out, int64_t row_bytes, int64_t batch, int64_t k, void *stream);
 
 /* argmax over the 16 gate weights -> uint8 gate id, first maximum on ties

@@ -120,3 +120,19 @@ def test_where_networks_run_that_do_not_fit_the_one_kernel(monkeypatch, dims, k,
             del run[:]
             assert np.array_equal(model(D.PackBitsTensor(x)).cpu().numpy(), want)
     assert run == route
+    if "folded" not in route and route[0] != "one kernel":      # built, found not to pay: nothing of it stays
+        assert layers[-1]._folded_network.program == ()
+
+
+def test_the_lists_are_all_that_stays():
+    """17 bytes per neuron; what the sweeps need besides is given back."""
+    layers = [tuple(t.cuda() for t in layer) for layer in _random_layers([100, 20000, 20000, 20000])]
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    network = ops.FoldedLayers(100, layers)
+    assert network.program.numel() == 17 * 60000 and torch.cuda.memory_allocated() - before == -(-17 * 60000 // 512) * 512
+
+
+def _random_layers(dims):
+    g = torch.Generator().manual_seed(1)
+    return [(*torch.randint(0, a, (2, b), generator=g), torch.randint(0, 16, (b,), generator=g).to(torch.uint8)) for a, b in zip(dims, dims[1:])]
