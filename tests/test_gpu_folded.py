@@ -19,7 +19,7 @@ CASES = [([5, 3, 4], 2, 16, 32, ALL), ([1, 1, 1, 1], 1, 3, 8, ALL), ([40, 257, 2
          ([300, 1001, 1001, 1001], 7, 24, 64, ALL), ([64, 3000, 500, 700], 1, 48, 64, ALL), ([64, 640, 640], 10, 512, 64, ALL),
          ([200, 4100, 4200], 2, 2064, 64, ALL), ([200] + 31 * [2050], 50, 528, 32, ALL), ([30, 400, 400, 400], 4, 1040, 64, (0, 15)),
          ([100, 40000, 40000], 1, 528, 64, ALL), ([64, 2500, 2600], 2, 4112, 64, ALL), ([20, 900, 900], 900, 1040, 64, ALL),
-         ([30, 400, 400, 400], 4, 1040, 64, (3, 5, 10, 12)), ([100, 900, 900, 900], 9, 640, 64, (1, 2, 4, 6, 7, 8, 9, 11, 13, 14))]
+         ([64, 9000, 18002], 2, 4112, 64, ALL), ([30, 400, 400, 400], 4, 1040, 64, (3, 5, 10, 12)), ([100, 900, 900, 900], 9, 640, 64, (1, 2, 4, 6, 7, 8, 9, 11, 13, 14))]
 
 
 @pytest.mark.parametrize("dims,k,row_bytes,bits,gates", CASES)
@@ -50,6 +50,33 @@ def test_counts_and_rows(dims, k, row_bytes, bits, gates):
     assert packed._folded_counts(network.sizes, network.rows, k) or row_bytes % 16 != 0
     if row_bytes % 16 == 0:
         assert torch.equal(ops.eval_folded(xd, network, batch, k), want)
+
+
+# Rows longer than those that tail_counts_kernel takes: classes by the table of what is not constant, whole or in parts (more than 2040
+# neurons), among them classes of constants only (some true, which are counted once) and of a few neurons.
+@pytest.mark.parametrize("m", [700, 2040, 2100, 9001])
+def test_classes_of_very_different_length(m):
+    g, k, row_bytes = torch.Generator().manual_seed(m), 5, 4112
+    dims = [64, 3000, k * m]
+    layers = []
+    for n_in, n_out in zip(dims[:-1], dims[1:]):
+        a, b = torch.randint(0, n_in, (2, n_out), generator=g)
+        layers.append([a, b, torch.randint(0, 16, (n_out,), generator=g).to(torch.uint8)])
+    gate = layers[1][2].view(k, m)
+    gate[1] = 15 * (gate[1] & 1)                            # constants only
+    gate[2] = 0
+    gate[3, 5:] = 15
+    gate[4] = 6                                             # all needed
+    layers[1][1] = (layers[1][0] + 1) % 3000
+    x = torch.from_numpy(torch.randint(0, 256, (64, row_bytes), generator=g, dtype=torch.uint8).numpy().view("int64"))
+    network, xd = ops.FoldedLayers(64, [tuple(t.cuda() for t in layer) for layer in layers]), x.cuda()
+    rows = x.numpy()
+    for a, b, gate in layers:
+        rows = O.eval_packed(rows, a.numpy(), b.numpy(), gate.numpy())
+    batch = row_bytes * 8 - 5
+    want = np.concatenate([O.group_bit_sum(rows[c * m:(c + 1) * m], 5, 1) for c in range(k)], 1)
+    for _ in range(2):
+        assert np.array_equal(ops.eval_folded(xd, network, batch, k).cpu().numpy(), want)
 
 
 def test_a_wide_network_is_folded(monkeypatch):

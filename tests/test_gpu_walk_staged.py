@@ -12,6 +12,20 @@ from tests.test_gpu_walk import _connections, _reference
 pytestmark = pytest.mark.gpu
 
 
+def assert_adam(w, grad, start, step, w_got, moments, lr=0.01, beta1=0.9, beta2=0.999, eps=1e-8):
+    """Weights and both moments of every neuron against the step in 64 bits from the same gradient and float constants.  Moments: one
+    rounding of each product and sum (2^-24 each).  Weights: one of the sum, and of the update 1 - beta2^step, in which the last place of a
+    power close to 1 is 6e-8 / 5e-3 = 1.2e-5 at step 5; twice that for a power that is two places off."""
+    beta1, beta2, lr, eps = (float(torch.tensor(v)) for v in (beta1, beta2, lr, eps))
+    w, grad, (m, v) = w.double().flatten(), grad.double().flatten(), [t.double() for t in start]
+    m_ref, v_ref = m + (grad - m) * (1 - beta1), v * beta2 + grad * grad * (1 - beta2)
+    update = lr / (1 - beta1 ** step) * m_ref / (v_ref.sqrt() / (1 - beta2 ** step) ** 0.5 + eps)
+    m_got, v_got = (t.cpu().double() for t in moments)
+    assert bool(((m_got - m_ref).abs() <= 2 ** -22 * (m.abs() + grad.abs())).all())
+    assert bool(((v_got - v_ref).abs() <= 2 ** -22 * v_ref).all())
+    assert bool(((w_got.cpu().double().flatten() - (w - update)).abs() <= 3e-5 * update.abs() + 2 ** -22 * m.abs() * lr / v_ref.sqrt() + 2 ** -23 * w.abs()).all())
+
+
 @pytest.mark.parametrize("batch", [4, 36, 128, 132, 256, 640, 1024, 1028, 1160, 2048])
 @pytest.mark.parametrize("case,classes", [(("square", 1, 1), 1), (("square", 9, 9), 9), (("square", 2500, 2500), 5), (("square", 19000, 19000), 19000),
                                           (("paths", 150, 70), 70), (("loops", 70, 65), 13), (("any", 40, 5000), 5000)])
@@ -26,18 +40,19 @@ def test_staged_backward(case, classes, batch):
     walk = ops.build_walk(a.cuda(), b.cuda(), n_in)
     xd, wd, gyd, coef = x.cuda(), w.cuda(), gyc.cuda(), ops.logic_coefs(w.cuda())
     for want_x in {False, walk.complete}:
-        moments = [torch.zeros(n_out * 16, device="cuda") for _ in range(2)]
-        state, w2 = torch.zeros(2, dtype=torch.int32, device="cuda"), wd.clone()
+        start = [0.1 * torch.randn(n_out * 16, generator=g), 0.01 * torch.rand(n_out * 16, generator=g)]
+        moments = [t.cuda() for t in start]
+        state, w2 = torch.tensor([4, 0], dtype=torch.int32, device="cuda"), wd.clone()      # the fifth step
         with N.tuning(N.TUNE_WALK_KERNEL, 2):
             gx, gw = ops.logic_backward_walk(xd, gyd, coef, wd, walk, 1.5, want_grad_x=want_x, rows_per_class=n_out // classes)
             gx2, _ = ops.logic_backward_walk(xd, gyd, coef, w2, walk, 1.5, want_grad_x=want_x, rows_per_class=n_out // classes,
                                              adam=dict(exp_avg=moments[0], exp_avg_sq=moments[1], state=state, lr=0.01, beta1=0.9, beta2=0.999,
-                                                       eps=1e-8, grad_scale=1.0))
+                                                       eps=1e-8, grad_scale=0.5))
         with N.tuning(N.TUNE_WALK_KERNEL, 1):
             gx_register, _ = ops.logic_backward_walk(xd, gyd, coef, wd, walk, 1.5, want_grad_x=want_x, rows_per_class=n_out // classes)
         assert_grad_close(gw, gw_ref, "grad_w")
-        assert_grad_close(moments[0].view(n_out, 16) * 10, gw_ref, "first moment")
-        assert state.tolist() == [1, 0] and not torch.equal(w2, wd)
+        assert state.tolist() == [5, 0]
+        assert_adam(w, gw.cpu() * 0.5, start, 5, w2, moments)
         if want_x:
             assert_grad_close(gx, gx_ref, "grad_x")
             assert torch.equal(gx, gx_register) and torch.equal(gx2, gx)      # the same two terms, wherever the walk is cut

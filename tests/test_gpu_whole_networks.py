@@ -60,9 +60,12 @@ def test_line_between_the_two(copies):
     assert int(program[3]) == 400 - copies and (program._dl_whole is not None) == (copies <= 100)
 
 
-def test_through_the_layers():
-    """Counts for one number of classes and another, and rows, of a model whose passes are remembered."""
+def test_through_the_layers(monkeypatch):
+    """Counts for one number of classes and another, and rows, of a model whose passes are remembered: every pass runs the evaluation
+    of all neurons."""
     torch.manual_seed(1)
+    evaluate, programs = ops.eval_network, []
+    monkeypatch.setattr(ops, "eval_network", lambda x, network, *a: programs.append(network.program) or evaluate(x, network, *a))
     model = [D.LogicLayer(30, 600), D.LogicLayer(600, 600)]
     with torch.no_grad():
         for layer in model:
@@ -74,7 +77,10 @@ def test_through_the_layers():
             got = torch.nn.Sequential(*model, D.GroupSum(k)).eval()(D.PackBitsTensor(x))
             want = O.packed_net_counts(x.cpu().numpy(), *[[t[i].cpu() for t in net] for i in range(2)], [t[2].cpu().numpy() for t in net], k, 32)
             assert np.array_equal(got.cpu().numpy(), want)
-        assert model[1]._network is None or model[1]._network.program is None or model[1]._network.program._dl_whole is not None
+        packed = model[1](model[0](D.PackBitsTensor(x)))
+        assert np.array_equal(ops.groupbitsum(packed.t, packed.pad_len, 6).cpu().numpy(), want)
+    # layers of 600 rows: built by the first pass; whoever changes k or reads rows finds the program there
+    assert len(programs) == 6 and all(p is model[1]._network.program and p._dl_whole is not None for p in programs)
 
 
 @pytest.mark.parametrize("fold", [True, False])
