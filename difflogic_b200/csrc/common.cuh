@@ -40,7 +40,22 @@ struct ClassRows {
 };
 static inline SplitRows split_rows(const void *x) { return {reinterpret_cast<const uint8_t *>(x), nullptr, INT64_MAX}; }
 
+static inline int current_sms() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    return n;
+}
+
 }  // namespace dl
+
+// Adds three bits in each of 32 places: h the carries, l the sums.
+#define DL_CSA32(h, l, a, b, c)        \
+    {                                  \
+        const uint32_t u_ = (a) ^ (b); \
+        const uint32_t c_ = (c);       \
+        h = ((a) & (b)) | (u_ & c_);   \
+        l = u_ ^ c_;                   \
+    }
 
 #define DL_REQUIRE(cond, code, ...)                       \
     do {                                                  \

@@ -171,14 +171,6 @@ constexpr int kTailWarps = kThreads / 32, kTailPlanes = 10, kTailShare = (1 << k
 constexpr int kTailSum = kTailPlanes + 3;                                                          // planes of a CTA's sums
 constexpr uint32_t kTailMore = 1u << 31;  // of an offset: in the second buffer
 
-#define DL_TAIL_CSA(h, l, a, b, c)     \
-    {                                  \
-        const uint32_t u_ = (a) ^ (b); \
-        const uint32_t c_ = (c);       \
-        h = ((a) & (b)) | (u_ & c_);   \
-        l = u_ ^ c_;                   \
-    }
-
 __global__ void __launch_bounds__(kThreads, 2)
 tail_counts_kernel(const SplitRows x, const int64_t *__restrict__ a, const int64_t *__restrict__ b, const uint8_t *__restrict__ gate,
                    const int32_t *__restrict__ start, const int32_t *__restrict__ ones, int32_t *__restrict__ out, int64_t row_bytes,
@@ -239,16 +231,16 @@ tail_counts_kernel(const SplitRows x, const int64_t *__restrict__ a, const int64
                 for (int w = 0; w < 4; ++w) {
                     const uint32_t v0 = gate32(a0[w], b0[w], {m0.x, m0.y, m0.z, m0.w}), v1 = gate32(a1[w], b1[w], {m1.x, m1.y, m1.z, m1.w});
                     uint32_t t, f;
-                    DL_TAIL_CSA(t, p[w][0], p[w][0], v0, v1);
+                    DL_CSA32(t, p[w][0], p[w][0], v0, v1);
                     if (q % 2 == 0) {
                         two[w] = t;
                     } else {
-                        DL_TAIL_CSA(f, p[w][1], p[w][1], two[w], t);
+                        DL_CSA32(f, p[w][1], p[w][1], two[w], t);
                         if (q == 1) {
                             four[w] = f;
                         } else {
                             uint32_t carry;
-                            DL_TAIL_CSA(carry, p[w][2], p[w][2], four[w], f);
+                            DL_CSA32(carry, p[w][2], p[w][2], four[w], f);
 #pragma unroll
                             for (int i = 3; i < kTailPlanes; ++i) {
                                 const uint32_t n = p[w][i] & carry;
@@ -277,7 +269,7 @@ tail_counts_kernel(const SplitRows x, const int64_t *__restrict__ a, const int64
 #pragma unroll
         for (int i = 0; i < kTailSum; ++i) {
             uint32_t h, l;
-            DL_TAIL_CSA(h, l, sum[i], i < kTailPlanes ? s_plane[r][i][word] : 0u, carry);
+            DL_CSA32(h, l, sum[i], i < kTailPlanes ? s_plane[r][i][word] : 0u, carry);
             sum[i] = l;
             carry = h;
         }
@@ -399,7 +391,7 @@ extern "C" DL_API int dl_eval_folded(const void *x, const void *lists, const int
         const ClassRows classes = {t.start, t.ones, longest > 0 ? (int)longest : 1};
         if (direct && (!staged || row_bytes <= kTailLongest)) {
             // parts: as many as leave the busiest of the CTAs that run at a time (two per SM) the fewest neurons; 200: what a part costs besides
-            const int64_t blocks = ceil_div(row_bytes, 512), slots = 2 * 148, fewest = ceil_div(classes.m, kTailShare * kTailWarps);
+            const int64_t blocks = ceil_div(row_bytes, 512), slots = 2 * current_sms(), fewest = ceil_div(classes.m, kTailShare * kTailWarps);
             int64_t parts = fewest, least = 0;
             for (int64_t p = fewest; p <= fewest + 64 && (p == fewest || p <= classes.m / 64); ++p) {
                 const int64_t cost = ceil_div(blocks * k * p, slots) * (ceil_div(classes.m, p) + 200);

@@ -185,7 +185,7 @@ static inline PackGrid pack_grid(const PackShape &sh) {
     };
     const PackGrid small = {0, grid(256, 8)}, large = {1, grid(64, 128)};
     const int64_t tiles = (int64_t)large.grid.x * large.grid.y;
-    return tiles >= 2 * 148 ? large : small;
+    return tiles >= 2 * current_sms() ? large : small;
 }
 
 }  // namespace dl

@@ -29,18 +29,4 @@ __device__ __forceinline__ uint32_t res_mask15(uint32_t w) {
     return m;
 }
 
-#define DL_CSA32(h, l, a, b, c)        \
-    {                                  \
-        const uint32_t u_ = (a) ^ (b); \
-        const uint32_t c_ = (c);       \
-        h = ((a) & (b)) | (u_ & c_);   \
-        l = u_ ^ c_;                   \
-    }
-
-inline int current_sms() {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
-    return n;
-}
-
 }  // namespace dl

@@ -711,11 +711,6 @@ static WalkShape walk_shape(int64_t batch) {
     while (s.wc > 1 && ceil_div(s.ncb, s.wc) * s.wc * 4 > (int64_t)s.ncb * 5) s.wc /= 2;
     return s;
 }
-static int walk_sms() {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
-    return n;
-}
 // The staged backward kernel: rows of whole 16-byte units (the caller sees to that) and at most 16 column blocks, once a warp has two
 // turns of eight steps to go; below, its start (two dependent loads and the first copies) shows.  Measured with Adam, us, register /
 // staged kernel (steps per warp): 16000 x 128 (7): 7.9 / 8.1; 16000 x 256 (14): 13.1 / 13.5; 20000 x 172 (17): 20.5 / 16.8; 40000 x 128 (17): 22.8 /
@@ -725,7 +720,7 @@ static bool walk_staged(int64_t batch, int64_t entries, int64_t rows) {
     const int force = tuning(DL_TUNE_WALK_KERNEL);
     const int64_t ncb = ceil_div(batch, 128);
     if (force == 1 || ncb > kStagedWarps || rows * (batch / 4) > INT32_MAX) return false;
-    return force == 2 || entries * ncb >= (int64_t)walk_sms() * kStagedWarps * 2 * kWalkSteps;
+    return force == 2 || entries * ncb >= (int64_t)current_sms() * kStagedWarps * 2 * kWalkSteps;
 }
 static int64_t walk_ctas(int G, int64_t entries) { return ceil_div(entries, (int64_t)kWalkWarps * (32 / G) * kWalkSteps); }
 
@@ -906,7 +901,7 @@ extern "C" DL_API int dl_backward_walk_f32(const float *x, const float *grad_y, 
     };
     if (vec && walk_staged(batch, entries, n_in > n_out ? n_in : n_out)) {
         const int wc = (int)ceil_div(batch, 128), groups = kStagedWarps / wc, warps = wc * groups;
-        const int64_t part = ceil_div(ceil_div(entries, (int64_t)walk_sms() * groups), kWalkSteps) * kWalkSteps;
+        const int64_t part = ceil_div(ceil_div(entries, (int64_t)current_sms() * groups), kWalkSteps) * kWalkSteps;
         const size_t smem = (size_t)warps * kStagedWarpBytes;
         auto staged = grad_x != nullptr ? walk_backward_staged_kernel<true> : walk_backward_staged_kernel<false>;
         if (cudaFuncSetAttribute(staged, cudaFuncAttributeMaxDynamicSharedMemorySize, kStagedWarps * kStagedWarpBytes) != cudaSuccess)
