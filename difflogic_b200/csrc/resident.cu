@@ -14,9 +14,9 @@
 //
 // Measured, whole kernel, all neurons in the program and their rows put into class order for the counts -> now, us: 784 -> 4 x 8000, 2^20
 // samples 826 -> 492 (1210 layer by layer); 784 -> 5 x 16000, 10000 samples 45 -> 23, 2^18 560 -> 248; 784 -> 12 x 12000, 2^17 451 -> 167;
-// 256 -> 12 x 4000, 2^18 201 -> 85; 784 -> 4 x 8000, 100 samples 14.4 -> 15.7 (four CTAs whose loads wait for one another). What is
-// left as gates: 40 % of the neurons with gates drawn evenly; networks of which three quarters are left run in resident_whole.cu.
-// Shared-memory pipe 59 %, issue 55 % busy: neither is what bounds it alone; a block goes through load, layers and counts one after
+// 256 -> 12 x 4000, 2^18 201 -> 85; 784 -> 4 x 8000, 100 samples 14.4 -> 15.7 (four CTAs whose loads wait for one another): so few
+// run in resident_whole.cu.  What is left as gates: 40 % of the neurons with gates drawn evenly; networks of which three quarters are left
+// run there as well.  Shared-memory pipe 59 %, issue 59 % busy: neither is what bounds it alone; a block goes through load, layers and counts one after
 // the other and two blocks share an SM.  Loading
 // the input four rows per thread at a time, and fetching the next block's into L2, changed nothing.
 //

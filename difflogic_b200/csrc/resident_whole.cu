@@ -1,4 +1,8 @@
-// The whole-network kernel for networks that folding leaves nearly as they are (resident.cu has the idea and the folded form).
+// The whole-network kernel for networks that folding leaves nearly as they are, and for small passes (resident.cu has the idea and the
+// folded form).
+//
+// Small passes: the host takes longer than either kernel, and this program is one launch per layer, where the folded one takes 26 launches
+// for four layers and a table: second pass of 784 -> 4 x 2000, 10000 samples, 66 us, 203 folded.
 //
 // Every neuron is evaluated and its row's slot is its position in the layer: no output slots to fetch, no row that waits for a later
 // reader, and the last layer's rows are put where their classes are, so that they are counted without a table.  That saves more

@@ -56,7 +56,9 @@ def _walk_pays(width, batch, training):
     leave lanes idle, which the gather kernels spread more finely, and with few columns the walk's longer chain from load to store
     shows.  Rows that are not whole 16-byte units are read value by value by the gather kernels, 1.15 to 2.4 times as slow.
 
-    Measured with four layers, walk / gather kernels, us.  Captured training step: 8000 wide, 256 columns: 80 / 73, 2048: 396 / 391;
+    Measured with four layers, walk / gather kernels, us; training steps with the backward kernel that holds its rows in registers, which
+    the staged one has replaced since for layers of 37888 neurons and one column block on (walk_staged, csrc/walk.cu): there the lines may
+    lie lower than drawn here.  Captured training step: 8000 wide, 256 columns: 80 / 73, 2048: 396 / 391;
     16000, 64: 77 / 65, 128: 77 / 80, 512: 167 / 218; 64000, 64: 149 / 151, 80: 205 / 199, 96: 207 / 207, 100: 212 / 230; 128000, 68:
     359 / 364; second wave (18945 neurons on): 19000, 128: 104 / 94, 192: 142 / 135, 256: 141 / 139; 22500, 128: 112 / 107, 192: 153 / 156;
     28000, 128: 116 / 118; up to 32 columns (75777 neurons on): 64000, 32: 120 / 124; 78000, 32: 175 / 156; 112000, 24: 191 / 178, 32: 194 /

@@ -127,17 +127,19 @@ class PackBitsTensor:
 
     def _network(self, batch, k, counts=True):
         """The pending layers as a program for the one-kernel evaluation, None when that kernel does not take them, False when it
-        is not their turn yet: where building the program takes longer than it saves one batch (PROGRAM_AT_ONCE_ROWS), it is built
-        when the same gates and connections are met a second time.  It stays with the last layer until a layer's gates or connections
+        is not their turn yet: where building the program takes longer than it saves one batch (PROGRAM_AT_ONCE_SAMPLES, _ROWS and
+        FOLD_AT_ONCE_BYTES draw the line), it is built when the same gates and connections are met a second time.  It stays with the last layer until a layer's gates or connections
         are others, one of each kind: which one a pass takes goes by its classes and the alignment of its rows, too.  Not while a CUDA
         graph is being captured: the graph would outlive a program that a change of the weights replaces."""
         layers = [layer.indices + (gate,) for layer, gate in self._pending]
         last = self._pending[-1][0]
-        kept = [network if network is not None and network.sizes[0] == self._t.shape[0] and network.matches(layers) else None
-                for network in (last._network, last._folded_network)]
-        for network in kept:
-            if network is not None and network.serves(self._t, k):
-                return network
+        kept = [last._network, last._folded_network]
+        for i, network in enumerate(kept):
+            if network is not None:
+                if not (network.sizes[0] == self._t.shape[0] and network.matches(layers)):
+                    kept[i] = None
+                elif network.serves(self._t, k):
+                    return network
         any_kept = kept[0] or kept[1]
         sizes = any_kept.sizes if any_kept is not None else ops.network_sizes(self._t.shape[0], layers)
         folded = not ops.eval_network_applicable(self._t, sizes, batch, k)
