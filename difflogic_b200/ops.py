@@ -555,6 +555,7 @@ class NetworkProgram:
 
     gates_ready = None
     counted = None      # number of classes to make a table for along with the program
+    layer_by_layer = False      # neither folded nor, all layers or the hidden ones, in one kernel, whatever the classes
     samples = None      # of the pass that it is built for; None: the form for large batches
     limit = None        # samples of a pass from which on that form is wanted and not there
 
@@ -659,6 +660,7 @@ class NetworkProgram:
 
 
 FOLDED_LAYERS = 32     # layers of a network that can be folded
+ONE_KERNEL_ROWS = 1 << 14     # rows of an input or a layer that the one-kernel evaluation takes at most
 
 
 class FoldedLayers(NetworkProgram):
@@ -708,8 +710,9 @@ class FoldedLayers(NetworkProgram):
         return super().serves(x, k) and self.pays
 
     def drop(self):
-        """What remains of a network that does not pay: that it does not."""
+        """What remains of a network that does not pay: that it does not, and whether that is all there is to ask."""
         self.program = ()
+        self.layer_by_layer = max(self.sizes[:-1]) > ONE_KERNEL_ROWS
 
 
 def row_counts(rows):

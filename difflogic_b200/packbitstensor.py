@@ -140,12 +140,15 @@ class PackBitsTensor:
                     kept[i] = None
                 elif network.serves(self._t, k):
                     return network
+                elif network.layer_by_layer:
+                    return False
         any_kept = kept[0] or kept[1]
         sizes = any_kept.sizes if any_kept is not None else ops.network_sizes(self._t.shape[0], layers)
-        folded = not ops.eval_network_applicable(self._t, sizes, batch, k)
+        narrow = max(sizes) <= ops.ONE_KERNEL_ROWS
+        folded = not (narrow and ops.eval_network_applicable(self._t, sizes, batch, k))
         if folded and not ops.eval_folded_applicable(self._t, sizes):
             return None
-        if folded and k > 1 and ops.eval_network_applicable(self._t, sizes, batch, 1) and not self._folded_counts(sizes, sum(sizes), k):
+        if folded and narrow and k > 1 and ops.eval_network_applicable(self._t, sizes, batch, 1) and not self._folded_counts(sizes, sum(sizes), k):
             return None                     # the classes are too many for the one kernel, not the layers
         network, samples = kept[folded], self._t.shape[1] * self.bit_count
         if network is None:

@@ -148,7 +148,7 @@ def test_where_networks_run_that_do_not_fit_the_one_kernel(monkeypatch, dims, k,
             assert np.array_equal(model(D.PackBitsTensor(x)).cpu().numpy(), want)
     assert run == route
     if "folded" not in route and route[0] != "one kernel":      # built, found not to pay: nothing of it stays
-        assert layers[-1]._folded_network.program == ()
+        assert layers[-1]._folded_network.program == () and layers[-1]._folded_network.layer_by_layer == (max(dims[:-1]) > 16384)
 
 
 def test_the_lists_are_all_that_stays():
